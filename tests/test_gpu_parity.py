@@ -237,6 +237,28 @@ def test_spmm_on_units_of_short_rows(w, longest):
     assert np.array_equal(C, C2)
 
 
+@pytest.mark.parametrize("w", [3, 5, 6, 9, 12, 31, 33, 41, 66, 100, 130, 260])
+def test_spmm_ragged_widths_and_rows_at_the_split(w):
+    # widths that fill their lane groups in part (one, two and four columns per lane, one and
+    # two panels per walk), rows of both sides of the limit a group walks alone, and operands
+    # that are not 16-byte aligned
+    sp = _sp()
+    n = 3000
+    rng = np.random.default_rng(w)
+    lengths = rng.integers(0, 20, size=n)
+    lengths[:8] = [127, 128, 129, 255, 1023, 1024, 1025, 2500]
+    ptr, ind, val = _rows_of_given_lengths(lengths, n, 11)
+    B = rng.standard_normal((n, w)).astype(np.float32)
+    ref64, refabs = oracle.spmm_f64(ptr, ind, val, B)
+    dp, di, dv = _dev(ptr), _dev(ind), _dev(val)
+    flat = torch.zeros(n * w + 1, device="cuda")
+    shifted = flat[1:].view(n, w)
+    shifted.copy_(torch.from_numpy(B))
+    for b in (_dev(B), shifted):
+        C = sp.spmm(dp, di, dv, b).cpu().numpy()
+        assert np.all(np.abs(C - ref64) <= 1e-5 * refabs + 1e-30)
+
+
 def test_spmm_is_linear_and_permutation_consistent():
     # size-independent properties at a larger size: A(x+y) = Ax + Ay, and
     # (P A P^T)(P x) = P (A x)
