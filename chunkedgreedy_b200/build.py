@@ -38,18 +38,15 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
-def build(force=False, verbose=False, profile_rounds=False, checked=False):
-    """``profile_rounds``: compile the chain kernel of the sketch stage with cycle counters per
-    phase of a round (-DCSG_ROUND_PROFILE; a diagnostic build, slower, never the default).
-    ``checked``: a second library, libsporder_b200_checked.so, in which every index a kernel
+def build(force=False, verbose=False, checked=False):
+    """``checked``: a second library, libsporder_b200_checked.so, in which every index a kernel
     derives from data of another kernel is tested before use (-DSPORDER_CHECKED); load it by
     setting SPORDER_B200_LIBRARY to its path."""
     if checked:
         return _build(LIB_CHECKED, "build_checked", ["-DSPORDER_CHECKED"], verbose)
-    if not force and not profile_rounds and not needs_build():
+    if not force and not needs_build():
         return LIB
-    extra = ["-DCSG_ROUND_PROFILE=%d" % int(profile_rounds)] if profile_rounds else []
-    return _build(LIB, "build", extra, verbose)
+    return _build(LIB, "build", [], verbose)
 
 
 def _build(lib, objdir, extra, verbose):
@@ -77,5 +74,4 @@ def _build(lib, objdir, extra, verbose):
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv,
-                profile_rounds=2 if "--profile-rounds=2" in sys.argv else int("--profile-rounds" in sys.argv),
                 checked="--checked" in sys.argv))

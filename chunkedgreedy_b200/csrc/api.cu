@@ -4,7 +4,6 @@
 
 #include <atomic>
 #include <chrono>
-#include <cstdlib>
 #include <cstring>
 
 #include "common.cuh"
@@ -146,7 +145,7 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   // streams of the heaviest rows
   const size_t span = static_cast<size_t>(p.chunk < n ? p.chunk : n);
   const size_t cap = transpose_only ? 1 : static_cast<size_t>(stream_capacity(ctx, z, span));
-  const size_t hmax = cap / (size_t(1) << (SKETCH_HEAVY_BUCKET - 1)) + 1;
+  const size_t hmax = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
   const size_t o_hs = ar.take(8 * cap), o_ho = ar.take(4 * (hmax + 1));
   const size_t o_hst = ar.take(4 * hmax * 2 * (p.M / 32) * 32);
   const size_t pmax = transpose_only ? 1 : z / SKETCH_PART_COLS + hmax + 1;  // column slices of the heavy rows
@@ -162,7 +161,7 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
     cap_p = ctx.stream_need_prio ? static_cast<size_t>(ctx.stream_need_prio + (ctx.stream_need_prio >> 3)) : cap / 2;
     if (cap_p > cap - cap / 4) cap_p = cap - cap / 4;
     if (cap_p < 1) cap_p = 1;
-    hmax_p = cap_p / (size_t(1) << (SKETCH_HEAVY_BUCKET - 1)) + 1;
+    hmax_p = cap_p / HEAVY_WORK + 1;
     if (hmax_p > span) hmax_p = span;
     pmax_p = z / SKETCH_PART_COLS + hmax_p + 1;
     o_p_list = ar.take(4 * span);
@@ -217,7 +216,7 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
     prio->heavy_max = static_cast<uint32_t>(hmax_p);
     s->hstream = s->hstream + cap_p;
     s->stream_cap = static_cast<uint32_t>(cap - cap_p);
-    const size_t hmax_r = (cap - cap_p) / (size_t(1) << (SKETCH_HEAVY_BUCKET - 1)) + 1;
+    const size_t hmax_r = (cap - cap_p) / HEAVY_WORK + 1 + CHAIN_ROWS;
     if (hmax_r < s->heavy_max) s->heavy_max = static_cast<uint32_t>(hmax_r);
   }
   return true;
@@ -262,37 +261,6 @@ bool finish_call(Context &ctx, const CsgScratch &s, const CsgScratch *prio = nul
   uint64_t need = ((static_cast<uint64_t>(h[CTRL_HEAVY_NEED + 1]) << 32) | h[CTRL_HEAVY_NEED]) + need_prio;
   if (need > STREAM_CAP_MAX) need = STREAM_CAP_MAX;
   if (need > ctx.stream_need_seen) ctx.stream_need_seen = need;
-#ifdef CSG_ROUND_PROFILE
-  if (getenv("CSG_ROUND_PROFILE")) {  // cycles per phase of the chain kernel's rounds, all warps
-    unsigned long long c[12];
-    if (cudaMemcpy(c, s.ctrl + CTRL_PROFILE, sizeof(c), cudaMemcpyDeviceToHost) == cudaSuccess && c[6])
-      fprintf(stderr,
-              "[rounds] %llu rounds, %.2f elements each; cycles per round: look-up %.0f, order %.0f, "
-              "resolve %.0f, targets %.0f, limits %.0f, apply %.0f\n",
-              c[6], double(c[7]) / c[6], double(c[0]) / c[6], double(c[1]) / c[6], double(c[2]) / c[6],
-              double(c[3]) / c[6], double(c[4]) / c[6], double(c[5]) / c[6]);
-    uint32_t heavy = 0;
-    cudaMemcpy(&heavy, s.ctrl + CTRL_HEAVY_ROWS, sizeof(heavy), cudaMemcpyDeviceToHost);
-    if (heavy > 4096) heavy = 4096;
-    static uint32_t kcyc[4096], work[4096];
-    static int32_t rows[4096];
-    if (heavy && cudaMemcpy(kcyc, s.heavy_off, heavy * 4, cudaMemcpyDeviceToHost) == cudaSuccess &&
-        cudaMemcpy(rows, s.row_list, heavy * 4, cudaMemcpyDeviceToHost) == cudaSuccess) {
-      for (uint32_t i = 0; i < heavy; ++i)
-        cudaMemcpy(&work[i], s.row_work + rows[i], 4, cudaMemcpyDeviceToHost);
-      fprintf(stderr, "[rounds] %u heavy rows; slowest (row: stream elements, Mcycles, cycles/element):", heavy);
-      for (int k = 0; k < 12; ++k) {
-        uint32_t best = 0;
-        for (uint32_t i = 1; i < heavy; ++i)
-          if (kcyc[i] > kcyc[best]) best = i;
-        fprintf(stderr, " [%d: %u, %.1f, %.0f]", rows[best], work[best], kcyc[best] * 1024e-6,
-                work[best] ? kcyc[best] * 1024.0 / work[best] : 0.0);
-        kcyc[best] = 0;
-      }
-      fprintf(stderr, "\n");
-    }
-  }
-#endif
   return true;
 }
 

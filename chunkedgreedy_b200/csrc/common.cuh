@@ -126,17 +126,21 @@ enum {
   CTRL_HEAVY_NEED = 10,    // and the word after it: stream elements of all rows of heavy weight (64-bit)
   CTRL_STREAM_OVERRUN = 12,  // set by heavy_expand_kernel when a slice would pass the stream buffer
   CTRL_CHECK = 13,         // checked build: site of the first index out of bounds, then the index (64-bit)
-  CTRL_BUCKET_COUNT = 16,  // 33 entries
+  CTRL_MID_END = 16,       // end of the rows of heavy weight in row_list (those past CTRL_HEAVY_ROWS did not fit)
+  CTRL_LANE_TICKET = 17,   // next row for the kernel that runs a row per lane
   CTRL_PRIO = 50,          // chunk whose heavy rows run ahead of the rest (PRIO_NONE: no such chunk)
-  CTRL_CRITICAL_ROWS = 51,  // rows at the head of the chunk ahead's list whose chains keep a scheduler each
-  CTRL_CRITICAL_TICKET = 52,
-  CTRL_LONGEST = 53,       // longest candidate stream of the chunk ahead
-  CTRL_BUCKET_BASE = 56,   // 33 entries
-  CTRL_BUCKET_FILL = 96,   // 33 entries
-  CTRL_STATS = 136,        // see greedy.cu (8-byte aligned)
-  CTRL_PROFILE = 168,      // 16 64-bit counters, written only by a build with -DCSG_ROUND_PROFILE
-  CTRL_WORDS = 200
+  CTRL_PRIO_WORK = 51,     // shortest candidate stream among the rows the chunk ahead lists
+  CTRL_STATS = 56,         // see greedy.cu (8-byte aligned)
+  CTRL_BUCKET_COUNT = 128,  // WORK_BUCKETS entries each
+  CTRL_BUCKET_BASE = 256,
+  CTRL_BUCKET_FILL = 384,
+  CTRL_WORDS = 512
 };
+
+// Rows are listed by the length of their candidate stream, in quarter octaves (bucket 4 e + f
+// holds the lengths in [2^e (1 + f/4), 2^e (1 + (f+1)/4)), longest bucket first): 32 consecutive
+// rows of the list, one per lane of a warp (sketch.cu), then differ by a quarter at most.
+constexpr int WORK_BUCKETS = 128;
 
 constexpr uint32_t PRIO_NONE = 0xFFFFFFFFu;
 // phases of a call that runs one chunk ahead: everything (no such split), the chunk ahead, the rest
@@ -145,7 +149,12 @@ enum CallPhase { PHASE_ALL = 0, PHASE_PRIO = 1, PHASE_REST = 2 };
 inline int prio_chain_blocks(int num_sms) { return num_sms / 4 > 0 ? num_sms / 4 : 1; }
 
 constexpr int SKETCH_PART_COLS = 128;   // columns of a heavy row whose stream one warp writes out
-constexpr int SKETCH_HEAVY_BUCKET = 17;  // rows streaming >= 65536 candidates are "heavy"
+// Rows that stream at least HEAVY_WORK candidates are "heavy": a warp of the chain kernel each.
+// Shorter rows join them, longest first, while the list of heavy rows stays within CHAIN_ROWS
+// and the stream has at least CHAIN_WORK_MIN elements (bucket_scan_kernel).
+constexpr uint32_t HEAVY_WORK = 1u << 16;
+constexpr uint32_t CHAIN_ROWS = 296;
+constexpr uint32_t CHAIN_WORK_MIN = 64;
 
 // stage launchers; all enqueue on ctx.stream and return false after set_error()
 bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
@@ -232,6 +241,12 @@ __device__ __forceinline__ unsigned match_digit(uint32_t d) {
     peers &= ((d >> b) & 1u) ? has : ~has;
   }
   return d < 256u ? peers : 1u << (threadIdx.x & 31);
+}
+
+// bucket of a row that streams t >= 1 candidates
+__device__ __forceinline__ int work_bucket(uint32_t t) {
+  const int e = 31 - __clz(t);
+  return 4 * e + static_cast<int>((e >= 2 ? t >> (e - 2) : t << (2 - e)) & 3u);
 }
 
 // packed entry of the top-k table; wire format of the reference

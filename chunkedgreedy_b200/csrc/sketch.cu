@@ -12,38 +12,24 @@
 //   top-k         :46-66,71-90 (per-lane selection sort by weight, then k rounds
 //                 of arg-max over the lanes' cursors, ties to the smaller lane)
 //
-// What differs is the machinery.  One warp consumes one row's stream, as in the
-// reference, but
-//  * rows come from a work list ordered heaviest first: the stream of one row is an
-//    order-dependent chain, so the longest rows must start first;
-//  * stream elements are PRODUCED in batches into shared memory - lane-parallel over the
-//    column groups of the chunk-local transpose, coalesced for long groups, Dice terms
-//    computed here - and CONSUMED from there in a tight loop, so group bookkeeping,
-//    address arithmetic, the divide and DRAM latency stay out of the dependent chain;
-//  * a step on a full sketch costs three redux.sync (the cheapest warp collective on
-//    this part): one hit test and two for the eviction victim of the NEXT miss, which
-//    is computed ahead of time from each lane's cached two smallest weights (see
-//    Sketch::add_full);
-//  * the rows with the longest streams set the run time of the whole call, and a warp
-//    that shares its scheduler with seven others takes 1.6x longer per step.  Those rows
-//    (65536 stream elements or more) take a path of their own: their streams are written
-//    out to memory by the whole grid (heavy_expand_kernel, one warp per 128 columns),
-//    then a chain kernel runs one warp per row and one warp per scheduler - one block per
-//    SM, kept alone there by its shared-memory request - doing nothing but consuming.  The
-//    kernel of all other rows follows as a programmatic dependent launch: it starts as
-//    soon as the chain kernel's blocks are running and fills the SMs that kernel leaves or
-//    frees;
-//  * for sketches of up to 128 slots the chain kernel does not step through the stream one
-//    element at a time: it resolves the longest prefix of the next 32 elements whose
-//    outcome can be read off the sketch as it stands, all lanes at once (see "the chains
-//    in rounds" below) - 16 elements per round on the longest R-MAT rows, at under half
-//    the cost of 16 sequential steps.  Larger sketches keep the element-wise chain
-//    (heavy_consume_kernel);
-//  * a large call runs in two parts (see run_csg): the chunk with the most nonzeros on a
-//    stream of its own, ahead of the rest.  Both parts go through launch_cells with their own
-//    lists and control words; their chain kernels have eight warps per block, and only the
-//    critical rows - those long enough to decide when the call ends - keep a scheduler to
-//    themselves.
+// What differs is the machinery:
+//  * rows come from a work list ordered by the length of their stream, longest first: a
+//    stream is an order-dependent chain;
+//  * the longest rows (65536 candidates or more, and shorter ones while they are few) set the
+//    run time.  Their streams are written out to memory by the whole grid (heavy_expand_kernel,
+//    one warp per 128 columns); then a group of warps works on each row and resolves up to 32
+//    candidates per round (see "the chains in rounds" below);
+//  * all other rows run side by side, one per LANE: the container of a row is a column of
+//    shared memory, a step of 32 rows costs a warp little more than a step of one row did, and
+//    further warps of the block produce the streams (see "a row per lane" below).  This
+//    kernel follows the chain kernel as a programmatic dependent launch, so that its blocks
+//    settle beside that kernel's on the same SMs;
+//  * sketches of more than 128 slots keep one warp per row, its slots in the lanes' registers;
+//    a step on a full sketch costs three redux.sync (see Sketch::add_full), and their heaviest
+//    rows run one warp per scheduler (heavy_consume_kernel);
+//  * a large call runs in two parts (see run_csg): the longest rows of the chunk with the most
+//    nonzeros on a stream of their own, ahead of the rest.  Both parts go through launch_cells
+//    with their own lists and control words.
 #include "common.cuh"
 
 namespace csg {
@@ -56,6 +42,7 @@ constexpr int S_RING = 256;    // stream elements per batch, light rows
 constexpr int H_PART = SKETCH_PART_COLS;  // columns of a heavy row expanded by one warp: small enough
                                          // that a slice of hub columns (up to chunk-1 candidates
                                          // each) does not become the last warp to finish
+constexpr int LANE_CELLS = 4;  // largest sketch (cells per lane) kept by one lane (rows_in_lanes_kernel)
 constexpr int S_LONG = 48;     // groups with at least this many pending entries are copied by the whole warp
 
 struct SketchArgs {
@@ -221,69 +208,6 @@ struct Sketch {
       lane_top2();
       if (slot / CELLS == gown) find_victim(l1w, l1c, gmin, gown, gcell);
     }
-  }
-
-  // this lane's smallest (weight, cell): all the victim search of the table steps needs
-  __device__ __forceinline__ void lane_min() {
-    l1w = __float_as_uint(w[0]);
-    l1c = 0;
-#pragma unroll
-    for (int c = 1; c < CELLS; ++c) {
-      const uint32_t x = __float_as_uint(w[c]);
-      const bool first = x < l1w;
-      l1w = first ? x : l1w;
-      l1c = first ? c : l1c;
-    }
-  }
-
-  // ---- steps with a key -> slot table --------------------------------------------------
-  // One byte per row of the chunk in shared memory (0 = not in the sketch, else slot + 1)
-  // answers "is the key there, and where" with one broadcast load instead of CELLS compares
-  // and a warp reduction, and the victim is only looked for when an element misses (two
-  // reductions per miss, none per hit).  Fewer instructions per element than add_full, which
-  // is what counts where many warps share a scheduler; add_full's speculation buys latency,
-  // which counts where a warp has a scheduler to itself.
-  __device__ __forceinline__ void add_filling_tab(int32_t s, float a, uint8_t *tab, int32_t cbase) {
-    const int q = tab[s - cbase];
-    if (q) {  // (same address in all lanes: the branch is uniform)
-      add_weight(q - 1, a);
-      return;
-    }
-    put(filled, s, a);
-    if (lane == 0) tab[s - cbase] = static_cast<uint8_t>(filled + 1);
-    ++filled;
-    if (filled == 32 * CELLS) lane_min();
-    __syncwarp();
-  }
-
-  __device__ __forceinline__ void add_full_tab(int32_t s, float a, uint8_t *tab, int32_t cbase) {
-    const int q = tab[s - cbase];
-    if (q) {  // hit
-      add_weight(q - 1, a);
-      lane_min();
-      return;
-    }
-    find_victim(l1w, l1c, gmin, gown, gcell);
-    const float wnew = __uint_as_float(gmin) + a;
-    const int32_t gslot = gown * CELLS + gcell;
-    if (lane == gown) {
-      int32_t old_key = key[0];
-#pragma unroll
-      for (int c = 1; c < CELLS; ++c) old_key = (c == gcell) ? key[c] : old_key;
-      tab[old_key - cbase] = 0;
-      tab[s - cbase] = static_cast<uint8_t>(gslot + 1);
-    }
-    put(gslot, s, wnew);
-    lane_min();
-    __syncwarp();
-  }
-
-  // the table is empty again for the next row
-  __device__ __forceinline__ void clear_tab(uint8_t *tab, int32_t cbase) const {
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c)
-      if (key[c] >= 0) tab[key[c] - cbase] = 0;
-    __syncwarp();
   }
 
   __device__ __forceinline__ void local_sort_descending() {
@@ -531,20 +455,10 @@ __device__ __forceinline__ void consume(Sketch<CELLS> &sk, const int32_t *bs, co
   }
 }
 
-// The same with the key -> slot table (see Sketch::add_full_tab).
 // A stream key as an index into a table over the chunk's rows: in the checked build a key
 // outside the chunk is recorded and replaced by the chunk's first row.
 __device__ __forceinline__ int32_t key_in_chunk(uint32_t *ctrl, int32_t s, int32_t cbase, int32_t span) {
   return index_ok(ctrl, CHK_KEY, static_cast<long long>(s) - cbase, span) ? s : cbase;
-}
-
-template <int CELLS>
-__device__ __forceinline__ void consume_tab(Sketch<CELLS> &sk, uint8_t *tab, int32_t cbase, const int32_t *bs,
-                                            const float *ba, int cnt, uint32_t *ctrl, int32_t span) {
-  int t = 0;
-  for (; t < cnt && sk.filled < 32 * CELLS; ++t) sk.add_filling_tab(key_in_chunk(ctrl, bs[t], cbase, span), ba[t], tab, cbase);
-#pragma unroll 1
-  for (; t < cnt; ++t) sk.add_full_tab(key_in_chunk(ctrl, bs[t], cbase, span), ba[t], tab, cbase);
 }
 
 __device__ __forceinline__ bool row_bounds_ok(const SketchArgs &a, int32_t rb, int32_t re) {
@@ -555,24 +469,10 @@ __device__ __forceinline__ bool row_bounds_ok(const SketchArgs &a, int32_t rb, i
   return true;
 }
 
-// All rows below the heavy threshold: one warp per row, producing and consuming in turn.
-// TAB: with a key -> slot table per warp (tab_bytes each, dynamic shared memory); without it
-// for chunks whose tables would not fit and for sketches of more than 224 slots (the table
-// holds slot numbers in a byte).
-template <int CELLS, bool TAB>
-__global__ void __launch_bounds__(S_THREADS) sketch_kernel(SketchArgs a, int after_primary, int tab_bytes) {
-  extern __shared__ __align__(16) unsigned char light_dyn[];
-  __shared__ int32_t ring_s[S_WARPS][S_RING];
-  __shared__ float ring_a[S_WARPS][S_RING];
-  const int lane = lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t listed = a.ctrl[CTRL_ROWS_LISTED];
-  int32_t *bs = ring_s[warp];
-  float *ba = ring_a[warp];
-  uint8_t *tab = light_dyn + static_cast<size_t>(warp) * tab_bytes;
-  if (TAB) {
-    for (int i = lane * 16; i < tab_bytes; i += 32 * 16) *reinterpret_cast<uint4 *>(tab + i) = make_uint4(0, 0, 0, 0);
-    __syncwarp();
-  }
+// Rows [ticket, end) of the list, one warp per row, producing and consuming in turn.
+template <int CELLS>
+__device__ __forceinline__ void rows_by_warp(const SketchArgs &a, uint32_t end, int32_t *bs, float *ba) {
+  const int lane = lane_id();
   Sketch<CELLS> sk;
   sk.bind_lane();
   Producer<S_RING> prod(a);
@@ -580,29 +480,554 @@ __global__ void __launch_bounds__(S_THREADS) sketch_kernel(SketchArgs a, int aft
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(&a.ctrl[CTRL_ROW_TICKET], 1u);  // starts after the heavy rows
     item = __shfl_sync(FULL, item, 0);
-    if (item >= listed) break;
+    if (item >= end) break;
     const int32_t r = a.row_list[item];
     if (!index_ok(a.ctrl, CHK_LIST, r, a.n)) continue;
     const int32_t rb = a.ptr[r], re = a.ptr[r + 1];
     if (!row_bounds_ok(a, rb, re)) continue;
-    const int32_t cbase = (r / a.chunk) * a.chunk;
     sk.clear();
     prod.begin(r, rb, re, re - rb);
     for (;;) {
       const int cnt = prod.produce(bs, ba);
       if (cnt == 0) break;
-      if (TAB)
-        consume_tab<CELLS>(sk, tab, cbase, bs, ba, cnt, a.ctrl, tab_bytes);
-      else
-        consume<CELLS>(sk, bs, ba, cnt);
+      consume<CELLS>(sk, bs, ba, cnt);
       __syncwarp();
     }
-    if (TAB) sk.clear_tab(tab, cbase);
     sk.select_top_k(a.k, a.table + static_cast<size_t>(r) * a.k, a.row_base);
   }
+}
+
+// all: every row the chain kernel leaves (sketches of more than LANE_CELLS cells per lane; the
+// others go to rows_in_lanes_kernel).  Otherwise only the rows of heavy weight that did not fit
+// the stream buffer.
+template <int CELLS>
+__global__ void __launch_bounds__(S_THREADS) sketch_kernel(SketchArgs a, int all, int after_primary) {
+  __shared__ int32_t ring_s[S_WARPS][S_RING];
+  __shared__ float ring_a[S_WARPS][S_RING];
+  const int warp = threadIdx.x >> 5;
+  rows_by_warp<CELLS>(a, a.ctrl[all ? CTRL_ROWS_LISTED : CTRL_MID_END], ring_s[warp], ring_a[warp]);
   // Launched as the programmatic dependent of the heavy-chain kernel, this kernel starts
   // while that one is still running; it must not be seen as finished before it.
   if (after_primary) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---- a row per lane -----------------------------------------------------------------------
+// Most candidates of a large call belong to rows of middling length, far more rows than the
+// GPU has warps.  What counts for them is instructions per candidate, and a warp that works on
+// one row spends all its 32 lanes on one candidate (56 warp instructions each, measured).  Here
+// every LANE has a row of its own: 32 sequential containers side by side, each in a column of
+// shared memory (word i of lane l at [i * 32 + l], so that lanes reading different places never
+// meet in a bank), some 170 instructions per step of up to 32 candidates.
+//   * W[code]: weight bits of slot `code` (cell * 32 + lane in the container's terms, so that
+//     the eviction order (weight, cell, lane) is (weight, code)), ~0 while the slot is empty;
+//   * an index from key to slot: a byte per row of the chunk (TableIndex), or for chunks whose
+//     tables would leave room for too few warps a chained hash table (ChainIndex);
+//   * the least weight of every eight slots, its slot, and the least of those in registers, so
+//     that a miss knows its victim.  Hits and misses then recompute one group's least and the
+//     least of all in the same way: lanes that do either run together.
+// 32 consecutive rows of the list differ by at most a quarter in length, so lanes idle little.
+// The containers belong to one warp of a block; four more warps produce the streams, 32
+// candidates of a row at a time, into a ring the first warp reads a phase later (a lane that
+// walks its row's columns by itself spends a memory latency per candidate: ten times slower).
+// At the end of a batch all warps select the rows' top k, by counting ranks.
+// What bounds it: the latency of a step (some 550 cycles; a warp alone on a scheduler issues
+// every other cycle, and the producing warps take slots as well), then the tail of the longest
+// rows.  R-MAT scale 22, everything but the heavy rows (297 M candidates): 25 ms of the GPU with a
+// warp per row, 11 ms this way.
+constexpr int L_RING = 32;         // candidates produced per row and phase, one per lane of a producing warp
+constexpr int L_PRODUCERS = 4;     // producing warps ...
+constexpr int L_WARPS = 1 + L_PRODUCERS;
+constexpr int L_ROWS = 32 / L_PRODUCERS;  // ... and rows of each
+constexpr int L_TABLE_MAX = 1024;  // largest chunk (rows) indexed by a byte table
+
+// Key -> slot by one byte per row of the chunk (0 = not there, else slot + 1).  Keys travel as
+// the byte's place in the lane's column of the table; those of the slots, 16 bits each, are
+// kept for evictions and for the selection.
+template <int CELLS>
+struct TableIndex {
+  static constexpr int M = 32 * CELLS;
+  static __host__ __device__ int quads(int64_t span) { return static_cast<int>((span + 3) / 4); }
+  static int words(int64_t span) { return M * 16 + (quads(span) + 1) * 32; }  // (one word more: what an empty slot's key names)
+  uint32_t *mem;  // this lane's column of the index's words
+  static __device__ __forceinline__ uint32_t encode(uint32_t s) { return (s >> 2) * 128u + (s & 3u); }
+  static __device__ __forceinline__ uint32_t decode(uint32_t e) { return (e >> 7) * 4u + (e & 3u); }
+  __device__ __forceinline__ uint8_t &place(uint32_t e) { return reinterpret_cast<uint8_t *>(mem + M * 16)[e]; }
+  __device__ __forceinline__ uint16_t &stored(int c) { return reinterpret_cast<uint16_t *>(mem + (c >> 1) * 32)[c & 1]; }
+  __device__ __forceinline__ uint32_t key(int c) { return decode(stored(c)); }
+  __device__ __forceinline__ void init(int64_t span) {
+    for (int i = 0; i <= quads(span); ++i) mem[M * 16 + i * 32] = 0u;
+    for (int c = 0; c < M; ++c) stored(c) = static_cast<uint16_t>(quads(span) * 128);
+  }
+  __device__ __forceinline__ int find(uint32_t e) { return static_cast<int>(place(e)); }
+  __device__ __forceinline__ void replace(int c, uint32_t e, bool) {
+    place(stored(c)) = 0;
+    stored(c) = static_cast<uint16_t>(e);
+    place(e) = static_cast<uint8_t>(c + 1);
+  }
+  __device__ __forceinline__ void forget(int c, int64_t span) {
+    place(stored(c)) = 0;
+    stored(c) = static_cast<uint16_t>(quads(span) * 128);
+  }
+  __device__ __forceinline__ void forget_all() {}
+};
+
+// Key -> slot by hashing: one byte per bucket names the first slot of its chain, a slot's word
+// holds its key (24 bits) and the next slot of the chain.  Four to sixteen buckets per slot: the 32
+// lanes of a warp wait for the longest chain among them.
+template <int CELLS>
+struct ChainIndex {
+  static constexpr int M = 32 * CELLS;
+  static constexpr int BITS = CELLS <= 2 ? 10 : 9;
+  static constexpr uint32_t NONE = 0xFFu;
+  static int words(int64_t) { return M * 32 + (1 << BITS) / 4 * 32; }
+  uint32_t *mem;
+  static __device__ __forceinline__ uint32_t encode(uint32_t s) { return s; }
+  __device__ __forceinline__ uint8_t &head(uint32_t s) {
+    const uint32_t b = (s * 0x9E3779B1u) >> (32 - BITS);
+    return reinterpret_cast<uint8_t *>(mem + M * 32 + (b >> 2) * 32)[b & 3u];
+  }
+  __device__ __forceinline__ uint32_t &entry(uint32_t c) { return mem[c * 32]; }
+  __device__ __forceinline__ uint32_t key(int c) { return entry(c) >> 8; }
+  __device__ __forceinline__ void init(int64_t) { forget_all(); }
+  __device__ __forceinline__ int find(uint32_t s) {  // slot + 1, 0 when the key is not there
+    uint32_t c = head(s);
+    while (c != NONE) {
+      const uint32_t e = entry(c);
+      if (e >> 8 == s) return static_cast<int>(c) + 1;
+      c = e & 0xFFu;
+    }
+    return 0;
+  }
+  __device__ __forceinline__ void replace(int c, uint32_t s, bool used) {
+    if (used) {  // out of its chain
+      const uint32_t e = entry(c), next = e & 0xFFu;
+      uint8_t &first = head(e >> 8);
+      uint32_t at = first;
+      if (at == static_cast<uint32_t>(c)) {
+        first = static_cast<uint8_t>(next);
+      } else {
+        while (at != NONE) {
+          const uint32_t f = entry(at);
+          if ((f & 0xFFu) == static_cast<uint32_t>(c)) {
+            entry(at) = (f & ~0xFFu) | next;
+            break;
+          }
+          at = f & 0xFFu;
+        }
+      }
+    }
+    uint8_t &first = head(s);
+    entry(c) = (s << 8) | first;
+    first = static_cast<uint8_t>(c);
+  }
+  __device__ __forceinline__ void forget(int, int64_t) {}
+  __device__ __forceinline__ void forget_all() {
+    for (int i = 0; i < (1 << BITS) / 4; ++i) mem[M * 32 + i * 32] = 0xFFFFFFFFu;
+  }
+};
+
+struct LaneShared {
+  uint32_t first;          // place in the list of the batch's first row
+  int32_t count[2][32];    // candidates in each row's part of the ring's buffers
+};
+
+// shared memory of a block, in words: weights, two buffers of the ring (keys, Dice terms), what
+// the warps tell one another, then the index.  Outside the phases the ring's words serve the
+// top-k selection.
+template <int CELLS>
+struct LaneLayout {
+  static constexpr int M = 32 * CELLS;
+  static constexpr int RING_OFF = M * 32;
+  static constexpr int BUFFER = 2 * L_RING * 32;
+  static constexpr int SHARED_OFF = RING_OFF + 2 * BUFFER;
+  static constexpr int I_OFF = SHARED_OFF + sizeof(LaneShared) / 4;
+  static_assert(L_WARPS * 2 * S_RING <= I_OFF, "rows_by_warp borrows the memory in front of the index for its rings");
+  static_assert(L_WARPS * M <= 2 * BUFFER, "the selection's copies of the weights fit the ring");
+};
+
+// Least of N values with what goes with it; the first of equal ones.  A tree, so that a step's
+// chain of dependent compares is three or four deep.
+template <int N>
+__device__ __forceinline__ void least_of(const uint32_t (&v)[N], const int32_t (&tag)[N], uint32_t &best,
+                                         int32_t &best_tag) {
+  if constexpr (N == 1) {
+    best = v[0];
+    best_tag = tag[0];
+  } else {
+    constexpr int H = (N + 1) / 2;
+    uint32_t h[H];
+    int32_t t[H];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      bool first;
+      h[i] = __vibmin_u32(v[2 * i], v[2 * i + 1], &first);  // minimum and which one it was, one instruction
+      t[i] = first ? tag[2 * i] : tag[2 * i + 1];
+    }
+    if constexpr (N % 2 == 1) {
+      h[H - 1] = v[N - 1];
+      t[H - 1] = tag[N - 1];
+    }
+    least_of<H>(h, t, best, best_tag);
+  }
+}
+
+template <int CELLS, typename Index>
+struct LaneSketch {
+  static constexpr int M = 32 * CELLS;
+  static constexpr int GROUPS = M / 8;
+  uint32_t *mem;         // this lane's column of the weights
+  Index index;
+  uint32_t gw[GROUPS];   // least weight of every eight slots ...
+  int32_t gc[GROUPS];    // ... and the first slot that has it
+  uint32_t low;          // the least of all of them, which the next miss takes ...
+  int32_t victim;        // ... and its slot
+
+  __device__ __forceinline__ uint32_t &weight(int c) { return mem[c * 32]; }
+  // The j-th slot to be filled.  While it is empty its weight is the j-th smallest bit pattern:
+  // a miss then takes the empty slots in order like any other victim, and that weight vanishes
+  // in the first Dice term added to it.
+  static __device__ __forceinline__ int code_of(int j) { return (j % CELLS) * 32 + j / CELLS; }
+
+  __device__ __forceinline__ void init(int64_t span) {
+    for (int j = 0; j < M; ++j) weight(code_of(j)) = static_cast<uint32_t>(j);
+    index.init(span);
+    fresh();
+  }
+  __device__ __forceinline__ void fresh() {
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      gw[g] = static_cast<uint32_t>((g * 8 % 32) * CELLS + g * 8 / 32);
+      gc[g] = g * 8;
+    }
+    low = 0;
+    victim = 0;
+  }
+  __device__ __forceinline__ void clear(int64_t span) {  // back to empty, at the price of what was filled
+    for (int j = 0; j < M && weight(code_of(j)) >= static_cast<uint32_t>(M); ++j) {
+      weight(code_of(j)) = static_cast<uint32_t>(j);
+      index.forget(code_of(j), span);
+    }
+    index.forget_all();
+    fresh();
+  }
+
+  // One candidate (e: its key as the index has it, p: what find(e) said), then the look-up of the
+  // next one, whose latency passes while this one's group and victim are worked out.
+  __device__ __forceinline__ int step(uint32_t e, float al, int p, uint32_t next) {
+    const int c = p ? p - 1 : victim;
+    const uint32_t held = weight(c);
+    if (p == 0) index.replace(c, e, low >= static_cast<uint32_t>(M));
+    weight(c) = __float_as_uint(__uint_as_float(held) + al);
+    const int found = index.find(next);
+    const int g8 = c & ~7;
+    uint32_t w[8];
+    int32_t tags[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      w[i] = weight(g8 + i);
+      tags[i] = i;
+    }
+    uint32_t least;
+    int32_t first;
+    least_of<8>(w, tags, least, first);
+    first += g8;
+#pragma unroll
+    for (int i = 0; i < GROUPS; ++i) {
+      gw[i] = 8 * i == g8 ? least : gw[i];
+      gc[i] = 8 * i == g8 ? first : gc[i];
+    }
+    least_of<GROUPS>(gw, gc, low, victim);
+    return found;
+  }
+};
+
+// The rows that did not fit the stream buffer, before the lanes' own (rare: a first call on
+// much larger rows than the context has seen, or a caller's bound on the buffer).
+template <int CELLS>
+__device__ __noinline__ void rows_that_did_not_fit(const SketchArgs &a, uint32_t end, uint32_t *mem) {
+  mem += (threadIdx.x >> 5) * 2 * S_RING;
+  rows_by_warp<CELLS>(a, end, reinterpret_cast<int32_t *>(mem), reinterpret_cast<float *>(mem + S_RING));
+}
+
+// A row as a producing warp keeps it: columns [p, re) are left, `q` candidates of column p are
+// produced already; rs is the row's length, cbase its chunk's first row.
+struct LaneRow {
+  int32_t r, p, re, q, rs, cbase;
+};
+__device__ __forceinline__ LaneRow lane_row(const SketchArgs &a, uint32_t item, uint32_t listed) {
+  LaneRow w = {-1, 0, 0, 0, 0, 0};
+  if (item < listed) {
+    w.r = a.row_list[item];
+    if (!index_ok(a.ctrl, CHK_LIST, w.r, a.n)) w.r = -1;
+  }
+  if (w.r >= 0) {
+    w.p = a.ptr[w.r];
+    w.re = a.ptr[w.r + 1];
+    if (w.p < 0 || w.re < w.p || w.re > a.nnz) {  // malformed row pointers: flag and skip
+      atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
+      w.r = -1;
+      w.p = w.re = 0;
+    }
+    w.rs = w.re - w.p;
+    w.cbase = (w.r / a.chunk) * a.chunk;
+  }
+  return w;
+}
+
+// Place of element u of row l in a ring buffer: shifted by u, so that neither a lane per row
+// (the reader) nor a lane per element (the producer) meets another in a bank.
+__device__ __forceinline__ int ring_at(int u, int l) { return u * 32 + ((l + u) & 31); }
+
+// A row while its part of a ring buffer is filled: the state of LaneRow, the columns in hand (one
+// per lane: group and place of the row in it) and the candidates produced so far.
+struct LaneFill {
+  int32_t p, q, re, rs, cbase, total;
+  int2 sg;
+  int32_t rank;
+};
+__device__ __forceinline__ void load_columns(const SketchArgs &a, LaneFill &f, int lane) {
+  f.sg = make_int2(0, 0);
+  f.rank = 0;
+  if (f.p + lane < f.re) {
+    f.sg = a.seg[f.p + lane];
+    f.rank = a.seg_rank[f.p + lane];
+  }
+}
+// One window of 32 columns for each of K rows (rows first, first + 1, .. of the batch), side by
+// side so that their latencies overlap: lengths, prefix sums, then lane t fetches candidate t,
+// whose column it finds by a search over the prefix sums.
+template <typename Index, int K>
+__device__ __forceinline__ void fill_window(const SketchArgs &a, LaneFill (&f)[K], int first, uint32_t span,
+                                            uint32_t *buffer, int lane) {
+  int32_t left[K], incl[K], all[K], take[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    left[k] = f[k].sg.y >= 2 ? f[k].sg.y - 1 : 0;  // candidates of this lane's column
+    if (lane == 0) left[k] -= f[k].q;
+    incl[k] = left[k];
+  }
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int32_t t = __shfl_up_sync(FULL, incl[k], off);
+      if (lane >= off) incl[k] += t;
+    }
+  }
+  int j[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    all[k] = __shfl_sync(FULL, incl[k], 31);
+    take[k] = min(all[k], L_RING - f[k].total);
+    j[k] = 0;
+  }
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int32_t v = __shfl_sync(FULL, incl[k], j[k] + step - 1);
+      j[k] += v <= lane - f[k].total ? step : 0;  // this lane fetches candidate lane - total of the window
+    }
+  }
+  int2 e[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int x = lane - f[k].total;
+    int32_t ord = x - __shfl_sync(FULL, incl[k] - left[k], j[k]) + (j[k] == 0 ? f[k].q : 0);
+    const int32_t start = __shfl_sync(FULL, f[k].sg.x, j[k]), own = __shfl_sync(FULL, f[k].rank, j[k]);
+    ord += ord >= own ? 1 : 0;  // the row itself is not its candidate
+    e[k] = make_int2(f[k].cbase, 1);
+    if (x >= 0 && x < take[k] && index_ok(a.ctrl, CHK_CAND, start + ord, a.nnz)) e[k] = a.cand[start + ord];
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (take[k] < all[k]) {  // the window holds more: go on from here next time
+      const int jj = __ffs(static_cast<int>(__ballot_sync(FULL, incl[k] > take[k]))) - 1;
+      f[k].q = take[k] - __shfl_sync(FULL, incl[k] - left[k], jj) + (jj == 0 ? f[k].q : 0);
+      f[k].p += jj;
+    } else {
+      f[k].p += 32;
+      f[k].q = 0;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int x = lane - f[k].total;
+    if (x >= 0 && x < take[k]) {
+      const int at = ring_at(lane, first + k);
+      // (a key outside the chunk only comes from rows that are not sorted: kept in bounds)
+      buffer[at] = Index::encode(
+          min(static_cast<uint32_t>(key_in_chunk(a.ctrl, e[k].x, f[k].cbase, a.chunk) - f[k].cbase), span - 1u));
+      buffer[L_RING * 32 + at] = __float_as_uint(2.0f / static_cast<float>(f[k].rs + e[k].y));
+    }
+    f[k].total += take[k];
+  }
+}
+
+// One phase of a producing warp: the next L_RING candidates of each of its rows.  `mine` is the
+// row of lane i < L_ROWS (row number first_row + i of the batch).  The descriptors of the next rows'
+// columns are on their way while a pair of rows is worked on.
+template <typename Index>
+__device__ __forceinline__ void produce_phase(const SketchArgs &a, LaneRow &mine, int first_row, uint32_t span,
+                                              uint32_t *buffer, int32_t *count) {
+  constexpr int K = 2;
+  const int lane = lane_id();
+  auto take_rows = [&](int i, LaneFill (&f)[K]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      f[k].p = __shfl_sync(FULL, mine.p, i + k);
+      f[k].q = __shfl_sync(FULL, mine.q, i + k);
+      f[k].re = __shfl_sync(FULL, mine.re, i + k);
+      f[k].total = 0;
+      load_columns(a, f[k], lane);
+    }
+  };
+  LaneFill next[K];
+  take_rows(0, next);
+#pragma unroll 1
+  for (int i = 0; i < L_ROWS; i += K) {
+    LaneFill f[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      f[k] = next[k];
+      f[k].rs = __shfl_sync(FULL, mine.rs, i + k);
+      f[k].cbase = __shfl_sync(FULL, mine.cbase, i + k);
+    }
+    if (i + K < L_ROWS) take_rows(i + K, next);
+    fill_window<Index, K>(a, f, first_row + i, span, buffer, lane);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {  // few candidates per column: more windows
+      while (f[k].total < L_RING && f[k].p < f[k].re) {
+        LaneFill one[1] = {f[k]};
+        load_columns(a, one[0], lane);
+        fill_window<Index, 1>(a, one, first_row + i + k, span, buffer, lane);
+        f[k] = one[0];
+      }
+      if (lane == i + k) {
+        mine.p = f[k].p;
+        mine.q = f[k].q;
+      }
+      if (lane == 0) count[first_row + i + k] = f[k].total;
+    }
+  }
+}
+
+// Top k of the rows owner = warp, warp + L_WARPS, ... of the batch.
+template <int CELLS, typename Index>
+__device__ __forceinline__ void select_phase(const SketchArgs &a, uint32_t *mem, const LaneRow &row_of_lane) {
+  using L = LaneLayout<CELLS>;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  uint32_t *const tw = mem + L::RING_OFF + warp * L::M;
+  for (int owner = warp; owner < 32; owner += L_WARPS) {
+    const int32_t row = __shfl_sync(FULL, row_of_lane.r, owner);
+    if (row < 0) continue;
+    const int32_t base = __shfl_sync(FULL, row_of_lane.cbase, owner) + a.row_base;
+    Sketch<CELLS> top;  // slot (lane, cell) of the container, as select_top_k has it
+    Index theirs;
+    theirs.mem = mem + L::I_OFF + owner;
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) {
+      const int code = c * 32 + lane;
+      const uint32_t bits = mem[code * 32 + owner];
+      const bool on = bits >= static_cast<uint32_t>(L::M);  // (below: an empty slot)
+      top.key[c] = on ? static_cast<int32_t>(theirs.key(code)) : -1;
+      top.w[c] = on ? __uint_as_float(bits) : 0.0f;
+    }
+    int have = 0;
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) have += __popc(__ballot_sync(FULL, top.key[c] >= 0));
+    top.local_sort_descending();
+    // Entry i of lane l is number l * CELLS + i; the selection takes the heaviest first, on
+    // ties the smaller number: an entry's place is how many come before it.
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) tw[lane * CELLS + c] = __float_as_uint(top.w[c]);
+    __syncwarp();
+    int place[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) place[c] = 0;
+    for (int i4 = 0; i4 * 4 < have; ++i4) {
+      const uint4 v = reinterpret_cast<const uint4 *>(tw)[i4];
+      const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e4 = 0; e4 < 4; ++e4)
+#pragma unroll
+        for (int c = 0; c < CELLS; ++c)
+          place[c] += x[e4] + (i4 * 4 + e4 < lane * CELLS + c ? 1u : 0u) > __float_as_uint(top.w[c]) ? 1 : 0;
+    }
+    uint64_t *const out = a.table + static_cast<size_t>(row) * a.k;
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c)
+      if (top.key[c] >= 0 && place[c] < a.k) out[place[c]] = pack_entry(top.key[c] + base, top.w[c]);
+    for (int j = have + lane; j < a.k; j += 32) out[j] = 0;  // the stages behind stop at the first empty entry
+  }
+}
+
+template <int CELLS, typename Index>
+// (four blocks per SM by registers, so that one also fits beside the 18 warps of a chain block at 128 slots)
+__global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchArgs a) {
+  using L = LaneLayout<CELLS>;
+  extern __shared__ __align__(16) uint32_t lanes_mem[];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t listed = a.ctrl[CTRL_ROWS_LISTED], mid_end = a.ctrl[CTRL_MID_END];
+  const uint32_t span = static_cast<uint32_t>(a.chunk < a.n ? a.chunk : a.n);
+  if (a.ctrl[CTRL_HEAVY_ROWS] < mid_end) rows_that_did_not_fit<CELLS>(a, mid_end, lanes_mem);
+  __syncthreads();
+  LaneShared &sh = *reinterpret_cast<LaneShared *>(lanes_mem + L::SHARED_OFF);
+  uint32_t *const ring = lanes_mem + L::RING_OFF;
+  LaneSketch<CELLS, Index> sk;
+  sk.mem = lanes_mem + lane;
+  sk.index.mem = lanes_mem + L::I_OFF + lane;
+  if (warp == 0) sk.init(span);
+  for (;;) {
+    if (threadIdx.x == 0) sh.first = atomicAdd(&a.ctrl[CTRL_LANE_TICKET], 32u);
+    __syncthreads();
+    const uint32_t first = sh.first;
+    if (first >= listed) break;
+    // (every warp reads all 32 rows: the producers need their own, the selection needs any)
+    const LaneRow row = lane_row(a, first + lane, listed);
+    const int first_row = (warp - 1) * L_ROWS;
+    LaneRow mine = row;
+    if (warp > 0) {
+      const int from = (first_row + lane) & 31;
+      mine.r = __shfl_sync(FULL, row.r, from);
+      mine.p = __shfl_sync(FULL, row.p, from);
+      mine.re = __shfl_sync(FULL, row.re, from);
+      mine.rs = __shfl_sync(FULL, row.rs, from);
+      mine.cbase = __shfl_sync(FULL, row.cbase, from);
+      produce_phase<Index>(a, mine, first_row, span, ring, sh.count[0]);
+    }
+    __syncthreads();
+    for (int b = 0;; b ^= 1) {
+      const int cnt = sh.count[b][lane];
+      const int most = __reduce_max_sync(FULL, cnt);
+      if (most == 0) break;  // the same in every warp: all rows are through
+      if (warp > 0) {
+        produce_phase<Index>(a, mine, first_row, span, ring + (b ^ 1) * L::BUFFER, sh.count[b ^ 1]);
+      } else {
+        const uint32_t *const in = ring + b * L::BUFFER;
+        uint32_t key = in[ring_at(0, lane)], term = in[L_RING * 32 + ring_at(0, lane)];
+        if (cnt == 0) key = 0;  // (no candidate: nothing was written here)
+        int found = sk.index.find(key);
+#pragma unroll 1
+        for (int u = 0; u < most; ++u) {
+          const uint32_t e = key;
+          const float al = __uint_as_float(term);
+          const int next = ring_at(u + 1 < L_RING ? u + 1 : u, lane);  // requested a step ahead
+          key = u + 1 < cnt ? in[next] : 0u;
+          term = in[L_RING * 32 + next];
+          if (u < cnt) found = sk.step(e, al, found, key);
+        }
+      }
+      __syncthreads();
+    }
+    select_phase<CELLS, Index>(a, lanes_mem, row);
+    __syncthreads();
+    if (warp == 0) sk.clear(span);
+  }
+  // Launched as the programmatic dependent of the heavy-chain kernel (see launch_cells): it must
+  // not be seen as finished before that one.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---- heavy rows through materialised streams ------------------------------------------
@@ -612,6 +1037,7 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
   __shared__ unsigned long long carry_s;
   __shared__ uint32_t count_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long lighter = 0;  // stream elements of the rows below HEAVY_WORK (the others are counted already)
   uint32_t H = a.ctrl[CTRL_HEAVY_ROWS];
   if (H > a.heavy_max) H = a.heavy_max;
   if (threadIdx.x == 0) {
@@ -626,6 +1052,7 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
       const int32_t r = a.row_list[i];
       v = a.row_work[r];
       np = static_cast<uint32_t>((a.ptr[r + 1] - a.ptr[r] + H_PART - 1) / H_PART);
+      if (v < HEAVY_WORK) lighter += v;
     }
     // parts first (same scan, second value packed in the high half of 64 bits)
     unsigned long long pk = (static_cast<unsigned long long>(np) << 43) | v;  // sums: < 2^21 parts, < 2^43 entries
@@ -657,6 +1084,10 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
     if (threadIdx.x == 0) carry_s = carry + tot;
     __syncthreads();
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) lighter += __shfl_down_sync(FULL, lighter, off);
+  if (lane == 0 && lighter)
+    atomicAdd(reinterpret_cast<unsigned long long *>(a.ctrl + CTRL_HEAVY_NEED), lighter);
   if (threadIdx.x == 0) {
     const uint32_t Hc = count_s;
     // parts of the rows that stay heavy: part_base[Hc] closes the table
@@ -853,77 +1284,95 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_consume_kernel(SketchArgs 
 // rewrites slot E_i, hits add their alpha (hits on one key all add the same alpha, so
 // their order is immaterial), and the next round starts L elements further on.  While the
 // sketch still has empty slots only (1) applies and miss number i fills the next i-th slot.
-// On the longest R-MAT rows a round resolves 16 elements on average in about 1000 cycles,
-// where 16 sequential steps take 2200.  State lives in shared memory: weights and keys by
-// slot code, a key -> slot table over the chunk's rows, and the per-round order.
-// Diagnostic builds (python -m chunkedgreedy_b200.build --profile-rounds[=2]), printed by the
-// host when CSG_ROUND_PROFILE is set in the environment: -DCSG_ROUND_PROFILE=1 records the
-// run time of every heavy row (two clock reads per row), =2 also the cycles per phase of the
-// longest row's whole-window rounds (which slows those rounds down).
-#if defined(CSG_ROUND_PROFILE) && CSG_ROUND_PROFILE >= 2
-#define PROF_DECL unsigned long long prof_t0 = clock64(), prof_t1
-#define PROF_MARK(i)                                \
-  do {                                              \
-    prof_t1 = clock64();                            \
-    prof[i] += prof_t1 - prof_t0;                   \
-    prof_t0 = prof_t1;                              \
-  } while (0)
-#define PROF_ADD(i, v) prof[i] += (v)
-#else
-#define PROF_DECL
-#define PROF_MARK(i)
-#define PROF_ADD(i, v)
-#endif
-
-constexpr int H_RING = 1024;    // stream elements staged per batch
-constexpr int ROUND_CELLS = 4;  // largest sketch (cells per lane) resolved in rounds
-// Whole-window rounds and the table steps of the light rows are used for sketches of 64 slots
-// (two cells per lane: k = 16 at the default oversampling, the benchmark's configuration).
-// With 128 slots both measured slower on the R-MAT GCN configuration (sketch stage 55.5 ms
-// without either, 62.4 with the whole-window rounds, 65.3 with the table steps, 72.0 with
-// both): the ranking of a round grows with the square of the sketch, and a step's work per
-// lane with its cells.  With 32 slots a window of 32 can take every entry.
-constexpr int WINDOW_CELLS = 2;
+// A group of warps works on one row: its first warp walks the stream and decides the rounds, the other
+// warps order the slots for it (rank_slots), which is most of the instructions of a round and
+// none of its dependent steps; meanwhile the first warp looks the window up.  State lives in
+// shared memory: weights and keys by slot code, a key -> slot table over the chunk's rows, and
+// the order of the round.  Cycles per candidate of the longest rows of R-MAT scale 20, symmetrised
+// (128 slots): 105 with one warp per row, 64 this way; of R-MAT scale 22 (64 slots) 53 and 52 - there
+// the dependent steps of the first warp are the bound and the order comes in their shadow.
+constexpr int H_RING = 512;      // stream elements staged per batch
+constexpr int ROUND_CELLS = 4;   // largest sketch (cells per lane) resolved in rounds
+constexpr int WINDOW_CELLS = 2;  // smallest sketch with whole-window rounds: with 32 slots a window of 32 can take every entry
+constexpr int MATES = 1024;      // words of the duplicate detector
+constexpr int ROUND_TAB_MAX = 65536;  // largest chunk (rows) with a key -> slot table
 constexpr int TRIAL_ROUNDS = 8;     // rounds of each kind a row times before it settles on one ...
 constexpr int COMMIT_ROUNDS = 160;  // ... for this many rounds
-constexpr int ROUND_RING_BYTES = S_WARPS * 2 * H_RING * 8;
+template <int CELLS>
+struct Helpers {
+  static constexpr int N = 2 * CELLS;                    // warps that order the slots, sixteen slots each
+  // Groups (rows) per block, one block per SM: with two the registers of an SM still hold two
+  // blocks of rows_in_lanes_kernel (one at 96 slots and more), which does most of the work of a large call.
+  static constexpr int ROWS = 2;
+  static constexpr int THREADS = 32 * (1 + N);           // of a group
+};
+// named barriers of a group: row in hand, state is ready to be ordered, the order is ready
+constexpr int BAR_ROW = 1, BAR_STATE = 2, BAR_ORDER = 3;
 
 template <int CELLS>
 struct RoundState {
   static constexpr int M = 32 * CELLS;
   __align__(16) uint32_t w[M];   // weight bits by slot code (cell * 32 + lane)
   __align__(16) int32_t key[M];
-  __align__(16) uint32_t sw[M];  // S0 in ascending (weight, code) order: weights ...
-  int32_t si[M];                 // ... and slot codes
-  int32_t rank[M];               // position of each slot in that order
-  int32_t sk[M];                 // ... and keys
+  int32_t rank[M];               // position of each slot in ascending (weight, code) order
+  uint32_t sw[32];               // the 32 lightest in that order: weights ...
+  int32_t si[32];                // ... slot codes ...
+  int32_t sk[32];                // ... and keys
+  uint32_t cw[32];               // the same without the entries that hits hold back
+  int32_t ci[32], ck[32], cr[32];
   int32_t miss_pos[32];          // lane of the i-th miss of the window
-  uint32_t fence_sink;           // see phase_fence
-#ifdef SPORDER_CHECKED
-  uint32_t *ctrl;                // checked build: where a key outside its chunk is recorded ...
-  int32_t span;                  // ... and the rows the key tables cover
-#endif
+  int32_t row_done;              // tells the other warps that the row is through
+  uint32_t item;                 // the row in hand (place in the list)
 };
 
-// The key of a stream element as the rounds use it: in the checked build a key outside the
-// chunk's table is recorded and replaced by the chunk's first row.
-template <int CELLS, bool TAB>
-__device__ __forceinline__ int32_t round_key(const RoundState<CELLS> &st, int32_t s, int32_t cbase) {
-#ifdef SPORDER_CHECKED
-  if (TAB) return key_in_chunk(st.ctrl, s, cbase, st.span);
-#endif
-  (void)st;
-  (void)cbase;
-  return s;
+// A group's shared memory: state, two stream buffers (the next batch lands while this one is
+// consumed), the duplicate detector (all zero between rounds), then the key -> slot table (slot
+// + 1, one byte per row of the chunk; none for very large chunks).  The rounds are functions of
+// their own; they get an offset and build their pointers from the array itself, so that the
+// compiler sees shared memory and not a generic address (slower by some ten cycles a load).
+extern __shared__ __align__(16) unsigned char heavy_dyn[];
+template <int CELLS>
+struct GroupMemory {
+  static constexpr int RING = (sizeof(RoundState<CELLS>) + 15) / 16 * 16;
+  static constexpr int MATE = RING + 2 * H_RING * 8;
+  static constexpr int TAB = MATE + MATES * 4;
+  static __device__ __forceinline__ RoundState<CELLS> &state(int base) {
+    return *reinterpret_cast<RoundState<CELLS> *>(heavy_dyn + base);
+  }
+  static __device__ __forceinline__ int2 *ring(int base, int buffer) {
+    return reinterpret_cast<int2 *>(heavy_dyn + base + RING) + buffer * H_RING;
+  }
+  static __device__ __forceinline__ uint32_t *mates(int base) {
+    return reinterpret_cast<uint32_t *>(heavy_dyn + base + MATE);
+  }
+  static __device__ __forceinline__ uint8_t *tab(int base) { return heavy_dyn + base + TAB; }
+};
+
+// what the rounds of a row need to know
+struct RoundRow {
+  int base;           // the group's place in shared memory
+  int32_t cbase;      // first row of the chunk
+  bool mates_hashed;  // the chunk has more than MATES rows: words are shared
+  uint32_t *ctrl;     // checked build: where a key outside its chunk is recorded ...
+  int32_t span;       // ... and the rows of a chunk
+  int bars;           // the group's named barriers are bars + BAR_*
+};
+
+template <int CELLS>
+__device__ __forceinline__ void bar_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(Helpers<CELLS>::THREADS) : "memory");
+}
+template <int CELLS>
+__device__ __forceinline__ void bar_wait(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(Helpers<CELLS>::THREADS) : "memory");
 }
 
-// Slot that holds key s, or -1.  With TAB from the key -> slot table of the chunk (one byte
-// per row); without it - chunks whose tables would not fit shared memory - by comparing s
-// with every slot's key (keys are unique in a sketch, empty slots hold -1).
+// Slot that holds key s (relative to the chunk), or -1.  With TAB from the key -> slot table;
+// without it by comparing s with every slot's key (unique in a sketch, empty slots hold -1).
 template <int CELLS, bool TAB>
-__device__ __forceinline__ int slot_of(const RoundState<CELLS> &st, const uint8_t *tab, int32_t cbase,
-                                       int32_t s) {
-  if (TAB) return static_cast<int>(tab[s - cbase]) - 1;
+__device__ __forceinline__ int slot_of(const RoundRow &row, int32_t s) {
+  if (TAB) return static_cast<int>(GroupMemory<CELLS>::tab(row.base)[s]) - 1;
+  const RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
   int q = -1;
 #pragma unroll
   for (int i4 = 0; i4 < 8 * CELLS; ++i4) {
@@ -936,98 +1385,122 @@ __device__ __forceinline__ int slot_of(const RoundState<CELLS> &st, const uint8_
   return q;
 }
 
-// Keeps the phases of a round apart in the instruction schedule.  Left alone, ptxas
-// interleaves the window look-up, the count and the limit look-ups, and the round takes
-// 1220 cycles; with a read of %clock between them (which it does not move code across, as
-// long as the value is used) it takes 995.  The values go to a word nobody reads.
-__device__ __forceinline__ void phase_fence(uint32_t &sink) {
-  uint32_t t;
-  asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
-  sink ^= t;
+// One of the other warps: the place of its sixteen slots in the (weight, code) order, the
+// number of entries (x, i) below (mine, slot).  Two lanes per slot, half of the entries each.
+// "x < mine" is counted as sat((mine - x) * 2^90), one fused multiply-add that is exactly 1 or 0:
+// weights lie in [2^-31, 2^32], so two different ones are at least 2^-54 apart.  An equal entry
+// is below for a smaller code; that choice is made per block of four entries (mine or the next
+// float above it), and the slot's own block is put right afterwards.
+template <int CELLS>
+__device__ __forceinline__ void rank_slots(int base, int helper, int lane) {
+  RoundState<CELLS> &st = GroupMemory<CELLS>::state(base);
+  constexpr int M = 32 * CELLS, QUADS = M / 8;  // blocks of four entries per half
+  constexpr float BIG = 1.2379400392853803e27f;  // 2^90
+  const int slot = helper * 16 + (lane & 15), half = lane >> 4, own = slot >> 2;
+  const float4 *const v4 = reinterpret_cast<const float4 *>(st.w);
+  const uint32_t bits = st.w[slot];
+  const int32_t key = st.key[slot];
+  const float mine = __uint_as_float(bits);
+  const float lt = mine * BIG, le = __uint_as_float(bits + 1u) * BIG;
+  const float4 mates = v4[own];
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float4 all[QUADS];  // (loaded in one go: left to itself the compiler waits for every load)
+#pragma unroll
+  for (int b = 0; b < QUADS; ++b) all[b] = v4[half * QUADS + b];
+#pragma unroll
+  for (int b = 0; b < QUADS; ++b) {
+    const float bar = half * QUADS + b < own ? le : lt;
+    acc[0] += __saturatef(fmaf(all[b].x, -BIG, bar));
+    acc[1] += __saturatef(fmaf(all[b].y, -BIG, bar));
+    acc[2] += __saturatef(fmaf(all[b].z, -BIG, bar));
+    acc[3] += __saturatef(fmaf(all[b].w, -BIG, bar));
+  }
+  int pos = static_cast<int>((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  if (own / QUADS == half) {
+    const int e = slot & 3;
+    pos += (e > 0 && mates.x == mine ? 1 : 0) + (e > 1 && mates.y == mine ? 1 : 0) + (e > 2 && mates.z == mine ? 1 : 0);
+  }
+  pos += __shfl_xor_sync(FULL, pos, 16);
+  if (half == 0) {
+    st.rank[slot] = pos;
+    if (pos < 32) st.sw[pos] = bits;
+  } else if (pos < 32) {
+    st.si[pos] = slot;
+    st.sk[pos] = key;
+  }
 }
 
-// One round on a full sketch; returns the number of stream elements resolved (>= 1).
+// The window of a round, one element per lane, as looked up before the order is known.
+template <int CELLS>
+struct Window {
+  bool valid;
+  int32_t s;      // key, relative to the chunk
+  float al;       // Dice term
+  int q;          // slot that holds the key, or -1
+  int32_t mate;   // word of the duplicate detector
+};
+
 template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_full(RoundState<CELLS> &st, uint8_t *tab, int32_t cbase,
-                                          const int2 *ring, int p, int cnt, int lane,
-                                          uint32_t &sink) {
-  constexpr int M = 32 * CELLS;
-  const uint32_t below = (1u << lane) - 1u;
-  phase_fence(sink);
-  const bool valid = p + lane < cnt;
-  const int2 elem = valid ? ring[p + lane] : make_int2(0, 0);
-  const int32_t s = round_key<CELLS, TAB>(st, elem.x, cbase);
-  const float al = __int_as_float(elem.y);
-  uint32_t mine[CELLS];
-  int32_t mykey[CELLS];
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) {
-    mine[c] = st.w[c * 32 + lane];
-    mykey[c] = st.key[c * 32 + lane];
-  }
-  const int q = valid ? slot_of<CELLS, TAB>(st, tab, cbase, s) : 0;
-  const bool miss = valid && q < 0;
-  const bool hit = valid && q >= 0;
-  // lanes carrying the same key: a second miss of a key ends the prefix (1); hits of one
-  // key are added by the first of them
-  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
-  const uint32_t wq = st.w[hit ? q : 0];
-  const uint32_t missing = __ballot_sync(FULL, miss);
-  const int mtot = __popc(missing);
-  const int mrank = __popc(missing & below);
-  phase_fence(sink);
-  // Position of this lane's slots in the (weight, code) order of S0: the number of entries
-  // (x, i) below (mine, code).  Weight bit patterns are below 2^31, so x < y is the sign of
-  // x - y, and "below" is x < mine + 1 for a smaller code i, x < mine for a larger one.
-  // Four chains per slot: one long chain would run at add latency.
-  int pos[CELLS];
-  {
-    int32_t acc[CELLS][4];
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0;
-    uint4 v[M / 4];
-#pragma unroll
-    for (int i4 = 0; i4 < M / 4; ++i4) v[i4] = reinterpret_cast<const uint4 *>(st.w)[i4];
-#pragma unroll
-    for (int i4 = 0; i4 < M / 4; ++i4) {
-      const uint32_t x[4] = {v[i4].x, v[i4].y, v[i4].z, v[i4].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = i4 * 4 + e, ci = i >> 5, li = i & 31;
-        const uint32_t lower = (below >> li) & 1u;  // code li of this cell is below this lane's
-#pragma unroll
-        for (int c = 0; c < CELLS; ++c) {
-          uint32_t d = x[e] - mine[c];
-          if (ci < c) d -= 1u;
-          else if (ci == c) d -= lower;
-          acc[c][e] += static_cast<int32_t>(d) >> 31;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c) pos[c] = -((acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]));
-  }
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) {
-    st.sw[pos[c]] = mine[c];
-    st.si[pos[c]] = c * 32 + lane;
-    st.sk[pos[c]] = mykey[c];
-    st.rank[c * 32 + lane] = pos[c];
-  }
-  phase_fence(sink);
-  if (miss) st.miss_pos[mrank] = lane;
+__device__ __forceinline__ Window<CELLS> look_up(const RoundRow &row, int buf, int p, int cnt, int lane) {
+  const int2 *const ring = GroupMemory<CELLS>::ring(row.base, buf);
+  Window<CELLS> w;
+  w.valid = p + lane < cnt;
+  const int2 elem = w.valid ? ring[p + lane] : make_int2(row.cbase, 0);
+  // (a key outside the chunk only comes from rows that are not sorted: kept in bounds)
+  w.s = static_cast<int32_t>(min(static_cast<uint32_t>(key_in_chunk(row.ctrl, elem.x, row.cbase, row.span) - row.cbase),
+                                 static_cast<uint32_t>(row.span) - 1u));
+  w.al = __int_as_float(elem.y);
+  // Lanes that carry the same key: every lane sets its bit in a word of shared memory under its
+  // key, and reads the word back later.  match.any, the instruction made for this, takes some
+  // 380 cycles here.
+  w.mate = row.mates_hashed ? static_cast<int32_t>((static_cast<uint32_t>(w.s) * 0x9E3779B1u) >> 22) : w.s;
+  if (w.valid) atomicOr(&GroupMemory<CELLS>::mates(row.base)[w.mate], 1u << lane);
+  w.q = w.valid ? slot_of<CELLS, TAB>(row, w.s) : -1;
+  return w;
+}
+
+// lanes of the window with this lane's key; clears the detector
+template <int CELLS>
+__device__ __forceinline__ unsigned same_key(const RoundRow &row, const Window<CELLS> &w, int lane) {
+  uint32_t *const mates = GroupMemory<CELLS>::mates(row.base);
   __syncwarp();
-  phase_fence(sink);
+  unsigned same = w.valid ? mates[w.mate] : 0u;
+  if (row.mates_hashed) {  // a word may stand for several keys: rare, then the slow instruction
+    const int32_t first = __shfl_sync(FULL, w.s, same ? __ffs(static_cast<int>(same)) - 1 : lane);
+    if (__any_sync(FULL, w.valid && first != w.s)) same = __match_any_sync(FULL, w.valid ? w.s : -1 - lane);
+    if (!w.valid) same = 0u;
+  }
+  __syncwarp();
+  if (w.valid) mates[w.mate] = 0u;
+  return same;
+}
+
+// One strict round on a full sketch; returns the number of stream elements resolved (>= 1).
+template <int CELLS, bool TAB>
+__device__ __forceinline__ int round_strict(const RoundRow &row, int buf, int p, int cnt, int lane) {
+  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
+  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
+  const uint32_t below = (1u << lane) - 1u;
+  bar_arrive<CELLS>(row.bars + BAR_STATE);
+  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
+  const bool miss = w.valid && w.q < 0, hit = w.valid && w.q >= 0;
+  const int q = hit ? w.q : 0;
+  const uint32_t wq = st.w[q];
+  const uint32_t missing = __ballot_sync(FULL, miss);
+  const int mtot = __popc(missing), mrank = __popc(missing & below);
+  if (miss) st.miss_pos[mrank] = lane;
+  const unsigned same = same_key<CELLS>(row, w, lane);
+  bar_wait<CELLS>(row.bars + BAR_ORDER);
   // every lane reads what either kind of element needs, then selects
-  const int rho = st.rank[hit ? q : 0];
-  const int tgt = st.si[mrank];
-  const uint32_t base = st.sw[mrank];
-  const int32_t old_key = st.sk[mrank];
+  const int rho = st.rank[q];
+  const int tgt = st.si[mrank & 31];
+  const uint32_t base = st.sw[mrank & 31];
+  const int32_t old_key = st.sk[mrank & 31];
   const uint32_t top = st.sw[mtot > 0 ? mtot - 1 : 0];
   const int at_hit = st.miss_pos[rho & 31];
   const int at_next = st.miss_pos[(mrank + 1) & 31];
-  const uint32_t nb = __float_as_uint(__uint_as_float(base) + al);
-  int lim = valid ? 32 : lane;
+  const uint32_t nb = __float_as_uint(__uint_as_float(base) + w.al);
+  int lim = w.valid ? 32 : lane;
   if (hit) {  // (2): this hit and the miss that takes its slot cannot share a prefix
     const int at = rho < mtot ? at_hit : 32;
     lim = at > lane ? at : lane;
@@ -1039,21 +1512,18 @@ __device__ __forceinline__ int round_full(RoundState<CELLS> &st, uint8_t *tab, i
     if (nb <= top) lim = nb > base ? (mrank + 1 < mtot ? at_next : 32) : lane;
     if (same & below) lim = lane;  // (1)
   }
-  phase_fence(sink);
   int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
   L = L < 1 ? 1 : L;  // one element alone is always resolved exactly
   const bool applies = lane < L;
   const unsigned mates = same & (L >= 32 ? FULL : (1u << L) - 1u);
   const int times = __popc(mates);
-  float wv = __uint_as_float(wq) + al;
-  if (times > 1) wv += al;
-  if (times > 2)
-    for (int t = 2; t < times; ++t) wv += al;
+  float wv = __uint_as_float(wq) + w.al;
+  for (int t = 1; t < times; ++t) wv += w.al;
   if (applies && miss) {
-    if (TAB) tab[old_key - cbase] = 0;
-    st.key[tgt] = s;
+    if (TAB) tab[old_key] = 0;
+    st.key[tgt] = w.s;
     st.w[tgt] = nb;
-    if (TAB) tab[s - cbase] = static_cast<uint8_t>(tgt + 1);
+    if (TAB) tab[w.s] = static_cast<uint8_t>(tgt + 1);
   }
   if (applies && hit && (mates & below) == 0u) st.w[q] = __float_as_uint(wv);  // first hit of its key
   __syncwarp();
@@ -1061,8 +1531,8 @@ __device__ __forceinline__ int round_full(RoundState<CELLS> &st, uint8_t *tab, i
 }
 
 // One round on a full sketch of 64 slots or more that resolves the WHOLE window.  The three
-// conditions of round_full end a prefix at the first element whose outcome cannot be read off
-// the order of S0 directly.  Almost all of those are hits on an entry that the misses of the
+// conditions of the strict round end a prefix at the first element whose outcome cannot be read
+// off the order of S0 directly.  Almost all of those are hits on an entry that the misses of the
 // window are about to take, and their outcome still follows from S0 by a little bookkeeping:
 //   * the misses take the entries of S0 in order, but skip an entry that a hit has made
 //     heavier before they reached it (put back one Dice term heavier, an entry lands behind
@@ -1076,100 +1546,44 @@ __device__ __forceinline__ int round_full(RoundState<CELLS> &st, uint8_t *tab, i
 // the entry is gone iff P + b > r.  Bounds on P + b settle most of them without looking at
 // the others (see "slack" below); a window where one stays undecided walks them in stream
 // order (a handful per window, state in two 32-bit masks, every lane computing the same).
-// The miss with i misses before it
-// then takes the (i+1)-th entry that no hit holds back.  The read-off is exact as long as
-// nothing put back or made heavier is light enough to be taken again inside the window; an
-// element whose new weight does not clear the heaviest entry taken ends the prefix before the
-// next miss behind it (before itself, if its weight did not grow at all).  On the heaviest
-// R-MAT rows that happens in one window of 32,000 (the row's own Dice terms dominate) to one
-// in ten (rows whose terms vary more), and a round resolves 32.0 resp. 29.3 elements where
-// round_full resolves 16.4 on the former; it costs about 1.8 times a round_full, which is why
+// The miss with i misses before it then takes the (i+1)-th entry that no hit holds back.  The
+// read-off is exact as long as nothing put back or made heavier is light enough to be taken
+// again inside the window; an element whose new weight does not clear the heaviest entry taken
+// ends the prefix before the next miss behind it (before itself, if its weight did not grow at
+// all).  On the heaviest R-MAT rows that happens in one window of 32,000 (the row's own Dice
+// terms dominate) to one in ten (rows whose terms vary more), and a round resolves 32.0 resp.
+// 29.3 elements where a strict one resolves 16.4 on the former; on rows whose terms vary widely
+// either kind ends after 6 to 13 and the strict round is the cheaper one, which is why
 // rounds_row times both kinds on every row and keeps the one that resolves more per cycle.
-#ifdef CSG_WINDOW_FENCES
-#define WINDOW_FENCE(s) phase_fence(s)
-#else
-#define WINDOW_FENCE(s)
-#endif
 template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_window(RoundState<CELLS> &st, uint8_t *tab, uint32_t *mates,
-                                            int32_t cbase, const int2 *ring, int p, int cnt, int lane,
-                                            uint32_t &sink, unsigned long long *prof) {
+__device__ __forceinline__ int round_window(const RoundRow &row, int buf, int p, int cnt, int lane) {
+  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
+  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
   constexpr int M = 32 * CELLS;
-  static_assert(CELLS >= 2, "a window of 32 needs more than 32 slots");
+  static_assert(CELLS >= WINDOW_CELLS, "a window of 32 needs more than 32 slots");
   const uint32_t below = (1u << lane) - 1u;
-  PROF_DECL;
-  WINDOW_FENCE(sink);
-  const bool valid = p + lane < cnt;
-  const int2 elem = valid ? ring[p + lane] : make_int2(0, 0);
-  const int32_t s = round_key<CELLS, TAB>(st, elem.x, cbase);
-  const float al = __int_as_float(elem.y);
-  // Lanes that carry the same key: every lane sets its bit in a word of shared memory under
-  // its key and reads the word back (cleared again at the end of the round).  match.any, the
-  // instruction made for this, takes some 380 cycles here; it serves chunks too large for
-  // the table.
-  if (mates != nullptr && valid) atomicOr(&mates[s - cbase], 1u << lane);
-  uint32_t mine[CELLS];
-  int32_t mykey[CELLS];
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) {
-    mine[c] = st.w[c * 32 + lane];
-    mykey[c] = st.key[c * 32 + lane];
-  }
-  const int q = valid ? slot_of<CELLS, TAB>(st, tab, cbase, s) : -1;
-  const bool present = valid && q >= 0;  // S0 holds the key
-  const uint32_t wq = st.w[present ? q : 0];
-  WINDOW_FENCE(sink);
-  PROF_MARK(0);
-  // position of this lane's slots in the (weight, code) order of S0 (see round_full)
-  int pos[CELLS];
-  {
-    int32_t acc[CELLS][4];
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0;
-    uint4 v[M / 4];
-#pragma unroll
-    for (int i4 = 0; i4 < M / 4; ++i4) v[i4] = reinterpret_cast<const uint4 *>(st.w)[i4];
-#pragma unroll
-    for (int i4 = 0; i4 < M / 4; ++i4) {
-      const uint32_t x[4] = {v[i4].x, v[i4].y, v[i4].z, v[i4].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = i4 * 4 + e, ci = i >> 5, li = i & 31;
-        const uint32_t lower = (below >> li) & 1u;
-#pragma unroll
-        for (int c = 0; c < CELLS; ++c) {
-          uint32_t d = x[e] - mine[c];
-          if (ci < c) d -= 1u;
-          else if (ci == c) d -= lower;
-          acc[c][e] += static_cast<int32_t>(d) >> 31;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c) pos[c] = -((acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]));
-  }
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) st.rank[c * 32 + lane] = pos[c];
-  __syncwarp();
-  WINDOW_FENCE(sink);
-  PROF_MARK(1);
+  bar_arrive<CELLS>(row.bars + BAR_STATE);
+  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
+  const bool present = w.valid && w.q >= 0;  // S0 holds the key
+  const int q = present ? w.q : 0;
+  const uint32_t wq = st.w[q];
+  const unsigned same = same_key<CELLS>(row, w, lane);
+  const bool leader = w.valid && (same & below) == 0u;  // first element of its key in the window
+  const uint32_t absent = __ballot_sync(FULL, leader && !present);
+  const int absent_before = __popc(absent & below);
+  bar_wait<CELLS>(row.bars + BAR_ORDER);
   const int rho = present ? st.rank[q] : M;
-  unsigned same;
-  if (mates != nullptr)
-    same = valid ? mates[s - cbase] : 0u;
-  else
-    same = __match_any_sync(FULL, valid ? s : -1 - lane);
-  const bool leader = valid && (same & below) == 0u;  // first element of its key in the window
+  const uint32_t my_w = st.sw[lane];  // the entry of rank `lane`
+  const int32_t my_i = st.si[lane], my_k = st.sk[lane];
   // Which leaders miss: those S0 does not hold, and those whose entry is gone by their turn.
   // An open element (leader, entry among the 32 lightest) with `before` certain misses and
   // `nth` open elements in front of it: at least `before`, at most `before + nth` entries
   // below its own are taken or skipped by its turn, so rank < before means gone and
   // rank >= before + nth means still there, whatever the open elements in front did.  Most
   // windows have only such elements; the others are walked in stream order.
-  const uint32_t absent = __ballot_sync(FULL, leader && !present);
   const bool open = leader && present && rho < 32;
   uint32_t open_set = __ballot_sync(FULL, open);
-  const int slack = rho - __popc(absent & below);
+  const int slack = rho - absent_before;
   const bool sure_gone = open && slack < 0;
   const bool sure_held = open && slack >= __popc(open_set & below);
   uint32_t flipped = __ballot_sync(FULL, sure_gone);  // lanes whose entry was taken before their turn
@@ -1189,86 +1603,67 @@ __device__ __forceinline__ int round_window(RoundState<CELLS> &st, uint8_t *tab,
         held |= 1u << r;
     }
   }
-  PROF_MARK(2);
   const uint32_t missing = absent | flipped;
   const int mtot = __popc(missing);
   const bool miss = (missing >> lane) & 1u;
-  // The i-th miss takes the i-th entry of the order that no hit holds back: the owners of those
-  // entries write them out in that numbering (rank minus the held ranks below it).
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) {
-    const int r = pos[c];
-    if (r < 32 && ((held >> r) & 1u) == 0u) {
-      const int at = r - __popc(held & ((1u << r) - 1u));
-      st.sw[at] = mine[c];
-      st.si[at] = c * 32 + lane;
-      st.sk[at] = mykey[c];
-      st.miss_pos[at] = r;
-    }
+  // the i-th miss takes the i-th entry of the order that no hit holds back
+  if (((held >> lane) & 1u) == 0u) {
+    const int at = lane - __popc(held & below);
+    st.cw[at] = my_w;
+    st.ci[at] = my_i;
+    st.ck[at] = my_k;
+    st.cr[at] = lane;
   }
-  __syncwarp();
-  WINDOW_FENCE(sink);
-  PROF_MARK(3);
   const int mine_i = miss ? __popc(missing & below) : 0;
   const int last_i = mtot > 0 ? mtot - 1 : 0;
-  const int tgt = st.si[mine_i];
-  const uint32_t base = st.sw[mine_i];
-  const int32_t old_key = st.sk[mine_i];
-  const uint32_t top = st.sw[last_i];
-  const int t_last = mtot > 0 ? st.miss_pos[last_i] : -1;  // rank of the heaviest entry taken
   const uint32_t behind = missing & ~(below | (1u << lane));
-  const int next_miss = behind ? __ffs(behind) - 1 : 32;
-  const uint32_t nb = __float_as_uint(__uint_as_float(base) + al);
-  const uint32_t hv = __float_as_uint(__uint_as_float(wq) + al);
-  int lim = valid ? 32 : lane;
+  const int next_miss = behind ? __ffs(static_cast<int>(behind)) - 1 : 32;
+  const uint32_t hv = __float_as_uint(__uint_as_float(wq) + w.al);
+  __syncwarp();
+  const uint32_t base = st.cw[mine_i];
+  const uint32_t top = st.cw[last_i];
+  const int t_last = mtot > 0 ? st.cr[last_i] : -1;  // rank of the heaviest entry taken
+  const int tgt = st.ci[mine_i];
+  const int32_t old_key = st.ck[mine_i];
+  const uint32_t nb = __float_as_uint(__uint_as_float(base) + w.al);
+  int lim = w.valid ? 32 : lane;
   if (mtot > 0) {
     if (miss && nb <= top) lim = nb > base ? next_miss : lane;
     if (leader && present && !miss && rho <= t_last && hv <= top) lim = hv > wq ? next_miss : lane;
   }
-  WINDOW_FENCE(sink);
   int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
   L = L < 1 ? 1 : L;  // one element alone is always resolved exactly
-  PROF_MARK(4);
   const bool applies = lane < L && leader;
   const int times = __popc(same & (L >= 32 ? FULL : (1u << L) - 1u));
   float wv = miss ? __uint_as_float(nb) : __uint_as_float(hv);
-  for (int k = 1; k < times; ++k) wv += al;  // later elements of the key, in stream order
-  if (TAB && applies && miss) tab[old_key - cbase] = 0;
-  if (mates != nullptr && valid) mates[s - cbase] = 0u;
+  for (int k = 1; k < times; ++k) wv += w.al;  // later elements of the key, in stream order
+  if (TAB && applies && miss) tab[old_key] = 0;
   // (a key taken by one miss may be put back by a later one, which then is a flipped lane:
   // clear first, then set)
   if (flipped) __syncwarp();
   if (applies && miss) {
-    st.key[tgt] = s;
+    st.key[tgt] = w.s;
     st.w[tgt] = __float_as_uint(wv);
-    if (TAB) tab[s - cbase] = static_cast<uint8_t>(tgt + 1);
+    if (TAB) tab[w.s] = static_cast<uint8_t>(tgt + 1);
   }
   if (applies && !miss) st.w[q] = __float_as_uint(wv);
   __syncwarp();
-  PROF_MARK(5);
-  PROF_ADD(6, 1);
-  PROF_ADD(7, L);
   return L;
 }
 
-// One round while the sketch has empty slots; `filled` is updated.
+// One round while the sketch has empty slots; `filled` is updated.  (No order needed.)
 template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_fill(RoundState<CELLS> &st, uint8_t *tab, int32_t cbase,
-                                          const int2 *ring, int p, int cnt, int lane,
-                                          int &filled) {
+__device__ __forceinline__ int round_fill(const RoundRow &row, int buf, int p, int cnt, int lane, int &filled) {
+  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
+  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
   constexpr int M = 32 * CELLS;
   const uint32_t below = (1u << lane) - 1u;
-  const bool valid = p + lane < cnt;
-  const int2 elem = valid ? ring[p + lane] : make_int2(0, 0);
-  const int32_t s = round_key<CELLS, TAB>(st, elem.x, cbase);
-  const float al = __int_as_float(elem.y);
-  const int q = valid ? slot_of<CELLS, TAB>(st, tab, cbase, s) : 0;
-  const bool miss = valid && q < 0;
-  const bool hit = valid && q >= 0;
+  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
+  const bool miss = w.valid && w.q < 0, hit = w.valid && w.q >= 0;
   const uint32_t missing = __ballot_sync(FULL, miss);
   const int mrank = __popc(missing & below);
-  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
-  int lim = valid ? 32 : lane;
+  const unsigned same = same_key<CELLS>(row, w, lane);
+  int lim = w.valid ? 32 : lane;
   if (miss && ((same & below) || mrank >= M - filled)) lim = lane;
   const int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
   const unsigned prefix = L >= 32 ? FULL : (1u << L) - 1u;
@@ -1276,13 +1671,13 @@ __device__ __forceinline__ int round_fill(RoundState<CELLS> &st, uint8_t *tab, i
     if (miss) {
       const int j = filled + mrank;  // j-th slot to be filled: lane j / CELLS, cell j % CELLS
       const int code = (j % CELLS) * 32 + j / CELLS;
-      st.key[code] = s;
-      st.w[code] = __float_as_uint(al);
-      if (TAB) tab[s - cbase] = static_cast<uint8_t>(code + 1);
+      st.key[code] = w.s;
+      st.w[code] = __float_as_uint(w.al);
+      if (TAB) tab[w.s] = static_cast<uint8_t>(code + 1);
     } else if (hit && ((same & prefix) & below) == 0u) {
-      float wv = __uint_as_float(st.w[q]);
-      for (int t = __popc(same & prefix); t > 0; --t) wv += al;
-      st.w[q] = __float_as_uint(wv);
+      float wv = __uint_as_float(st.w[w.q]);
+      for (int t = __popc(same & prefix); t > 0; --t) wv += w.al;
+      st.w[w.q] = __float_as_uint(wv);
     }
   }
   filled += __popc(missing & prefix);
@@ -1290,9 +1685,6 @@ __device__ __forceinline__ int round_fill(RoundState<CELLS> &st, uint8_t *tab, i
   return L;
 }
 
-// Same contract as heavy_consume_kernel (one warp per heavy row, one block per SM, final
-// sketch to heavy_state), resolving the stream in rounds.  The dynamic shared memory that
-// keeps the block alone on its SM holds the key -> slot tables, `tab_bytes` per warp.
 // copies `cnt` stream elements into a ring buffer without passing through registers
 __device__ __forceinline__ void stage_batch(int2 *ring, const int2 *in, int cnt, int lane) {
   for (int i = lane; i < cnt; i += 32) {
@@ -1302,52 +1694,47 @@ __device__ __forceinline__ void stage_batch(int2 *ring, const int2 *in, int cnt,
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// The whole-window rounds as a function of their own (like rounds_row below: compiled into one
-// body with the strict rounds, each kind loses speed to the other's registers and schedule).
-// Whole-window rounds on [p, cnt) of a batch, at most `left` of them.
+// Rounds of one kind on [p, cnt) of a batch, at most `left` of them; returns where they got to
+// and how many are left.  Functions of their own:
+// compiled into one body each kind loses speed to the other's registers and schedule.
 template <int CELLS, bool TAB>
-__device__ __noinline__ int window_rounds(RoundState<CELLS> &st, uint8_t *tab, uint32_t *mates,
-                                          int32_t cbase, const int2 *ring, int p, int cnt, int &left,
-                                          unsigned long long *prof) {
+__device__ __noinline__ int2 window_rounds(const RoundRow row, int buf, int p, int cnt, int left) {
   const int lane = lane_id();
-  uint32_t sink = 0;
   while (p < cnt && left > 0) {
-    p += round_window<CELLS, TAB>(st, tab, mates, cbase, ring, p, cnt, lane, sink, prof);
+    p += round_window<CELLS, TAB>(row, buf, p, cnt, lane);
     --left;
   }
-  if (lane == 0) st.fence_sink = sink;
-  return p;
+  return make_int2(p, left);
+}
+template <int CELLS, bool TAB>
+__device__ __noinline__ int2 strict_rounds(const RoundRow row, int buf, int p, int cnt, int left) {
+  const int lane = lane_id();
+  while (p < cnt && left > 0) {
+    p += round_strict<CELLS, TAB>(row, buf, p, cnt, lane);
+    --left;
+  }
+  return make_int2(p, left);
 }
 
-// One heavy row, start to finish: stream batches in, rounds, final sketch out.  Not
-// inlined: compiled as part of the kernel's ticket loop the same rounds take 1280 cycles
-// instead of 1000.
+// One heavy row, start to finish, by the first warp: stream batches in, rounds, final sketch out.
 template <int CELLS, bool TAB>
-__device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, int32_t cbase,
-                                        RoundState<CELLS> &st, uint8_t *tab, uint32_t *mates, int2 *ring0,
-                                        int2 *ring1, int32_t *out, unsigned long long *prof_out) {
+__device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, const RoundRow row, int32_t *out) {
+  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
+  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
+  int2 *const ring0 = GroupMemory<CELLS>::ring(row.base, 0), *const ring1 = GroupMemory<CELLS>::ring(row.base, 1);
   constexpr int M = 32 * CELLS;
   const int lane = lane_id();
-  unsigned long long prof[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  (void)prof;
-  (void)prof_out;
 #pragma unroll
   for (int c = 0; c < CELLS; ++c) {
     st.key[c * 32 + lane] = -1;
     st.w[c * 32 + lane] = 0u;
   }
   int filled = 0, buf = 0;
-  // (see the loop below) kind of round in use, rounds left in the stretch, the trial being
-  // booked (0 window, 1 strict, -1 none), and what the trials resolved in how many cycles
-#ifdef CSG_STRICT_ONLY
-  int mode = 1, left = 1 << 30, trial = -1;
-#else
+  // (see the loop below) kind of round in use (0 window, 1 strict), rounds left in the stretch,
+  // the trial being booked (-1 none), and what the trials resolved in how many cycles
   int mode = 0, left = TRIAL_ROUNDS, trial = 0;
-
-#endif
   long long got[2] = {0, 0}, took[2] = {0, 0};
   int streak = 0, last_mode = -1;
-  uint32_t sink = 0;
   __syncwarp();
   stage_batch(ring0, in, static_cast<int>(total < H_RING ? total : H_RING), lane);
   for (uint32_t base = 0; base < total; base += H_RING) {
@@ -1359,10 +1746,9 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, int32_t 
       asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest group: this batch is in
     __syncwarp();
-    const int2 *ring = buf ? ring1 : ring0;
     int p = 0;
-    while (p < cnt && filled < M) p += round_fill<CELLS, TAB>(st, tab, cbase, ring, p, cnt, lane, filled);
-    if constexpr (CELLS == WINDOW_CELLS) {
+    while (p < cnt && filled < M) p += round_fill<CELLS, TAB>(row, buf, p, cnt, lane, filled);
+    if constexpr (CELLS >= WINDOW_CELLS) {
       // Which kind of round is faster depends on the row: a whole-window round costs more and
       // pays where it resolves (nearly) the whole window - rows whose own length dominates their
       // Dice terms.  Where the terms vary widely, entries put back light are taken again at
@@ -1373,14 +1759,10 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, int32_t 
       while (p < cnt) {
         const int before = p;
         const long long t0 = clock64();
-        if (mode == 0) {
-          p = window_rounds<CELLS, TAB>(st, tab, mates, cbase, ring, p, cnt, left, prof);
-        } else {  // (in line: as a function of its own this kind runs a tenth slower)
-          while (p < cnt && left > 0) {
-            p += round_full<CELLS, TAB>(st, tab, cbase, ring, p, cnt, lane, sink);
-            --left;
-          }
-        }
+        const int2 at = mode == 0 ? window_rounds<CELLS, TAB>(row, buf, p, cnt, left)
+                                  : strict_rounds<CELLS, TAB>(row, buf, p, cnt, left);
+        p = at.x;
+        left = at.y;
         if (trial >= 0) {  // a trial stretch: book it
           got[trial] += p - before;
           took[trial] += clock64() - t0;
@@ -1390,27 +1772,24 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, int32_t 
             trial = 1;
             mode = 1;
             left = TRIAL_ROUNDS;
-          } else {
-            if (trial == 1)  // both tried: elements per cycle, compared without dividing
-              mode = got[0] * took[1] >= got[1] * took[0] ? 0 : 1;
-            if (trial == 1) {
-              // the stretch grows while the same kind keeps winning (up to 16 times as long)
-              streak = mode == last_mode ? (streak < 4 ? streak + 1 : 4) : 0;
-              last_mode = mode;
-              trial = -1;
-              left = COMMIT_ROUNDS << streak;
-            } else {  // a committed stretch is over: measure again
-              trial = 0;
-              mode = 0;
-              left = TRIAL_ROUNDS;
-              got[0] = got[1] = 0;
-              took[0] = took[1] = 0;
-            }
+          } else if (trial == 1) {  // both tried: elements per cycle, compared without dividing
+            mode = got[0] * took[1] >= got[1] * took[0] ? 0 : 1;
+            // the stretch grows while the same kind keeps winning (up to 16 times as long)
+            streak = mode == last_mode ? (streak < 4 ? streak + 1 : 4) : 0;
+            last_mode = mode;
+            trial = -1;
+            left = COMMIT_ROUNDS << streak;
+          } else {  // a committed stretch is over: measure again
+            trial = 0;
+            mode = 0;
+            left = TRIAL_ROUNDS;
+            got[0] = got[1] = 0;
+            took[0] = took[1] = 0;
           }
         }
       }
-    } else {  // other sketch sizes: strict rounds (see WINDOW_CELLS)
-      while (p < cnt) p += round_full<CELLS, TAB>(st, tab, cbase, ring, p, cnt, lane, sink);
+    } else {
+      strict_rounds<CELLS, TAB>(row, buf, p, cnt, 1 << 30);
     }
     buf ^= 1;
   }
@@ -1418,109 +1797,64 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, int32_t 
 #pragma unroll
   for (int c = 0; c < CELLS; ++c) {
     const int32_t kk = st.key[c * 32 + lane];
-    out[(2 * c) * 32 + lane] = kk;
+    out[(2 * c) * 32 + lane] = kk >= 0 ? kk + row.cbase : -1;
     out[(2 * c + 1) * 32 + lane] = static_cast<int32_t>(st.w[c * 32 + lane]);
-    if (TAB && kk >= 0) tab[kk - cbase] = 0;  // the table is empty again for the next row
+    if (TAB && kk >= 0) tab[kk] = 0;  // the table is empty again for the next row
   }
-  if (lane == 0) st.fence_sink = sink;
-#ifdef CSG_ROUND_PROFILE
-  if (lane == 0 && prof_out != nullptr)
-    for (int i = 0; i < 12; ++i) atomicAdd(prof_out + i, prof[i]);
-#endif
   __syncwarp();
 }
 
-// WARPS per block: four (a scheduler each) for the chains that decide how long the call
-// takes; eight, two to a scheduler, for the chains of the rest of a call that runs one chunk
-// ahead - they have time to spare and then hold half as many SMs.
-template <int CELLS, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 1) heavy_rounds_kernel(SketchArgs a, int tab_bytes, int mates_words) {
-  // dynamic shared memory: two stream buffers per warp (the next batch lands while this
-  // one is consumed), then the key tables
-  extern __shared__ __align__(16) unsigned char heavy_dyn[];
-  constexpr int RING_BYTES = WARPS * 2 * H_RING * 8;
-  int2(*rings)[2][H_RING] = reinterpret_cast<int2(*)[2][H_RING]>(heavy_dyn);
-  __shared__ RoundState<CELLS> state[WARPS];
-  const int lane = lane_id(), warp = threadIdx.x >> 5;
+// A group of warps per heavy row, in list order (longest first).  Several groups to a block, so
+// that the chains of a call that runs one chunk ahead fill few SMs while the rest of the call
+// is transposed on the others.
+template <int CELLS>
+__global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS) __maxnreg__(CELLS <= 2 ? 88 : 72)
+    heavy_rounds_kernel(SketchArgs a, int tab_bytes) {
+  constexpr int THREADS = Helpers<CELLS>::THREADS;
+  using G = GroupMemory<CELLS>;
+  const int group = threadIdx.x / THREADS, in_group = threadIdx.x % THREADS;
+  const int base = group * (G::TAB + tab_bytes);
+  RoundState<CELLS> &st = G::state(base);
+  const int lane = lane_id(), warp = in_group >> 5, bars = 3 * group;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
-  uint8_t *tab = heavy_dyn + RING_BYTES + static_cast<size_t>(warp) * tab_bytes;
-  // (behind the four key tables: a word per row of the chunk and warp for round_window's
-  // duplicate detection, when it fits)
-  uint32_t *mates = mates_words > 0
-                        ? reinterpret_cast<uint32_t *>(heavy_dyn + RING_BYTES + static_cast<size_t>(WARPS) * tab_bytes) +
-                              static_cast<size_t>(warp) * mates_words
-                        : nullptr;
-  for (int i = lane; i < mates_words; i += 32) mates[i] = 0u;
-
-#ifdef SPORDER_CHECKED
-  if (lane == 0) {
-    state[warp].ctrl = a.ctrl;
-    state[warp].span = tab_bytes;
-  }
-  __syncwarp();
-#endif
-  for (int i = lane * 16; i < tab_bytes; i += 32 * 16) *reinterpret_cast<uint4 *>(tab + i) = make_uint4(0, 0, 0, 0);
-  // Blocks of eight warps (a call that runs one chunk ahead): the first blocks take the critical
-  // rows at the head of the list with four of their warps (the other four leave at once, so
-  // those chains have a scheduler each); the blocks behind them take the other rows eight at a
-  // time, in list order, so that the rows fill as few SMs as they can and blocks without rows
-  // leave at once.  Blocks of four warps draw tickets.
-  auto run_row = [&](uint32_t item) {
+  for (int i = in_group * 16; i < MATES * 4 + tab_bytes; i += THREADS * 16)
+    *reinterpret_cast<uint4 *>(heavy_dyn + base + G::MATE + i) = make_uint4(0, 0, 0, 0);
+  const int32_t span = a.chunk < a.n ? a.chunk : a.n;
+  for (;;) {
+    if (in_group == 0) {
+      st.item = atomicAdd(&a.ctrl[CTRL_HEAVY_TICKET + 1], 1u);
+      st.row_done = 0;
+    }
+    bar_wait<CELLS>(bars + BAR_ROW);
+    const uint32_t item = st.item;
+    if (item >= heavy) break;
     const int32_t r = a.row_list[item];
     // checked build: the row, its place in the state array and its stream's extent
-    if (!index_ok(a.ctrl, CHK_LIST, r, a.n) || !index_ok(a.ctrl, CHK_STATE, item, a.heavy_max) ||
-        !index_ok(a.ctrl, CHK_STREAM, static_cast<long long>(a.heavy_off[item]) + a.row_work[r],
-                  static_cast<long long>(a.stream_cap) + 1))
-      return;
-    int32_t *out = a.heavy_state + static_cast<size_t>(item) * (2 * CELLS * 32);
-#ifdef CSG_ROUND_PROFILE
-    const unsigned long long row_t0 = clock64();
-    const uint32_t row_off = a.heavy_off[item];
-#endif
-    if (tab_bytes > 0)
-      rounds_row<CELLS, true>(a.hstream + a.heavy_off[item], a.row_work[r], (r / a.chunk) * a.chunk,
-                              state[warp], tab, mates, rings[warp][0], rings[warp][1], out,
-                              item == 0 ? reinterpret_cast<unsigned long long *>(a.ctrl + CTRL_PROFILE)
-                                        : nullptr);  // (profile build: the longest row only)
-    else  // chunk too large for key tables in shared memory
-      rounds_row<CELLS, false>(a.hstream + a.heavy_off[item], a.row_work[r], 0, state[warp], nullptr,
-                               nullptr, rings[warp][0], rings[warp][1], out,
-                               reinterpret_cast<unsigned long long *>(a.ctrl + CTRL_PROFILE));
-#ifdef CSG_ROUND_PROFILE
-    // the row's stream offset is no longer needed: its place takes the row's run time (in
-    // units of 1024 cycles), for the host to list the slowest rows
-    (void)row_off;
-    if (lane == 0) a.heavy_off[item] = static_cast<uint32_t>((clock64() - row_t0) >> 10);
-#endif
-  };
-  if constexpr (WARPS == S_WARPS) {
-    for (;;) {
-      uint32_t item = 0;
-      if (lane == 0) item = atomicAdd(&a.ctrl[CTRL_HEAVY_TICKET + 1], 1u);
-      item = __shfl_sync(FULL, item, 0);
-      if (item >= heavy) break;
-      run_row(item);
-    }
-  } else {
-    uint32_t crit = a.ctrl[CTRL_CRITICAL_ROWS];
-    crit = crit < heavy ? crit : heavy;
-    uint32_t sparse_blocks = (crit + S_WARPS - 1) / S_WARPS;
-    if (sparse_blocks >= gridDim.x) {  // no block left for other rows: all rows alike
-      sparse_blocks = gridDim.x;
-      crit = heavy;
-    }
-    uint32_t item, stride, last = heavy;
-    if (blockIdx.x < sparse_blocks) {
-      if (warp >= S_WARPS) return;
-      item = blockIdx.x * S_WARPS + warp;
-      stride = sparse_blocks * S_WARPS;
-      last = crit;
+    const bool ok = index_ok(a.ctrl, CHK_LIST, r, a.n) && index_ok(a.ctrl, CHK_STATE, item, a.heavy_max) &&
+                    index_ok(a.ctrl, CHK_STREAM, static_cast<long long>(a.heavy_off[item]) + a.row_work[r],
+                             static_cast<long long>(a.stream_cap) + 1);
+    if (warp > 0) {
+      for (;;) {
+        bar_wait<CELLS>(bars + BAR_STATE);
+        if (*static_cast<volatile int32_t *>(&st.row_done)) break;
+        rank_slots<CELLS>(base, warp - 1, lane);
+        bar_arrive<CELLS>(bars + BAR_ORDER);
+      }
     } else {
-      item = crit + (blockIdx.x - sparse_blocks) * WARPS + warp;
-      stride = (gridDim.x - sparse_blocks) * WARPS;
+      if (ok) {
+        const RoundRow row = {base, (r / a.chunk) * a.chunk, span > MATES, a.ctrl, span, bars};
+        int32_t *out = a.heavy_state + static_cast<size_t>(item) * (2 * CELLS * 32);
+        if (tab_bytes > 0)
+          rounds_row<CELLS, true>(a.hstream + a.heavy_off[item], a.row_work[r], row, out);
+        else
+          rounds_row<CELLS, false>(a.hstream + a.heavy_off[item], a.row_work[r], row, out);
+      }
+      if (lane == 0) st.row_done = 1;
+      __syncwarp();
+      bar_arrive<CELLS>(bars + BAR_STATE);
     }
-    for (; item < last; item += stride) run_row(item);
+    bar_wait<CELLS>(bars + BAR_ROW);
   }
 }
 
@@ -1551,9 +1885,6 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase) {
   // with the other three quarters (a chain block takes a whole SM, and the kernel of the other
   // rows starts only when every chain block has one).
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
-  const int chain_blocks = phase == PHASE_PRIO   ? prio_chain_blocks(ctx.num_sms)
-                           : phase == PHASE_REST ? ctx.num_sms - prio_chain_blocks(ctx.num_sms)
-                                                 : ctx.num_sms;
   heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
   heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
@@ -1566,85 +1897,71 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase) {
   // ahead, next in their stream, hold their SMs, and the kernel of the other rows cannot
   // settle on them first)
   if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
-  // The chain kernel asks for all the shared memory of an SM, so that it runs one block
-  // per SM.  Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, with key
-  // tables for a block's four warps (one byte per row of a chunk each) when they fit in there.
-  bool in_rounds = false;
-  if constexpr (CELLS <= ROUND_CELLS) {
-    auto launch_rounds = [&](auto kernel, int warps, int blocks, bool must_fit, bool *launched) -> bool {
-      cudaFuncAttributes fa;
-      CSG_CUDA(cudaFuncGetAttributes(&fa, kernel));
-      const int pad = ctx.smem_optin - 1024 - static_cast<int>(fa.sharedSizeBytes);
-      const int64_t ring_bytes = static_cast<int64_t>(warps) * 2 * H_RING * 8;
-      int64_t tab_bytes = (static_cast<int64_t>(a.chunk) + 15) / 16 * 16;
-      if (ring_bytes + tab_bytes * warps > pad) tab_bytes = 0;  // slots found by comparing keys
-      // round_window's duplicate detector: four bytes per row of the chunk and warp, if they fit too
-      int64_t mates_words = tab_bytes;
-      if (tab_bytes == 0 || ring_bytes + 5 * tab_bytes * warps > pad) mates_words = 0;
-      *launched = false;
-      if (must_fit && (mates_words == 0 || pad < ring_bytes)) return true;  // (the caller falls back)
-      CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
-      kernel<<<blocks, 32 * warps, pad, st>>>(a, static_cast<int>(tab_bytes), static_cast<int>(mates_words));
-      CSG_CUDA(cudaGetLastError());
-      *launched = true;
-      return true;
-    };
-    if (phase != PHASE_ALL && CELLS == WINDOW_CELLS) {
-      // eight chains to an SM, if all their tables fit, critical rows apart (see the kernel)
-      if (!launch_rounds(heavy_rounds_kernel<CELLS, 2 * S_WARPS>, 2 * S_WARPS, chain_blocks, true, &in_rounds))
-        return false;
-    }
-    if (!in_rounds &&
-        !launch_rounds(heavy_rounds_kernel<CELLS, S_WARPS>, S_WARPS, chain_blocks, false, &in_rounds))
-      return false;
+  // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a block per row.
+  constexpr bool in_rounds = CELLS <= ROUND_CELLS;
+  if constexpr (in_rounds) {
+    const int64_t span = a.chunk < a.n ? a.chunk : a.n;
+    const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
+    // (groups per block: as many as their tables leave room for)
+    const int group_bytes = GroupMemory<CELLS>::TAB + tab_bytes;
+    const int room = ctx.smem_optin - 1024;
+    int groups = Helpers<CELLS>::ROWS;
+    while (groups > 1 && groups * group_bytes > room) --groups;
+    CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    // (all of an SM's memory as shared: a block of another split cannot move in beside this one)
+    CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  cudaSharedmemCarveoutMaxShared));
+    heavy_rounds_kernel<CELLS><<<ctx.num_sms, Helpers<CELLS>::THREADS * groups, groups * group_bytes, st>>>(a, tab_bytes);
+    CSG_CUDA(cudaGetLastError());
   }
-  if (!in_rounds) {
+  if constexpr (!in_rounds) {
     const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
     CSG_CUDA(cudaFuncSetAttribute(heavy_consume_kernel<CELLS>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
-    heavy_consume_kernel<CELLS><<<chain_blocks, S_THREADS, pad, st>>>(a);
+    heavy_consume_kernel<CELLS><<<phase == PHASE_PRIO ? prio_chain_blocks(ctx.num_sms) : phase == PHASE_REST ? ctx.num_sms - prio_chain_blocks(ctx.num_sms) : ctx.num_sms, S_THREADS, pad, st>>>(a);
     CSG_CUDA(cudaGetLastError());
   }
   // The other rows run beside the heavy chains: their kernel follows in the same stream
   // as a programmatic dependent launch, so its blocks are placed only after every block
   // of the chain kernel is running (and has its SM to itself), and it fills the SMs that
   // stay or fall free.  It waits for the chain kernel before it ends (see sketch_kernel).
-  // key -> slot tables for its warps when a chunk's table is small enough that the blocks of an
-  // SM still fit (16 KB per block) and slot numbers fit a byte
-  int light_tab = 0;
-  if constexpr (CELLS == WINDOW_CELLS) {
-    const int64_t want = (static_cast<int64_t>(a.chunk < a.n ? a.chunk : a.n) + 15) / 16 * 16;
-    if (want <= 4096) light_tab = static_cast<int>(want);
-  }
-  auto launch_light = [&](auto kernel, int tab_bytes) -> bool {
-    const int dyn = tab_bytes * S_WARPS;
+  auto launch_light = [&](auto kernel, int threads, int smem, bool dependent, auto... args) -> bool {
+    if (smem > 48 * 1024)
+      CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     int per_sm = 0;
-    CSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S_THREADS, dyn));
+    CSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (per_sm < 1) per_sm = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctx.num_sms * per_sm);
-    cfg.blockDim = dim3(S_THREADS);
-    cfg.dynamicSmemBytes = dyn;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    // The chunk ahead has listed only its heavy rows: its kernel of the other rows has work
-    // only if some of them did not fit the stream buffer.  It runs behind the chains in plain
-    // stream order, where its idle blocks would otherwise sit on the SMs until the chains end.
-    cfg.numAttrs = phase == PHASE_PRIO ? 0 : 1;
-    CSG_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, phase == PHASE_PRIO ? 0 : 1, tab_bytes));
+    cfg.numAttrs = dependent ? 1 : 0;
+    CSG_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, args...));
     return true;
   };
-  if constexpr (CELLS == WINDOW_CELLS) {
-    if (light_tab > 0) {
-      if (!launch_light(sketch_kernel<CELLS, true>, light_tab)) return false;
-    } else if (!launch_light(sketch_kernel<CELLS, false>, 0)) {
+  // The chunk ahead has listed only its heavy rows: there is other work only if some of them did
+  // not fit the stream buffer.  That runs behind the chains in plain stream order, where its
+  // idle blocks would otherwise sit on the SMs until the chains end.
+  const int64_t span = a.chunk < a.n ? a.chunk : a.n;
+  if (phase == PHASE_PRIO || CELLS > LANE_CELLS || span > (1 << 24)) {
+    if (!launch_light(sketch_kernel<CELLS>, S_THREADS, 0, phase != PHASE_PRIO, phase == PHASE_PRIO ? 0 : 1,
+                      phase == PHASE_PRIO ? 0 : 1))
+      return false;
+  } else if constexpr (CELLS <= LANE_CELLS) {
+    auto lanes = [&](auto kernel, int index_words) {
+      return launch_light(kernel, 32 * L_WARPS, (LaneLayout<CELLS>::I_OFF + index_words) * 4, true);
+    };
+    if (span <= L_TABLE_MAX) {
+      if (!lanes(rows_in_lanes_kernel<CELLS, TableIndex<CELLS>>, TableIndex<CELLS>::words(span))) return false;
+    } else if (!lanes(rows_in_lanes_kernel<CELLS, ChainIndex<CELLS>>, ChainIndex<CELLS>::words(span))) {
       return false;
     }
-  } else if (!launch_light(sketch_kernel<CELLS, false>, 0)) {
-    return false;
   }
   heavy_topk_kernel<CELLS><<<ctx.num_sms, S_THREADS, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());

@@ -347,32 +347,35 @@ __global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, Tr
   }
 }
 
-// Work list of the chunk ahead: its rows that stream 65,536 candidates or more (the other
-// rows of the chunk go with everybody else's), longest stream first, so that the eight rows a
-// block of the chain kernel takes are of a length and the block is done when they are.  The
-// critical rows - at least half as long as the longest, the ones that can decide when the call
-// ends; their chains keep a scheduler to themselves - are then the head of the list.  One block;
-// a chunk has at most PRIO_MAX_CHUNK rows.
+// Work list of the chunk ahead: its rows within a factor of four of its longest stream (and of
+// HEAVY_WORK candidates or more), longest first.  Those can decide when the call ends; the other
+// rows of the chunk go with everybody else's.  One block; a chunk has at most PRIO_MAX_CHUNK rows.
 constexpr int PRIO_MAX_CHUNK = 4096;
 __global__ void __launch_bounds__(1024) priority_rows_kernel(TransposeArgs ap, int32_t *row_list) {
   __shared__ int32_t s_row[PRIO_MAX_CHUNK];
   __shared__ uint32_t s_work[PRIO_MAX_CHUNK];
-  __shared__ uint32_t count, critical;
+  __shared__ uint32_t count, longest;
   __shared__ unsigned long long need;
   if (threadIdx.x == 0) {
     count = 0;
     need = 0;
-    critical = 0;
+    longest = 0;
   }
   __syncthreads();
   const uint32_t prio = ap.ctrl[CTRL_PRIO];
-  uint32_t longest = 0;
+  uint32_t least = 0;
   if (prio != PRIO_NONE && ap.chunk <= PRIO_MAX_CHUNK) {
     const int64_t start = static_cast<int64_t>(prio) * ap.chunk;
     const int64_t end = start + ap.chunk < ap.n ? start + ap.chunk : ap.n;
+    uint32_t top = 0;
+    for (int64_t r = start + threadIdx.x; r < end; r += blockDim.x) top = max(top, ap.row_work[r]);
+    top = __reduce_max_sync(FULL, top);
+    if ((threadIdx.x & 31) == 0 && top) atomicMax(&longest, top);
+    __syncthreads();
+    least = longest / 4 > HEAVY_WORK ? longest / 4 : HEAVY_WORK;
     for (int64_t r = start + threadIdx.x; r < end; r += blockDim.x) {
       const uint32_t t = ap.row_work[r];
-      if (t >= (1u << (SKETCH_HEAVY_BUCKET - 1))) {
+      if (t >= least) {
         const uint32_t at = atomicAdd(&count, 1u);
         s_row[at] = static_cast<int32_t>(r);
         s_work[at] = t;
@@ -391,29 +394,14 @@ __global__ void __launch_bounds__(1024) priority_rows_kernel(TransposeArgs ap, i
         before += (wj > w || (wj == w && s_row[j] < r)) ? 1u : 0u;
       }
       row_list[before] = r;
-      if (before == 0) longest = w;
     }
-    // (the thread that placed the first row knows the longest stream)
-    const uint32_t top = __reduce_max_sync(FULL, longest);
-    if ((threadIdx.x & 31) == 0 && top) atomicMax(&critical, top);  // borrowed as a maximum for a moment
-    __syncthreads();
-    longest = critical;
-    __syncthreads();
-    if (threadIdx.x == 0) critical = 0;
-    __syncthreads();
-    const uint32_t bar = longest - longest / 2;
-    uint32_t mine = 0;
-    for (uint32_t i = threadIdx.x; i < H; i += blockDim.x) mine += s_work[i] >= bar ? 1u : 0u;
-    mine = __reduce_add_sync(FULL, mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&critical, mine);
-    __syncthreads();
   }
   if (threadIdx.x == 0) {
     ap.ctrl[CTRL_ROWS_LISTED] = count;
     ap.ctrl[CTRL_HEAVY_ROWS] = count;
-    ap.ctrl[CTRL_CRITICAL_ROWS] = critical;
-    ap.ctrl[CTRL_CRITICAL_TICKET] = 0;
-    ap.ctrl[CTRL_LONGEST] = longest;
+    ap.ctrl[CTRL_MID_END] = count;
+    ap.ctrl[CTRL_LANE_TICKET] = count;
+    ap.ctrl[CTRL_PRIO_WORK] = least;
     ap.ctrl[CTRL_ROW_TICKET] = count;
     ap.ctrl[CTRL_HEAVY_TICKET] = 0;
     ap.ctrl[CTRL_HEAVY_TICKET + 1] = 0;
@@ -778,81 +766,94 @@ __global__ void __launch_bounds__(Y_THREADS) symmetric_groups_kernel(TransposeAr
   }
 }
 
-// rows per power-of-two bucket of row_work
 // rows of the chunk that runs ahead which that part of the call takes itself
-__device__ __forceinline__ bool taken_ahead(uint32_t prio, int32_t chunk, int32_t r, uint32_t work) {
-  return prio != PRIO_NONE && work >= (1u << (SKETCH_HEAVY_BUCKET - 1)) &&
-         static_cast<uint32_t>(r / chunk) == prio;
+__device__ __forceinline__ bool taken_ahead(uint32_t prio, uint32_t least, int32_t chunk, int32_t r, uint32_t work) {
+  return prio != PRIO_NONE && work >= least && static_cast<uint32_t>(r / chunk) == prio;
 }
 
+// rows per bucket of row_work
 __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint32_t *row_work,
-                                                           uint32_t *ctrl, int32_t chunk, bool skip_prio) {
-  __shared__ uint32_t bucket[33];
+                                                           uint32_t *ctrl, int32_t chunk, const uint32_t *ctrl_ahead) {
+  __shared__ uint32_t bucket[WORK_BUCKETS];
   __shared__ unsigned long long need;
-  if (threadIdx.x < 33) bucket[threadIdx.x] = 0;
+  if (threadIdx.x < WORK_BUCKETS) bucket[threadIdx.x] = 0;
   if (threadIdx.x == 0) need = 0;
   __syncthreads();
-  const uint32_t prio = skip_prio ? ctrl[CTRL_PRIO] : PRIO_NONE;
+  const uint32_t prio = ctrl_ahead ? ctrl_ahead[CTRL_PRIO] : PRIO_NONE;
+  const uint32_t least = ctrl_ahead ? ctrl_ahead[CTRL_PRIO_WORK] : 0u;
   for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     uint32_t t = __ldcg(row_work + r);
-    if (taken_ahead(prio, chunk, r, t)) t = 0;
-    if (t) atomicAdd(&bucket[32 - __clz(t)], 1u);
+    if (taken_ahead(prio, least, chunk, r, t)) t = 0;
+    if (t) atomicAdd(&bucket[work_bucket(t)], 1u);
     // stream elements of the rows heavy enough for a materialised stream: what the stream
     // buffer would have to hold for all of them (the host sizes the next call's buffer by it)
-    if (t >= (1u << (SKETCH_HEAVY_BUCKET - 1))) atomicAdd(&need, static_cast<unsigned long long>(t));
+    if (t >= HEAVY_WORK) atomicAdd(&need, static_cast<unsigned long long>(t));
   }
   __syncthreads();
-  if (threadIdx.x < 33 && bucket[threadIdx.x])
+  if (threadIdx.x < WORK_BUCKETS && bucket[threadIdx.x])
     atomicAdd(&ctrl[CTRL_BUCKET_COUNT + threadIdx.x], bucket[threadIdx.x]);
   if (threadIdx.x == 0 && need)
     atomicAdd(reinterpret_cast<unsigned long long *>(ctrl + CTRL_HEAVY_NEED), need);
 }
 
-// Heaviest bucket first: rows with 2^(b-1) <= work < 2^b sit in bucket b.
-// ctrl_ahead: the control words of the chunk that runs ahead, when the call has one.  The rows
-// of this list that are within a factor of four of the longest stream of the whole call (their
-// bucket is the top one or the one below) count as critical like the long rows of the chunk
-// ahead: their chains keep a scheduler to themselves (see heavy_rounds_kernel).
-__global__ void bucket_scan_kernel(uint32_t *ctrl, const uint32_t *ctrl_ahead) {
-  if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    int top = 0;
-    for (int b = 32; b >= 1; --b) {
-      ctrl[CTRL_BUCKET_BASE + b] = run;
-      run += ctrl[CTRL_BUCKET_COUNT + b];
-      ctrl[CTRL_BUCKET_FILL + b] = 0;
-      if (top == 0 && ctrl[CTRL_BUCKET_COUNT + b]) top = b;
-    }
-    if (ctrl_ahead) {
-      const uint32_t longest = ctrl_ahead[CTRL_LONGEST];
-      const int top_ahead = longest ? 32 - __clz(longest) : 0;
-      top = top_ahead > top ? top_ahead : top;
-      int from = top - 1 > SKETCH_HEAVY_BUCKET ? top - 1 : SKETCH_HEAVY_BUCKET;
-      ctrl[CTRL_CRITICAL_ROWS] = from <= 32 ? ctrl[CTRL_BUCKET_BASE + from - 1] : 0u;  // rows of buckets >= from
-      ctrl[CTRL_CRITICAL_TICKET] = 0;
-    }
-    ctrl[CTRL_ROWS_LISTED] = run;
-    // rows with at least 2^(SKETCH_HEAVY_BUCKET-1) stream elements head the list; the
-    // heavy sketch kernel takes them, the other kernel's tickets start behind them
-    const uint32_t heavy = ctrl[CTRL_BUCKET_BASE + SKETCH_HEAVY_BUCKET - 1];
+// Longest bucket first (one warp, lane l counts the buckets 127 - 4 l .. 124 - 4 l).
+// Which rows get a warp of the chain kernel each: all rows of HEAVY_WORK candidates or more,
+// and below that the longest buckets that keep the list within CHAIN_ROWS rows.  A row resolved
+// in rounds takes 40 to 200 cycles per candidate and half an SM; run by one lane among 32 it takes
+// about 600, so in a call with few long rows the lanes would be waiting for the longest one.
+// CHAIN_ROWS = two rows on each of 148 SMs: beyond one wave of them the chains only queue, and
+// what they do the lanes do with a sixth of the SM time (R-MAT scale 22 took 42 ms with 1184 rows
+// here).
+__global__ void bucket_scan_kernel(uint32_t *ctrl) {
+  const int lane = threadIdx.x;
+  uint32_t c[4], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    c[j] = ctrl[CTRL_BUCKET_COUNT + WORK_BUCKETS - 1 - (4 * lane + j)];
+    sum += c[j];
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, off);
+    if (lane >= off) incl += t;
+  }
+  uint32_t run = incl - sum;
+  uint32_t heavy = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int b = WORK_BUCKETS - 1 - (4 * lane + j);
+    ctrl[CTRL_BUCKET_BASE + b] = run;
+    run += c[j];
+    ctrl[CTRL_BUCKET_FILL + b] = 0;
+    if (b >= work_bucket(HEAVY_WORK) || (b >= work_bucket(CHAIN_WORK_MIN) && run <= CHAIN_ROWS)) heavy = run;
+  }
+  heavy = __reduce_max_sync(FULL, heavy);
+  const uint32_t listed = __shfl_sync(FULL, run, 31);
+  if (lane == 0) {
+    ctrl[CTRL_ROWS_LISTED] = listed;
     ctrl[CTRL_HEAVY_ROWS] = heavy;
+    ctrl[CTRL_MID_END] = heavy;
+    ctrl[CTRL_LANE_TICKET] = heavy;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
   }
 }
 
 __global__ void row_list_kernel(int32_t n, const uint32_t *__restrict__ row_work, uint32_t *ctrl,
-                                int32_t *__restrict__ row_list, int32_t chunk, bool skip_prio) {
+                                int32_t *__restrict__ row_list, int32_t chunk,
+                                const uint32_t *ctrl_ahead) {
   const int lane = threadIdx.x & 31;
   const int32_t total = gridDim.x * blockDim.x;
-  const uint32_t prio = skip_prio ? ctrl[CTRL_PRIO] : PRIO_NONE;
+  const uint32_t prio = ctrl_ahead ? ctrl_ahead[CTRL_PRIO] : PRIO_NONE;
+  const uint32_t least = ctrl_ahead ? ctrl_ahead[CTRL_PRIO_WORK] : 0u;
   for (int32_t base = blockIdx.x * blockDim.x; base < n; base += total) {
     const int32_t r = base + threadIdx.x;
     uint32_t t = r < n ? row_work[r] : 0u;
-    if (r < n && taken_ahead(prio, chunk, r, t)) t = 0;
-    const uint32_t bkt = t ? (32 - __clz(t)) : 0u;
-    const unsigned peers = __match_any_sync(FULL, bkt);
-    if (bkt) {
+    if (r < n && taken_ahead(prio, least, chunk, r, t)) t = 0;
+    const int bkt = t ? work_bucket(t) : -1;
+    const unsigned peers = match_digit(t ? static_cast<uint32_t>(bkt) : 256u);
+    if (t) {
       const int leader = __ffs(peers) - 1;
       uint32_t pre = 0;
       if (lane == leader) pre = atomicAdd(&ctrl[CTRL_BUCKET_FILL + bkt], __popc(peers));
@@ -938,11 +939,11 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
     if (ygrid > ctx.num_sms * 8) ygrid = ctx.num_sms * 8;
     symmetric_groups_kernel<<<ygrid, Y_THREADS, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
-    bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, false);
+    bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, nullptr);
     CSG_CUDA(cudaGetLastError());
-    bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl, nullptr);
+    bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl);
     CSG_CUDA(cudaGetLastError());
-    row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, false);
+    row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, nullptr);
     CSG_CUDA(cudaGetLastError());
     count_launches(4);
     return true;
@@ -980,11 +981,11 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   transpose_kernel<<<grid, T_THREADS, smem, st>>>(a);
   CSG_CUDA(cudaGetLastError());
   if (phase == PHASE_REST) CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[6], 0));
-  bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, phase == PHASE_REST);
+  bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
-  bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl, phase == PHASE_REST ? ctrl_ahead : nullptr);
+  bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl);
   CSG_CUDA(cudaGetLastError());
-  row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, phase == PHASE_REST);
+  row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
   count_launches(7 + 3 * a.passes);
   return true;

@@ -53,6 +53,26 @@ def test_csg_larger_cases_against_oracle(name):
     assert np.array_equal(order.cpu().numpy(), o_or)
 
 
+@pytest.mark.parametrize("k", [8, 16, 24, 32])  # one to four cells per lane
+@pytest.mark.parametrize("chunk", [5, 300, 1024, 1025, 3000])
+def test_rows_in_lanes_and_in_rounds_against_oracle(chunk, k):
+    # a row per lane with the byte table (chunks of up to 1024 rows) and with the hash chains
+    # (above), the last batch of lanes partly empty; on repeated contexts the rows that get a
+    # group of the chain kernel change with the buffer the context has learnt to plan
+    sp = _sp()
+    from chunkedgreedy_b200 import synth
+    ptr, ind, _ = synth.random_sparse(3001, 14, 17, hub_cols=60, hub_frac=0.5, empty_rows=0.05)
+    o_or, t_or = oracle.csg(ptr, ind, False, with_table=True, k=k, chunk_size=chunk)
+    ctx = sp.Context()
+    dp, di = _dev(ptr), _dev(ind)
+    for limit in (0, 5000, 1):  # streams that fit, some that do not, none
+        ctx.set_stream_limit(limit)
+        order, table = sp.csg_table(dp, di, k=k, chunk_size=chunk, ctx=ctx)
+        assert np.array_equal(table.cpu().numpy().view(np.uint64), t_or)
+        assert np.array_equal(order.cpu().numpy(), o_or)
+    ctx.close()
+
+
 @pytest.mark.parametrize("name", ["hubsym", "rmat12", "m512", "bigchunk", "rmat16", "dense_ties",
                                   "dense_fill", "dense_m32", "dense_ragged", "dense_m96",
                                   "dense_m128", "dense_m128_ties", "zipf65k"])
