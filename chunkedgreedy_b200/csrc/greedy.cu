@@ -7,10 +7,10 @@
 // (sporder/src/common/warp_visited_bitmap.cuh:99-111).  The visiting order is the
 // permutation (new2old).
 //
-// One warp per chunk as in the reference; what changes: rows whose candidate
-// stream was empty are known from the transpose (row_work == 0) and need no table
-// load, the restart scan keeps a monotone cursor instead of rescanning the bitmap,
-// the arg-max is two warp reductions, and the order is written 32 entries at a time.
+// One warp runs a chunk's chain as in the reference; what changes: rows whose candidate
+// stream was empty are known from the transpose (row_work == 0) and never enter the chain
+// (see greedy_lists_kernel), the chain runs on short lists in shared memory, and the order
+// leaves the block in one coalesced copy.
 #include "common.cuh"
 
 namespace csg {
@@ -41,11 +41,8 @@ struct ChainStats {  // lives at ctrl[CTRL_STATS ...]
   double in_chunk_weight;  // table weights whose candidate lies in the row's own chunk
 };
 
-// The chain of chunk q = rows [start, end), run by one warp.  STAGED: the chunk's rows of the
-// table were copied to shared memory (`staged`, row-major like the table) by the block.
-template <bool STAGED>
-__device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited,
-                                            const uint64_t *staged) {
+// The chain of rows [start, end), run by one warp on the table itself.
+__device__ __noinline__ void chain_chunk(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited) {
   const int lane = lane_id();
   const int32_t size = end - start;
   const int32_t words = (size + 31) >> 5;
@@ -73,8 +70,7 @@ __device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, 
 
     int32_t best_c = -1;
     if (nonempty[loc >> 5] & (1u << (loc & 31))) {
-      const uint64_t *row = STAGED ? staged + static_cast<size_t>(loc) * a.k
-                                   : a.table + static_cast<size_t>(cur) * a.k;
+      const uint64_t *row = a.table + static_cast<size_t>(cur) * a.k;
       uint32_t best_w = 0;  // weight bits; real weights are positive
       for (int32_t j = lane; j < a.k; j += 32) {
         const uint64_t e = row[j];
@@ -86,7 +82,7 @@ __device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, 
         // The next row of the chain is one of these candidates, and its list is needed as
         // soon as the arg-max below is known: ask for every candidate's list now, so that the
         // one dependent load per step finds it in L1 instead of waiting on L2.
-        if (!STAGED) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.table + static_cast<size_t>(cand) * a.k));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.table + static_cast<size_t>(cand) * a.k));
         const uint32_t wb = entry_weight_bits(e);
         if (wb > best_w || (wb == best_w && cand < best_c)) {
           best_w = wb;
@@ -173,6 +169,7 @@ __device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, 
   }
 }
 
+// Chunks whose lists do not fit shared memory: a warp each.
 __global__ void __launch_bounds__(G_WARPS * 32) greedy_kernel(GreedyArgs a) {
   extern __shared__ uint32_t g_smem[];
   const int warp = threadIdx.x >> 5;
@@ -184,27 +181,255 @@ __global__ void __launch_bounds__(G_WARPS * 32) greedy_kernel(GreedyArgs a) {
   // two bitmaps per chunk: visited, and "row has a non-empty top-k list"
   uint32_t *visited = a.gbitmaps ? a.gbitmaps + static_cast<size_t>(q) * 2 * a.words
                                  : g_smem + static_cast<size_t>(warp) * 2 * a.words;
-  chain_chunk<false>(a, start, end, visited, nullptr);
+  chain_chunk(a, start, end, visited);
 }
 
-// With no more chunks than SMs there are too few chains to hide one another's latency, and a
-// step is one dependent read of a table row: a block per chunk copies the chunk's rows of the
-// table into shared memory first (1024 rows x 16 entries = 128 KB), and one warp runs the
-// chain on that copy.
-constexpr int GS_THREADS = 256;
-__global__ void __launch_bounds__(GS_THREADS, 1) greedy_staged_kernel(GreedyArgs a) {
-  extern __shared__ __align__(16) uint32_t g_smem[];
+// A block per chunk.  A chunk is one dependent chain of up to 1024 steps, so what counts is the
+// latency of a step.
+//  * Rows without a list ("bare") stay out of the chain: the chain would emit one only when it
+//    restarts there, and change nothing by it.  The rows with a list are numbered 0 .. m-1 in
+//    index order.  Restarts go to ascending rows, and a bare row comes out just before
+//    the first restart at a row behind it: once the chain is known, every bare row's place
+//    follows from the number of rows the chain had emitted at that restart.
+//  * The block first writes every list out as 16-bit row numbers in the order in which the chain
+//    would try them (weight, on ties the smaller index; the table has the weights in order, only
+//    ties have to be put right), candidates outside the chunk as a row that counts as visited.
+//  * A step is then: read the current row's list, read those rows' flags, one warp minimum over
+//    (place in the list, row) of the free ones.  Lanes without a list entry look at the rows behind
+//    the restart cursor meanwhile, and the same minimum says where to restart if no entry is free.
+//    All else is kept out of the loop: a lone warp waits four to six cycles for every instruction
+//    that needs the one before it, and written without care the step takes 460 cycles instead of 135.
+// On a B200, per call: power-law band of 65,536 rows 320 -> 74 us (64 chains, the longest of 900
+// steps), R-MAT scale 22 646 -> 258 us (4096 chains).
+// A candidate without a list of its own (only a false promise of symmetry makes one) would let
+// the chain reach bare rows: such a chunk runs on the table.
+constexpr int GS_MAX_SPAN = 32768;   // rows of a chunk: their numbers must fit 15 bits
+constexpr uint32_t BARE = 0x8000u;   // in `place`: a bare row's place in the chunk, else a numbered row
+constexpr int GS_WINDOW = 32;        // flags behind the last row that read as visited
+
+struct ListLayout {  // shared memory, in bytes
+  int flags, row_of, place, mark, window, words, lists, total;
+};
+__host__ __device__ inline ListLayout list_layout(int32_t span, int32_t k) {
+  ListLayout l;
+  int at = 0;
+  auto take = [&](int bytes) {
+    const int o = at;
+    at += (bytes + 15) & ~15;
+    return o;
+  };
+  const int words = (span + 31) / 32;
+  l.flags = take(span + GS_WINDOW + 1);  // per numbered row: emitted
+  l.row_of = take(2 * (span + 1));       // its place in the chunk
+  l.place = take(2 * span);              // the order: who goes to each place
+  l.mark = take(2 * (span + 1));         // per numbered row: 1 + rows emitted before the restart at it, 0 without one
+  l.window = take(2 * 32);               // what lanes without a list entry look at
+  l.words = take(8 * words);             // per 32 rows: which have a list; how many in front have one
+  l.lists = take(2 * span * k);
+  l.total = at;
+  return l;
+}
+
+// Shared memory by its own 32-bit addresses, in program order.
+__device__ __forceinline__ uint32_t lds_u16(uint32_t at) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds_s8(uint32_t at) {  // sign-extended
+  int32_t v;
+  asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(at));
+  return static_cast<uint32_t>(v);
+}
+__device__ __forceinline__ void sts_u8(uint32_t at, uint32_t v) {
+  asm volatile("st.shared.u8 [%0], %1;" ::"r"(at), "r"(v));
+}
+__device__ __forceinline__ void sts_u16(uint32_t at, uint32_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(static_cast<uint16_t>(v)));
+}
+
+// LONG: lists of more than 32 entries.
+template <bool STATS, bool LONG>
+__global__ void greedy_lists_kernel(GreedyArgs a) {
+  extern __shared__ __align__(16) unsigned char gl_smem[];
+  __shared__ int32_t odd, count;
+  const int lane = lane_id(), warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int32_t q = blockIdx.x;
   const int64_t start64 = static_cast<int64_t>(q) * a.chunk;
   const int32_t start = static_cast<int32_t>(start64);
   const int32_t end = (start64 + a.chunk > a.n) ? a.n : static_cast<int32_t>(start64 + a.chunk);
-  uint32_t *visited = g_smem;
-  uint64_t *staged = reinterpret_cast<uint64_t *>(g_smem + ((2 * a.words + 3) & ~3));
-  const size_t entries = static_cast<size_t>(end - start) * a.k;
-  const uint64_t *src = a.table + static_cast<size_t>(start) * a.k;
-  for (size_t i = threadIdx.x; i < entries; i += GS_THREADS) staged[i] = src[i];
+  const int32_t size = end - start, words = (size + 31) >> 5;
+  const int k = a.k;
+  const ListLayout lay = list_layout(a.chunk < a.n ? a.chunk : a.n, k);
+  uint8_t *const flags = gl_smem + lay.flags;
+  uint16_t *const row_of = reinterpret_cast<uint16_t *>(gl_smem + lay.row_of);
+  uint16_t *const place = reinterpret_cast<uint16_t *>(gl_smem + lay.place);
+  uint16_t *const mark = reinterpret_cast<uint16_t *>(gl_smem + lay.mark);
+  uint32_t *const has = reinterpret_cast<uint32_t *>(gl_smem + lay.words);
+  uint32_t *const before = has + words;
+  uint16_t *const lists = reinterpret_cast<uint16_t *>(gl_smem + lay.lists);
+  if (threadIdx.x == 0) odd = 0;
+  for (int32_t w = warp; w < words; w += warps) {
+    const int32_t i = (w << 5) + lane;
+    const unsigned m = __ballot_sync(FULL, i < size && a.row_work[start + i] != 0);
+    if (lane == 0) has[w] = m;
+  }
   __syncthreads();
-  if (threadIdx.x < 32) chain_chunk<true>(a, start, end, visited, staged);
+  if (warp == 0) {  // numbers: exclusive sums over the words
+    int32_t run = 0;
+    for (int32_t w0 = 0; w0 < words; w0 += 32) {
+      const int32_t v = w0 + lane < words ? __popc(has[w0 + lane]) : 0;
+      int32_t incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int32_t t = __shfl_up_sync(FULL, incl, off);
+        if (lane >= off) incl += t;
+      }
+      if (w0 + lane < words) before[w0 + lane] = run + incl - v;
+      run += __shfl_sync(FULL, incl, 31);
+    }
+    if (lane == 0) count = run;
+  }
+  __syncthreads();
+  const int32_t m = count;
+  for (int32_t i = threadIdx.x; i < size; i += blockDim.x) {
+    const uint32_t w = has[i >> 5], bit = 1u << (i & 31);
+    if (w & bit) row_of[before[i >> 5] + __popc(w & (bit - 1u))] = static_cast<uint16_t>(i);
+  }
+  for (int32_t i = threadIdx.x; i < m + GS_WINDOW + 1; i += blockDim.x)
+    if (i <= a.chunk + GS_WINDOW) flags[i] = i < m ? 0 : 0xFF;
+  for (int32_t i = threadIdx.x; i <= m; i += blockDim.x) mark[i] = static_cast<uint16_t>(i < m ? 0 : m + 1);
+  __syncthreads();
+  // lists: G lanes a row (16 while a list fits them), U rows of a group in flight
+  {
+    constexpr int U = 4;
+    const int G = k <= 16 ? 16 : 32, groups = blockDim.x / G, group = threadIdx.x / G, gl = threadIdx.x % G;
+    bool strange = false;
+    for (int32_t r0 = 0; r0 < m; r0 += groups * U) {
+      for (int j0 = 0; j0 < k; j0 += G) {
+        const int j = j0 + gl;
+        uint64_t e[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int32_t r = r0 + u * groups + group;
+          e[u] = r < m && j < k ? a.table[static_cast<size_t>(start + row_of[r]) * k + j] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int32_t r = r0 + u * groups + group;
+          const uint32_t wb = entry_weight_bits(e[u]), id = static_cast<uint32_t>(e[u]);
+          int pos = j;
+          // among equal weights the smaller index comes first
+          if (k <= G) {
+            for (int d = 1; d < G; ++d) {
+              const uint32_t uw = __shfl_up_sync(FULL, wb, d, 32), ui = __shfl_up_sync(FULL, id, d, 32);
+              const uint32_t dw = __shfl_down_sync(FULL, wb, d, 32), di = __shfl_down_sync(FULL, id, d, 32);
+              const bool up = gl >= d && wb && uw == wb, down = gl + d < G && wb && dw == wb;
+              if (!__any_sync(FULL, up || down)) break;
+              pos += (down && di < id ? 1 : 0) - (up && ui > id ? 1 : 0);
+            }
+          } else if (wb) {
+            const uint64_t *row = a.table + static_cast<size_t>(start + row_of[r]) * k;
+            for (int t = j - 1; t >= 0 && entry_weight_bits(row[t]) == wb; --t)
+              pos -= static_cast<uint32_t>(row[t]) > id ? 1 : 0;
+            for (int t = j + 1; t < k && entry_weight_bits(row[t]) == wb; ++t)
+              pos += static_cast<uint32_t>(row[t]) < id ? 1 : 0;
+          }
+          if (r < m && j < k) {
+            const int32_t cand = entry_index(e[u]) - a.row_base - start;
+            uint32_t number = static_cast<uint32_t>(m);  // reads as visited
+            if (wb && cand >= 0 && cand < size) {
+              const uint32_t w = has[cand >> 5], bit = 1u << (cand & 31);
+              number = before[cand >> 5] + __popc(w & (bit - 1u));
+              strange |= (w & bit) == 0u;
+            }
+            lists[r * k + pos] = static_cast<uint16_t>(number);
+          }
+        }
+      }
+    }
+    if (strange) odd = 1;
+  }
+  __syncthreads();
+  if (odd) {
+    if (warp == 0) chain_chunk(a, start, end, has);  // (its two bitmaps fit the words)
+    return;
+  }
+  if (warp == 0 && m > 0) {
+    const uint32_t s_flags = static_cast<uint32_t>(__cvta_generic_to_shared(flags));
+    const uint32_t s_place = static_cast<uint32_t>(__cvta_generic_to_shared(place));
+    const uint32_t s_mark = static_cast<uint32_t>(__cvta_generic_to_shared(mark));
+    const uint32_t s_row_of = static_cast<uint32_t>(__cvta_generic_to_shared(row_of));
+    // a lane reads its entry of the list, or behind the list its place of the cursor's window
+    const bool mine = lane < k;
+    const uint32_t s_list =
+        static_cast<uint32_t>(__cvta_generic_to_shared(gl_smem + (mine ? lay.lists : lay.window))) + 2 * lane;
+    const uint32_t stride = mine ? 2 * k : 0;
+    const uint32_t tag = mine ? static_cast<uint32_t>(lane) << 15 : 0x80000000u;
+    int32_t segments = 0, t = 0;
+    float link_w = 0.0f;
+    uint32_t c = 0;  // the chain begins with a restart at number 0
+    for (;;) {
+      // a restart at c: everything in front of it that is not emitted yet is bare
+      const uint32_t shift = lds_u16(s_row_of + 2 * c) - c;
+      sts_u16(s_mark + 2 * c, t + 1);
+      uint32_t cursor = c + 1, next;
+      if (!mine) sts_u16(s_list, min(cursor + lane - k, m));
+      ++segments;
+      const uint32_t out0 = s_place + 2 * shift;
+      uint32_t out = out0 + 2 * t;
+      for (;;) {
+        // (all lanes store the same values, so each sees its own and no barrier is needed)
+        sts_u8(s_flags + c, 0xFFu);
+        uint32_t at = lds_u16(s_list + c * stride);
+        sts_u16(out, c);
+        out += 2;
+        uint32_t found = lds_s8(s_flags + at) | (tag | at);  // all ones when that row is out already
+        if (LONG)
+          for (int j = lane + 32; j < k && found == 0xFFFFFFFFu; j += 32) {
+            at = lds_u16(s_list + c * stride + 2 * (j - lane));
+            found = lds_s8(s_flags + at) | (static_cast<uint32_t>(j) << 15 | at);
+          }
+        next = __reduce_min_sync(FULL, found);
+        if (next >= 0x80000000u) break;
+        if (STATS)
+          link_w += __uint_as_float(
+              entry_weight_bits(a.table[static_cast<size_t>(start + row_of[c]) * k + (next >> 15)]));
+        c = next & 0x7FFFu;
+      }
+      t = static_cast<int32_t>(out - out0) >> 1;
+      while (next == 0xFFFFFFFFu && static_cast<int32_t>(cursor) < m) {  // nobody free in the cursor's window
+        const uint32_t at = min(cursor + lane, m);
+        next = __reduce_min_sync(FULL, lds_s8(s_flags + at) | (0x80000000u | at));
+        cursor += 32;
+      }
+      if (next == 0xFFFFFFFFu) break;
+      c = next & 0x7FFFFFFFu;
+    }
+    if (STATS && lane == 0) {
+      ChainStats *st = reinterpret_cast<ChainStats *>(a.ctrl + CTRL_STATS);
+      atomicAdd(&st->restarts, size - m + segments - 1);  // every bare row is one; the first row is none
+      atomicAdd(&st->links, m - segments);
+      atomicAdd(&st->link_weight_sum, static_cast<double>(link_w));
+    }
+  } else if (STATS && warp == 0 && lane == 0) {
+    atomicAdd(&reinterpret_cast<ChainStats *>(a.ctrl + CTRL_STATS)->restarts, size - 1);
+  }
+  __syncthreads();
+  for (int32_t i = threadIdx.x; i < size; i += blockDim.x) {  // the bare rows' places
+    const uint32_t w = has[i >> 5], bit = 1u << (i & 31);
+    if (w & bit) continue;
+    const int32_t number = before[i >> 5] + __popc(w & (bit - 1u));
+    int32_t x = number;  // the first restart behind it (the mark behind the last row ends the search)
+    while (mark[x] == 0) ++x;
+    const int32_t at = i - number + mark[x] - 1;
+    if (index_ok(a.ctrl_all, CHK_ORDER, at, size)) place[at] = static_cast<uint16_t>(i | BARE);
+  }
+  __syncthreads();
+  for (int32_t i = threadIdx.x; i < size; i += blockDim.x) {
+    const uint32_t v = place[i];
+    a.order[start + i] = start + static_cast<int32_t>(v & BARE ? v & ~BARE : row_of[v]) + a.row_base;
+  }
 }
 
 // sporder/src/common/similarity_top_k.cu:120-157
@@ -301,16 +526,21 @@ bool launch_greedy(Context &ctx, int32_t n, const CsgParams &p, CsgScratch &s,
     a.gbitmaps = s.gbitmaps;
     smem = 0;
   }
-  // few chunks: one block per chunk with the chunk's table rows in shared memory, if they fit
-  const size_t staged_bytes = static_cast<size_t>((2 * a.words + 3) & ~3) * sizeof(uint32_t) +
-                              static_cast<size_t>(span) * p.k * sizeof(uint64_t);
-  if (a.num_chunks <= ctx.num_sms && staged_bytes + 1024 <= static_cast<size_t>(ctx.smem_optin)) {
-    CSG_CUDA(cudaFuncSetAttribute(greedy_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(staged_bytes)));
-    greedy_staged_kernel<<<a.num_chunks, GS_THREADS, staged_bytes, ctx.stream>>>(a);
-    CSG_CUDA(cudaGetLastError());
-    count_launches(1);
-    return true;
+  // a block per chunk on lists in shared memory, if they fit
+  if (span <= GS_MAX_SPAN && p.k <= 256) {
+    const int bytes = list_layout(span, p.k).total;
+    if (bytes + 1024 <= ctx.smem_optin) {
+      const bool lng = p.k > 32;
+      auto kernel = with_stats ? (lng ? greedy_lists_kernel<true, true> : greedy_lists_kernel<true, false>)
+                               : (lng ? greedy_lists_kernel<false, true> : greedy_lists_kernel<false, false>);
+      CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      // many chunks: several blocks to an SM; few: more warps to write the lists of each
+      const int threads = a.num_chunks <= 2 * ctx.num_sms ? 512 : 256;
+      kernel<<<a.num_chunks, threads, bytes, ctx.stream>>>(a);
+      CSG_CUDA(cudaGetLastError());
+      count_launches(1);
+      return true;
+    }
   }
   const int grid = (a.num_chunks + G_WARPS - 1) / G_WARPS;
   greedy_kernel<<<grid, G_WARPS * 32, smem, ctx.stream>>>(a);

@@ -73,6 +73,29 @@ def test_rows_in_lanes_and_in_rounds_against_oracle(chunk, k):
     ctx.close()
 
 
+@pytest.mark.parametrize("k", [1, 15, 16, 17, 31, 32, 33, 64])
+@pytest.mark.parametrize("chunk", [1, 32, 33, 700])
+def test_greedy_chains_on_lists_against_oracle(chunk, k):
+    # lists shorter than, as long as and longer than half a warp and a warp (what is left of the
+    # warp watches for the next restart), weights that tie all the time, rows without a list
+    # between the others, a chunk of one row; with and without statistics
+    sp = _sp()
+    from chunkedgreedy_b200 import synth
+    rng = np.random.default_rng(k)
+    n = 2111
+    lengths = np.where(rng.random(n) < 0.3, 0, 3)
+    rows = np.repeat(np.arange(n), lengths)
+    ptr, ind, _ = synth.coo_to_csr(n, rows, rng.integers(0, 400, rows.size))
+    want, stats = oracle.csg(ptr, ind, False, with_stats=True, k=k, chunk_size=chunk)
+    dp, di = _dev(ptr), _dev(ind)
+    got = sp.chunk_similarity_greedy(dp, di, k=k, chunk_size=chunk)
+    assert np.array_equal(got.cpu().numpy(), want)
+    got, st = sp.chunk_similarity_greedy(dp, di, k=k, chunk_size=chunk, with_stats=True)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert st["chain_restarts"] == stats["chain_restarts"]
+    assert abs(st["avg_followed_weight"] - stats["avg_followed_weight"]) <= 1e-5
+
+
 @pytest.mark.parametrize("name", ["hubsym", "rmat12", "m512", "bigchunk", "rmat16", "dense_ties",
                                   "dense_fill", "dense_m32", "dense_ragged", "dense_m96",
                                   "dense_m128", "dense_m128_ties", "zipf65k"])
