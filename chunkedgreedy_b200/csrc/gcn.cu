@@ -1,0 +1,447 @@
+// The dense part of a two-layer GCN around the library's SpMM, forward and backward, fp32.
+//
+// The caller's model is Linear(in, hidden) -> A -> ReLU -> A -> Linear(hidden, classes)
+// (experiments/e2e_gcn.py:126-137).  With P = A x and the row sums s = A 1 computed first, and the
+// second product taken behind the second linear layer (it is narrower there), what is left
+// between the two sparse products is
+//   forward   H = relu(P W1^T + s b1^T),  U = H W2^T
+//   backward  (G = dL/dU)  D = (G W2) * (H > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T H.
+// One kernel each way: H leaves the first with bias and ReLU applied, D never exists in memory.
+// Both are bound by fp32 multiply-adds (2 n in hidden each way, against three passes over n rows
+// of 128 floats): blocks are persistent, one per SM, operands staged with cp.async a tile ahead,
+// 8 x 8 results per thread.  Per pass on 1.05 M rows, 128 -> 128 -> 16, on a B200: GCN_FIGURES
+#include "../../include/sporder_b200.h"
+#include "common.cuh"
+
+namespace csg {
+
+namespace {
+
+constexpr int D_THREADS = 256;
+constexpr int F_ROWS = 128;  // rows per tile, forward
+constexpr int B_ROWS = 32;   // ... and backward
+constexpr int MAX_CLASSES = 48;
+
+struct DenseArgs {
+  int32_t n, in, hid, cls;
+  const float *P, *s, *W1, *b1, *W2;
+  float *H, *U;       // outputs of the forward pass, H an input of the backward pass
+  const float *G;
+  float *part;        // backward: a block's sums
+  float *dW1, *db1, *dW2;
+};
+
+// 16 (4) bytes global -> shared without registers; zeros when off
+__device__ __forceinline__ void copy16(float *dst, const float *src, bool on) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy4(float *dst, const float *src, bool on) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(on ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// ROWS rows of `cols` floats (a multiple of 4) from row r0 of src into dst, COLS_T + 4 apart, zeros
+// behind the last column and the last row
+template <int ROWS, int COLS_T>
+__device__ __forceinline__ void stage_rows(float *dst, const float *src, int64_t r0, int32_t n, int32_t cols) {
+  constexpr int PER_ROW = COLS_T / 4;
+  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += D_THREADS) {
+    const int r = i / PER_ROW, c = (i % PER_ROW) * 4;
+    const bool on = r0 + r < n && c < cols;
+    copy16(dst + r * (COLS_T + 4) + c, src + (on ? (r0 + r) * cols + c : 0), on);
+  }
+}
+
+template <int IN_T, int HID_T>
+struct ForwardShared {
+  static constexpr int PS = IN_T + 4, HS = HID_T + 4;
+  static constexpr int TILE = F_ROWS * (PS > HS ? PS : HS);  // holds a tile of P, then of H
+  static constexpr int W1 = 0, W2 = W1 + IN_T * HID_T, B1 = W2 + MAX_CLASSES * HS, S = B1 + HID_T,
+                       TILES = S + 2 * F_ROWS, FLOATS = TILES + 2 * TILE;
+};
+
+template <int IN_T, int HID_T>
+__global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) {
+  using L = ForwardShared<IN_T, HID_T>;
+  constexpr int NC = HID_T / 16, V = NC < 4 ? NC : 4, Q = NC / V;  // columns per thread: Q runs of V
+  extern __shared__ __align__(16) float dense_smem[];
+  float *const w1 = dense_smem + L::W1, *const w2 = dense_smem + L::W2, *const b1 = dense_smem + L::B1;
+  float *const s = dense_smem + L::S;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < IN_T * HID_T; i += D_THREADS) {  // W1 with a column of the result per column
+    const int k = i / HID_T, j = i % HID_T;
+    w1[i] = k < a.in && j < a.hid ? a.W1[static_cast<size_t>(j) * a.in + k] : 0.0f;
+  }
+  for (int i = tid; i < MAX_CLASSES * L::HS; i += D_THREADS) {
+    const int c = i / L::HS, j = i % L::HS;
+    w2[i] = c < a.cls && j < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + j] : 0.0f;
+  }
+  for (int i = tid; i < HID_T; i += D_THREADS) b1[i] = i < a.hid ? a.b1[i] : 0.0f;
+  const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
+  auto stage = [&](int64_t t, int buf) {
+    if (t < tiles) {
+      stage_rows<F_ROWS, IN_T>(dense_smem + L::TILES + buf * L::TILE, a.P, t * F_ROWS, a.n, a.in);
+      for (int i = tid; i < F_ROWS; i += D_THREADS) {
+        const bool on = t * F_ROWS + i < a.n;
+        copy4(s + buf * F_ROWS + i, a.s + (on ? t * F_ROWS + i : 0), on);
+      }
+    }
+    copies_commit();
+  };
+  stage(blockIdx.x, 0);
+  int buf = 0;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, buf ^= 1) {
+    stage(t + gridDim.x, buf ^ 1);
+    copies_wait<1>();
+    __syncthreads();
+    float *const tile = dense_smem + L::TILES + buf * L::TILE;
+    float acc[8][NC];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) acc[i][j] = 0.0f;
+#pragma unroll 2
+    for (int k = 0; k < IN_T; k += 4) {
+      float4 p[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) p[i] = *reinterpret_cast<const float4 *>(tile + (ty + 16 * i) * L::PS + k);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float w[NC];
+#pragma unroll
+        for (int qq = 0; qq < Q; ++qq) {
+          const float *src = w1 + (k + kk) * HID_T + qq * (HID_T / Q) + tx * V;
+          if constexpr (V == 4) *reinterpret_cast<float4 *>(w + qq * V) = *reinterpret_cast<const float4 *>(src);
+          else *reinterpret_cast<float2 *>(w + qq * V) = *reinterpret_cast<const float2 *>(src);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float x = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+#pragma unroll
+          for (int j = 0; j < NC; ++j) acc[i][j] = fmaf(x, w[j], acc[i][j]);
+        }
+      }
+    }
+    __syncthreads();  // P of this tile is done with: its place takes H
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = ty + 16 * i;
+      const float si = s[buf * F_ROWS + r];
+#pragma unroll
+      for (int qq = 0; qq < Q; ++qq)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const int j = qq * (HID_T / Q) + tx * V + v;
+          tile[r * L::HS + j] = fmaxf(fmaf(si, b1[j], acc[i][qq * V + v]), 0.0f);
+        }
+    }
+    __syncthreads();
+    const int64_t r0 = t * F_ROWS;
+    for (int i = tid; i < F_ROWS * (HID_T / 4); i += D_THREADS) {
+      const int r = i / (HID_T / 4), c = (i % (HID_T / 4)) * 4;
+      if (r0 + r < a.n && c < a.hid)
+        __stcs(reinterpret_cast<float4 *>(a.H + (r0 + r) * a.hid + c), *reinterpret_cast<const float4 *>(tile + r * L::HS + c));
+    }
+    // U: two threads per row, every other group of four classes each
+    {
+      const int r = tid >> 1;
+      if (r0 + r < a.n) {
+        for (int c0 = (tid & 1) * 4; c0 < a.cls; c0 += 8) {
+          float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+          for (int k = 0; k < HID_T; k += 4) {
+            const float4 h = *reinterpret_cast<const float4 *>(tile + r * L::HS + k);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float4 w = *reinterpret_cast<const float4 *>(w2 + (c0 + c) * L::HS + k);
+              u[c] = fmaf(h.x, w.x, fmaf(h.y, w.y, fmaf(h.z, w.z, fmaf(h.w, w.w, u[c]))));
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c0 + c < a.cls) a.U[(r0 + r) * a.cls + c0 + c] = u[c];
+        }
+      }
+    }
+    __syncthreads();  // the tile's place is free for the copies of the round after next
+  }
+  copies_wait<0>();
+}
+
+template <int IN_T, int HID_T, int CLS_T>
+struct BackwardShared {
+  static constexpr int PS = IN_T + 4, HS = HID_T + 4;
+  static constexpr int D = 0, BUF = D + B_ROWS * HS;
+  static constexpr int P = 0, H = P + B_ROWS * PS, G = H + B_ROWS * HS, S = G + B_ROWS * CLS_T, BUF_FLOATS = S + B_ROWS;
+  static constexpr int FLOATS = BUF + 2 * BUF_FLOATS;
+};
+// a block's sums in `part`: dW1 (HID_T x IN_T), dW2 (CLS_T x HID_T), then db1 from each of the
+// D_THREADS / HID_T groups of threads
+template <int IN_T, int HID_T, int CLS_T>
+struct PartLayout {
+  static constexpr int W2 = HID_T * IN_T, B1 = W2 + CLS_T * HID_T, FLOATS = B1 + D_THREADS;
+};
+
+template <int IN_T, int HID_T, int CLS_T>
+__global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a) {
+  using L = BackwardShared<IN_T, HID_T, CLS_T>;
+  using O = PartLayout<IN_T, HID_T, CLS_T>;
+  constexpr int NJ = HID_T / 16, VJ = NJ < 4 ? NJ : 4, QJ = NJ / VJ;
+  constexpr int NI = IN_T / 16, VI = 4, QI = NI / VI;
+  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS;  // dW2: PER classes of one hidden unit per thread
+  extern __shared__ __align__(16) float dense_smem[];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int hj = tid % HID_T, group = tid / HID_T;
+  float w2[CLS_T];  // this thread's hidden unit's column of W2
+#pragma unroll
+  for (int c = 0; c < CLS_T; ++c)
+    w2[c] = c < a.cls && hj < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + hj] : 0.0f;
+  float acc[NJ][NI], acc2[PER], accb = 0.0f;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) acc[j][i] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) acc2[c] = 0.0f;
+  for (int i = tid; i < 2 * L::BUF_FLOATS; i += D_THREADS) dense_smem[L::BUF + i] = 0.0f;  // classes behind the last
+  __syncthreads();
+  const int64_t tiles = (static_cast<int64_t>(a.n) + B_ROWS - 1) / B_ROWS;
+  auto stage = [&](int64_t t, int buf) {
+    if (t < tiles) {
+      float *const b = dense_smem + L::BUF + buf * L::BUF_FLOATS;
+      const int64_t r0 = t * B_ROWS;
+      stage_rows<B_ROWS, IN_T>(b + L::P, a.P, r0, a.n, a.in);
+      stage_rows<B_ROWS, HID_T>(b + L::H, a.H, r0, a.n, a.hid);
+      for (int i = tid; i < B_ROWS * a.cls; i += D_THREADS) {
+        const int r = i / a.cls, c = i % a.cls;
+        const bool on = r0 + r < a.n;
+        copy4(b + L::G + r * CLS_T + c, a.G + (on ? r0 * a.cls + i : 0), on);
+      }
+      for (int i = tid; i < B_ROWS; i += D_THREADS) copy4(b + L::S + i, a.s + (r0 + i < a.n ? r0 + i : 0), r0 + i < a.n);
+    }
+    copies_commit();
+  };
+  stage(blockIdx.x, 0);
+  int buf = 0;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, buf ^= 1) {
+    stage(t + gridDim.x, buf ^ 1);
+    copies_wait<1>();
+    __syncthreads();
+    const float *const b = dense_smem + L::BUF + buf * L::BUF_FLOATS;
+    const float *const p = b + L::P, *const h = b + L::H, *const g = b + L::G, *const s = b + L::S;
+    float *const d = dense_smem + L::D;
+#pragma unroll 4
+    for (int r = group; r < B_ROWS; r += GROUPS) {
+      float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int c = 0; c < CLS_T; c += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(g + r * CLS_T + c);
+        x[0] = fmaf(q.x, w2[c], x[0]);
+        x[1] = fmaf(q.y, w2[c + 1], x[1]);
+        x[2] = fmaf(q.z, w2[c + 2], x[2]);
+        x[3] = fmaf(q.w, w2[c + 3], x[3]);
+      }
+      const float y = h[r * L::HS + hj] > 0.0f ? (x[0] + x[1]) + (x[2] + x[3]) : 0.0f;
+      d[r * L::HS + hj] = y;
+      accb = fmaf(y, s[r], accb);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int r = 0; r < B_ROWS; ++r) {
+      float dj[NJ], pi[NI];
+#pragma unroll
+      for (int q = 0; q < QJ; ++q) {
+        const float *src = d + r * L::HS + q * (HID_T / QJ) + ty * VJ;
+        if constexpr (VJ == 4) *reinterpret_cast<float4 *>(dj + q * VJ) = *reinterpret_cast<const float4 *>(src);
+        else *reinterpret_cast<float2 *>(dj + q * VJ) = *reinterpret_cast<const float2 *>(src);
+      }
+#pragma unroll
+      for (int q = 0; q < QI; ++q)
+        *reinterpret_cast<float4 *>(pi + q * VI) = *reinterpret_cast<const float4 *>(p + r * L::PS + q * (IN_T / QI) + tx * VI);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) acc[j][i] = fmaf(dj[j], pi[i], acc[j][i]);
+      const float hv = h[r * L::HS + hj];
+#pragma unroll
+      for (int c = 0; c < PER; ++c) acc2[c] = fmaf(g[r * CLS_T + group * PER + c], hv, acc2[c]);
+    }
+    __syncthreads();
+  }
+  copies_wait<0>();
+  float *const out = a.part + static_cast<size_t>(blockIdx.x) * O::FLOATS;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int row = (j / VJ) * (HID_T / QJ) + ty * VJ + j % VJ, col = (i / VI) * (IN_T / QI) + tx * VI + i % VI;
+      out[row * IN_T + col] = acc[j][i];
+    }
+#pragma unroll
+  for (int c = 0; c < PER; ++c) out[O::W2 + (group * PER + c) * HID_T + hj] = acc2[c];
+  out[O::B1 + tid] = accb;
+}
+
+// the blocks' sums, always in the same order
+template <int IN_T, int HID_T, int CLS_T>
+__global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) {
+  using O = PartLayout<IN_T, HID_T, CLS_T>;
+  const int w1 = a.hid * a.in, w2 = a.cls * a.hid, total = w1 + w2 + a.hid;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    int at, times = 1;
+    float *to;
+    if (i < w1) {
+      at = i / a.in * IN_T + i % a.in;
+      to = a.dW1 + i;
+    } else if (i < w1 + w2) {
+      const int x = i - w1;
+      at = O::W2 + x / a.hid * HID_T + x % a.hid;
+      to = a.dW2 + x;
+    } else {
+      at = O::B1 + i - w1 - w2;
+      to = a.db1 + (i - w1 - w2);
+      times = D_THREADS / HID_T;
+    }
+    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int g = 0; g < times; ++g) {
+      const float *src = a.part + at + g * HID_T;
+      int b = 0;
+      for (; b + 4 <= blocks; b += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sum[u] += src[static_cast<size_t>(b + u) * O::FLOATS];
+      for (; b < blocks; ++b) sum[0] += src[static_cast<size_t>(b) * O::FLOATS];
+    }
+    *to = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+  }
+}
+
+// A 1: a warp per row, rows in turn
+__global__ void __launch_bounds__(256) row_sums_kernel(int32_t n, int32_t nnz, const int32_t *__restrict__ ptr,
+                                                       const float *__restrict__ val, float *__restrict__ out) {
+  // eight lanes a row: most rows are short, and the few long ones are read at full width all the same
+  constexpr int G = 8;
+  const int gl = threadIdx.x % G;
+  const int64_t groups = static_cast<int64_t>(gridDim.x) * blockDim.x / G;
+  const int64_t rounds = (static_cast<int64_t>(n) + groups - 1) / groups;
+  int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / G;
+  for (int64_t i = 0; i < rounds; ++i, r += groups) {
+    int32_t b = 0, e = 0;
+    if (r < n) {
+      b = ptr[r];
+      e = ptr[r + 1];
+      if (b < 0 || e < b || e > nnz) e = b = 0;  // malformed row pointers: an empty row
+    }
+    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int32_t p = b + gl;
+    for (; p + 3 * G < e; p += 4 * G)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] += val[p + u * G];
+    for (; p < e; p += G) x[0] += val[p];
+    float v = (x[0] + x[1]) + (x[2] + x[3]);
+#pragma unroll
+    for (int off = G / 2; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
+    if (gl == 0 && r < n) out[r] = v;
+  }
+}
+
+template <typename Kernel>
+bool dense_smem_limit(Kernel kernel, size_t bytes) {
+  CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  return true;
+}
+
+template <int IN_T, int HID_T>
+bool forward_variant(Context &ctx, const DenseArgs &a) {
+  const size_t smem = sizeof(float) * ForwardShared<IN_T, HID_T>::FLOATS;
+  if (!dense_smem_limit(gcn_forward_kernel<IN_T, HID_T>, smem)) return false;
+  const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
+  const int grid = static_cast<int>(tiles < ctx.num_sms ? tiles : ctx.num_sms);
+  gcn_forward_kernel<IN_T, HID_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(1);
+  return true;
+}
+
+template <int IN_T, int HID_T, int CLS_T>
+bool backward_variant(Context &ctx, DenseArgs a) {
+  const size_t smem = sizeof(float) * BackwardShared<IN_T, HID_T, CLS_T>::FLOATS;
+  if (!dense_smem_limit(gcn_backward_kernel<IN_T, HID_T, CLS_T>, smem)) return false;
+  const int64_t tiles = (static_cast<int64_t>(a.n) + B_ROWS - 1) / B_ROWS;
+  const int grid = static_cast<int>(tiles < ctx.num_sms ? tiles : ctx.num_sms);
+  if (!ensure_workspace(ctx, sizeof(float) * PartLayout<IN_T, HID_T, CLS_T>::FLOATS * static_cast<size_t>(grid))) return false;
+  a.part = reinterpret_cast<float *>(ctx.ws);
+  gcn_backward_kernel<IN_T, HID_T, CLS_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
+  CSG_CUDA(cudaGetLastError());
+  const int total = a.hid * a.in + a.cls * a.hid + a.hid;
+  gcn_sums_kernel<IN_T, HID_T, CLS_T><<<(total + 255) / 256, 256, 0, ctx.stream>>>(a, grid);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(2);
+  return true;
+}
+
+bool check_dense(const DenseArgs &a) {
+  CSG_REQUIRE(a.n >= 1 && a.in >= 4 && a.in <= 128 && a.in % 4 == 0 && a.hid >= 4 && a.hid <= 128 && a.hid % 4 == 0 &&
+                  a.cls >= 1 && a.cls <= MAX_CLASSES,
+              "gcn: expect in and hidden in multiples of 4 up to 128 and up to %d classes (got %d, %d, %d)", MAX_CLASSES,
+              a.in, a.hid, a.cls);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(a.P) | reinterpret_cast<uintptr_t>(a.H);
+  CSG_REQUIRE(all % 16 == 0, "gcn: P and H must be 16-byte aligned");
+  return true;
+}
+
+bool run_forward(Context &ctx, const DenseArgs &a) {
+  if (!check_dense(a)) return false;
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  if (a.in <= 64)
+    return a.hid <= 32 ? forward_variant<64, 32>(ctx, a) : a.hid <= 64 ? forward_variant<64, 64>(ctx, a) : forward_variant<64, 128>(ctx, a);
+  return a.hid <= 32 ? forward_variant<128, 32>(ctx, a) : a.hid <= 64 ? forward_variant<128, 64>(ctx, a) : forward_variant<128, 128>(ctx, a);
+}
+
+template <int CLS_T>
+bool run_backward_classes(Context &ctx, const DenseArgs &a) {
+  if (a.in <= 64)
+    return a.hid <= 32   ? backward_variant<64, 32, CLS_T>(ctx, a)
+           : a.hid <= 64 ? backward_variant<64, 64, CLS_T>(ctx, a)
+                         : backward_variant<64, 128, CLS_T>(ctx, a);
+  return a.hid <= 32   ? backward_variant<128, 32, CLS_T>(ctx, a)
+         : a.hid <= 64 ? backward_variant<128, 64, CLS_T>(ctx, a)
+                       : backward_variant<128, 128, CLS_T>(ctx, a);
+}
+
+bool run_backward(Context &ctx, const DenseArgs &a) {
+  if (!check_dense(a)) return false;
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  return a.cls <= 16 ? run_backward_classes<16>(ctx, a) : run_backward_classes<MAX_CLASSES>(ctx, a);
+}
+
+bool run_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *ptr, const float *val, float *out) {
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  int64_t grid = (static_cast<int64_t>(n) * 8 + 255) / 256;
+  if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
+  row_sums_kernel<<<static_cast<int>(grid), 256, 0, ctx.stream>>>(n, nnz, ptr, val, out);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(1);
+  return true;
+}
+
+}  // namespace
+
+bool launch_gcn_forward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *P, const float *s,
+                        const float *W1, const float *b1, const float *W2, float *H, float *U) {
+  DenseArgs a = {n, in, hid, cls, P, s, W1, b1, W2, H, U, nullptr, nullptr, nullptr, nullptr, nullptr};
+  return run_forward(ctx, a);
+}
+bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *G, const float *H,
+                         const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2) {
+  DenseArgs a = {n, in, hid, cls, P, s, nullptr, nullptr, W2, const_cast<float *>(H), nullptr, G, nullptr, dW1, db1, dW2};
+  return run_backward(ctx, a);
+}
+bool launch_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr, const float *d_val, float *d_out) {
+  return run_row_sums(ctx, n, nnz, d_ptr, d_val, d_out);
+}
+
+}  // namespace csg

@@ -20,7 +20,7 @@ import time
 import torch
 import torch.nn.functional as F
 
-from . import chunk_similarity_greedy, reorder, spmm
+from . import _ctx, _enter, _lib, chunk_similarity_greedy, reorder, spmm
 
 __all__ = ["SpMMFn", "GraphOperator", "GCN", "train", "reorder_and_train", "breakeven_epochs"]
 
@@ -57,6 +57,17 @@ class GraphOperator:
         self._pending.append((e0, e1))
         return out
 
+    def row_sums(self):
+        """A 1, one float per row."""
+        out = torch.empty(self.ptr.numel() - 1, dtype=torch.float32, device=self.ptr.device)
+        ctx = _ctx(self.ctx, self.ptr)
+        with torch.cuda.device(self.ptr.device):
+            _enter(ctx, self.ptr)
+            if _lib.load().sporder_row_sums(ctx.handle, out.numel(), self.val.numel(), self.ptr.data_ptr(),
+                                            self.val.data_ptr(), out.data_ptr()) != 0:
+                _lib.check()
+        return out
+
     def collect(self):
         torch.cuda.synchronize()
         self.spmm_ms += sum(a.elapsed_time(b) for a, b in self._pending)
@@ -64,14 +75,76 @@ class GraphOperator:
         return self.spmm_ms
 
 
+class DenseFn(torch.autograd.Function):
+    """relu(P W1^T + s b1^T) W2^T, in one kernel forward and one backward; no gradient for P
+    and s."""
+
+    @staticmethod
+    def forward(ctx, P, s, w1, b1, w2, lib_ctx):
+        n, hidden, classes = P.shape[0], w1.shape[0], w2.shape[0]
+        P, w1, b1, w2 = P.contiguous(), w1.contiguous(), b1.contiguous(), w2.contiguous()
+        H = torch.empty((n, hidden), dtype=torch.float32, device=P.device)
+        U = torch.empty((n, classes), dtype=torch.float32, device=P.device)
+        ctx.lib_ctx = _ctx(lib_ctx, P)
+        with torch.cuda.device(P.device):
+            _enter(ctx.lib_ctx, P)
+            if _lib.load().sporder_gcn_forward(ctx.lib_ctx.handle, n, P.shape[1], hidden, classes, P.data_ptr(),
+                                               s.data_ptr(), w1.data_ptr(), b1.data_ptr(), w2.data_ptr(),
+                                               H.data_ptr(), U.data_ptr()) != 0:
+                _lib.check()
+        ctx.save_for_backward(P, s, H, w2)
+        return U
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, g):
+        P, s, H, w2 = ctx.saved_tensors
+        n, in_dim, hidden, classes = P.shape[0], P.shape[1], H.shape[1], w2.shape[0]
+        g = g.contiguous()
+        dw1 = torch.empty((hidden, in_dim), dtype=torch.float32, device=P.device)
+        db1 = torch.empty(hidden, dtype=torch.float32, device=P.device)
+        dw2 = torch.empty((classes, hidden), dtype=torch.float32, device=P.device)
+        with torch.cuda.device(P.device):
+            _enter(ctx.lib_ctx, P)
+            if _lib.load().sporder_gcn_backward(ctx.lib_ctx.handle, n, in_dim, hidden, classes, g.data_ptr(),
+                                                H.data_ptr(), P.data_ptr(), s.data_ptr(), w2.data_ptr(),
+                                                dw1.data_ptr(), db1.data_ptr(), dw2.data_ptr()) != 0:
+                _lib.check()
+        return None, None, dw1, db1, dw2, None
+
+
 class GCN(torch.nn.Module):
+    """Linear -> op -> ReLU -> op -> Linear.  The sparse products are taken where they are
+    narrowest, which does not change what is computed: op is linear in its columns, so
+    op(x W1^T + b1) = op(x) W1^T + op(1) b1^T and op(h) W2^T = op(h W2^T).  With the operator in front of
+    the first layer, training needs no product for that layer's gradient at all (features carry
+    none)."""
+
     def __init__(self, in_dim, hidden, classes):
         super().__init__()
         self.w1 = torch.nn.Linear(in_dim, hidden)
         self.w2 = torch.nn.Linear(hidden, classes)
 
     def forward(self, x, op):
-        h = F.relu(SpMMFn.apply(self.w1(x), op))
+        hidden, in_dim = self.w1.weight.shape
+        classes = self.w2.weight.shape[0]
+        training = torch.is_grad_enabled()
+        # columns of sparse products, operator first against layer first, forward and backward
+        first = in_dim * (2 if training and x.requires_grad else 1)
+        if first <= hidden * (2 if training else 1) and self.w1.bias is not None:
+            p = SpMMFn.apply(x, op)
+            s = op.row_sums() if hasattr(op, "row_sums") else op(torch.ones_like(x[:, :1]))[:, 0].contiguous()
+            # limits of the fused kernels; others, and features that want a gradient, by torch
+            if (not p.requires_grad and in_dim % 4 == 0 and in_dim <= 128 and hidden % 4 == 0
+                    and hidden <= 128 and classes <= 48 and classes <= hidden
+                    and all(t.is_cuda and t.dtype == torch.float32 for t in (p, s, self.w1.weight, self.w2.weight))):
+                u = DenseFn.apply(p, s, self.w1.weight, self.w1.bias, self.w2.weight, getattr(op, "ctx", None))
+                return SpMMFn.apply(u, op) + self.w2.bias
+            h = F.relu(torch.addr(F.linear(p, self.w1.weight), s, self.w1.bias))
+        else:
+            h = F.relu(SpMMFn.apply(self.w1(x), op))
+        if classes < hidden:
+            return SpMMFn.apply(F.linear(h, self.w2.weight), op) + self.w2.bias
         return self.w2(SpMMFn.apply(h, op))
 
 

@@ -510,6 +510,39 @@ def test_gcn_gradients_match_dense_reference_and_reordering_is_equivalent():
     assert sorted(res["order"].cpu().tolist()) == list(range(n))
 
 
+@pytest.mark.parametrize("n", [1, 31, 128, 129, 40_000])
+@pytest.mark.parametrize("sizes", [(4, 4, 1), (64, 32, 7), (100, 64, 16), (128, 128, 17), (68, 36, 3), (64, 128, 48),
+                                   (128, 32, 33), (300, 32, 5), (33, 64, 80)])
+@pytest.mark.parametrize("want_x", [False, True])
+def test_gcn_model_against_fp64(n, sizes, want_x):
+    # the fused dense kernels at the edges of their tiles, and the sizes and gradients they leave to torch
+    from chunkedgreedy_b200 import gcn, synth
+    in_dim, hidden, classes = sizes
+    if n == 1:
+        ptr, ind = np.array([0, 1], dtype=np.int32), np.zeros(1, dtype=np.int32)
+    else:
+        ptr, ind, _ = synth.random_sparse(n, 3, 5, symmetric=True, hub_cols=2, hub_frac=0.2)
+    dp, di = _dev(ptr), _dev(ind)
+    op = gcn.GraphOperator(dp, di, gcn.normalised_values(dp, di))
+    torch.manual_seed(3)
+    model = gcn.GCN(in_dim, hidden, classes).cuda()
+    x = torch.randn((n, in_dim), device="cuda", requires_grad=want_x)
+    target = torch.randn((n, classes), device="cuda")
+    z = model(x, op)
+    (z * target).sum().backward()
+    a = torch.sparse_csr_tensor(dp.long(), di.long(), op.val.double(), size=(n, n))
+    wide = [p.detach().double().requires_grad_(True) for p in model.parameters()]
+    xr = x.detach().double().requires_grad_(want_x)
+    w1, b1, w2, b2 = wide
+    zr = a @ torch.relu(a @ (xr @ w1.t() + b1)) @ w2.t() + b2
+    (zr * target.double()).sum().backward()
+    pairs = [(z, zr)] + [(p.grad, q.grad) for p, q in zip(model.parameters(), wide)]
+    if want_x:
+        pairs.append((x.grad, xr.grad))
+    for got, want in pairs:
+        assert float((got.double() - want).norm()) <= 2e-5 * float(want.norm()) + 1e-6
+
+
 @pytest.mark.parametrize("name", ["stencil1024", "road2m"])
 def test_full_size_streaming_workloads_bit_exact(name):
     # benchmark configurations 2 and 3 at their full sizes (1.05 M / 2 M rows): the oracle
