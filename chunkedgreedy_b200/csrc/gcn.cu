@@ -9,7 +9,9 @@
 // One kernel each way: H leaves the first with bias and ReLU applied, D never exists in memory.
 // Both are bound by fp32 multiply-adds (2 n in hidden each way, against three passes over n rows
 // of 128 floats): blocks are persistent, one per SM, operands staged with cp.async a tile ahead,
-// 8 x 8 results per thread.  Per pass on 1.05 M rows, 128 -> 128 -> 16, on a B200: GCN_FIGURES
+// 8 x 8 results per thread.  Per pass on 1.05 M rows,
+// 128 -> 128 -> 16, on a B200: 0.95 ms forward, 1.09 ms backward (53 % of the fp32 pipes; two warps per
+// scheduler, and the phases of a tile do not overlap); one torch kernel per operation took 1.8 and 2.4 ms.
 #include "../../include/sporder_b200.h"
 #include "common.cuh"
 
@@ -17,7 +19,8 @@ namespace csg {
 
 namespace {
 
-constexpr int D_THREADS = 256;
+constexpr int F_THREADS = 256;  // threads of a block, forward
+constexpr int D_THREADS = 256;  // ... and backward
 constexpr int F_ROWS = 128;  // rows per tile, forward
 constexpr int B_ROWS = 32;   // ... and backward
 constexpr int MAX_CLASSES = 48;
@@ -46,14 +49,22 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_grou
 
 // ROWS rows of `cols` floats (a multiple of 4) from row r0 of src into dst, COLS_T + 4 apart, zeros
 // behind the last column and the last row
-template <int ROWS, int COLS_T>
+template <int ROWS, int COLS_T, int THREADS>
 __device__ __forceinline__ void stage_rows(float *dst, const float *src, int64_t r0, int32_t n, int32_t cols) {
   constexpr int PER_ROW = COLS_T / 4;
-  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += D_THREADS) {
+  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += THREADS) {
     const int r = i / PER_ROW, c = (i % PER_ROW) * 4;
     const bool on = r0 + r < n && c < cols;
     copy16(dst + r * (COLS_T + 4) + c, src + (on ? (r0 + r) * cols + c : 0), on);
   }
+}
+
+// acc.x += a.x * b.x, acc.y += a.y * b.y in one instruction
+__device__ __forceinline__ void fma2(float2 &acc, float2 a, float2 b) {
+  unsigned long long &c = reinterpret_cast<unsigned long long &>(acc);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(c)
+      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
 }
 
 template <int IN_T, int HID_T>
@@ -65,27 +76,29 @@ struct ForwardShared {
 };
 
 template <int IN_T, int HID_T>
-__global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) {
+__global__ void __launch_bounds__(F_THREADS, 1) gcn_forward_kernel(DenseArgs a) {
   using L = ForwardShared<IN_T, HID_T>;
-  constexpr int NC = HID_T / 16, V = NC < 4 ? NC : 4, Q = NC / V;  // columns per thread: Q runs of V
+  constexpr int NC = HID_T / 16;               // columns per thread, in pairs
+  constexpr int TY = F_THREADS / 16, RPT = F_ROWS / TY;  // rows per thread, TY apart
   extern __shared__ __align__(16) float dense_smem[];
   float *const w1 = dense_smem + L::W1, *const w2 = dense_smem + L::W2, *const b1 = dense_smem + L::B1;
   float *const s = dense_smem + L::S;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int i = tid; i < IN_T * HID_T; i += D_THREADS) {  // W1 with a column of the result per column
-    const int k = i / HID_T, j = i % HID_T;
+  // W1 with a column of the result per column, entries of two successive inputs side by side
+  for (int i = tid; i < IN_T * HID_T; i += F_THREADS) {
+    const int k = i / (2 * HID_T) * 2 + (i & 1), j = i % (2 * HID_T) >> 1;
     w1[i] = k < a.in && j < a.hid ? a.W1[static_cast<size_t>(j) * a.in + k] : 0.0f;
   }
-  for (int i = tid; i < MAX_CLASSES * L::HS; i += D_THREADS) {
+  for (int i = tid; i < MAX_CLASSES * L::HS; i += F_THREADS) {
     const int c = i / L::HS, j = i % L::HS;
     w2[i] = c < a.cls && j < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + j] : 0.0f;
   }
-  for (int i = tid; i < HID_T; i += D_THREADS) b1[i] = i < a.hid ? a.b1[i] : 0.0f;
+  for (int i = tid; i < HID_T; i += F_THREADS) b1[i] = i < a.hid ? a.b1[i] : 0.0f;
   const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
   auto stage = [&](int64_t t, int buf) {
     if (t < tiles) {
-      stage_rows<F_ROWS, IN_T>(dense_smem + L::TILES + buf * L::TILE, a.P, t * F_ROWS, a.n, a.in);
-      for (int i = tid; i < F_ROWS; i += D_THREADS) {
+      stage_rows<F_ROWS, IN_T, F_THREADS>(dense_smem + L::TILES + buf * L::TILE, a.P, t * F_ROWS, a.n, a.in);
+      for (int i = tid; i < F_ROWS; i += F_THREADS) {
         const bool on = t * F_ROWS + i < a.n;
         copy4(s + buf * F_ROWS + i, a.s + (on ? t * F_ROWS + i : 0), on);
       }
@@ -99,58 +112,54 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) 
     copies_wait<1>();
     __syncthreads();
     float *const tile = dense_smem + L::TILES + buf * L::TILE;
-    float acc[8][NC];
+    float2 acc[RPT][NC];  // sums over the even and over the odd inputs
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RPT; ++i)
 #pragma unroll
-      for (int j = 0; j < NC; ++j) acc[i][j] = 0.0f;
+      for (int j = 0; j < NC; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll 2
     for (int k = 0; k < IN_T; k += 4) {
-      float4 p[8];
+      float4 p[RPT];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) p[i] = *reinterpret_cast<const float4 *>(tile + (ty + 16 * i) * L::PS + k);
+      for (int i = 0; i < RPT; ++i) p[i] = *reinterpret_cast<const float4 *>(tile + (ty + TY * i) * L::PS + k);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        float w[NC];
+      for (int kk = 0; kk < 4; kk += 2) {
+        float2 w[NC];
 #pragma unroll
-        for (int qq = 0; qq < Q; ++qq) {
-          const float *src = w1 + (k + kk) * HID_T + qq * (HID_T / Q) + tx * V;
-          if constexpr (V == 4) *reinterpret_cast<float4 *>(w + qq * V) = *reinterpret_cast<const float4 *>(src);
-          else *reinterpret_cast<float2 *>(w + qq * V) = *reinterpret_cast<const float2 *>(src);
-        }
+        for (int j = 0; j < NC; j += 2)
+          *reinterpret_cast<float4 *>(w + j) = *reinterpret_cast<const float4 *>(w1 + (k + kk) * HID_T + 2 * (j / 2 * 32 + tx * 2));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float x = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+        for (int i = 0; i < RPT; ++i) {
+          const float2 x = kk == 0 ? make_float2(p[i].x, p[i].y) : make_float2(p[i].z, p[i].w);
 #pragma unroll
-          for (int j = 0; j < NC; ++j) acc[i][j] = fmaf(x, w[j], acc[i][j]);
+          for (int j = 0; j < NC; ++j) fma2(acc[i][j], x, w[j]);
         }
       }
     }
     __syncthreads();  // P of this tile is done with: its place takes H
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = ty + 16 * i;
+    for (int i = 0; i < RPT; ++i) {
+      const int r = ty + TY * i;
       const float si = s[buf * F_ROWS + r];
 #pragma unroll
-      for (int qq = 0; qq < Q; ++qq)
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const int j = qq * (HID_T / Q) + tx * V + v;
-          tile[r * L::HS + j] = fmaxf(fmaf(si, b1[j], acc[i][qq * V + v]), 0.0f);
-        }
+      for (int jj = 0; jj < NC; ++jj) {
+        const int j = jj / 2 * 32 + tx * 2 + (jj & 1);
+        tile[r * L::HS + j] = fmaxf(fmaf(si, b1[j], acc[i][jj].x + acc[i][jj].y), 0.0f);
+      }
     }
     __syncthreads();
     const int64_t r0 = t * F_ROWS;
-    for (int i = tid; i < F_ROWS * (HID_T / 4); i += D_THREADS) {
+    for (int i = tid; i < F_ROWS * (HID_T / 4); i += F_THREADS) {
       const int r = i / (HID_T / 4), c = (i % (HID_T / 4)) * 4;
       if (r0 + r < a.n && c < a.hid)
         __stcs(reinterpret_cast<float4 *>(a.H + (r0 + r) * a.hid + c), *reinterpret_cast<const float4 *>(tile + r * L::HS + c));
     }
     // U: two threads per row, every other group of four classes each
     {
-      const int r = tid >> 1;
+      constexpr int TPR = F_THREADS / F_ROWS;
+      const int r = tid / TPR;
       if (r0 + r < a.n) {
-        for (int c0 = (tid & 1) * 4; c0 < a.cls; c0 += 8) {
+        for (int c0 = tid % TPR * 4; c0 < a.cls; c0 += 4 * TPR) {
           float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 4
           for (int k = 0; k < HID_T; k += 4) {
@@ -190,9 +199,9 @@ template <int IN_T, int HID_T, int CLS_T>
 __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a) {
   using L = BackwardShared<IN_T, HID_T, CLS_T>;
   using O = PartLayout<IN_T, HID_T, CLS_T>;
-  constexpr int NJ = HID_T / 16, VJ = NJ < 4 ? NJ : 4, QJ = NJ / VJ;
-  constexpr int NI = IN_T / 16, VI = 4, QI = NI / VI;
-  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS;  // dW2: PER classes of one hidden unit per thread
+  constexpr int NJ = HID_T / 16, VJ = NJ < 4 ? NJ : 4, QJ = NJ / VJ;  // hidden units per thread, QJ runs of VJ
+  constexpr int NI = IN_T / 16, VI = 4, QI = NI / VI;   // inputs per thread, in fours
+  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS, VC = PER % 4 == 0 ? 4 : 2;  // dW2: PER classes of one hidden unit per thread
   extern __shared__ __align__(16) float dense_smem[];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int hj = tid % HID_T, group = tid / HID_T;
@@ -200,11 +209,12 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
 #pragma unroll
   for (int c = 0; c < CLS_T; ++c)
     w2[c] = c < a.cls && hj < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + hj] : 0.0f;
-  float acc[NJ][NI], acc2[PER], accb = 0.0f;
+  float2 acc[NJ][NI / 2];
+  float acc2[PER], accb = 0.0f;
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
 #pragma unroll
-    for (int i = 0; i < NI; ++i) acc[j][i] = 0.0f;
+    for (int i = 0; i < NI / 2; ++i) acc[j][i] = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int c = 0; c < PER; ++c) acc2[c] = 0.0f;
   for (int i = tid; i < 2 * L::BUF_FLOATS; i += D_THREADS) dense_smem[L::BUF + i] = 0.0f;  // classes behind the last
@@ -214,8 +224,8 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
     if (t < tiles) {
       float *const b = dense_smem + L::BUF + buf * L::BUF_FLOATS;
       const int64_t r0 = t * B_ROWS;
-      stage_rows<B_ROWS, IN_T>(b + L::P, a.P, r0, a.n, a.in);
-      stage_rows<B_ROWS, HID_T>(b + L::H, a.H, r0, a.n, a.hid);
+      stage_rows<B_ROWS, IN_T, D_THREADS>(b + L::P, a.P, r0, a.n, a.in);
+      stage_rows<B_ROWS, HID_T, D_THREADS>(b + L::H, a.H, r0, a.n, a.hid);
       for (int i = tid; i < B_ROWS * a.cls; i += D_THREADS) {
         const int r = i / a.cls, c = i % a.cls;
         const bool on = r0 + r < a.n;
@@ -252,7 +262,8 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
     __syncthreads();
 #pragma unroll 4
     for (int r = 0; r < B_ROWS; ++r) {
-      float dj[NJ], pi[NI];
+      float dj[NJ];
+      float2 pi[NI / 2];
 #pragma unroll
       for (int q = 0; q < QJ; ++q) {
         const float *src = d + r * L::HS + q * (HID_T / QJ) + ty * VJ;
@@ -261,14 +272,20 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
       }
 #pragma unroll
       for (int q = 0; q < QI; ++q)
-        *reinterpret_cast<float4 *>(pi + q * VI) = *reinterpret_cast<const float4 *>(p + r * L::PS + q * (IN_T / QI) + tx * VI);
+        *reinterpret_cast<float4 *>(pi + 2 * q) = *reinterpret_cast<const float4 *>(p + r * L::PS + q * (IN_T / QI) + tx * VI);
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
-        for (int i = 0; i < NI; ++i) acc[j][i] = fmaf(dj[j], pi[i], acc[j][i]);
+        for (int i = 0; i < NI / 2; ++i) fma2(acc[j][i], make_float2(dj[j], dj[j]), pi[i]);
       const float hv = h[r * L::HS + hj];
 #pragma unroll
-      for (int c = 0; c < PER; ++c) acc2[c] = fmaf(g[r * CLS_T + group * PER + c], hv, acc2[c]);
+      for (int c = 0; c < PER; c += VC) {
+        float gv[VC];
+        if constexpr (VC == 4) *reinterpret_cast<float4 *>(gv) = *reinterpret_cast<const float4 *>(g + r * CLS_T + group * PER + c);
+        else *reinterpret_cast<float2 *>(gv) = *reinterpret_cast<const float2 *>(g + r * CLS_T + group * PER + c);
+#pragma unroll
+        for (int x = 0; x < VC; ++x) acc2[c + x] = fmaf(gv[x], hv, acc2[c + x]);
+      }
     }
     __syncthreads();
   }
@@ -279,7 +296,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int row = (j / VJ) * (HID_T / QJ) + ty * VJ + j % VJ, col = (i / VI) * (IN_T / QI) + tx * VI + i % VI;
-      out[row * IN_T + col] = acc[j][i];
+      out[row * IN_T + col] = i & 1 ? acc[j][i / 2].y : acc[j][i / 2].x;
     }
 #pragma unroll
   for (int c = 0; c < PER; ++c) out[O::W2 + (group * PER + c) * HID_T + hj] = acc2[c];
@@ -319,10 +336,12 @@ __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) 
   }
 }
 
-// A 1: a warp per row, rows in turn
+// A 1.  Eight lanes a row; rows of more than SUM_SPLIT entries are queued in pieces for a second
+// kernel, where a warp adds a piece at a time (one row of a power-law graph holds 10^5 entries).
+constexpr int SUM_SPLIT = 512, SUM_PIECE = 2048;
 __global__ void __launch_bounds__(256) row_sums_kernel(int32_t n, int32_t nnz, const int32_t *__restrict__ ptr,
-                                                       const float *__restrict__ val, float *__restrict__ out) {
-  // eight lanes a row: most rows are short, and the few long ones are read at full width all the same
+                                                       const float *__restrict__ val, float *__restrict__ out,
+                                                       uint32_t *queued, int2 *queue) {
   constexpr int G = 8;
   const int gl = threadIdx.x % G;
   const int64_t groups = static_cast<int64_t>(gridDim.x) * blockDim.x / G;
@@ -335,16 +354,39 @@ __global__ void __launch_bounds__(256) row_sums_kernel(int32_t n, int32_t nnz, c
       e = ptr[r + 1];
       if (b < 0 || e < b || e > nnz) e = b = 0;  // malformed row pointers: an empty row
     }
-    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int32_t p = b + gl;
-    for (; p + 3 * G < e; p += 4 * G)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] += val[p + u * G];
-    for (; p < e; p += G) x[0] += val[p];
-    float v = (x[0] + x[1]) + (x[2] + x[3]);
+    float v = 0.0f;
+    if (e - b > SUM_SPLIT) {
+      if (gl == 0) {
+        const int32_t pieces = (e - b + SUM_PIECE - 1) / SUM_PIECE;
+        uint32_t at = atomicAdd(queued, static_cast<uint32_t>(pieces));
+        for (int32_t p = b; p < e; p += SUM_PIECE) queue[at++] = make_int2(static_cast<int32_t>(r), p);
+      }
+    } else {
+      for (int32_t p = b + gl; p < e; p += G) v += val[p];
+    }
 #pragma unroll
     for (int off = G / 2; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
     if (gl == 0 && r < n) out[r] = v;
+  }
+}
+
+__global__ void __launch_bounds__(256) row_pieces_kernel(const int32_t *__restrict__ ptr, const float *__restrict__ val,
+                                                         float *__restrict__ out, const uint32_t *queued,
+                                                         const int2 *queue) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t total = *queued, warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
+    const int2 q = queue[i];
+    const int32_t end = min(ptr[q.x + 1], q.y + SUM_PIECE);
+    float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int32_t p = q.y + lane; p < end; p += 256)
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (p + 32 * u < end) x[u] += val[p + 32 * u];
+    float v = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
+    if (lane == 0) atomicAdd(out + q.x, v);
   }
 }
 
@@ -360,7 +402,7 @@ bool forward_variant(Context &ctx, const DenseArgs &a) {
   if (!dense_smem_limit(gcn_forward_kernel<IN_T, HID_T>, smem)) return false;
   const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
   const int grid = static_cast<int>(tiles < ctx.num_sms ? tiles : ctx.num_sms);
-  gcn_forward_kernel<IN_T, HID_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
+  gcn_forward_kernel<IN_T, HID_T><<<grid, F_THREADS, smem, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(1);
   return true;
@@ -420,11 +462,18 @@ bool run_backward(Context &ctx, const DenseArgs &a) {
 
 bool run_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *ptr, const float *val, float *out) {
   CSG_CUDA(cudaSetDevice(ctx.device));
-  int64_t grid = (static_cast<int64_t>(n) * 8 + 255) / 256;
+  int64_t grid = (static_cast<int64_t>(n) + 31) / 32;
   if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
-  row_sums_kernel<<<static_cast<int>(grid), 256, 0, ctx.stream>>>(n, nnz, ptr, val, out);
+  // at most nnz / SUM_SPLIT pieces: a piece shorter than that is the end of a row with a full one
+  if (!ensure_workspace(ctx, 256 + sizeof(int2) * (static_cast<size_t>(nnz) / SUM_SPLIT + 1))) return false;
+  uint32_t *const queued = reinterpret_cast<uint32_t *>(ctx.ws);
+  int2 *const queue = reinterpret_cast<int2 *>(ctx.ws + 256);
+  CSG_CUDA(cudaMemsetAsync(queued, 0, sizeof(uint32_t), ctx.stream));
+  row_sums_kernel<<<static_cast<int>(grid), 256, 0, ctx.stream>>>(n, nnz, ptr, val, out, queued, queue);
   CSG_CUDA(cudaGetLastError());
-  count_launches(1);
+  row_pieces_kernel<<<ctx.num_sms, 256, 0, ctx.stream>>>(ptr, val, out, queued, queue);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(2);
   return true;
 }
 
