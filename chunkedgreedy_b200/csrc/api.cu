@@ -129,16 +129,18 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   const size_t o_payA = ar.take(4 * z), o_payB = ar.take(4 * z);
   const size_t o_cand = ar.take(8 * z), o_seg = ar.take(8 * z), o_rank = ar.take(4 * z);
   const size_t o_work = ar.take(4 * static_cast<size_t>(n));
+  const size_t o_rseg = ar.take(4 * static_cast<size_t>(n)), o_rcols = ar.take(4 * static_cast<size_t>(n));
   const size_t o_list = ar.take(4 * static_cast<size_t>(n));
   const size_t o_ctrl = ar.take(4 * CTRL_WORDS);
   // (the greedy stage may run with another chunk size than the sketch: chunk_greedy)
   size_t bw = transpose_only ? 0 : greedy_bitmap_words(n, p.chunk);
   if (greedy_chunk > 0 && greedy_bitmap_words(n, greedy_chunk) > bw) bw = greedy_bitmap_words(n, greedy_chunk);
   const size_t o_bm = ar.take(4 * (bw ? bw : 1));
-  // heavy chunks hold more than 15360 nonzeros each and are cut into tiles of 4096
+  // heavy chunks hold more than 10240 nonzeros or 2048 rows each and are cut into tiles of 4096
   const size_t chunks = (static_cast<size_t>(n) + p.chunk - 1) / p.chunk;
-  size_t heavy_max = z / 15360 + 1;
+  size_t heavy_max = p.chunk > 2048 ? chunks : z / 10240 + 1;
   if (heavy_max > chunks) heavy_max = chunks;
+  const size_t o_nc = ar.take(4 * chunks);
   const size_t tiles_max = z / 4096 + heavy_max + 1;
   const size_t o_hc = ar.take(4 * heavy_max), o_htb = ar.take(4 * (heavy_max + 1));
   const size_t o_th = ar.take(4 * 256 * tiles_max), o_db = ar.take(4 * 256 * heavy_max);
@@ -184,6 +186,9 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   s->seg = reinterpret_cast<int2 *>(ctx.ws + o_seg);
   s->seg_rank = reinterpret_cast<int32_t *>(ctx.ws + o_rank);
   s->row_work = reinterpret_cast<uint32_t *>(ctx.ws + o_work);
+  s->row_seg = reinterpret_cast<int32_t *>(ctx.ws + o_rseg);
+  s->row_cols = reinterpret_cast<int32_t *>(ctx.ws + o_rcols);
+  s->next_chunk = reinterpret_cast<int32_t *>(ctx.ws + o_nc);
   s->row_list = reinterpret_cast<int32_t *>(ctx.ws + o_list);
   s->ctrl = reinterpret_cast<uint32_t *>(ctx.ws + o_ctrl);
   s->table = user_table ? user_table : reinterpret_cast<uint64_t *>(ctx.ws + o_table);
@@ -270,7 +275,7 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
              const int32_t *d_ptr, const int32_t *d_ind,
              int32_t k, float ovs, int32_t chunk, int32_t *d_new_order, uint64_t *d_table,
              uint64_t table_capacity, sporder_csg_timing_t *timing, sporder_csg_stats_t *stats,
-             int32_t *k_used, bool symmetric = false) {
+             int32_t *k_used) {
   const auto wall0 = std::chrono::steady_clock::now();
   CsgParams p;
   if (!resolve_params(n, nnz, k, ovs, chunk, &p)) return false;
@@ -292,8 +297,6 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
               static_cast<unsigned long long>(table_capacity),
               static_cast<unsigned long long>(static_cast<uint64_t>(n) * p.k));
   CSG_CUDA(cudaSetDevice(ctx.device));
-  // (a row block of a larger matrix does not hold the rows its columns name: no shortcut there)
-  const bool sym_path = symmetric && row_base == 0 && n == ncols;
   // Large calls run one chunk ahead.  On power-law inputs the rows with the longest candidate
   // streams - the dependent chains that decide how long the call takes - sit in the chunk
   // with the most nonzeros, and all their chains need is that chunk's own transposition.  So
@@ -301,13 +304,14 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
   // there while the context's stream transposes everything else; the two meet before the
   // greedy stage.  Results do not depend on the split (the same kernels on the same rows).
   // By default for calls of 2^24 nonzeros in 64 chunks or more, whose chunk ahead must hold 2^17
-  // nonzeros: smaller calls do not pay for the second pipeline's fifteen launches.  A caller's
+  // nonzeros: smaller calls do not pay for the second pipeline's fifteen launches, and with larger
+  // sketches the chains of the two parts only slow each other (R-MAT scale 20, 128 slots: 43.5 ms ahead, 40.3 not).  A caller's
   // own threshold (sporder_context_set_ahead_threshold) applies to any call of two chunks.
   const int64_t chunks = (static_cast<int64_t>(n) + p.chunk - 1) / p.chunk;
-  bool ahead = !sym_path && ctx.side_stream != nullptr && p.chunk <= 4096;
+  bool ahead = ctx.side_stream != nullptr && p.chunk <= 4096;
   int32_t ahead_chunk_nnz = 1 << 17;
   if (ctx.ahead_min_nnz == 0) {
-    ahead = ahead && nnz >= AHEAD_MIN_NNZ && chunks >= 64;
+    ahead = ahead && nnz >= AHEAD_MIN_NNZ && chunks >= 64 && p.M <= 64;
   } else {
     ahead = ahead && ctx.ahead_min_nnz > 0 && nnz >= ctx.ahead_min_nnz && chunks >= 2;
     ahead_chunk_nnz = 0;
@@ -319,7 +323,7 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
 
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[0], st));
   if (!ahead) {
-    if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s, sym_path)) return false;
+    if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s)) return false;
     if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
     if (!launch_sketch(ctx, n, nnz, p, d_ptr, s, row_base, zero_table)) return false;
   } else {
@@ -330,10 +334,10 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
       CSG_CUDA(cudaEventRecord(ctx.ev[5], st));
       CSG_CUDA(cudaStreamWaitEvent(ctx.side_stream, ctx.ev[5], 0));
       // the chunk ahead: queued first, so that the host's launches of the rest do not delay it
-      if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, sp, false, PHASE_PRIO, s.ctrl)) return false;
+      if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, sp, PHASE_PRIO, s.ctrl)) return false;
       if (!launch_sketch(ctx, n, nnz, p, d_ptr, sp, row_base, false, PHASE_PRIO)) return false;
       CSG_CUDA(cudaEventRecord(ctx.ev[7], ctx.side_stream));
-      if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s, false, PHASE_REST, sp.ctrl)) return false;
+      if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s, PHASE_REST, sp.ctrl)) return false;
       if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
       CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[8], 0));
       if (!launch_sketch(ctx, n, nnz, p, d_ptr, s, row_base, false, PHASE_REST)) return false;
@@ -397,8 +401,7 @@ __global__ void __launch_bounds__(256) unpack_table_kernel(size_t count, const u
 // other defaults (k = min(32, max(16, 2 nnz / n)), oversampling 2), results unpacked.
 bool run_similarity_graph(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr, const int32_t *d_ind,
                           int32_t k, float ovs, int32_t *d_indices, float *d_weights,
-                          sporder_sim_timing_t *timing, sporder_sim_stats_t *stats, int32_t *k_used,
-                          bool symmetric = false) {
+                          sporder_sim_timing_t *timing, sporder_sim_stats_t *stats, int32_t *k_used) {
   const auto wall0 = std::chrono::steady_clock::now();
   CSG_REQUIRE(n >= 1, "n must be >= 1 (got %d)", n);
   CSG_REQUIRE(nnz >= 0, "nnz must be >= 0 (got %d)", nnz);
@@ -424,7 +427,7 @@ bool run_similarity_graph(Context &ctx, int32_t n, int32_t nnz, const int32_t *d
   if (!plan_scratch(ctx, n, nnz, p, nullptr, &s)) return false;
   cudaStream_t st = ctx.stream;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[0], st));
-  if (!launch_transpose(ctx, n, n, nnz, p.chunk, d_ptr, d_ind, s, symmetric)) return false;
+  if (!launch_transpose(ctx, n, n, nnz, p.chunk, d_ptr, d_ind, s)) return false;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
   if (!launch_sketch(ctx, n, nnz, p, d_ptr, s, 0, true)) return false;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[2], st));
@@ -463,7 +466,7 @@ bool run_similarity_graph(Context &ctx, int32_t n, int32_t nnz, const int32_t *d
 // chunks of chunk_size rows, candidates outside the chunk skipped.
 bool run_chunk_greedy(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr, const int32_t *d_ind,
                       int32_t k, float ovs, int32_t chunk, int32_t *d_new_order,
-                      sporder_cg_timing_t *timing, sporder_cg_stats_t *stats, bool symmetric = false) {
+                      sporder_cg_timing_t *timing, sporder_cg_stats_t *stats) {
   const auto wall0 = std::chrono::steady_clock::now();
   CsgParams pg;  // greedy: the caller's chunk; also resolves k and oversampling
   if (!resolve_params(n, nnz, k, ovs, chunk, &pg)) return false;
@@ -482,7 +485,7 @@ bool run_chunk_greedy(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr
   if (!plan_scratch(ctx, n, nnz, ps, nullptr, &s, pg.chunk)) return false;
   cudaStream_t st = ctx.stream;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[0], st));
-  if (!launch_transpose(ctx, n, n, nnz, ps.chunk, d_ptr, d_ind, s, symmetric)) return false;
+  if (!launch_transpose(ctx, n, n, nnz, ps.chunk, d_ptr, d_ind, s)) return false;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
   if (!launch_sketch(ctx, n, nnz, ps, d_ptr, s, 0, stats != nullptr)) return false;
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[2], st));
@@ -547,12 +550,11 @@ bool run_count_pillars(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_pt
     if (!resolve_params(n, nnz, 1, 1.0f, height, &p)) return false;  // k = 1: smallest table the layout allows
     CsgScratch s;
     if (!plan_scratch(ctx, n, nnz, p, nullptr, &s, 0, true)) return false;
-    if (!launch_transpose(ctx, n, n, nnz, p.chunk, d_ptr, d_ind, s)) return false;
-    // the counter takes the place of the (now unused) sort buffer; the transpose set the flag word
-    d_count = reinterpret_cast<unsigned long long *>(s.keyA);
+    // the counter takes the place of the (here unused) candidates
+    d_count = reinterpret_cast<unsigned long long *>(s.cand);
     d_bad = s.ctrl + CTRL_BAD_INPUT;
     CSG_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), ctx.stream));
-    if (!launch_pillars_groups(ctx, nnz, s.seg_rank, d_count)) return false;
+    if (!launch_transpose(ctx, n, n, nnz, p.chunk, d_ptr, d_ind, s, PHASE_ALL, nullptr, d_count)) return false;
   }
   unsigned long long *h = reinterpret_cast<unsigned long long *>(ctx.h_pinned + 16);
   CSG_CUDA(cudaMemcpyAsync(h, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx.stream));
@@ -657,7 +659,7 @@ void sporder_chunk_similarity_greedy(sporder_context_t ctx, int32_t n, int32_t n
     return;
   }
   csg::run_csg(ctx->c, n, n, 0, nnz, d_ptr, d_ind, k, oversampling, chunk_size, d_new_order, nullptr, 0,
-               timing, stats, nullptr, is_symmetric);
+               timing, stats, nullptr);
 }
 
 int32_t sporder_csg_with_table(sporder_context_t ctx, int32_t n, int32_t nnz, const int32_t *d_ptr,
@@ -672,7 +674,7 @@ int32_t sporder_csg_with_table(sporder_context_t ctx, int32_t n, int32_t nnz, co
   }
   int32_t k_used = -1;
   if (!csg::run_csg(ctx->c, n, n, 0, nnz, d_ptr, d_ind, k, oversampling, chunk_size, d_new_order, d_table,
-                    d_table_capacity, timing, stats, &k_used, is_symmetric))
+                    d_table_capacity, timing, stats, &k_used))
     return -1;
   return k_used;
 }
@@ -731,7 +733,7 @@ int32_t sporder_chunk_similarity_greedy_host(sporder_context_t ctx, int32_t n, i
       CSG_CUDA(cudaMemcpyAsync(d_ind, h_ind, sizeof(int32_t) * static_cast<size_t>(nnz),
                                cudaMemcpyHostToDevice, c.stream));
     const bool ok = csg::run_csg(c, n, n, 0, nnz, d_ptr, d_ind, k, oversampling, chunk_size, d_order,
-                                 nullptr, 0, timing, stats, nullptr, is_symmetric);
+                                 nullptr, 0, timing, stats, nullptr);
     if (ok)
       CSG_CUDA(cudaMemcpyAsync(h_new_order, d_order, sizeof(int32_t) * static_cast<size_t>(n),
                                cudaMemcpyDeviceToHost, c.stream));
@@ -751,7 +753,7 @@ void sporder_chunk_greedy(sporder_context_t ctx, int32_t n, int32_t nnz, const i
     return;
   }
   csg::run_chunk_greedy(ctx->c, n, nnz, d_ptr, d_ind, k, oversampling, chunk_size, d_new_order, timing,
-                        stats, is_symmetric);
+                        stats);
 }
 
 int32_t sporder_similarity_graph(sporder_context_t ctx, int32_t n, int32_t nnz, const int32_t *d_ptr,
@@ -765,7 +767,7 @@ int32_t sporder_similarity_graph(sporder_context_t ctx, int32_t n, int32_t nnz, 
   }
   int32_t k_used = -1;
   if (!csg::run_similarity_graph(ctx->c, n, nnz, d_ptr, d_ind, k, oversampling, d_indices, d_weights,
-                                 timing, stats, &k_used, is_symmetric))
+                                 timing, stats, &k_used))
     return -1;
   return k_used;
 }

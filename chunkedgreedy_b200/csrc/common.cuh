@@ -95,8 +95,9 @@ struct CsgScratch {
   // chunk-local transpose (see transpose.cu)
   uint32_t *keyA, *keyB, *payA, *payB;  // ping-pong buffers of the global sort path
   int2 *cand;                           // (row, row length) grouped by (chunk, column), rows ascending
-  int2 *seg;                            // per nonzero: (first index into cand, group length)
-  int32_t *seg_rank;                    // per nonzero: index of its own row inside that group
+  int2 *seg;                            // per row and shared column: (first index into cand, group length)
+  int32_t *seg_rank;                    // ... and the place of the row itself inside that group
+  int32_t *row_seg, *row_cols;          // per row: its first entry of seg, and how many
   uint32_t *row_work;                   // candidates each row will see
   // work list of rows with candidates, heaviest bucket first
   int32_t *row_list;
@@ -109,8 +110,9 @@ struct CsgScratch {
   int32_t *heavy_state;
   uint32_t stream_cap, heavy_max;
   uint32_t *part_base, *part_off;
-  // tiled sort of heavy chunks (see transpose.cu)
-  int32_t *heavy_chunk, *heavy_tile_base;
+  bool no_heavy_rows = false;  // known on the host already: nothing for the chain kernel
+  // compact_kernel's second list, tiled sort of heavy chunks (see transpose.cu)
+  int32_t *next_chunk, *heavy_chunk, *heavy_tile_base;
   uint32_t *tile_hist, *digit_base;
 };
 enum {
@@ -128,6 +130,8 @@ enum {
   CTRL_CHECK = 13,         // checked build: site of the first index out of bounds, then the index (64-bit)
   CTRL_MID_END = 16,       // end of the rows of heavy weight in row_list (those past CTRL_HEAVY_ROWS did not fit)
   CTRL_LANE_TICKET = 17,   // next row for the kernel that runs a row per lane
+  CTRL_NEXT_COUNT = 18,    // chunks compact_kernel's small form left to the large one, and that one's ticket
+  CTRL_NEXT_TICKET = 19,
   CTRL_PRIO = 50,          // chunk whose heavy rows run ahead of the rest (PRIO_NONE: no such chunk)
   CTRL_PRIO_WORK = 51,     // shortest candidate stream among the rows the chunk ahead lists
   CTRL_STATS = 56,         // see greedy.cu (8-byte aligned)
@@ -158,8 +162,8 @@ constexpr uint32_t CHAIN_WORK_MIN = 64;
 
 // stage launchers; all enqueue on ctx.stream and return false after set_error()
 bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
-                      const int32_t *d_ind, CsgScratch &s, bool symmetric = false, int phase = PHASE_ALL,
-                      uint32_t *ctrl_other = nullptr);
+                      const int32_t *d_ind, CsgScratch &s, int phase = PHASE_ALL, uint32_t *ctrl_other = nullptr,
+                      unsigned long long *d_count = nullptr);
 // start of a call that runs one chunk ahead: clears the counters of both parts and names the chunk
 bool launch_priority_pick(Context &ctx, int32_t n, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
                           CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz);
@@ -169,7 +173,6 @@ bool launch_greedy(Context &ctx, int32_t n, const CsgParams &p, CsgScratch &s,
                    int32_t *d_new_order, bool with_stats, int32_t row_base);
 bool launch_pillars_search(Context &ctx, int32_t n, int32_t nnz, int32_t height, const int32_t *d_ptr,
                            const int32_t *d_ind, unsigned long long *d_count, uint32_t *d_bad);
-bool launch_pillars_groups(Context &ctx, int32_t nnz, const int32_t *seg_rank, unsigned long long *d_count);
 bool launch_in_chunk_weight(Context &ctx, int32_t n, int32_t k, int32_t chunk, const uint64_t *table,
                             uint32_t *ctrl);
 bool launch_table_stats(Context &ctx, int32_t n, int32_t k, const uint64_t *table, uint32_t *ctrl);

@@ -56,18 +56,6 @@ __global__ void __launch_bounds__(256) pillars_search_kernel(int32_t n, int32_t 
   if (lane == 0 && mine) atomicAdd(count, mine);
 }
 
-// column groups of the chunk-local transpose = nonzeros that come first in their group
-__global__ void __launch_bounds__(256) pillars_groups_kernel(int32_t nnz, const int32_t *__restrict__ seg_rank,
-                                                             unsigned long long *count) {
-  const int lane = threadIdx.x & 31;
-  unsigned long long mine = 0;
-  for (int32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += gridDim.x * blockDim.x)
-    mine += seg_rank[p] == 0 ? 1u : 0u;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mine += __shfl_down_sync(FULL, mine, off);
-  if (lane == 0 && mine) atomicAdd(count, mine);
-}
-
 }  // namespace
 
 bool launch_pillars_search(Context &ctx, int32_t n, int32_t nnz, int32_t height, const int32_t *d_ptr,
@@ -75,15 +63,6 @@ bool launch_pillars_search(Context &ctx, int32_t n, int32_t nnz, int32_t height,
   int grid = (n + 7) / 8;
   if (grid > ctx.num_sms * 16) grid = ctx.num_sms * 16;
   pillars_search_kernel<<<grid, 256, 0, ctx.stream>>>(n, nnz, height, d_ptr, d_ind, d_count, d_bad);
-  CSG_CUDA(cudaGetLastError());
-  count_launches(1);
-  return true;
-}
-
-bool launch_pillars_groups(Context &ctx, int32_t nnz, const int32_t *seg_rank, unsigned long long *d_count) {
-  int grid = (nnz + 255) / 256;
-  if (grid > ctx.num_sms * 16) grid = ctx.num_sms * 16;
-  pillars_groups_kernel<<<grid, 256, 0, ctx.stream>>>(nnz, seg_rank, d_count);
   CSG_CUDA(cudaGetLastError());
   count_launches(1);
   return true;

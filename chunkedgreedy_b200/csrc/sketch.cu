@@ -49,7 +49,7 @@ struct SketchArgs {
   int32_t n, nnz, k, row_base, chunk;
   const int32_t *ptr;
   const int2 *seg;
-  const int32_t *seg_rank;
+  const int32_t *seg_rank, *row_seg, *row_cols;
   const int2 *cand;
   const int32_t *row_list;
   const uint32_t *row_work;
@@ -486,7 +486,7 @@ __device__ __forceinline__ void rows_by_warp(const SketchArgs &a, uint32_t end, 
     const int32_t rb = a.ptr[r], re = a.ptr[r + 1];
     if (!row_bounds_ok(a, rb, re)) continue;
     sk.clear();
-    prod.begin(r, rb, re, re - rb);
+    prod.begin(r, a.row_seg[r], a.row_seg[r] + a.row_cols[r], re - rb);
     for (;;) {
       const int cnt = prod.produce(bs, ba);
       if (cnt == 0) break;
@@ -769,6 +769,10 @@ __device__ __forceinline__ LaneRow lane_row(const SketchArgs &a, uint32_t item, 
       w.p = w.re = 0;
     }
     w.rs = w.re - w.p;
+    if (w.r >= 0) {
+      w.p = a.row_seg[w.r];
+      w.re = w.p + a.row_cols[w.r];
+    }
     w.cbase = (w.r / a.chunk) * a.chunk;
   }
   return w;
@@ -1051,7 +1055,7 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
     if (i < H) {
       const int32_t r = a.row_list[i];
       v = a.row_work[r];
-      np = static_cast<uint32_t>((a.ptr[r + 1] - a.ptr[r] + H_PART - 1) / H_PART);
+      np = static_cast<uint32_t>((a.row_cols[r] + H_PART - 1) / H_PART);
       if (v < HEAVY_WORK) lighter += v;
     }
     // parts first (same scan, second value packed in the high half of 64 bits)
@@ -1119,14 +1123,10 @@ __device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, 
   PartRef p;
   p.item = lo;
   p.r = a.row_list[lo];
-  const int32_t rb = a.ptr[p.r], re = a.ptr[p.r + 1];
-  p.row_size = re - rb;
+  const int32_t rb = a.row_seg[p.r], re = rb + a.row_cols[p.r];
+  p.row_size = a.ptr[p.r + 1] - a.ptr[p.r];
   p.pb = rb + static_cast<int32_t>(part - a.part_base[lo]) * H_PART;
   p.pe = p.pb + H_PART < re ? p.pb + H_PART : re;
-  if (rb < 0 || re < rb || re > a.nnz) {  // malformed row pointers: nothing to do
-    atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
-    p.pe = p.pb;
-  }
   return p;
 }
 
@@ -1879,47 +1879,49 @@ __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
 }
 
 template <int CELLS>
-bool launch_cells(Context &ctx, const SketchArgs &a, int phase) {
+bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_rows) {
   // A call that runs one chunk ahead has two of these sequences in flight: the chunk ahead on
   // the side stream with a quarter of the SMs for its chains, the rest on the context's stream
   // with the other three quarters (a chain block takes a whole SM, and the kernel of the other
   // rows starts only when every chain block has one).
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
-  heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  heavy_part_scan_kernel<<<1, 1024, 0, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  heavy_expand_kernel<<<ctx.num_sms * 8, S_THREADS, 0, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  // (the rest of the call starts its own chains only behind this point: by then the chains
-  // ahead, next in their stream, hold their SMs, and the kernel of the other rows cannot
-  // settle on them first)
-  if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
-  // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a block per row.
   constexpr bool in_rounds = CELLS <= ROUND_CELLS;
-  if constexpr (in_rounds) {
-    const int64_t span = a.chunk < a.n ? a.chunk : a.n;
-    const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
-    // (groups per block: as many as their tables leave room for)
-    const int group_bytes = GroupMemory<CELLS>::TAB + tab_bytes;
-    const int room = ctx.smem_optin - 1024;
-    int groups = Helpers<CELLS>::ROWS;
-    while (groups > 1 && groups * group_bytes > room) --groups;
-    CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
-    // (all of an SM's memory as shared: a block of another split cannot move in beside this one)
-    CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  cudaSharedmemCarveoutMaxShared));
-    heavy_rounds_kernel<CELLS><<<ctx.num_sms, Helpers<CELLS>::THREADS * groups, groups * group_bytes, st>>>(a, tab_bytes);
+  if (!no_heavy_rows) {
+    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
-  }
-  if constexpr (!in_rounds) {
-    const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
-    CSG_CUDA(cudaFuncSetAttribute(heavy_consume_kernel<CELLS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
-    heavy_consume_kernel<CELLS><<<phase == PHASE_PRIO ? prio_chain_blocks(ctx.num_sms) : phase == PHASE_REST ? ctx.num_sms - prio_chain_blocks(ctx.num_sms) : ctx.num_sms, S_THREADS, pad, st>>>(a);
+    heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
+    heavy_part_scan_kernel<<<1, 1024, 0, st>>>(a);
+    CSG_CUDA(cudaGetLastError());
+    heavy_expand_kernel<<<ctx.num_sms * 8, S_THREADS, 0, st>>>(a);
+    CSG_CUDA(cudaGetLastError());
+    // (the rest of the call starts its own chains only behind this point: by then the chains
+    // ahead, next in their stream, hold their SMs, and the kernel of the other rows cannot
+    // settle on them first)
+    if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
+    // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a group of warps per row.
+    if constexpr (in_rounds) {
+      const int64_t span = a.chunk < a.n ? a.chunk : a.n;
+      const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
+      // (groups per block: as many as their tables leave room for)
+      const int group_bytes = GroupMemory<CELLS>::TAB + tab_bytes;
+      const int room = ctx.smem_optin - 1024;
+      int groups = Helpers<CELLS>::ROWS;
+      while (groups > 1 && groups * group_bytes > room) --groups;
+      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+      // (all of an SM's memory as shared: a block of another split cannot move in beside this one)
+      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    cudaSharedmemCarveoutMaxShared));
+      heavy_rounds_kernel<CELLS><<<ctx.num_sms, Helpers<CELLS>::THREADS * groups, groups * group_bytes, st>>>(a, tab_bytes);
+      CSG_CUDA(cudaGetLastError());
+    }
+    if constexpr (!in_rounds) {
+      const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
+      CSG_CUDA(cudaFuncSetAttribute(heavy_consume_kernel<CELLS>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
+      heavy_consume_kernel<CELLS><<<phase == PHASE_PRIO ? prio_chain_blocks(ctx.num_sms) : phase == PHASE_REST ? ctx.num_sms - prio_chain_blocks(ctx.num_sms) : ctx.num_sms, S_THREADS, pad, st>>>(a);
+      CSG_CUDA(cudaGetLastError());
+    }
   }
   // The other rows run beside the heavy chains: their kernel follows in the same stream
   // as a programmatic dependent launch, so its blocks are placed only after every block
@@ -1950,12 +1952,12 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase) {
   // idle blocks would otherwise sit on the SMs until the chains end.
   const int64_t span = a.chunk < a.n ? a.chunk : a.n;
   if (phase == PHASE_PRIO || CELLS > LANE_CELLS || span > (1 << 24)) {
-    if (!launch_light(sketch_kernel<CELLS>, S_THREADS, 0, phase != PHASE_PRIO, phase == PHASE_PRIO ? 0 : 1,
+    if (!launch_light(sketch_kernel<CELLS>, S_THREADS, 0, phase != PHASE_PRIO && !no_heavy_rows, phase == PHASE_PRIO ? 0 : 1,
                       phase == PHASE_PRIO ? 0 : 1))
       return false;
   } else if constexpr (CELLS <= LANE_CELLS) {
     auto lanes = [&](auto kernel, int index_words) {
-      return launch_light(kernel, 32 * L_WARPS, (LaneLayout<CELLS>::I_OFF + index_words) * 4, true);
+      return launch_light(kernel, 32 * L_WARPS, (LaneLayout<CELLS>::I_OFF + index_words) * 4, !no_heavy_rows);
     };
     if (span <= L_TABLE_MAX) {
       if (!lanes(rows_in_lanes_kernel<CELLS, TableIndex<CELLS>>, TableIndex<CELLS>::words(span))) return false;
@@ -1963,9 +1965,11 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase) {
       return false;
     }
   }
+  count_launches(1);
+  if (no_heavy_rows) return true;
   heavy_topk_kernel<CELLS><<<ctx.num_sms, S_THREADS, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
-  count_launches(7);
+  count_launches(6);
   return true;
 }
 
@@ -1982,6 +1986,8 @@ bool launch_sketch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, con
   a.ptr = d_ptr;
   a.seg = s.seg;
   a.seg_rank = s.seg_rank;
+  a.row_seg = s.row_seg;
+  a.row_cols = s.row_cols;
   a.cand = s.cand;
   a.row_list = s.row_list;
   a.row_work = s.row_work;
@@ -2002,7 +2008,7 @@ bool launch_sketch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, con
   switch (p.M / 32) {
 #define CSG_CASE(C) \
   case C:           \
-    return launch_cells<C>(ctx, a, phase);
+    return launch_cells<C>(ctx, a, phase, s.no_heavy_rows);
     CSG_CASE(1) CSG_CASE(2) CSG_CASE(3) CSG_CASE(4) CSG_CASE(5) CSG_CASE(6) CSG_CASE(7) CSG_CASE(8)
     CSG_CASE(9) CSG_CASE(10) CSG_CASE(11) CSG_CASE(12) CSG_CASE(13) CSG_CASE(14) CSG_CASE(15)
     CSG_CASE(16)

@@ -4,27 +4,23 @@
 // (sporder/src/common/csr2csc.cu:38-115) and then, per row, scans whole column
 // lists to pick out the rows of the row's own chunk
 // (sporder/src/common/chunk_similarity_top_k.cu:52-84).  Candidates never leave
-// the chunk, so this library transposes every chunk on its own: the chunk's
-// (column, position) pairs are sorted by column with a stable LSD radix sort,
-// column groups are found, and the kernels emit
-//   cand[]  : the chunk's rows grouped by column, rows ascending inside a group,
-//             each with its row length (what the Dice term needs);
-//   seg[p]  : for nonzero p (CSR order) the group of its column: (first, length),
-//             and seg_rank[p], the place of p's own row inside that group;
-//   row_work: per row, how many candidates its stream will hold.
-// Chunks of up to T_LS nonzeros are handled start to finish by one thread block in
-// shared memory (one read of the CSR slice, no intermediate traffic).  Heavier
-// chunks - on power-law inputs a handful of chunks hold millions of nonzeros, and
-// the rows with the longest streams live in exactly those - are cut into tiles and
-// sorted by the whole grid: per pass a tile histogram, a per-chunk scan and a
-// stable tile scatter, then a group search per element.
-// A caller-promised symmetric pattern needs no sort at all: column c's rows inside a chunk
-// are the entries of ROW c that fall into the chunk's row range, already ascending, so the
-// CSR arrays themselves serve as cand[] (with the row lengths looked up) and a group is a
-// sub-range of row c found by binary search (symmetric_groups_kernel).  The reference takes
-// the same promise and reads the aliased CSR arrays as the CSC
-// (sporder/src/common/csr2csc.h:52-54); like there, a false promise gives a different
-// (still valid) permutation, never an out-of-range access.
+// the chunk, so this library transposes every chunk on its own, and only the part of it
+// that matters: a column that a single row of the chunk holds brings no candidate.  The
+// kernels emit, with "group" for the rows of a chunk that share a column,
+//   cand[]  : the rows of every group, ascending, each with its row length (what the Dice term
+//             needs);
+//   seg[]   : per row, one after the other and columns ascending, its groups: (first, length);
+//             and seg_rank[], the place of the row itself inside the group;
+//   row_seg, row_cols: where a row's groups are in seg[], and how many;
+//   row_work: how many candidates the row's stream will hold.
+// Chunks of up to C_NNZ nonzeros in which few enough of them lie in groups are handled start
+// to finish by one thread block, without a sort (compact_kernel).  Heavier chunks - on power-law
+// inputs a handful of chunks hold millions of nonzeros, and the rows with the longest streams
+// live in exactly those - are cut into tiles and sorted by the whole grid: per pass a tile
+// histogram, a per-chunk scan and a stable tile scatter, then a group search per element (there
+// every column of a row gets an entry of seg[]).
+// The reference can be promised a symmetric pattern and then reads the CSR arrays as the CSC
+// (sporder/src/common/csr2csc.h:52-54); nothing here needs the promise.
 #include "common.cuh"
 
 namespace csg {
@@ -35,18 +31,20 @@ constexpr int T_THREADS = 512;
 constexpr int T_WARPS = T_THREADS / 32;
 constexpr int T_IPT = 8;
 constexpr int T_TILE = T_THREADS * T_IPT;  // 4096
-constexpr int T_LS = 15360;                // largest chunk (nonzeros) sorted in shared memory
-constexpr int T_RP = 2048;                 // largest chunk (rows) with row tables in shared memory
+constexpr int C_NNZ = 65536;               // largest chunk (nonzeros) that compact_kernel looks at ...
+constexpr int C_ROWS = 2048;               // ... and its rows
 
 struct TransposeArgs {
   int32_t n, nnz, chunk, num_chunks, passes;
   const int32_t *ptr, *ind;
   uint32_t *keyA, *keyB, *payA, *payB;
   int2 *cand, *seg;
-  int32_t *seg_rank;
+  int32_t *seg_rank, *row_seg, *row_cols;
   uint32_t *row_work;
   uint32_t *ctrl;
-  // heavy chunks (more than T_LS nonzeros)
+  unsigned long long *count;  // only count the groups, rows alone in a column included (nullptr: transpose)
+  int32_t *next_chunk;        // chunks compact_kernel's small form passed on to the large one
+  // heavy chunks (those that compact_kernel passes on)
   int32_t *heavy_chunk;      // chunk ids, in arrival order
   int32_t *heavy_tile_base;  // first tile of each heavy chunk, plus the total
   uint32_t *tile_hist;       // [tile][256] digit counts, then offsets
@@ -76,106 +74,6 @@ __device__ __forceinline__ ChunkSpan chunk_span(const TransposeArgs &a, int32_t 
   return c;
 }
 
-struct Shared {
-  uint32_t wc[T_WARPS * 256];
-  uint32_t hist[256];
-  uint32_t binbase[256];
-  int32_t warp_last[T_WARPS];
-  int32_t carry;
-  int32_t ticket;
-  int32_t sptr[T_RP + 1];
-  uint32_t row_work[T_RP];
-  uint32_t skey[2][T_LS];
-  uint16_t spay[2][T_LS];
-};
-
-// One stable counting pass on an 8-bit digit.  FIRST reads the keys from the CSR
-// column array and uses the position as payload.
-template <typename PayT, bool FIRST>
-__device__ void radix_pass(const uint32_t *kin, const PayT *pin, uint32_t *kout, PayT *pout,
-                           int L, int shift, Shared &sh, uint32_t *ctrl) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 256) sh.hist[tid] = 0;
-  __syncthreads();
-  for (int i = tid; i < L; i += T_THREADS) atomicAdd(&sh.hist[(kin[i] >> shift) & 255u], 1u);
-  __syncthreads();
-  if (warp == 0) {  // exclusive scan of 256 bins, 8 per lane
-    uint32_t v[8], s = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[j] = sh.hist[lane * 8 + j];
-      s += v[j];
-    }
-    uint32_t incl = s;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      uint32_t t = __shfl_up_sync(FULL, incl, off);
-      if (lane >= off) incl += t;
-    }
-    uint32_t run = incl - s;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      sh.binbase[lane * 8 + j] = run;
-      run += v[j];
-    }
-  }
-  __syncthreads();
-
-  for (int tb = 0; tb < L; tb += T_TILE) {
-    for (int j = tid; j < T_WARPS * 256; j += T_THREADS) sh.wc[j] = 0;
-    __syncthreads();
-    uint32_t key[T_IPT], rk[T_IPT];
-    PayT pay[T_IPT];
-    const int wbase = tb + warp * (32 * T_IPT);
-#pragma unroll
-    for (int i = 0; i < T_IPT; ++i) {
-      const int idx = wbase + i * 32 + lane;
-      const bool valid = idx < L;
-      key[i] = valid ? kin[idx] : 0u;
-      if (FIRST)
-        pay[i] = static_cast<PayT>(idx);
-      else
-        pay[i] = valid ? pin[idx] : PayT(0);
-      const uint32_t d = valid ? ((key[i] >> shift) & 255u) : 256u;
-      const unsigned peers = match_digit(d);
-      const int leader = __ffs(peers) - 1;
-      uint32_t pre = 0;
-      if (lane == leader && valid) {
-        pre = sh.wc[warp * 256 + d];
-        sh.wc[warp * 256 + d] = pre + __popc(peers);
-      }
-      pre = __shfl_sync(FULL, pre, leader);
-      rk[i] = pre + __popc(peers & ((1u << lane) - 1u));
-      __syncwarp();
-    }
-    __syncthreads();
-    if (tid < 256) {  // per digit: running offsets over the warps, carried over tiles
-      uint32_t run = sh.binbase[tid];
-#pragma unroll
-      for (int w = 0; w < T_WARPS; ++w) {
-        const uint32_t t = sh.wc[w * 256 + tid];
-        sh.wc[w * 256 + tid] = run;
-        run += t;
-      }
-      sh.binbase[tid] = run;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < T_IPT; ++i) {
-      const int idx = wbase + i * 32 + lane;
-      if (idx < L) {
-        const uint32_t d = (key[i] >> shift) & 255u;
-        const uint32_t dst = sh.wc[warp * 256 + d] + rk[i];
-        if (index_ok(ctrl, CHK_SORT, dst, L)) {
-          kout[dst] = key[i];
-          pout[dst] = pay[i];
-        }
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // Row that owns CSR position x: largest row with ptr[row] <= x, searched in
 // [row_lo, row_hi] over either the shared copy of the chunk's row pointers or the
 // global array.
@@ -191,130 +89,252 @@ __device__ __forceinline__ int32_t row_of(const int32_t *p, int32_t lo, int32_t 
   return lo;
 }
 
-// After the sort: K = sorted columns, P = positions (chunk-local).  S / LN are the
-// free ping-pong buffers, reused for the group start of every element and the
-// group length stored at the group's first element.
-template <typename PayT>
-__device__ void emit_groups(const uint32_t *K, const PayT *P, uint32_t *S, PayT *LN, int L,
-                            int32_t b, int32_t cs, int32_t rows, bool rows_in_smem,
-                            const TransposeArgs &a, Shared &sh) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) sh.carry = 0;
+// One block per chunk, no sort:
+//  1. every column sets a bit of a hashed bit map, and a second time a bit of another map: what
+//     has not set the second bit is alone in its column (most nonzeros of a mesh or a road);
+//  2. the others are numbered in CSR order and entered into a hash table, which counts each
+//     column's rows;
+//  3. the table's counts of two and more become places in cand[];
+//  4. every member writes its row to its group, in any order, and then counts the smaller rows
+//     of the group: its place.  (That is one comparison per candidate the sketch stage will have to
+//     work through, so it never dominates.)
+//  5. members go out with their groups in CSR order, which is the order seg[] wants.
+// Two sizes: blocks of 512 threads, two to an SM, for up to 4096 numbered nonzeros; chunks with
+// more go on to blocks of 1024 threads for up to 10,240, those with more again to the tiled sort.
+// On a B200, 1.05 M rows of the shuffled mesh: 227 us with the groups read off the promised
+// symmetry, 170 without any promise; 65,536 rows of the power-law band: 173 -> 87 us.
+template <int THREADS_, int CAP_, int TABLE_BITS_, int FILTER_BITS_>
+struct CompactSize {
+  static constexpr int THREADS = THREADS_, WARPS = THREADS / 32, CAP = CAP_, TABLE_BITS = TABLE_BITS_, FILTER_BITS = FILTER_BITS_;
+  static constexpr int TABLE = 1 << TABLE_BITS, FILTER = (1 << FILTER_BITS) / 32;  // entries; words of each map
+  struct Shared {
+    uint32_t key[TABLE];          // columns, then how many members wrote their row
+    uint32_t cnt[TABLE];          // rows per column, then (place << 12) | rows, 0 for a column with one
+    union {
+      uint32_t filter[2][FILTER];
+      uint16_t member[CAP];       // rows of the groups
+    };
+    uint16_t slot[CAP];           // table entry of each numbered nonzero
+    uint16_t row[CAP];            // its position, then its row
+    int32_t sptr[C_ROWS + 1];
+    uint32_t work[C_ROWS];
+    uint32_t cols[C_ROWS / 2];    // 16 bits a row
+    int32_t warp_sum[32];
+    int32_t ticket;
+  };
+};
+using CompactSmall = CompactSize<512, 4096, 13, 16>;
+using CompactLarge = CompactSize<1024, 10240, 14, 17>;
+
+// exclusive sum over the block's threads; *total is the sum of all
+template <int WARPS>
+__device__ __forceinline__ int32_t block_sum(int32_t v, int32_t *warp_sum, int32_t *total) {
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  int32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t t = __shfl_up_sync(FULL, incl, off);
+    if (lane >= off) incl += t;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
-  for (int tb = 0; tb < L; tb += T_TILE) {
-    const int wbase = tb + warp * (32 * T_IPT);
-    int32_t last = -1;
-    int32_t st[T_IPT];
-    uint32_t key[T_IPT];
+  const int32_t w = lane < WARPS ? warp_sum[lane] : 0;
+  int32_t wi = w;
 #pragma unroll
-    for (int i = 0; i < T_IPT; ++i) {
-      const int idx = wbase + i * 32 + lane;
-      const bool valid = idx < L;
-      key[i] = valid ? K[idx] : 0u;
-      const uint32_t prev = (valid && idx > 0) ? K[idx - 1] : 0u;
-      const bool head = valid && (idx == 0 || key[i] != prev);
-      const unsigned hm = __ballot_sync(FULL, head);
-      const unsigned le = hm & (FULL >> (31 - lane));
-      st[i] = le ? (wbase + i * 32 + (31 - __clz(le))) : last;
-      if (hm) last = wbase + i * 32 + (31 - __clz(hm));
-    }
-    if (lane == 0) sh.warp_last[warp] = last;
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t t = __shfl_up_sync(FULL, wi, off);
+    if (lane >= off) wi += t;
+  }
+  *total = __shfl_sync(FULL, wi, 31);
+  const int32_t base = __shfl_sync(FULL, wi - w, warp);
+  __syncthreads();
+  return base + incl - v;
+}
+
+__device__ __forceinline__ uint32_t column_hash(uint32_t c) { return c * 0x9E3779B1u; }
+
+// LARGE: the chunks that the small form left (ctrl[CTRL_NEXT_COUNT] of them); what does not fit
+// goes to the tiled sort.
+template <typename S, bool LARGE>
+__global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typename S::Shared &sh = *reinterpret_cast<typename S::Shared *>(smem_raw);
+  constexpr int THREADS = S::THREADS, U = 4;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (;;) {
     __syncthreads();
-    int32_t carry = sh.carry;
-    for (int w = 0; w < warp; ++w) {
-      const int32_t t = sh.warp_last[w];
-      if (t >= 0) carry = t;
+    if (tid == 0) sh.ticket = static_cast<int32_t>(atomicAdd(&a.ctrl[LARGE ? CTRL_NEXT_TICKET : CTRL_CHUNK_TICKET], 1u));
+    __syncthreads();
+    if (sh.ticket >= (LARGE ? static_cast<int32_t>(a.ctrl[CTRL_NEXT_COUNT]) : a.num_chunks)) break;
+    const int32_t q = LARGE ? a.next_chunk[sh.ticket] : sh.ticket;
+    if (a.skip_prio && static_cast<uint32_t>(q) == a.ctrl_main[CTRL_PRIO]) continue;
+    const ChunkSpan c = chunk_span(a, q);
+    const int32_t b = c.b, rows = c.rows;
+    const int L = c.L;
+    if (L > C_NNZ || rows > C_ROWS) {
+      if (tid == 0) a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
+      continue;
     }
+    bool ordered = true;
+    for (int i = tid; i < rows; i += THREADS) {
+      const int32_t x = a.ptr[c.cs + i], y = a.ptr[c.cs + i + 1];
+      sh.sptr[i] = x;
+      if (i == rows - 1) sh.sptr[rows] = y;
+      ordered &= x <= y;
+      sh.work[i] = 0;
+      if (i < C_ROWS / 2) sh.cols[i] = 0;
+    }
+    if (!ordered) atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
+    for (int i = tid * 4; i < S::TABLE; i += THREADS * 4) {
+      *reinterpret_cast<uint4 *>(sh.key + i) = make_uint4(FULL, FULL, FULL, FULL);
+      *reinterpret_cast<uint4 *>(sh.cnt + i) = make_uint4(0, 0, 0, 0);
+    }
+    for (int i = tid * 4; i < 2 * S::FILTER; i += THREADS * 4)
+      *reinterpret_cast<uint4 *>(&sh.filter[0][0] + i) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const uint32_t *const ind = reinterpret_cast<const uint32_t *>(a.ind + b);
+    for (int i0 = tid; i0 < L; i0 += THREADS * U) {
+      uint32_t col[U];
 #pragma unroll
-    for (int i = 0; i < T_IPT; ++i) {
-      const int idx = wbase + i * 32 + lane;
-      if (idx < L) {
-        const int32_t s = st[i] >= 0 ? st[i] : carry;
-        S[idx] = static_cast<uint32_t>(s);
-        const bool tail = (idx == L - 1) || (K[idx + 1] != key[i]);
-        if (tail) LN[s] = static_cast<PayT>(idx + 1 - s);
+      for (int u = 0; u < U; ++u) col[u] = i0 + u * THREADS < L ? __ldg(ind + i0 + u * THREADS) : 0u;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * THREADS < L) {
+          const uint32_t h = column_hash(col[u]) >> (32 - S::FILTER_BITS), bit = 1u << (h & 31);
+          if (atomicOr(&sh.filter[0][h >> 5], bit) & bit) atomicOr(&sh.filter[1][h >> 5], bit);
+        }
+    }
+    __syncthreads();
+    // number what may share its column, in CSR order: a warp's elements are consecutive
+    int32_t numbered = 0;
+    for (int tb = 0; tb < L && numbered <= S::CAP; tb += THREADS * U) {
+      const int first = tb + (tid >> 5) * (32 * U) + lane;
+      uint32_t col[U];
+      unsigned on[U];
+      int32_t mine = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) col[u] = first + u * 32 < L ? __ldg(ind + first + u * 32) : 0u;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t h = column_hash(col[u]) >> (32 - S::FILTER_BITS);
+        on[u] = __ballot_sync(FULL, first + u * 32 < L && ((sh.filter[1][h >> 5] >> (h & 31)) & 1u) != 0u);
+        mine += __popc(on[u]);
+      }
+      int32_t tile_total;
+      int32_t at = numbered + block_sum<S::WARPS>(lane == 0 ? mine : 0, sh.warp_sum, &tile_total);
+      at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int32_t s = at + __popc(on[u] & ((1u << lane) - 1u));
+        at += __popc(on[u]);
+        if (((on[u] >> lane) & 1u) && s < S::CAP) {
+          uint32_t t = column_hash(col[u]) >> (32 - S::TABLE_BITS);
+          for (;;) {  // (fewer numbered nonzeros than table entries: an empty one is found)
+            const uint32_t seen = atomicCAS(&sh.key[t], FULL, col[u]);
+            if (seen == FULL || seen == col[u]) break;
+            t = (t + 1) & (S::TABLE - 1);
+          }
+          atomicAdd(&sh.cnt[t], 1u);
+          sh.slot[s] = static_cast<uint16_t>(t);
+          sh.row[s] = static_cast<uint16_t>(first + u * 32);
+        }
+      }
+      numbered += tile_total;
+    }
+    if (numbered > S::CAP) {  // (the same in all threads)
+      if (tid == 0) {
+        if (LARGE)
+          a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
+        else
+          a.next_chunk[atomicAdd(&a.ctrl[CTRL_NEXT_COUNT], 1u)] = q;
+      }
+      continue;
+    }
+    __syncthreads();
+    // places of the groups: each thread a stretch of the table
+    {
+      constexpr int PER = S::TABLE / THREADS;
+      uint32_t v[PER];
+      int32_t mine = 0, repeats = 0;
+#pragma unroll
+      for (int i = 0; i < PER; i += 4) {
+        *reinterpret_cast<uint4 *>(v + i) = *reinterpret_cast<const uint4 *>(sh.cnt + tid * PER + i);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (v[i + j] > 4095u) {  // (only with columns repeated inside rows)
+            atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
+            v[i + j] = 0;
+          }
+          mine += v[i + j] >= 2 ? static_cast<int32_t>(v[i + j]) : 0;
+          repeats += v[i + j] >= 2 ? static_cast<int32_t>(v[i + j]) - 1 : 0;
+        }
+      }
+      if (a.count) {
+        repeats = __reduce_add_sync(FULL, repeats);
+        if (lane == 0 && repeats) atomicAdd(a.count, static_cast<unsigned long long>(-static_cast<long long>(repeats)));
+        if (tid == 0) atomicAdd(a.count, static_cast<unsigned long long>(L));
+        continue;
+      }
+      int32_t total;
+      int32_t run = block_sum<S::WARPS>(mine, sh.warp_sum, &total);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const uint32_t n = v[i];
+        sh.cnt[tid * PER + i] = n >= 2 ? (static_cast<uint32_t>(run) << 12) | n : 0u;
+        sh.key[tid * PER + i] = 0u;
+        run += n >= 2 ? static_cast<int32_t>(n) : 0;
       }
     }
     __syncthreads();
-    if (tid == 0) {
-      int32_t c = sh.carry;
-      for (int w = 0; w < T_WARPS; ++w)
-        if (sh.warp_last[w] >= 0) c = sh.warp_last[w];
-      sh.carry = c;
+    for (int s = tid; s < numbered; s += THREADS) {
+      const uint32_t t = sh.slot[s], g = sh.cnt[t];
+      if (g == 0u) continue;
+      const int32_t r = row_of(sh.sptr, 0, rows, b + sh.row[s]);
+      sh.row[s] = static_cast<uint16_t>(r);
+      const uint32_t at = (g >> 12) + atomicAdd(&sh.key[t], 1u);
+      if (index_ok(a.ctrl, CHK_GROUP, at, S::CAP)) sh.member[at] = static_cast<uint16_t>(r);
+      atomicAdd(&sh.work[r], (g & 4095u) - 1u);
     }
     __syncthreads();
-  }
-  for (int i = tid; i < L; i += T_THREADS) {
-    const int32_t p = static_cast<int32_t>(P[i]);
-    const int32_t st = static_cast<int32_t>(S[i]);
-    if (!index_ok(a.ctrl, CHK_GROUP, p, L) || !index_ok(a.ctrl, CHK_GROUP, st, L)) continue;
-    const int32_t len = static_cast<int32_t>(LN[st]);
-    int32_t row;
-    if (rows_in_smem)
-      row = cs + row_of(sh.sptr, 0, rows, b + p);
-    else
-      row = row_of(a.ptr, cs, cs + rows, b + p);
-    const int32_t rl = rows_in_smem ? (sh.sptr[row - cs + 1] - sh.sptr[row - cs])
-                                    : (a.ptr[row + 1] - a.ptr[row]);
-    a.cand[b + i] = make_int2(row, rl);
-    a.seg[b + p] = make_int2(b + st, len);
-    a.seg_rank[b + p] = i - st;
-    if (len >= 2) {
-      // (a row's count can pass 32 bits when the chunk is the whole matrix: it sticks at the
-      // ceiling, which the sketch stage reads as "does not fit the stream buffer")
-      if (rows_in_smem)
-        saturating_add(&sh.row_work[row - cs], static_cast<uint32_t>(len - 1));
-      else
-        saturating_add(&a.row_work[row], static_cast<uint32_t>(len - 1));
-    }
-  }
-}
-
-__global__ void __launch_bounds__(T_THREADS, 1) transpose_kernel(TransposeArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
-  const int tid = threadIdx.x;
-  for (;;) {
-    __syncthreads();
-    if (tid == 0) sh.ticket = static_cast<int32_t>(atomicAdd(&a.ctrl[CTRL_CHUNK_TICKET], 1u));
-    __syncthreads();
-    const int32_t q = sh.ticket;
-    if (q >= a.num_chunks) break;
-    const ChunkSpan c = chunk_span(a, q);
-    const int32_t cs = c.cs, rows = c.rows, b = c.b;
-    const int L = c.L;
-    if (L > T_LS || L == 0) continue;  // heavy chunks go through the tiled kernels
-    const bool rows_in_smem = rows <= T_RP;
-    if (rows_in_smem) {
-      for (int i = tid; i <= rows; i += T_THREADS) sh.sptr[i] = a.ptr[cs + i];
-      for (int i = tid; i < rows; i += T_THREADS) sh.row_work[i] = 0;
+    int32_t written = 0;
+    for (int tb = 0; tb < numbered; tb += THREADS) {
+      const int s = tb + tid;
+      uint32_t g = 0;
+      int32_t r = 0, rank = 0;
+      if (s < numbered) {
+        g = sh.cnt[sh.slot[s]];
+        r = sh.row[s];
+      }
+      const int32_t start = static_cast<int32_t>(g >> 12), len = static_cast<int32_t>(g & 4095u);
+      for (int32_t i = 0; i < len; ++i) rank += sh.member[start + i] < r ? 1 : 0;
+      int32_t tile_total;
+      const int32_t at = written + block_sum<S::WARPS>(g ? 1 : 0, sh.warp_sum, &tile_total);
+      written += tile_total;
+      if (g) {
+        a.cand[b + start + rank] = make_int2(c.cs + r, sh.sptr[r + 1] - sh.sptr[r]);
+        a.seg[b + at] = make_int2(b + start, len);
+        a.seg_rank[b + at] = rank;
+        atomicAdd(&sh.cols[r >> 1], 1u << (16 * (r & 1)));
+      }
     }
     __syncthreads();
-    const uint32_t *kin0 = reinterpret_cast<const uint32_t *>(a.ind + b);
-    const int P = a.passes;
-    radix_pass<uint16_t, true>(kin0, nullptr, sh.skey[0], sh.spay[0], L, 0, sh, a.ctrl);
-    for (int ps = 1; ps < P; ++ps)
-      radix_pass<uint16_t, false>(sh.skey[(ps - 1) & 1], sh.spay[(ps - 1) & 1], sh.skey[ps & 1],
-                                  sh.spay[ps & 1], L, 8 * ps, sh, a.ctrl);
-    const int f = (P - 1) & 1;
-    emit_groups<uint16_t>(sh.skey[f], sh.spay[f], sh.skey[f ^ 1], sh.spay[f ^ 1], L, b, cs, rows,
-                          rows_in_smem, a, sh);
-    __syncthreads();
-    if (rows_in_smem)
-      for (int i = tid; i < rows; i += T_THREADS) a.row_work[cs + i] = sh.row_work[i];
+    int32_t before = 0;  // (rows come in order: where a row's groups start is the sum of the rows in front)
+    for (int r0 = 0; r0 < rows; r0 += THREADS) {
+      const int r = r0 + tid;
+      const int32_t n = r < rows ? static_cast<int32_t>((sh.cols[r >> 1] >> (16 * (r & 1))) & 0xFFFFu) : 0;
+      int32_t tile_total;
+      const int32_t at = before + block_sum<S::WARPS>(n, sh.warp_sum, &tile_total);
+      before += tile_total;
+      if (r < rows) {
+        a.row_seg[c.cs + r] = b + at;
+        a.row_cols[c.cs + r] = n;
+        a.row_work[c.cs + r] = sh.work[r];
+      }
+    }
   }
 }
 
 // ---- heavy chunks: tiled, whole-grid sort ----------------------------------------
-
-__global__ void classify_chunks_kernel(TransposeArgs a) {
-  for (int32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < a.num_chunks;
-       q += gridDim.x * blockDim.x) {
-    const ChunkSpan c = chunk_span(a, q);
-    if (a.skip_prio && static_cast<uint32_t>(q) == a.ctrl_main[CTRL_PRIO]) continue;
-    if (c.L > T_LS) a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
-  }
-}
 
 // The chunk that runs ahead of the rest: the one with the most nonzeros, if it is a heavy
 // chunk of at least min_nnz nonzeros (a row that streams 65,536 candidates or more needs a
@@ -339,7 +359,7 @@ __global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, Tr
     for (int w = 1; w < 32; ++w) mine = best[w] > mine ? best[w] : mine;
     const int32_t L = static_cast<int32_t>(mine >> 32);
     const uint32_t q = 0xFFFFFFFFu - static_cast<uint32_t>(mine);
-    const bool on = L > T_LS && L >= min_nnz;
+    const bool on = L > CompactLarge::CAP && L >= min_nnz;
     a.ctrl[CTRL_PRIO] = on ? q : PRIO_NONE;
     ap.ctrl[CTRL_PRIO] = on ? q : PRIO_NONE;
     ap.ctrl[CTRL_HEAVY_COUNT] = on ? 1u : 0u;
@@ -615,6 +635,15 @@ __global__ void __launch_bounds__(T_THREADS) heavy_emit_kernel(TransposeArgs a) 
     const uint32_t *P = (f ? a.payB : a.payA) + r.b;
     const bool staged = r.rows <= E_ROWS;
     int32_t w0 = 0;  // first sorted position held in skey
+    if (r.off == 0 && !a.count)  // every column of a row of such a chunk has an entry of seg[]
+      for (int32_t j = threadIdx.x; j < r.rows; j += T_THREADS) {
+        const int32_t x = a.ptr[r.cs + j], y = a.ptr[r.cs + j + 1];
+        const bool ok = x >= r.b && x <= y && y <= r.b + r.L;
+        if (!ok) atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
+        a.row_seg[r.cs + j] = ok ? x : r.b;
+        a.row_cols[r.cs + j] = ok ? y - x : 0;
+      }
+    int32_t firsts = 0;
     if (staged) {
       w0 = r.off - (r.rows - 1) < 0 ? 0 : r.off - (r.rows - 1);
       const int32_t w1 = r.off + r.cnt + (r.rows - 1) < r.L ? r.off + r.cnt + (r.rows - 1) : r.L;
@@ -635,6 +664,10 @@ __global__ void __launch_bounds__(T_THREADS) heavy_emit_kernel(TransposeArgs a) 
           hi = mid;
       }
       const int32_t st = lo;
+      if (a.count) {
+        firsts += i == st ? 1 : 0;
+        continue;
+      }
       lo = i + 1;
       hi = i + r.rows < r.L ? i + r.rows : r.L;  // first index with K > key
       while (lo < hi) {
@@ -662,106 +695,15 @@ __global__ void __launch_bounds__(T_THREADS) heavy_emit_kernel(TransposeArgs a) 
       a.seg[r.b + p] = make_int2(r.b + st, len);
       a.seg_rank[r.b + p] = i - st;
     }
+    if (a.count) {
+      firsts = __reduce_add_sync(FULL, firsts);
+      if (lane_id() == 0 && firsts) atomicAdd(a.count, static_cast<unsigned long long>(firsts));
+    }
     if (staged) {
       __syncthreads();
       for (int32_t j = threadIdx.x; j < r.rows; j += T_THREADS)
         if (swork[j]) saturating_add(&a.row_work[r.cs + j], swork[j]);
       __syncthreads();
-    }
-  }
-}
-
-// ---- symmetric pattern: groups read off the CSR arrays --------------------------------
-// One thread per nonzero p = (r, c): cand[p] = (c, length of row c) - cand is the column
-// array with lengths attached - and the group of column c in r's chunk is the part of row c
-// inside [chunk start, chunk end), found with three binary searches over row c that run in
-// step (the two ends and r's own place).  Blocks take tiles of Y_TILE positions; the rows a
-// tile touches are found once per tile and their pointers staged in shared memory.
-constexpr int Y_THREADS = 256;
-constexpr int Y_TILE = 2048;
-constexpr int Y_ROWS = 2048;  // rows of a tile with pointers in shared memory (more: searched in global memory)
-
-__global__ void __launch_bounds__(Y_THREADS) symmetric_groups_kernel(TransposeArgs a) {
-  __shared__ int32_t sptr[Y_ROWS + 1];
-  __shared__ int32_t span[2];
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int32_t tiles = (a.nnz + Y_TILE - 1) / Y_TILE;
-  if (a.ptr[0] != 0 || a.ptr[a.n] != a.nnz) {  // the row search below relies on both ends
-    if (tid == 0) atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
-    return;
-  }
-  for (int32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int32_t p_first = tile * Y_TILE;
-    const int32_t p_end = a.nnz - p_first < Y_TILE ? a.nnz : p_first + Y_TILE;
-    __syncthreads();
-    if (tid < 2) span[tid] = row_of(a.ptr, 0, a.n, tid ? p_end - 1 : p_first);
-    __syncthreads();
-    const int32_t r_first = span[0], r_last = span[1] < span[0] ? span[0] : span[1];
-    const int32_t nrows = r_last - r_first + 1;
-    const bool staged = nrows <= Y_ROWS;
-    if (staged)
-      for (int32_t i = tid; i <= nrows; i += Y_THREADS) sptr[i] = a.ptr[r_first + i];
-    __syncthreads();
-    for (int32_t p0 = p_first; p0 < p_end; p0 += Y_THREADS) {
-      const int32_t p = p0 + tid;
-      int32_t r = -1;
-      uint32_t add = 0;
-      if (p < p_end) {
-        r = staged ? r_first + row_of(sptr, 0, nrows, p) : row_of(a.ptr, r_first, r_last + 1, p);
-        const int32_t rb = a.ptr[r], re = a.ptr[r + 1];
-        const int32_t c = a.ind[p];
-        int32_t pc = 0, pe = 0;
-        bool ok = p >= rb && p < re && c >= 0 && c < a.n;  // (row pointers that are not ascending fail here)
-        if (ok) {
-          pc = a.ptr[c];
-          pe = a.ptr[c + 1];
-          ok = pc >= 0 && pe >= pc && pe <= a.nnz;
-        }
-        if (!ok) {
-          atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
-          a.cand[p] = make_int2(r, 1);
-          a.seg[p] = make_int2(p, 0);
-          a.seg_rank[p] = 0;
-        } else {
-          a.cand[p] = make_int2(c, pe - pc);
-          const int64_t q0 = static_cast<int64_t>(r / a.chunk) * a.chunk;
-          const int64_t q1 = q0 + a.chunk;
-          // first entries of row c not below the chunk start, the chunk end and r
-          int32_t lo_a = pc, hi_a = pe, lo_b = pc, hi_b = pe, lo_r = pc, hi_r = pe;
-          while (lo_a < hi_a || lo_b < hi_b || lo_r < hi_r) {
-            const int32_t ma = (lo_a + hi_a) >> 1, mb = (lo_b + hi_b) >> 1, mr = (lo_r + hi_r) >> 1;
-            const int32_t va = lo_a < hi_a ? a.ind[ma] : 0;
-            const int32_t vb = lo_b < hi_b ? a.ind[mb] : 0;
-            const int32_t vr = lo_r < hi_r ? a.ind[mr] : 0;
-            if (lo_a < hi_a) {
-              if (va < q0) lo_a = ma + 1; else hi_a = ma;
-            }
-            if (lo_b < hi_b) {
-              if (vb < q1) lo_b = mb + 1; else hi_b = mb;
-            }
-            if (lo_r < hi_r) {
-              if (vr < r) lo_r = mr + 1; else hi_r = mr;
-            }
-          }
-          // (rows that are not sorted can cross the three results: keep them ordered)
-          const int32_t first = lo_a;
-          const int32_t last = lo_b < first ? first : lo_b;
-          int32_t at = lo_r < first ? first : lo_r;
-          at = at > last ? last : at;
-          const int32_t len = last - first;
-          a.seg[p] = make_int2(first, len);
-          a.seg_rank[p] = at - first;
-          if (len >= 2) add = static_cast<uint32_t>(len - 1);
-        }
-      }
-      // the candidates each row will see: one atomic per warp where the warp sits in one row
-      const int32_t r_lead = __shfl_sync(FULL, r, 0);
-      if (__all_sync(FULL, r == r_lead || r < 0) && r_lead >= 0 && __all_sync(FULL, add < (1u << 26))) {
-        const uint32_t sum = __reduce_add_sync(FULL, add);
-        if (lane == 0 && sum) saturating_add(&a.row_work[r_lead], sum);
-      } else if (add) {
-        saturating_add(&a.row_work[r], add);
-      }
     }
   }
 }
@@ -885,8 +827,12 @@ TransposeArgs transpose_args(int32_t n, int32_t ncols, int32_t nnz, int32_t chun
   a.cand = s.cand;
   a.seg = s.seg;
   a.seg_rank = s.seg_rank;
+  a.row_seg = s.row_seg;
+  a.row_cols = s.row_cols;
   a.row_work = s.row_work;
   a.ctrl = s.ctrl;
+  a.count = nullptr;
+  a.next_chunk = s.next_chunk;
   a.heavy_chunk = s.heavy_chunk;
   a.heavy_tile_base = s.heavy_tile_base;
   a.tile_hist = s.tile_hist;
@@ -911,55 +857,12 @@ bool launch_priority_pick(Context &ctx, int32_t n, int32_t nnz, int32_t chunk, c
   return true;
 }
 
-// phase PHASE_ALL: the whole transposition on the context's stream.  PHASE_PRIO (on the side
-// stream, `s` = the scratch of the part that runs ahead): the one chunk launch_priority_pick
-// named, then that chunk's list of heavy rows; ctx.ev[6] marks the end of its transposition.
-// PHASE_REST (context's stream): every other chunk, then - once ev[6] has passed, because the
-// lists read the work counters of all rows - the lists of everything the part ahead left.
-bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
-                      const int32_t *d_ind, CsgScratch &s, bool symmetric, int phase, uint32_t *ctrl_other) {
-  // ctrl_other: the control words of the other part of a call that runs one chunk ahead
-  TransposeArgs a = transpose_args(n, ncols, nnz, chunk, d_ptr, d_ind, s);
-  a.ctrl_main = phase == PHASE_PRIO && ctrl_other ? ctrl_other : s.ctrl;
-  const uint32_t *ctrl_ahead = phase == PHASE_REST ? ctrl_other : nullptr;
-  a.skip_prio = phase == PHASE_REST;
-  const size_t smem = sizeof(Shared);
-  CSG_CUDA(cudaFuncSetAttribute(transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
-  if (phase == PHASE_ALL) {
-    CSG_CUDA(cudaMemsetAsync(s.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
-    CSG_CUDA(cudaMemsetAsync(s.row_work, 0, sizeof(uint32_t) * static_cast<size_t>(n), st));
-  }
-  int lgrid = (n + 255) / 256;
-  if (lgrid > ctx.num_sms * 8) lgrid = ctx.num_sms * 8;
-  if (phase == PHASE_ALL && symmetric && n == ncols && nnz > 0) {
-    // the caller's promise: the pattern is its own transpose
-    int ygrid = (nnz + Y_TILE - 1) / Y_TILE;
-    if (ygrid > ctx.num_sms * 8) ygrid = ctx.num_sms * 8;
-    symmetric_groups_kernel<<<ygrid, Y_THREADS, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
-    bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, nullptr);
-    CSG_CUDA(cudaGetLastError());
-    bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl);
-    CSG_CUDA(cudaGetLastError());
-    row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, nullptr);
-    CSG_CUDA(cudaGetLastError());
-    count_launches(4);
-    return true;
-  }
-  if (phase != PHASE_PRIO) {  // (the part ahead got its one heavy chunk from launch_priority_pick)
-    int cgrid = (a.num_chunks + 255) / 256;
-    if (cgrid > ctx.num_sms * 4) cgrid = ctx.num_sms * 4;
-    classify_chunks_kernel<<<cgrid, 256, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
-  }
+namespace {
+bool launch_heavy(Context &ctx, const TransposeArgs &a, bool one_chunk, cudaStream_t st) {
   heavy_tiles_kernel<<<1, 1024, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
-  // heavy chunks first: the rows with the longest streams live in them
   const int hgrid = ctx.num_sms * 2;
-  int sgrid = a.num_chunks < ctx.num_sms ? a.num_chunks : ctx.num_sms;
-  if (phase == PHASE_PRIO) sgrid = 1;
+  const int sgrid = one_chunk ? 1 : a.num_chunks < ctx.num_sms ? a.num_chunks : ctx.num_sms;
   for (int ps = 0; ps < a.passes; ++ps) {
     heavy_hist_kernel<<<hgrid, T_THREADS, 0, st>>>(a, ps);
     CSG_CUDA(cudaGetLastError());
@@ -970,24 +873,86 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   }
   heavy_emit_kernel<<<hgrid * 2, T_THREADS, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
+  count_launches(2 + 3 * a.passes);
+  return true;
+}
+
+bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
+  auto launch = [&](auto kernel, int threads, size_t smem, int per_sm) -> bool {
+    CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    const int grid = a.num_chunks < ctx.num_sms * per_sm ? a.num_chunks : ctx.num_sms * per_sm;
+    kernel<<<grid, threads, smem, st>>>(a);
+    CSG_CUDA(cudaGetLastError());
+    return true;
+  };
+  if (!launch(compact_kernel<CompactSmall, false>, CompactSmall::THREADS, sizeof(CompactSmall::Shared), 2)) return false;
+  if (!launch(compact_kernel<CompactLarge, true>, CompactLarge::THREADS, sizeof(CompactLarge::Shared), 1)) return false;
+  count_launches(2);
+  return true;
+}
+
+// the rows with candidates, longest stream first
+bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead) {
+  int grid = (n + 255) / 256;
+  if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
+  bucket_count_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
+  CSG_CUDA(cudaGetLastError());
+  bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl);
+  CSG_CUDA(cudaGetLastError());
+  row_list_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(3);
+  return true;
+}
+}  // namespace
+
+// phase PHASE_ALL: the whole transposition on the context's stream.  PHASE_PRIO (on the side
+// stream, `s` = the scratch of the part that runs ahead): the one chunk launch_priority_pick
+// named, then that chunk's list of heavy rows; ctx.ev[6] marks the end of its transposition.
+// PHASE_REST (context's stream): every other chunk, then - once ev[6] has passed, because the
+// lists read the work counters of all rows - the lists of everything the part ahead left.
+// A PHASE_ALL call looks at the outcome of compact_kernel on the host: without chunks for the
+// tiled sort (none on meshes, roads and most small matrices) its dozen launches are left out.
+// d_count: only the number of (chunk, column) pairs is wanted, and added there.
+bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
+                      const int32_t *d_ind, CsgScratch &s, int phase, uint32_t *ctrl_other,
+                      unsigned long long *d_count) {
+  // ctrl_other: the control words of the other part of a call that runs one chunk ahead
+  TransposeArgs a = transpose_args(n, ncols, nnz, chunk, d_ptr, d_ind, s);
+  a.ctrl_main = phase == PHASE_PRIO && ctrl_other ? ctrl_other : s.ctrl;
+  a.skip_prio = phase == PHASE_REST;
+  a.count = d_count;
   if (phase == PHASE_PRIO) {
+    cudaStream_t st = ctx.side_stream;
+    if (!launch_heavy(ctx, a, true, st)) return false;
     priority_rows_kernel<<<1, 1024, 0, st>>>(a, s.row_list);
     CSG_CUDA(cudaGetLastError());
+    count_launches(1);
     CSG_CUDA(cudaEventRecord(ctx.ev[6], st));  // the rest may read this chunk's work counters and its longest stream
-    count_launches(3 + 3 * a.passes);
     return true;
   }
-  const int grid = a.num_chunks < ctx.num_sms ? a.num_chunks : ctx.num_sms;
-  transpose_kernel<<<grid, T_THREADS, smem, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  if (phase == PHASE_REST) CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[6], 0));
-  bucket_count_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
-  CSG_CUDA(cudaGetLastError());
-  bucket_scan_kernel<<<1, 32, 0, st>>>(s.ctrl);
-  CSG_CUDA(cudaGetLastError());
-  row_list_kernel<<<lgrid, 256, 0, st>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
-  CSG_CUDA(cudaGetLastError());
-  count_launches(7 + 3 * a.passes);
+  cudaStream_t st = ctx.stream;
+  if (phase == PHASE_REST) {
+    if (!launch_compact(ctx, a, st) || !launch_heavy(ctx, a, false, st)) return false;
+    CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[6], 0));
+    return launch_lists(ctx, n, chunk, s, ctrl_other);
+  }
+  CSG_CUDA(cudaMemsetAsync(s.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
+  CSG_CUDA(cudaMemsetAsync(s.row_work, 0, sizeof(uint32_t) * static_cast<size_t>(n), st));
+  if (!launch_compact(ctx, a, st)) return false;
+  if (d_count) return launch_heavy(ctx, a, false, st);
+  if (!launch_lists(ctx, n, chunk, s, nullptr)) return false;
+  uint32_t *h = reinterpret_cast<uint32_t *>(ctx.h_pinned);
+  CSG_CUDA(cudaMemcpyAsync(h, s.ctrl, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  CSG_CUDA(cudaStreamSynchronize(st));
+  s.no_heavy_rows = h[CTRL_HEAVY_ROWS] == 0;
+  if (h[CTRL_HEAVY_COUNT] != 0) {
+    s.no_heavy_rows = false;
+    if (!launch_heavy(ctx, a, false, st)) return false;
+    CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, sizeof(uint32_t) * WORK_BUCKETS, st));
+    CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_HEAVY_NEED, 0, 2 * sizeof(uint32_t), st));
+    return launch_lists(ctx, n, chunk, s, nullptr);
+  }
   return true;
 }
 
