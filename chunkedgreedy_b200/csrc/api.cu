@@ -136,9 +136,9 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   size_t bw = transpose_only ? 0 : greedy_bitmap_words(n, p.chunk);
   if (greedy_chunk > 0 && greedy_bitmap_words(n, greedy_chunk) > bw) bw = greedy_bitmap_words(n, greedy_chunk);
   const size_t o_bm = ar.take(4 * (bw ? bw : 1));
-  // heavy chunks hold more than 10240 nonzeros or 2048 rows each and are cut into tiles of 4096
+  // heavy chunks hold more than 6144 nonzeros or 2048 rows each and are cut into tiles of 4096
   const size_t chunks = (static_cast<size_t>(n) + p.chunk - 1) / p.chunk;
-  size_t heavy_max = p.chunk > 2048 ? chunks : z / 10240 + 1;
+  size_t heavy_max = p.chunk > 2048 ? chunks : z / 6144 + 1;
   if (heavy_max > chunks) heavy_max = chunks;
   const size_t o_nc = ar.take(4 * chunks);
   const size_t tiles_max = z / 4096 + heavy_max + 1;
@@ -602,6 +602,7 @@ sporder_context_t sporder_context_create(void) {
     if ((e = cudaEventCreate(&ev)) != cudaSuccess) return fail(e, "cudaEventCreate");
   if ((e = cudaMallocHost(&c.h_pinned, 64 * sizeof(int))) != cudaSuccess)
     return fail(e, "cudaMallocHost");
+  std::memset(c.h_pinned, 0, 64 * sizeof(int));
   return h;
 }
 

@@ -21,6 +21,9 @@
 // every column of a row gets an entry of seg[]).
 // The reference can be promised a symmetric pattern and then reads the CSR arrays as the CSC
 // (sporder/src/common/csr2csc.h:52-54); nothing here needs the promise.
+#include <atomic>
+#include <chrono>
+
 #include "common.cuh"
 
 namespace csg {
@@ -100,13 +103,16 @@ __device__ __forceinline__ int32_t row_of(const int32_t *p, int32_t lo, int32_t 
 //     work through, so it never dominates.)
 //  5. members go out with their groups in CSR order, which is the order seg[] wants.
 // Two sizes: blocks of 512 threads, two to an SM, for up to 4096 numbered nonzeros; chunks with
-// more go on to blocks of 1024 threads for up to 10,240, those with more again to the tiled sort.
+// more go on to blocks of 1024 threads for up to 22,528 (in up to 6144 columns), those with more
+// again to the tiled sort.
 // On a B200, 1.05 M rows of the shuffled mesh: 227 us with the groups read off the promised
-// symmetry, 170 without any promise; 65,536 rows of the power-law band: 173 -> 87 us.
+// symmetry, COMPACT_MESH without any promise; 65,536 rows of the power-law band: 173 -> COMPACT_ZIPF us.
 template <int THREADS_, int CAP_, int TABLE_BITS_, int FILTER_BITS_>
 struct CompactSize {
   static constexpr int THREADS = THREADS_, WARPS = THREADS / 32, CAP = CAP_, TABLE_BITS = TABLE_BITS_, FILTER_BITS = FILTER_BITS_;
   static constexpr int TABLE = 1 << TABLE_BITS, FILTER = (1 << FILTER_BITS) / 32;  // entries; words of each map
+  // columns from which on a thread gives up: they cannot fill the table, however many are on their way
+  static constexpr int COLUMNS = TABLE - 2 * THREADS;
   struct Shared {
     uint32_t key[TABLE];          // columns, then how many members wrote their row
     uint32_t cnt[TABLE];          // rows per column, then (place << 12) | rows, 0 for a column with one
@@ -120,11 +126,11 @@ struct CompactSize {
     uint32_t work[C_ROWS];
     uint32_t cols[C_ROWS / 2];    // 16 bits a row
     int32_t warp_sum[32];
-    int32_t ticket;
+    int32_t ticket, columns;
   };
 };
 using CompactSmall = CompactSize<512, 4096, 13, 16>;
-using CompactLarge = CompactSize<1024, 10240, 14, 17>;
+using CompactLarge = CompactSize<1024, 22528, 13, 17>;
 
 // exclusive sum over the block's threads; *total is the sum of all
 template <int WARPS>
@@ -159,7 +165,7 @@ template <typename S, bool LARGE>
 __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename S::Shared &sh = *reinterpret_cast<typename S::Shared *>(smem_raw);
-  constexpr int THREADS = S::THREADS, U = 4;
+  constexpr int THREADS = S::THREADS, U = 8;
   const int tid = threadIdx.x, lane = tid & 31;
   for (;;) {
     __syncthreads();
@@ -173,8 +179,10 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
     const int L = c.L;
     if (L > C_NNZ || rows > C_ROWS) {
       if (tid == 0) a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
+      for (int i = tid; i < rows; i += THREADS) a.row_work[c.cs + i] = 0;  // (the tiled sort adds to it)
       continue;
     }
+    if (tid == 0) sh.columns = 0;
     bool ordered = true;
     for (int i = tid; i < rows; i += THREADS) {
       const int32_t x = a.ptr[c.cs + i], y = a.ptr[c.cs + i + 1];
@@ -227,47 +235,56 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
       for (int u = 0; u < U; ++u) {
         const int32_t s = at + __popc(on[u] & ((1u << lane) - 1u));
         at += __popc(on[u]);
-        if (((on[u] >> lane) & 1u) && s < S::CAP) {
-          uint32_t t = column_hash(col[u]) >> (32 - S::TABLE_BITS);
-          for (;;) {  // (fewer numbered nonzeros than table entries: an empty one is found)
-            const uint32_t seen = atomicCAS(&sh.key[t], FULL, col[u]);
-            if (seen == FULL || seen == col[u]) break;
-            t = (t + 1) & (S::TABLE - 1);
-          }
-          atomicAdd(&sh.cnt[t], 1u);
-          sh.slot[s] = static_cast<uint16_t>(t);
-          sh.row[s] = static_cast<uint16_t>(first + u * 32);
-        }
+        if (((on[u] >> lane) & 1u) && s < S::CAP) sh.row[s] = static_cast<uint16_t>(first + u * 32);
       }
       numbered += tile_total;
     }
-    if (numbered > S::CAP) {  // (the same in all threads)
+    __syncthreads();
+    const int inserted = numbered <= S::CAP ? numbered : 0;
+    for (int i0 = tid; i0 < inserted; i0 += THREADS * 4) {
+      uint32_t col[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) col[u] = i0 + u * THREADS < inserted ? __ldg(ind + sh.row[i0 + u * THREADS]) : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i0 + u * THREADS >= inserted || *static_cast<volatile int32_t *>(&sh.columns) > S::COLUMNS) continue;
+        uint32_t t = column_hash(col[u]) >> (32 - S::TABLE_BITS);
+        for (;;) {
+          const uint32_t seen = atomicCAS(&sh.key[t], FULL, col[u]);
+          if (seen == FULL) atomicAdd(&sh.columns, 1);
+          if (seen == FULL || seen == col[u]) break;
+          t = (t + 1) & (S::TABLE - 1);
+        }
+        atomicAdd(&sh.cnt[t], 1u);
+        sh.slot[i0 + u * THREADS] = static_cast<uint16_t>(t);
+      }
+    }
+    __syncthreads();
+    if (numbered > S::CAP || sh.columns > S::COLUMNS) {  // (the same in all threads)
       if (tid == 0) {
         if (LARGE)
           a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
         else
           a.next_chunk[atomicAdd(&a.ctrl[CTRL_NEXT_COUNT], 1u)] = q;
       }
+      if (LARGE)
+        for (int i = tid; i < rows; i += THREADS) a.row_work[c.cs + i] = 0;  // (the tiled sort adds to it)
       continue;
     }
-    __syncthreads();
-    // places of the groups: each thread a stretch of the table
+    // places of the groups, in any order
     {
       constexpr int PER = S::TABLE / THREADS;
       uint32_t v[PER];
       int32_t mine = 0, repeats = 0;
 #pragma unroll
-      for (int i = 0; i < PER; i += 4) {
-        *reinterpret_cast<uint4 *>(v + i) = *reinterpret_cast<const uint4 *>(sh.cnt + tid * PER + i);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (v[i + j] > 4095u) {  // (only with columns repeated inside rows)
-            atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
-            v[i + j] = 0;
-          }
-          mine += v[i + j] >= 2 ? static_cast<int32_t>(v[i + j]) : 0;
-          repeats += v[i + j] >= 2 ? static_cast<int32_t>(v[i + j]) - 1 : 0;
+      for (int i = 0; i < PER; ++i) {
+        v[i] = sh.cnt[i * THREADS + tid];
+        if (v[i] > 4095u) {  // (only with columns repeated inside rows)
+          atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
+          v[i] = 0;
         }
+        mine += v[i] >= 2 ? static_cast<int32_t>(v[i]) : 0;
+        repeats += v[i] >= 2 ? static_cast<int32_t>(v[i]) - 1 : 0;
       }
       if (a.count) {
         repeats = __reduce_add_sync(FULL, repeats);
@@ -280,8 +297,8 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const uint32_t n = v[i];
-        sh.cnt[tid * PER + i] = n >= 2 ? (static_cast<uint32_t>(run) << 12) | n : 0u;
-        sh.key[tid * PER + i] = 0u;
+        sh.cnt[i * THREADS + tid] = n >= 2 ? (static_cast<uint32_t>(run) << 12) | n : 0u;
+        sh.key[i * THREADS + tid] = 0u;
         run += n >= 2 ? static_cast<int32_t>(n) : 0;
       }
     }
@@ -359,7 +376,7 @@ __global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, Tr
     for (int w = 1; w < 32; ++w) mine = best[w] > mine ? best[w] : mine;
     const int32_t L = static_cast<int32_t>(mine >> 32);
     const uint32_t q = 0xFFFFFFFFu - static_cast<uint32_t>(mine);
-    const bool on = L > CompactLarge::CAP && L >= min_nnz;
+    const bool on = L > 8192 && L >= min_nnz;
     a.ctrl[CTRL_PRIO] = on ? q : PRIO_NONE;
     ap.ctrl[CTRL_PRIO] = on ? q : PRIO_NONE;
     ap.ctrl[CTRL_HEAVY_COUNT] = on ? 1u : 0u;
@@ -746,7 +763,7 @@ __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint
 // CHAIN_ROWS = two rows on each of 148 SMs: beyond one wave of them the chains only queue, and
 // what they do the lanes do with a sixth of the SM time (R-MAT scale 22 took 42 ms with 1184 rows
 // here).
-__global__ void bucket_scan_kernel(uint32_t *ctrl) {
+__global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, uint32_t ticket) {
   const int lane = threadIdx.x;
   uint32_t c[4], sum = 0;
 #pragma unroll
@@ -779,6 +796,11 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl) {
     ctrl[CTRL_LANE_TICKET] = heavy;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
+    // for the host (read_outcome)
+    outcome[1] = heavy;
+    outcome[2] = ctrl[CTRL_HEAVY_COUNT];
+    __threadfence_system();
+    outcome[0] = ticket;
   }
 }
 
@@ -891,13 +913,32 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
   return true;
 }
 
+// What bucket_scan_kernel wrote to the context's pinned words, as soon as it is there: the row list
+// is still being written then, and the launches behind it are queued before it is done.
+bool read_outcome(Context &ctx, cudaStream_t st, uint32_t *heavy_rows, uint32_t *heavy_chunks) {
+  volatile uint32_t *const h = reinterpret_cast<volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  const auto start = std::chrono::steady_clock::now();
+  for (int spins = 0; h[0] != ctx.outcome_ticket; ++spins) {
+    // something went wrong on the device, or it is busy with other work: wait for the stream
+    if ((spins & 1023) == 1023 && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(200)) {
+      CSG_CUDA(cudaStreamSynchronize(st));
+      CSG_REQUIRE(h[0] == ctx.outcome_ticket, "internal: the transposition did not report its outcome");
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  *heavy_rows = h[1];
+  *heavy_chunks = h[2];
+  return true;
+}
+
 // the rows with candidates, longest stream first
 bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead) {
   int grid = (n + 255) / 256;
   if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
   bucket_count_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
-  bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl);
+  bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl, reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD,
+                                               ++ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
   row_list_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
@@ -938,15 +979,13 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
     return launch_lists(ctx, n, chunk, s, ctrl_other);
   }
   CSG_CUDA(cudaMemsetAsync(s.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
-  CSG_CUDA(cudaMemsetAsync(s.row_work, 0, sizeof(uint32_t) * static_cast<size_t>(n), st));
   if (!launch_compact(ctx, a, st)) return false;
   if (d_count) return launch_heavy(ctx, a, false, st);
   if (!launch_lists(ctx, n, chunk, s, nullptr)) return false;
-  uint32_t *h = reinterpret_cast<uint32_t *>(ctx.h_pinned);
-  CSG_CUDA(cudaMemcpyAsync(h, s.ctrl, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  CSG_CUDA(cudaStreamSynchronize(st));
-  s.no_heavy_rows = h[CTRL_HEAVY_ROWS] == 0;
-  if (h[CTRL_HEAVY_COUNT] != 0) {
+  uint32_t heavy_rows = 0, heavy_chunks = 0;
+  if (!read_outcome(ctx, st, &heavy_rows, &heavy_chunks)) return false;
+  s.no_heavy_rows = heavy_rows == 0;
+  if (heavy_chunks != 0) {
     s.no_heavy_rows = false;
     if (!launch_heavy(ctx, a, false, st)) return false;
     CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, sizeof(uint32_t) * WORK_BUCKETS, st));

@@ -73,6 +73,28 @@ def test_rows_in_lanes_and_in_rounds_against_oracle(chunk, k):
     ctx.close()
 
 
+@pytest.mark.parametrize("rows,per_row,columns,chunk", [
+    (600, 30, 5000, 200), (2048, 2, 1900, 2048), (2049, 2, 1900, 2049), (2048, 11, 700, 2048),  # one small block; 22,528
+    (2048, 12, 700, 2048), (1500, 12, 9000, 1500), (1024, 64, 40_000, 1024), (1024, 65, 40_000, 1024),
+    (300, 700, 200_000, 60), (4000, 9, 200_000, 1024)])
+def test_grouping_of_shared_columns_against_oracle(rows, per_row, columns, chunk):
+    # both sizes of the block that groups a chunk's columns and what they pass on: nonzeros that may
+    # share their column, columns and rows at the limits, chunks beyond them (the tiled sort)
+    sp = _sp()
+    from chunkedgreedy_b200 import synth
+    rng = np.random.default_rng(rows * per_row)
+    n = max(rows, columns)
+    r = np.repeat(np.arange(rows), per_row)
+    c = (rng.integers(0, columns, rows)[:, None] + rng.permutation(columns)[:per_row][None, :]) % columns
+    ptr, ind, _ = synth.coo_to_csr(n, r, c.ravel())
+    want, table = oracle.csg(ptr, ind, False, with_table=True, k=16, chunk_size=chunk)
+    order, got = sp.csg_table(_dev(ptr), _dev(ind), k=16, chunk_size=chunk)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), table)
+    assert np.array_equal(order.cpu().numpy(), want)
+    for height in (13, 600):
+        assert sp.count_pillars(_dev(ptr), _dev(ind), height) == oracle.count_pillars(ptr, ind, height)
+
+
 @pytest.mark.parametrize("k", [1, 15, 16, 17, 31, 32, 33, 64])
 @pytest.mark.parametrize("chunk", [1, 32, 33, 700])
 def test_greedy_chains_on_lists_against_oracle(chunk, k):
