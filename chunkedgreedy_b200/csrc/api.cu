@@ -51,6 +51,20 @@ bool ensure_workspace(Context &ctx, size_t bytes) {
   return true;
 }
 
+bool wait_outcome(Context &ctx, cudaStream_t st) {
+  volatile uint32_t *const h = reinterpret_cast<volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  const auto start = std::chrono::steady_clock::now();
+  for (int spins = 0; h[0] != ctx.outcome_ticket; ++spins) {
+    // something went wrong on the device, or it is busy with other work: wait for the stream
+    if ((spins & 1023) == 1023 && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(200)) {
+      CSG_CUDA(cudaStreamSynchronize(st));
+      CSG_REQUIRE(h[0] == ctx.outcome_ticket, "internal: a kernel did not report its outcome");
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
+}
+
 // sporder/src/sporder.cpp:147-161 and the checks of
 // sporder/src/common/chunk_similarity_top_k.cu:143-147
 bool resolve_params(int32_t n, int32_t nnz, int32_t k, float ovs, int32_t chunk, CsgParams *out) {

@@ -50,7 +50,7 @@ struct Context {
   size_t ws_bytes = 0;
   cudaEvent_t ev[10] = {};  // [0..4] stage times; [5..8] fork, joins and order of a call that runs one chunk ahead
   int *h_pinned = nullptr;  // small pinned host buffer for counters (64 ints)
-  uint32_t outcome_ticket = 0;  // what h_pinned[OUTCOME_WORD] reads once the newest row lists are counted
+  uint32_t outcome_ticket = 0;  // the newest one handed to a kernel (see OUTCOME_WORD)
   char *stage = nullptr;    // device copies of host inputs (host-buffer entry point), kept between calls
   size_t stage_bytes = 0;
   // Buffer for the materialised candidate streams of the heaviest rows (sketch.cu), in stream
@@ -69,7 +69,10 @@ struct Context {
   uint64_t stream_limit = 0;       // caller's upper bound (sporder_context_set_stream_limit), 0 = none
 };
 
-constexpr int OUTCOME_WORD = 48;  // in h_pinned, written by the device: ticket, heavy rows, heavy chunks
+// In h_pinned, written by the device: a ticket, then what a kernel found out that decides about the
+// launches behind it.  wait_outcome returns once the ticket is ctx.outcome_ticket.
+constexpr int OUTCOME_WORD = 48;
+bool wait_outcome(Context &ctx, cudaStream_t st);
 
 bool ensure_workspace(Context &ctx, size_t bytes);
 

@@ -22,14 +22,13 @@
 //     sorted the same way into a scratch copy by as many blocks as there are tiles, then one
 //     pass that places every entry at the sum of its ranks in all tiles of its row.
 // A permutation that keeps every row and column inside its block of 1024 (every csg order
-// with the default chunk size does) needs less: the old row is sorted by column, so the new
-// row is already sorted block by block and only the entries of one block have to be ordered
-// among themselves.  ptr_new_kernel notices such a permutation, and rows of more than 32
-// entries then go through apply_runs_kernel: slices of 2048 entries, remapped into shared
-// memory with a halo, every entry placed at the start of its block's run plus the number of
-// smaller entries in the run (rows of up to 256 entries: the same by one warp per row).
-// No row is gathered by a single warp any more (that alone cost 6 ms on a row of 98 k
-// entries), and no sort runs on global memory (the in-place network cost another 17 ms).
+// with the default chunk size does) needs none of this: the old row is sorted by column, so the
+// new row is already sorted block by block and only the entries of one block have to be ordered
+// among themselves.  ptr_new_kernel notices such a permutation and tells the host, which then
+// launches apply_flat_kernel instead of the kernels above.  That one, which also does the copy
+// of the rows-only mode, cuts the output into tiles of 2048 entries whatever rows they belong to.
+#include <cstddef>
+
 #include "common.cuh"
 
 namespace csg {
@@ -40,6 +39,7 @@ constexpr int R_THREADS = 256;
 constexpr int R_SCAN_IPT = 8;
 constexpr int R_SCAN_TILE = R_THREADS * R_SCAN_IPT;  // rows per scan block
 constexpr int LOCAL_BITS = 10;                       // blocks of 1024 rows / columns: the default csg chunk
+constexpr int FLAT_TILE = 2048;                      // output entries per tile of apply_flat_kernel
 constexpr int R_WARP = 256;                          // longest row sorted by one warp in registers
 constexpr int R_MED = 4096;                          // longest row (and tile of a longer row) sorted in shared memory
 
@@ -118,62 +118,103 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32
 }
 
 __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
-    int32_t n, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
+    int32_t n, int32_t nnz, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
     const int32_t *__restrict__ block_sums, int32_t *__restrict__ ptr_new,
-    int32_t *__restrict__ old2new, uint32_t *__restrict__ leaves_block) {
-  __shared__ int32_t sm[R_THREADS / 32];
+    int32_t *__restrict__ old2new, uint32_t *__restrict__ leaves_block, int32_t *__restrict__ tile_row,
+    int32_t *__restrict__ row_delta,
+    volatile uint32_t *outcome, uint32_t ticket) {
+  constexpr int WARPS = R_THREADS / 32;
+  __shared__ int32_t sums[R_SCAN_IPT * WARPS];  // of 32 rows each, in row order
   __shared__ int moved;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) moved = 0;
   __syncthreads();
-  // thread t owns R_SCAN_IPT consecutive rows so that one block scan suffices
-  const int32_t first = blockIdx.x * R_SCAN_TILE + threadIdx.x * R_SCAN_IPT;
-  int32_t len[R_SCAN_IPT], s = 0;
+  const int32_t first = blockIdx.x * R_SCAN_TILE + threadIdx.x;
+  int32_t len[R_SCAN_IPT], from[R_SCAN_IPT], incl[R_SCAN_IPT];
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
-    const int32_t p = first + i;
-    len[i] = 0;
+    const int32_t p = first + i * R_THREADS;
+    len[i] = from[i] = 0;
     if (p < n) {
       const int32_t src = new_order[p];
-      len[i] = ptr_old[src + 1] - ptr_old[src];
+      from[i] = ptr_old[src];
+      len[i] = ptr_old[src + 1] - from[i];
       if (old2new) old2new[src] = p;
       if ((src >> LOCAL_BITS) != (p >> LOCAL_BITS)) moved = 1;  // leaves its block of 1024
     }
-    s += len[i];
+    incl[i] = len[i];
   }
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+    for (int i = 0; i < R_SCAN_IPT; ++i) {
+      const int32_t t = __shfl_up_sync(FULL, incl[i], off);
+      if (lane >= off) incl[i] += t;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R_SCAN_IPT; ++i)
+    if (lane == 31) sums[i * WARPS + warp] = incl[i];
   __syncthreads();
   if (threadIdx.x == 0 && moved) atomicExch(leaves_block, 1u);
-  int32_t tot;
-  int32_t run = block_sums[blockIdx.x] + block_exclusive_scan(s, &tot, sm);
+  if (warp == 0) {  // sums -> what lies in front of each 32 rows
+    static_assert(R_SCAN_IPT * WARPS == 64, "two per lane");
+    const int32_t x = sums[2 * lane], y = sums[2 * lane + 1];
+    int32_t run = x + y;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int32_t t = __shfl_up_sync(FULL, run, off);
+      if (lane >= off) run += t;
+    }
+    run += block_sums[blockIdx.x];
+    sums[2 * lane] = run - x - y;
+    sums[2 * lane + 1] = run - y;
+  }
+  __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) ptr_new[0] = 0;
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
-    const int32_t p = first + i;
-    run += len[i];
-    if (p < n) ptr_new[p + 1] = run;
+    const int32_t p = first + i * R_THREADS;
+    const int32_t run = sums[i * WARPS + warp] + incl[i] - len[i];
+    // the row that holds the first entry of a tile
+    for (int64_t t = (static_cast<int64_t>(run) + FLAT_TILE - 1) / FLAT_TILE;
+         t * FLAT_TILE < static_cast<int64_t>(run) + len[i] && t * FLAT_TILE < nnz; ++t)
+      tile_row[t] = p;
+    if (p < n) {
+      row_delta[p] = from[i] - run;
+      ptr_new[p + 1] = run + len[i];
+    }
+  }
+  if (outcome) {  // the last block tells the host whether any row left its block of 1024
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(leaves_block + 1, 1u) == gridDim.x - 1) {
+      outcome[1] = atomicAdd(leaves_block, 0u);
+      __threadfence_system();
+      outcome[0] = ticket;
+    }
   }
 }
 
 struct ApplyArgs {
-  int32_t n;
+  int32_t n, nnz;
   const int32_t *ptr_old, *ind_old;
   const float *val_old;      // nullptr: pattern only
   const int32_t *new_order;
-  const int32_t *old2new;    // nullptr: rows only (no remap, no sort)
+  const int32_t *old2new;    // nullptr: rows only (apply_flat_kernel<true>)
   const int32_t *ptr_new;
   int32_t *ind_new;
   float *val_new;
   int32_t *queue_warp, *queue_block;  // new rows of 33..R_WARP entries / of up to R_MED
   int2 *queue_long;                   // longer rows: (new row, number of its first tile)
-  int2 *queue_runs;                   // block-local permutation, rows past R_WARP: (new row, slice)
+  const int32_t *tile_row;            // per tile of the output: the row its first entry belongs to
+  const int32_t *row_delta;           // per new row: where it was less where it is
   uint32_t *counters;                 // [0] warp rows, [1] block rows, [2..3] packed (long rows, tiles),
-                                      // [4] set when the permutation leaves blocks of 1024,
-                                      // [6] slices in queue_runs
+                                      // [4] set when the permutation leaves blocks of 1024, [5] blocks that looked
   int32_t *tmp_key;                   // scratch copy of the long rows' sorted tiles, indexed like ind_new
   float *tmp_val;
 };
-constexpr int CNT_WARP = 0, CNT_BLOCK = 1, CNT_LONG = 2, CNT_MOVED = 4, CNT_RUNS = 6;
-constexpr int RUN_SLICE = 2048;                      // entries of a row one block orders at a time
-constexpr int RUN_HALO = (1 << LOCAL_BITS) - 1;      // a run holds at most 1024 entries
+constexpr int CNT_WARP = 0, CNT_BLOCK = 1, CNT_LONG = 2, CNT_MOVED = 4;
 
 // Rows of up to W entries, 32 / W of them at a time: each row in a segment of W lanes.
 // `mask` names the lanes whose row (src, len, dst) belongs to this size class.
@@ -195,24 +236,21 @@ __device__ __forceinline__ void apply_class(const ApplyArgs &a, unsigned mask, i
     int32_t key = 0x7FFFFFFF;
     float v = 0.0f;
     if (mine) {
-      const int32_t c = a.ind_old[s + j];
-      key = a.old2new ? a.old2new[c] : c;
+      key = a.old2new[a.ind_old[s + j]];
       if (a.val_new) v = a.val_old[s + j];
     }
-    if (a.old2new) {
 #pragma unroll
-      for (int k = 2; k <= W; k <<= 1) {
+    for (int k = 2; k <= W; k <<= 1) {
 #pragma unroll
-        for (int x = k >> 1; x > 0; x >>= 1) {
-          const int32_t ok = __shfl_xor_sync(FULL, key, x);
-          const float ov = __shfl_xor_sync(FULL, v, x);
-          const bool up = (j & k) == 0;
-          const bool lower = (j & x) == 0;
-          const bool take = (up == lower) ? (ok < key) : (ok > key);
-          if (take) {
-            key = ok;
-            v = ov;
-          }
+      for (int x = k >> 1; x > 0; x >>= 1) {
+        const int32_t ok = __shfl_xor_sync(FULL, key, x);
+        const float ov = __shfl_xor_sync(FULL, v, x);
+        const bool up = (j & k) == 0;
+        const bool lower = (j & x) == 0;
+        const bool take = (up == lower) ? (ok < key) : (ok > key);
+        if (take) {
+          key = ok;
+          v = ov;
         }
       }
     }
@@ -238,11 +276,7 @@ __global__ void __launch_bounds__(R_THREADS) apply_short_kernel(ApplyArgs a) {
       len = a.ptr_old[src_row + 1] - src;
       dst = a.ptr_new[p];
     }
-    if (len > R_WARP && a.old2new && a.counters[CNT_MOVED] == 0u) {  // block-local permutation
-      const uint32_t slices = static_cast<uint32_t>((len + RUN_SLICE - 1) / RUN_SLICE);
-      const uint32_t first = atomicAdd(&a.counters[CNT_RUNS], slices);
-      for (uint32_t t = 0; t < slices; ++t) a.queue_runs[first + t] = make_int2(p, static_cast<int32_t>(t));
-    } else if (len > 32) {
+    if (len > 32) {
       if (len <= R_WARP) {
         a.queue_warp[atomicAdd(&a.counters[CNT_WARP], 1u)] = p;
       } else if (len <= R_MED) {
@@ -335,66 +369,240 @@ __device__ __forceinline__ void warp_row(const ApplyArgs &a, int32_t src, int32_
   }
 }
 
-// One warp per queued row of 33..R_WARP entries.
-// Block-local permutation, rows of more than R_WARP entries: one block per slice of RUN_SLICE
-// entries.  The old row is sorted by column and the permutation keeps every column in its
-// block of 1024, so the remapped row is a sequence of runs, one per block, in the right
-// order; an entry's place is the start of its run plus the number of smaller entries in the
-// run.  The slice is staged with a halo of 1023 entries on either side: no run is longer
-// than 1024.
-__global__ void __launch_bounds__(R_THREADS) apply_runs_kernel(ApplyArgs a) {
-  __shared__ int32_t skey[RUN_SLICE + 2 * RUN_HALO];
-  if (!a.old2new || a.counters[CNT_MOVED] != 0u) return;
-  const int32_t total = static_cast<int32_t>(a.counters[CNT_RUNS]);
-  for (int32_t id = blockIdx.x; id < total; id += gridDim.x) {
-    const int2 q = a.queue_runs[id];  // (new row, slice)
-    const int32_t src_row = a.new_order[q.x];
-    const int32_t src = a.ptr_old[src_row], L = a.ptr_old[src_row + 1] - src;
-    const int32_t dst = a.ptr_new[q.x];
-    const int32_t s0 = q.y * RUN_SLICE;
-    const int32_t s1 = s0 + RUN_SLICE < L ? s0 + RUN_SLICE : L;
-    const int32_t w0 = s0 - RUN_HALO < 0 ? 0 : s0 - RUN_HALO;
-    const int32_t w1 = s1 + RUN_HALO < L ? s1 + RUN_HALO : L;
+// ---- tiles of the output ---------------------------------------------------------------------
+// A block per tile of FLAT_TILE consecutive output entries, rows in order.  ROWS: a copy of the
+// old rows in their new order.  Otherwise (a permutation that keeps rows and columns in their
+// blocks of 1024) an entry's place is the start of its run - the entries of its row in its column's
+// block - plus the number of smaller entries in the run, found by comparing where the run is
+// short and in a bit map of the block where it is long.  Runs belong to the tile that holds their
+// first entry; a tile reads on behind its end as far as its last run goes.
+// All rows cost the same per entry this way.  By kinds of rows (bitonic networks up to 32 entries,
+// run scans by a warp and by a block above) the reordered R-MAT scale 22 took 1.17 ms here, 0.95 this
+// way; bound by instructions (some 270 per entry, the passes over the tile in shared memory) at four blocks per SM.
+constexpr int FLAT_HALO = 1 << LOCAL_BITS;  // a run holds at most 1024 entries
+constexpr int FLAT_LONG = 48;               // shortest run that gets a bit map
+constexpr int FLAT_MAX = FLAT_TILE + FLAT_HALO;
+struct FlatShared {
+  int32_t delta[FLAT_TILE];               // at the first entry of a row: where it comes from, relative
+  uint32_t row_head[FLAT_TILE / 32];      // bit per entry: first of its row
+  int16_t row_before[FLAT_TILE / 32];     // last such entry in the words in front, -1: none in the tile
+  // (the copy of the rows-only mode needs no more than this)
+  uint32_t run_head[FLAT_MAX / 32];       // the same for runs
+  int16_t run_before[FLAT_MAX / 32];
+  int32_t key[FLAT_MAX];
+  float val[FLAT_TILE];
+  uint16_t run_end[FLAT_MAX];             // at the first entry of a run; FLAT_MAPPED + its bit map for a long one
+  uint32_t map[FLAT_MAX / FLAT_LONG][32];
+  uint16_t map_before[FLAT_MAX / FLAT_LONG][32];
+  int32_t maps;
+};
+constexpr uint32_t FLAT_MAPPED = 0x8000u;
+
+// last set bit at or below lane `lane` of word w, or what the words in front say
+__device__ __forceinline__ int32_t last_head(const uint32_t *heads, const int16_t *before, int w, int lane) {
+  const uint32_t m = heads[w] & (FULL >> (31 - lane));
+  return m ? w * 32 + 31 - __clz(static_cast<int>(m)) : before[w];
+}
+// `before` of `words` words, by one warp
+__device__ __forceinline__ void heads_before(const uint32_t *heads, int16_t *before, int words) {
+  const int lane = lane_id();
+  int carry = -1;
+  for (int w0 = 0; w0 < words; w0 += 32) {
+    const int w = w0 + lane;
+    const uint32_t h = w < words ? heads[w] : 0u;
+    const int mine = h ? w * 32 + 31 - __clz(static_cast<int>(h)) : -1;
+    int incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, off);
+      if (lane >= off) incl = max(incl, t);
+    }
+    int prev = __shfl_up_sync(FULL, incl, 1);
+    if (lane == 0) prev = -1;
+    if (w < words) before[w] = static_cast<int16_t>(max(prev, carry));
+    carry = max(carry, __shfl_sync(FULL, incl, 31));
+  }
+}
+
+template <bool ROWS>
+__global__ void __launch_bounds__(R_THREADS, 4) apply_flat_kernel(ApplyArgs a) {
+  extern __shared__ __align__(16) unsigned char flat_smem[];
+  FlatShared &sh = *reinterpret_cast<FlatShared *>(flat_smem);
+  constexpr int PER = FLAT_TILE / R_THREADS;  // entries per thread: 32 consecutive ones per warp and turn
+  const int tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  const int32_t nnz = min(a.ptr_new[a.n], a.nnz);
+  const int32_t tiles = nnz / FLAT_TILE + (nnz % FLAT_TILE ? 1 : 0);
+  for (int32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int32_t t0 = t * FLAT_TILE, cnt = nnz - t0 < FLAT_TILE ? nnz - t0 : FLAT_TILE, t1 = t0 + cnt;
+    const int32_t ra = a.tile_row[t], rb = t + 1 < tiles ? a.tile_row[t + 1] : a.n - 1;
     __syncthreads();
-    for (int32_t j = w0 + threadIdx.x; j < w1; j += R_THREADS) skey[j - w0] = a.old2new[a.ind_old[src + j]];
+    if (tid < FLAT_TILE / 32) sh.row_head[tid] = 0;
+    if (!ROWS && tid == 0) sh.maps = 0;
     __syncthreads();
-    for (int32_t i = s0 + threadIdx.x; i < s1; i += R_THREADS) {
-      const int32_t x = skey[i - w0];
-      const int32_t blk = x >> LOCAL_BITS;
-      int32_t below = 0;
-      int32_t j = i - 1;
-      for (; j >= w0 && (skey[j - w0] >> LOCAL_BITS) == blk; --j) below += skey[j - w0] < x ? 1 : 0;
-      const int32_t run_start = j + 1;
-      for (j = i + 1; j < w1 && (skey[j - w0] >> LOCAL_BITS) == blk; ++j) below += skey[j - w0] < x ? 1 : 0;
-      a.ind_new[dst + run_start + below] = x;
-      if (a.val_new) a.val_new[dst + run_start + below] = a.val_old[src + i];
+    const int32_t delta0 = a.row_delta[ra];
+    const int32_t rb_start = a.ptr_new[rb], rb_end = a.ptr_new[rb + 1];  // (rb holds entry t1, if there is one)
+    for (int32_t p = ra + tid; p <= rb; p += R_THREADS) {
+      const int32_t b = a.ptr_new[p], e = a.ptr_new[p + 1], d = a.row_delta[p];
+      if (b >= t1) break;  // (behind the last row with entries there may be many without)
+      if (b >= t0 && e > b) {
+        sh.delta[b - t0] = d;
+        atomicOr(&sh.row_head[(b - t0) >> 5], 1u << ((b - t0) & 31));
+      }
+    }
+    __syncthreads();
+    if (warp == 0) heads_before(sh.row_head, sh.row_before, FLAT_TILE / 32);
+    __syncthreads();
+    int32_t from[PER], key[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int w = warp * PER + u, e = w * 32 + lane;
+      const int32_t h = last_head(sh.row_head, sh.row_before, w, lane);
+      from[u] = t0 + e + (h >= 0 ? sh.delta[h] : delta0);
+      key[u] = e < cnt ? a.ind_old[from[u]] : 0;
+    }
+    if (ROWS) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) {
+        const int e = (warp * PER + u) * 32 + lane;
+        if (e < cnt) {
+          a.ind_new[t0 + e] = key[u];
+          if (a.val_new) a.val_new[t0 + e] = a.val_old[from[u]];
+        }
+      }
+      continue;
+    }
+    // In the same trip: the values, straight to shared memory; the entry in front of the tile, if
+    // its row goes on here; and the entries behind the tile, if the row that ends it goes on there.
+    if (a.val_new) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) {
+        const int e = (warp * PER + u) * 32 + lane;
+        if (e < cnt) {
+          const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(&sh.val[e]));
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(a.val_old + from[u]) : "memory");
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int32_t last = last_head(sh.row_head, sh.row_before, (cnt - 1) >> 5, (cnt - 1) & 31);
+    const int32_t last_delta = last >= 0 ? sh.delta[last] : delta0;
+    const bool goes_on = t1 < nnz && rb_start < t1, comes_in = (sh.row_head[0] & 1u) == 0u;
+    int32_t prev = comes_in ? a.ind_old[t0 - 1 + delta0] : 0;
+    bool in = goes_on && t1 + tid < rb_end;
+    int32_t more = in ? a.ind_old[t1 + tid + last_delta] : 0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = (warp * PER + u) * 32 + lane;
+      key[u] = e < cnt ? a.old2new[key[u]] : 0x7FFFFFFF;
+    }
+    if (comes_in) prev = a.old2new[prev];
+    if (in) more = a.old2new[more];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) sh.key[(warp * PER + u) * 32 + lane] = key[u];
+    __syncthreads();
+    const bool joined = comes_in && (prev >> LOCAL_BITS) == (sh.key[0] >> LOCAL_BITS);  // a run of the tile before
+    int32_t ext = 0;  // entries of the last run behind the tile's end
+    if (goes_on) {
+      const int32_t blk = sh.key[cnt - 1] >> LOCAL_BITS;
+      for (;;) {
+        const bool same = in && (more >> LOCAL_BITS) == blk;
+        if (same) sh.key[cnt + ext + tid] = more;
+        const int got = __syncthreads_count(same);
+        ext += got;
+        if (got < R_THREADS || ext >= FLAT_HALO) break;
+        in = t1 + ext + tid < rb_end && ext + tid < FLAT_HALO;
+        if (in) more = a.old2new[a.ind_old[t1 + ext + tid + last_delta]];
+      }
+    }
+    const int32_t total = cnt + ext;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int w = warp * PER + u, e = w * 32 + lane;
+      bool head = false;
+      if (e < cnt)
+        head = e == 0 ? !joined
+                      : ((sh.row_head[w] >> lane) & 1u) != 0u || (sh.key[e - 1] >> LOCAL_BITS) != (key[u] >> LOCAL_BITS);
+      const unsigned m = __ballot_sync(FULL, head);
+      if (lane == 0) sh.run_head[w] = m;
+    }
+    if (tid < FLAT_HALO / 32) sh.run_head[FLAT_TILE / 32 + tid] = 0;
+    __syncthreads();
+    if (warp == 0) heads_before(sh.run_head, sh.run_before, FLAT_MAX / 32);
+    __syncthreads();
+    // ends of the runs.  (A tile that is not full is the last one and has nothing behind it.)
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int w = warp * PER + u, e = w * 32 + lane;
+      if (e > 0 && e < cnt && ((sh.run_head[w] >> lane) & 1u)) {
+        const int32_t s = last_head(sh.run_head, sh.run_before, (e - 1) >> 5, (e - 1) & 31);
+        if (s >= 0) sh.run_end[s] = static_cast<uint16_t>(e);
+      }
+    }
+    if (tid == 0) {
+      const int32_t s = last_head(sh.run_head, sh.run_before, (cnt - 1) >> 5, (cnt - 1) & 31);
+      if (s >= 0) sh.run_end[s] = static_cast<uint16_t>(total);
+    }
+    __syncthreads();
+    // bit maps of the long runs
+    bool any_long = false;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int w = warp * PER + u, e = w * 32 + lane;
+      if (e < cnt && ((sh.run_head[w] >> lane) & 1u) && sh.run_end[e] - e >= FLAT_LONG) {
+        const int32_t id = atomicAdd(&sh.maps, 1);
+        sh.run_end[e] = static_cast<uint16_t>(FLAT_MAPPED + id);
+        any_long = true;
+      }
+    }
+    if (__syncthreads_or(any_long)) {
+      for (int i = tid; i < sh.maps * 32; i += R_THREADS) sh.map[i >> 5][i & 31] = 0u;
+      __syncthreads();
+      for (int e = tid; e < total; e += R_THREADS) {
+        const int32_t s = last_head(sh.run_head, sh.run_before, e >> 5, e & 31);
+        const uint32_t end = s >= 0 ? sh.run_end[s] : 0u;
+        if (end >= FLAT_MAPPED) {
+          const int32_t k = sh.key[e];
+          atomicOr(&sh.map[end - FLAT_MAPPED][(k >> 5) & 31], 1u << (k & 31));
+        }
+      }
+      __syncthreads();
+      for (int m = warp; m < sh.maps; m += R_THREADS / 32) {
+        const int c = __popc(sh.map[m][lane]);
+        int incl = c;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const int x = __shfl_up_sync(FULL, incl, off);
+          if (lane >= off) incl += x;
+        }
+        sh.map_before[m][lane] = static_cast<uint16_t>(incl - c);
+      }
+      __syncthreads();
+    }
+    if (a.val_new) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
+#pragma unroll 2
+    for (int e = tid; e < total; e += R_THREADS) {
+      const int32_t s = last_head(sh.run_head, sh.run_before, e >> 5, e & 31), k = sh.key[e];
+      if (s < 0) continue;  // the tile before does it
+      const uint32_t end = sh.run_end[s];
+      int32_t rank = 0;
+      if (end >= FLAT_MAPPED) {
+        const uint32_t m = end - FLAT_MAPPED, w = (k >> 5) & 31;
+        rank = sh.map_before[m][w] + __popc(sh.map[m][w] & ((1u << (k & 31)) - 1u));
+      } else if (end - s > 1) {
+        for (int32_t j = s; j < static_cast<int32_t>(end); ++j) rank += sh.key[j] < k ? 1 : 0;
+      }
+      a.ind_new[t0 + s + rank] = k;
+      if (a.val_new) a.val_new[t0 + s + rank] = e < cnt ? sh.val[e] : a.val_old[t0 + e + last_delta];
     }
   }
 }
 
-// The same for a row of up to R_WARP entries, by one warp: the whole row is staged.
-__device__ __forceinline__ void warp_row_runs(const ApplyArgs &a, int32_t *skey, int32_t src, int32_t L,
-                                              int32_t dst, int lane) {
-  __syncwarp();
-  for (int32_t j = lane; j < L; j += 32) skey[j] = a.old2new[a.ind_old[src + j]];
-  __syncwarp();
-  for (int32_t i = lane; i < L; i += 32) {
-    const int32_t x = skey[i];
-    const int32_t blk = x >> LOCAL_BITS;
-    int32_t below = 0;
-    int32_t j = i - 1;
-    for (; j >= 0 && (skey[j] >> LOCAL_BITS) == blk; --j) below += skey[j] < x ? 1 : 0;
-    const int32_t run_start = j + 1;
-    for (j = i + 1; j < L && (skey[j] >> LOCAL_BITS) == blk; ++j) below += skey[j] < x ? 1 : 0;
-    a.ind_new[dst + run_start + below] = x;
-    if (a.val_new) a.val_new[dst + run_start + below] = a.val_old[src + i];
-  }
-}
-
+// One warp per queued row of 33..R_WARP entries.
 __global__ void __launch_bounds__(R_THREADS) apply_warp_kernel(ApplyArgs a) {
-  __shared__ int32_t staged[R_THREADS / 32][R_WARP];
   const int lane = threadIdx.x & 31;
-  const bool local = a.old2new && a.counters[CNT_MOVED] == 0u;  // block-local permutation
   const uint32_t count = a.counters[CNT_WARP];
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < count; item += warps) {
@@ -402,14 +610,7 @@ __global__ void __launch_bounds__(R_THREADS) apply_warp_kernel(ApplyArgs a) {
     const int32_t src_row = a.new_order[p];
     const int32_t src = a.ptr_old[src_row], L = a.ptr_old[src_row + 1] - src;
     const int32_t dst = a.ptr_new[p];
-    if (!a.old2new) {  // rows only: a copy
-      for (int32_t i = lane; i < L; i += 32) {
-        a.ind_new[dst + i] = a.ind_old[src + i];
-        if (a.val_new) a.val_new[dst + i] = a.val_old[src + i];
-      }
-    } else if (local) {
-      warp_row_runs(a, staged[threadIdx.x >> 5], src, L, dst, lane);
-    } else if (L <= 64) {
+    if (L <= 64) {
       warp_row<2>(a, src, L, dst, lane);
     } else if (L <= 128) {
       warp_row<4>(a, src, L, dst, lane);
@@ -503,13 +704,6 @@ __global__ void __launch_bounds__(R_THREADS) apply_block_kernel(ApplyArgs a) {
     const int32_t src_row = a.new_order[p];
     const int32_t src = a.ptr_old[src_row], L = a.ptr_old[src_row + 1] - src;
     const int32_t dst = a.ptr_new[p];
-    if (!a.old2new) {  // rows only: a copy
-      for (int32_t i = threadIdx.x; i < L; i += R_THREADS) {
-        a.ind_new[dst + i] = a.ind_old[src + i];
-        if (a.val_new) a.val_new[dst + i] = a.val_old[src + i];
-      }
-      continue;
-    }
     block_sort(
         sh, L, a.val_new != nullptr,
         [&](int32_t i, int32_t &k, float &v) {
@@ -549,8 +743,7 @@ __device__ __forceinline__ LongTile long_tile(const ApplyArgs &a, int32_t id, in
   return t;
 }
 
-// One block per tile of R_MED entries of a long row: remapped and sorted into the scratch copy
-// (rows only: copied straight to the output).
+// One block per tile of R_MED entries of a long row: remapped and sorted into the scratch copy.
 __global__ void __launch_bounds__(R_THREADS) apply_tiles_kernel(ApplyArgs a) {
   extern __shared__ __align__(16) unsigned char apply_smem[];
   BlockSortShared &sh = *reinterpret_cast<BlockSortShared *>(apply_smem);
@@ -560,13 +753,6 @@ __global__ void __launch_bounds__(R_THREADS) apply_tiles_kernel(ApplyArgs a) {
     const LongTile t = long_tile(a, id, queued);
     const int32_t off = t.tile * R_MED;
     const int32_t len = t.L - off < R_MED ? t.L - off : R_MED;
-    if (!a.old2new) {
-      for (int32_t i = threadIdx.x; i < len; i += R_THREADS) {
-        a.ind_new[t.dst + off + i] = a.ind_old[t.src + off + i];
-        if (a.val_new) a.val_new[t.dst + off + i] = a.val_old[t.src + off + i];
-      }
-      continue;
-    }
     block_sort(
         sh, len, a.val_new != nullptr,
         [&](int32_t i, int32_t &k, float &v) {
@@ -583,7 +769,6 @@ __global__ void __launch_bounds__(R_THREADS) apply_tiles_kernel(ApplyArgs a) {
 // One block per tile again: every entry goes to the sum of its ranks in all tiles of its row
 // (its own index in its own tile).
 __global__ void __launch_bounds__(R_THREADS) apply_merge_kernel(ApplyArgs a) {
-  if (!a.old2new) return;
   const int32_t queued = static_cast<int32_t>(a.counters[CNT_LONG + 1]);
   const int32_t total = static_cast<int32_t>(a.counters[CNT_LONG]);
   for (int32_t id = blockIdx.x; id < total; id += gridDim.x) {
@@ -615,7 +800,8 @@ size_t reorder_workspace_bytes(int32_t n, int32_t nnz, int mode) {
   ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / 32 + 1));      // rows of 33..R_WARP entries
   ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / R_WARP + 1));  // rows of up to R_MED
   ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_MED + 1));      // longer rows
-  ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_WARP + 1));     // slices of a block-local permutation
+  ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / FLAT_TILE + 2));  // first row of every output tile
+  ar.take(sizeof(int32_t) * static_cast<size_t>(n));                     // row_delta
   if (mode == 1) {
     ar.take(sizeof(int32_t) * static_cast<size_t>(n));  // old2new
     ar.take(sizeof(int32_t) * static_cast<size_t>(nnz > 0 ? nnz : 1));  // sorted tiles: keys
@@ -635,6 +821,7 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   int32_t *block_sums = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nb) + 1)));
   ApplyArgs a;
   a.n = n;
+  a.nnz = nnz;
   a.ptr_old = d_ptr_old;
   a.ind_old = d_ind_old;
   a.val_old = with_vals ? d_val_old : nullptr;
@@ -646,7 +833,10 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   a.queue_warp = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / 32 + 1)));
   a.queue_block = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / R_WARP + 1)));
   a.queue_long = reinterpret_cast<int2 *>(ctx.ws + ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_MED + 1)));
-  a.queue_runs = reinterpret_cast<int2 *>(ctx.ws + ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_WARP + 1)));
+  int32_t *tile_row = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / FLAT_TILE + 2)));
+  a.tile_row = tile_row;
+  int32_t *row_delta = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * static_cast<size_t>(n)));
+  a.row_delta = row_delta;
   a.old2new = nullptr;
   a.tmp_key = nullptr;
   a.tmp_val = nullptr;
@@ -657,23 +847,42 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
     a.tmp_key = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * static_cast<size_t>(nnz > 0 ? nnz : 1)));
     a.tmp_val = reinterpret_cast<float *>(ctx.ws + ar.take(sizeof(float) * static_cast<size_t>(nnz > 0 ? nnz : 1)));
   }
-  const int sort_smem = static_cast<int>(sizeof(BlockSortShared));
-  CSG_CUDA(cudaFuncSetAttribute(apply_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem));
-  CSG_CUDA(cudaFuncSetAttribute(apply_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem));
   CSG_CUDA(cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), ctx.stream));
   len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums);
   CSG_CUDA(cudaGetLastError());
   scan_block_sums_kernel<<<1, 1024, 0, ctx.stream>>>(nb, block_sums);
   CSG_CUDA(cudaGetLastError());
-  ptr_new_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, d_ptr_new,
-                                                   old2new, a.counters + CNT_MOVED);
+  uint32_t *const outcome = reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  ++ctx.outcome_ticket;
+  ptr_new_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, nnz, d_ptr_old, d_new_order, block_sums, d_ptr_new,
+                                                   old2new, a.counters + CNT_MOVED, tile_row, row_delta,
+                                                   symmetric ? outcome : nullptr, ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
+  count_launches(3);
+  if (nnz == 0) return true;
+  bool local = false;
+  if (symmetric) {
+    if (!wait_outcome(ctx, ctx.stream)) return false;
+    local = reinterpret_cast<volatile uint32_t *>(outcome)[1] == 0u;
+  }
+  if (!symmetric || local) {
+    int64_t grid = (static_cast<int64_t>(nnz) + FLAT_TILE - 1) / FLAT_TILE;
+    if (grid > ctx.num_sms * 32) grid = ctx.num_sms * 32;
+    const int smem = symmetric ? static_cast<int>(sizeof(FlatShared)) : static_cast<int>(offsetof(FlatShared, run_head));
+    auto kernel = symmetric ? apply_flat_kernel<false> : apply_flat_kernel<true>;
+    CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<static_cast<int>(grid), R_THREADS, smem, ctx.stream>>>(a);
+    CSG_CUDA(cudaGetLastError());
+    count_launches(1);
+    return true;
+  }
+  const int sort_smem = static_cast<int>(sizeof(BlockSortShared));
+  CSG_CUDA(cudaFuncSetAttribute(apply_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem));
+  CSG_CUDA(cudaFuncSetAttribute(apply_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem));
   int64_t want = ((static_cast<int64_t>(n) + 31) / 32 * 32 + R_THREADS - 1) / R_THREADS;
   int grid = static_cast<int>(want < ctx.num_sms * 8 ? want : ctx.num_sms * 8);
   if (grid < 1) grid = 1;
   apply_short_kernel<<<grid, R_THREADS, 0, ctx.stream>>>(a);
-  CSG_CUDA(cudaGetLastError());
-  apply_runs_kernel<<<ctx.num_sms * 8, R_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   apply_warp_kernel<<<ctx.num_sms * 6, R_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
@@ -683,7 +892,7 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   CSG_CUDA(cudaGetLastError());
   apply_merge_kernel<<<ctx.num_sms * 4, R_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
-  count_launches(9);
+  count_launches(5);
   return true;
 }
 

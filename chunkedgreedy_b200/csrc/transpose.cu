@@ -21,9 +21,6 @@
 // every column of a row gets an entry of seg[]).
 // The reference can be promised a symmetric pattern and then reads the CSR arrays as the CSC
 // (sporder/src/common/csr2csc.h:52-54); nothing here needs the promise.
-#include <atomic>
-#include <chrono>
-
 #include "common.cuh"
 
 namespace csg {
@@ -106,7 +103,7 @@ __device__ __forceinline__ int32_t row_of(const int32_t *p, int32_t lo, int32_t 
 // more go on to blocks of 1024 threads for up to 22,528 (in up to 6144 columns), those with more
 // again to the tiled sort.
 // On a B200, 1.05 M rows of the shuffled mesh: 227 us with the groups read off the promised
-// symmetry, COMPACT_MESH without any promise; 65,536 rows of the power-law band: 173 -> COMPACT_ZIPF us.
+// symmetry, 115 without any promise; 65,536 rows of the power-law band: 173 -> 84 us.
 template <int THREADS_, int CAP_, int TABLE_BITS_, int FILTER_BITS_>
 struct CompactSize {
   static constexpr int THREADS = THREADS_, WARPS = THREADS / 32, CAP = CAP_, TABLE_BITS = TABLE_BITS_, FILTER_BITS = FILTER_BITS_;
@@ -796,7 +793,7 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     ctrl[CTRL_LANE_TICKET] = heavy;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
-    // for the host (read_outcome)
+    // for the host (wait_outcome)
     outcome[1] = heavy;
     outcome[2] = ctrl[CTRL_HEAVY_COUNT];
     __threadfence_system();
@@ -913,24 +910,6 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
   return true;
 }
 
-// What bucket_scan_kernel wrote to the context's pinned words, as soon as it is there: the row list
-// is still being written then, and the launches behind it are queued before it is done.
-bool read_outcome(Context &ctx, cudaStream_t st, uint32_t *heavy_rows, uint32_t *heavy_chunks) {
-  volatile uint32_t *const h = reinterpret_cast<volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
-  const auto start = std::chrono::steady_clock::now();
-  for (int spins = 0; h[0] != ctx.outcome_ticket; ++spins) {
-    // something went wrong on the device, or it is busy with other work: wait for the stream
-    if ((spins & 1023) == 1023 && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(200)) {
-      CSG_CUDA(cudaStreamSynchronize(st));
-      CSG_REQUIRE(h[0] == ctx.outcome_ticket, "internal: the transposition did not report its outcome");
-    }
-  }
-  std::atomic_thread_fence(std::memory_order_acquire);
-  *heavy_rows = h[1];
-  *heavy_chunks = h[2];
-  return true;
-}
-
 // the rows with candidates, longest stream first
 bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead) {
   int grid = (n + 255) / 256;
@@ -982,10 +961,11 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   if (!launch_compact(ctx, a, st)) return false;
   if (d_count) return launch_heavy(ctx, a, false, st);
   if (!launch_lists(ctx, n, chunk, s, nullptr)) return false;
-  uint32_t heavy_rows = 0, heavy_chunks = 0;
-  if (!read_outcome(ctx, st, &heavy_rows, &heavy_chunks)) return false;
-  s.no_heavy_rows = heavy_rows == 0;
-  if (heavy_chunks != 0) {
+  // (the row list is still being written then, and the launches behind it are queued in time)
+  if (!wait_outcome(ctx, st)) return false;
+  const volatile uint32_t *const outcome = reinterpret_cast<const volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  s.no_heavy_rows = outcome[1] == 0;
+  if (outcome[2] != 0) {
     s.no_heavy_rows = false;
     if (!launch_heavy(ctx, a, false, st)) return false;
     CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, sizeof(uint32_t) * WORK_BUCKETS, st));

@@ -155,6 +155,35 @@ def test_reorder_bit_exact(name, symmetric, golden):
         assert np.array_equal(_sha(gv.cpu().numpy()), golden[name + "/sym_val_sha256"])
 
 
+@pytest.mark.parametrize("nnz_cut", [0, 1, 2047, 2048, 2049, 4096, None])
+@pytest.mark.parametrize("with_val", [True, False])
+def test_reorder_in_tiles_of_the_output(nnz_cut, with_val):
+    # permutations inside blocks of 1024: runs (entries of a row in one block of columns) of every
+    # length up to a full block, across the ends of tiles, rows longer than a tile, rows without entries
+    sp = _sp()
+    rng = np.random.default_rng(5)
+    n = 5000
+    lens = rng.integers(0, 9, n)
+    lens[rng.choice(n, 60, replace=False)] = rng.integers(30, 120, 60)
+    lens[[7, 8, 1500, 4000]] = [4900, 3000, 1100, 2048]
+    lens[2000:2600] = 0
+    rows = np.repeat(np.arange(n), lens)
+    cols = np.concatenate([np.sort(rng.choice(n, l, replace=False)) for l in lens])
+    cols[rows == 1500] = 1024 + np.arange(1100)
+    if nnz_cut is not None:
+        rows, cols = rows[:nnz_cut], cols[:nnz_cut]
+    from chunkedgreedy_b200.synth import coo_to_csr
+    ptr, ind, val = coo_to_csr(n, rows, cols, rng.standard_normal(rows.size))
+    order = np.concatenate([b + rng.permutation(min(1024, n - b)) for b in range(0, n, 1024)]).astype(np.int32)
+    for symmetric in (True, False):
+        rp, ri, rv = oracle.reorder(ptr, ind, order, val, symmetric=symmetric)
+        got = sp.reorder(_dev(ptr), _dev(ind), _dev(order), val=_dev(val) if with_val else None, symmetric=symmetric)
+        assert np.array_equal(got[0].cpu().numpy(), rp)
+        assert np.array_equal(got[1].cpu().numpy(), ri)
+        if with_val:
+            assert np.array_equal(got[2].cpu().numpy(), rv)
+
+
 def test_reorder_random_permutation_long_rows():
     # rows of every size class: <= 32 (warp), <= 2048 (shared memory), longer (global)
     sp = _sp()
