@@ -1035,8 +1035,79 @@ __global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchAr
 }
 
 // ---- heavy rows through materialised streams ------------------------------------------
-// offsets of the heavy rows' streams in hstream; trims the heavy set to what fits
-__global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
+// part -> (heavy row, column range).  Uniform over the warp.
+struct PartRef {
+  uint32_t item;
+  int32_t r, pb, pe, row_size;
+};
+__device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, uint32_t heavy) {
+  uint32_t lo = 0, hi = heavy;  // part_base[lo] <= part < part_base[hi]
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a.part_base[mid] <= part)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  PartRef p;
+  p.item = lo;
+  p.r = a.row_list[lo];
+  const int32_t rb = a.row_seg[p.r], re = rb + a.row_cols[p.r];
+  p.row_size = a.ptr[p.r + 1] - a.ptr[p.r];
+  p.pb = rb + static_cast<int32_t>(part - a.part_base[lo]) * H_PART;
+  p.pe = p.pb + H_PART < re ? p.pb + H_PART : re;
+  return p;
+}
+
+// stream entries a part (H_PART columns of a heavy row) will produce; one warp
+__device__ __forceinline__ void count_part(const SketchArgs &a, uint32_t part, uint32_t heavy) {
+  const int lane = lane_id();
+  const PartRef p = part_ref(a, part, heavy);
+  uint32_t cnt = 0;
+  for (int32_t q = p.pb + lane; q < p.pe; q += 32) {
+    const int32_t len = a.seg[q].y;
+    cnt += len >= 2 ? static_cast<uint32_t>(len - 1) : 0u;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) cnt += __shfl_down_sync(FULL, cnt, off);
+  if (lane == 0) a.part_off[part] = cnt;
+}
+
+// counts -> offsets (exclusive scan in place, one block of 1024)
+__device__ __forceinline__ void scan_parts(const SketchArgs &a, uint32_t parts) {
+  __shared__ uint32_t sm[32];
+  __shared__ uint32_t carry_s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry_s = 0;
+  __syncthreads();
+  for (uint32_t base = 0; base < parts; base += 1024) {
+    const uint32_t i = base + threadIdx.x;
+    const uint32_t v = i < parts ? a.part_off[i] : 0u;
+    uint32_t incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(FULL, incl, off);
+      if (lane >= off) incl += t;
+    }
+    if (lane == 31) sm[warp] = incl;
+    __syncthreads();
+    uint32_t wbase = 0, tot = 0;
+    for (int w = 0; w < 32; ++w) {
+      const uint32_t t = sm[w];
+      if (w < warp) wbase += t;
+      tot += t;
+    }
+    const uint32_t carry = carry_s;
+    if (i < parts) a.part_off[i] = carry + wbase + incl - v;
+    __syncthreads();
+    if (threadIdx.x == 0) carry_s = carry + tot;
+    __syncthreads();
+  }
+}
+
+// Offsets of the heavy rows' streams in hstream; trims the heavy set to what fits.  with_parts:
+// the parts' offsets as well, which kernels of their own do in calls with many.
+__global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a, int with_parts) {
   __shared__ unsigned long long sm[32];
   __shared__ unsigned long long carry_s;
   __shared__ uint32_t count_s;
@@ -1104,82 +1175,22 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
     a.ctrl[CTRL_HEAVY_TICKET] = 0;
     a.ctrl[CTRL_HEAVY_TICKET + 1] = 0;
   }
+  if (!with_parts) return;
+  __syncthreads();
+  const uint32_t heavy = count_s, parts = a.ctrl[CTRL_HEAVY_PARTS];
+  for (uint32_t part = warp; part < parts; part += 32) count_part(a, part, heavy);
+  __syncthreads();
+  scan_parts(a, parts);
 }
 
-// part -> (heavy row, column range).  Uniform over the warp.
-struct PartRef {
-  uint32_t item;
-  int32_t r, pb, pe, row_size;
-};
-__device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, uint32_t heavy) {
-  uint32_t lo = 0, hi = heavy;  // part_base[lo] <= part < part_base[hi]
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a.part_base[mid] <= part)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  PartRef p;
-  p.item = lo;
-  p.r = a.row_list[lo];
-  const int32_t rb = a.row_seg[p.r], re = rb + a.row_cols[p.r];
-  p.row_size = a.ptr[p.r + 1] - a.ptr[p.r];
-  p.pb = rb + static_cast<int32_t>(part - a.part_base[lo]) * H_PART;
-  p.pe = p.pb + H_PART < re ? p.pb + H_PART : re;
-  return p;
-}
-
-// stream entries every part (H_PART columns of a heavy row) will produce
 __global__ void __launch_bounds__(256) heavy_part_count_kernel(SketchArgs a) {
-  const int lane = lane_id();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS], parts = a.ctrl[CTRL_HEAVY_PARTS];
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; part < parts; part += warps) {
-    const PartRef p = part_ref(a, part, heavy);
-    uint32_t cnt = 0;
-    for (int32_t q = p.pb + lane; q < p.pe; q += 32) {
-      const int32_t len = a.seg[q].y;
-      cnt += len >= 2 ? static_cast<uint32_t>(len - 1) : 0u;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) cnt += __shfl_down_sync(FULL, cnt, off);
-    if (lane == 0) a.part_off[part] = cnt;
-  }
+  for (uint32_t part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; part < parts; part += warps)
+    count_part(a, part, heavy);
 }
 
-// counts -> offsets (exclusive scan in place, one block)
-__global__ void __launch_bounds__(1024) heavy_part_scan_kernel(SketchArgs a) {
-  __shared__ uint32_t sm[32];
-  __shared__ uint32_t carry_s;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t parts = a.ctrl[CTRL_HEAVY_PARTS];
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < parts; base += 1024) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < parts ? a.part_off[i] : 0u;
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (lane == 31) sm[warp] = incl;
-    __syncthreads();
-    uint32_t wbase = 0, tot = 0;
-    for (int w = 0; w < 32; ++w) {
-      const uint32_t t = sm[w];
-      if (w < warp) wbase += t;
-      tot += t;
-    }
-    const uint32_t carry = carry_s;
-    if (i < parts) a.part_off[i] = carry + wbase + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + tot;
-    __syncthreads();
-  }
-}
+__global__ void __launch_bounds__(1024) heavy_part_scan_kernel(SketchArgs a) { scan_parts(a, a.ctrl[CTRL_HEAVY_PARTS]); }
 
 // one warp per part: its slice of the row's stream, written out in order
 __global__ void __launch_bounds__(S_THREADS) heavy_expand_kernel(SketchArgs a) {
@@ -1887,12 +1898,17 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
   constexpr bool in_rounds = CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
-    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
+    // (up to a million nonzeros there are a few thousand parts at most, less than a launch's worth)
+    const bool one_kernel = a.nnz <= 1 << 20;
+    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a, one_kernel ? 1 : 0);
     CSG_CUDA(cudaGetLastError());
-    heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
-    heavy_part_scan_kernel<<<1, 1024, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
+    if (!one_kernel) {
+      heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
+      CSG_CUDA(cudaGetLastError());
+      heavy_part_scan_kernel<<<1, 1024, 0, st>>>(a);
+      CSG_CUDA(cudaGetLastError());
+      count_launches(2);
+    }
     heavy_expand_kernel<<<ctx.num_sms * 8, S_THREADS, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
     // (the rest of the call starts its own chains only behind this point: by then the chains
@@ -1969,7 +1985,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   if (no_heavy_rows) return true;
   heavy_topk_kernel<CELLS><<<ctx.num_sms, S_THREADS, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
-  count_launches(6);
+  count_launches(4);
   return true;
 }
 

@@ -99,7 +99,7 @@ __device__ __forceinline__ int32_t row_of(const int32_t *p, int32_t lo, int32_t 
 //     of the group: its place.  (That is one comparison per candidate the sketch stage will have to
 //     work through, so it never dominates.)
 //  5. members go out with their groups in CSR order, which is the order seg[] wants.
-// Two sizes: blocks of 512 threads, two to an SM, for up to 4096 numbered nonzeros; chunks with
+// Two sizes: blocks of 512 threads, two to an SM, for up to 6144 numbered nonzeros (in up to 3072 columns); chunks with
 // more go on to blocks of 1024 threads for up to 22,528 (in up to 6144 columns), those with more
 // again to the tiled sort.
 // On a B200, 1.05 M rows of the shuffled mesh: 227 us with the groups read off the promised
@@ -126,7 +126,7 @@ struct CompactSize {
     int32_t ticket, columns;
   };
 };
-using CompactSmall = CompactSize<512, 4096, 13, 16>;
+using CompactSmall = CompactSize<512, 6144, 12, 17>;
 using CompactLarge = CompactSize<1024, 22528, 13, 17>;
 
 // exclusive sum over the block's threads; *total is the sum of all
