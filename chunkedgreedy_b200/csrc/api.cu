@@ -869,26 +869,25 @@ int32_t sporder_row_sums(sporder_context_t ctx, int32_t n, int32_t nnz, const in
   return csg::launch_row_sums(ctx->c, n, nnz, d_ptr, d_val, d_out) ? 0 : -1;
 }
 
-int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, int32_t classes,
-                            const float *d_P, const float *d_s, const float *d_W1, const float *d_b1,
-                            const float *d_W2, float *d_H, float *d_U) {
+int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, const float *d_Z,
+                            const float *d_W2, float *d_U) {
   csg::clear_error();
-  if (!ctx || !d_P || !d_s || !d_W1 || !d_b1 || !d_W2 || !d_H || !d_U) {
+  if (!ctx || !d_Z || !d_W2 || !d_U) {
     csg::set_error("gcn_forward: bad arguments");
     return -1;
   }
-  return csg::launch_gcn_forward(ctx->c, n, in_dim, hidden, classes, d_P, d_s, d_W1, d_b1, d_W2, d_H, d_U) ? 0 : -1;
+  return csg::launch_gcn_forward(ctx->c, n, hidden, classes, d_Z, d_W2, d_U) ? 0 : -1;
 }
 
 int32_t sporder_gcn_backward(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, int32_t classes,
-                             const float *d_G, const float *d_H, const float *d_P, const float *d_s,
+                             const float *d_G, const float *d_Z, const float *d_P, const float *d_s,
                              const float *d_W2, float *d_dW1, float *d_db1, float *d_dW2) {
   csg::clear_error();
-  if (!ctx || !d_G || !d_H || !d_P || !d_s || !d_W2 || !d_dW1 || !d_db1 || !d_dW2) {
+  if (!ctx || !d_G || !d_Z || !d_P || !d_s || !d_W2 || !d_dW1 || !d_db1 || !d_dW2) {
     csg::set_error("gcn_backward: bad arguments");
     return -1;
   }
-  return csg::launch_gcn_backward(ctx->c, n, in_dim, hidden, classes, d_G, d_H, d_P, d_s, d_W2, d_dW1, d_db1, d_dW2) ? 0 : -1;
+  return csg::launch_gcn_backward(ctx->c, n, in_dim, hidden, classes, d_G, d_Z, d_P, d_s, d_W2, d_dW1, d_db1, d_dW2) ? 0 : -1;
 }
 
 }  // extern "C"

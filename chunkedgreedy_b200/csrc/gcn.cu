@@ -1,17 +1,15 @@
-// The dense part of a two-layer GCN around the library's SpMM, forward and backward, fp32.
+// Dense parts of a two-layer GCN around the library's SpMM, fp32.
 //
 // The caller's model is Linear(in, hidden) -> A -> ReLU -> A -> Linear(hidden, classes)
-// (experiments/e2e_gcn.py:126-137).  With P = A x and the row sums s = A 1 computed first, and the
-// second product taken behind the second linear layer (it is narrower there), what is left
-// between the two sparse products is
-//   forward   H = relu(P W1^T + s b1^T),  U = H W2^T
-//   backward  (G = dL/dU)  D = (G W2) * (H > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T H.
-// One kernel each way: H leaves the first with bias and ReLU applied, D never exists in memory.
-// Both are bound by fp32 multiply-adds (2 n in hidden each way, against three passes over n rows
-// of 128 floats): blocks are persistent, one per SM, operands staged with cp.async a tile ahead,
-// 8 x 8 results per thread.  Per pass on 1.05 M rows,
-// 128 -> 128 -> 16, on a B200: 0.95 ms forward, 1.09 ms backward (53 % of the fp32 pipes; two warps per
-// scheduler, and the phases of a tile do not overlap); one torch kernel per operation took 1.8 and 2.4 ms.
+// (experiments/e2e_gcn.py:126-137).  With Z the first sparse product, P = A x and s = A 1 (the row
+// sums), and the second sparse product taken behind the second linear layer (it is narrower there):
+//   forward   U = relu(Z) W2^T
+//   backward  (G = dL/dU)  D = (G W2) * (Z > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T relu(Z).
+// One kernel each way; D never exists in memory.  The backward pass is bound by fp32 multiply-adds
+// (2 n in hidden of them, against three passes over n rows of 128 floats): blocks are persistent, one
+// per SM, operands staged with cp.async a tile ahead, 8 x 8 results per thread.  On 1.05 M rows,
+// 128 -> 128 -> 16, on a B200: 1.09 ms (53 % of the fp32 pipes; two warps per scheduler, and the
+// phases of a tile do not overlap); one torch kernel per operation took 2.4 ms.
 #include "../../include/sporder_b200.h"
 #include "common.cuh"
 
@@ -19,16 +17,15 @@ namespace csg {
 
 namespace {
 
-constexpr int F_THREADS = 256;  // threads of a block, forward
-constexpr int D_THREADS = 256;  // ... and backward
+constexpr int D_THREADS = 256;
 constexpr int F_ROWS = 128;  // rows per tile, forward
 constexpr int B_ROWS = 32;   // ... and backward
 constexpr int MAX_CLASSES = 48;
 
 struct DenseArgs {
   int32_t n, in, hid, cls;
-  const float *P, *s, *W1, *b1, *W2;
-  float *H, *U;       // outputs of the forward pass, H an input of the backward pass
+  const float *P, *s, *W2, *Z;
+  float *U;
   const float *G;
   float *part;        // backward: a block's sums
   float *dW1, *db1, *dW2;
@@ -67,42 +64,27 @@ __device__ __forceinline__ void fma2(float2 &acc, float2 a, float2 b) {
       : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
 }
 
-template <int IN_T, int HID_T>
+template <int HID_T>
 struct ForwardShared {
-  static constexpr int PS = IN_T + 4, HS = HID_T + 4;
-  static constexpr int TILE = F_ROWS * (PS > HS ? PS : HS);  // holds a tile of P, then of H
-  static constexpr int W1 = 0, W2 = W1 + IN_T * HID_T, B1 = W2 + MAX_CLASSES * HS, S = B1 + HID_T,
-                       TILES = S + 2 * F_ROWS, FLOATS = TILES + 2 * TILE;
+  static constexpr int HS = HID_T + 4;
+  static constexpr int W2 = 0, TILES = MAX_CLASSES * HS, FLOATS = TILES + 2 * F_ROWS * HS;
 };
 
-template <int IN_T, int HID_T>
-__global__ void __launch_bounds__(F_THREADS, 1) gcn_forward_kernel(DenseArgs a) {
-  using L = ForwardShared<IN_T, HID_T>;
-  constexpr int NC = HID_T / 16;               // columns per thread, in pairs
-  constexpr int TY = F_THREADS / 16, RPT = F_ROWS / TY;  // rows per thread, TY apart
+// Two threads per row, every other group of four classes each.  Bound by shared memory: a row of
+// Z and the weights are read from there once per group.
+template <int HID_T>
+__global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) {
+  using L = ForwardShared<HID_T>;
   extern __shared__ __align__(16) float dense_smem[];
-  float *const w1 = dense_smem + L::W1, *const w2 = dense_smem + L::W2, *const b1 = dense_smem + L::B1;
-  float *const s = dense_smem + L::S;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // W1 with a column of the result per column, entries of two successive inputs side by side
-  for (int i = tid; i < IN_T * HID_T; i += F_THREADS) {
-    const int k = i / (2 * HID_T) * 2 + (i & 1), j = i % (2 * HID_T) >> 1;
-    w1[i] = k < a.in && j < a.hid ? a.W1[static_cast<size_t>(j) * a.in + k] : 0.0f;
-  }
-  for (int i = tid; i < MAX_CLASSES * L::HS; i += F_THREADS) {
+  float *const w2 = dense_smem + L::W2;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < MAX_CLASSES * L::HS; i += D_THREADS) {
     const int c = i / L::HS, j = i % L::HS;
     w2[i] = c < a.cls && j < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + j] : 0.0f;
   }
-  for (int i = tid; i < HID_T; i += F_THREADS) b1[i] = i < a.hid ? a.b1[i] : 0.0f;
   const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
   auto stage = [&](int64_t t, int buf) {
-    if (t < tiles) {
-      stage_rows<F_ROWS, IN_T, F_THREADS>(dense_smem + L::TILES + buf * L::TILE, a.P, t * F_ROWS, a.n, a.in);
-      for (int i = tid; i < F_ROWS; i += F_THREADS) {
-        const bool on = t * F_ROWS + i < a.n;
-        copy4(s + buf * F_ROWS + i, a.s + (on ? t * F_ROWS + i : 0), on);
-      }
-    }
+    if (t < tiles) stage_rows<F_ROWS, HID_T, D_THREADS>(dense_smem + L::TILES + buf * F_ROWS * L::HS, a.Z, t * F_ROWS, a.n, a.hid);
     copies_commit();
   };
   stage(blockIdx.x, 0);
@@ -111,70 +93,23 @@ __global__ void __launch_bounds__(F_THREADS, 1) gcn_forward_kernel(DenseArgs a) 
     stage(t + gridDim.x, buf ^ 1);
     copies_wait<1>();
     __syncthreads();
-    float *const tile = dense_smem + L::TILES + buf * L::TILE;
-    float2 acc[RPT][NC];  // sums over the even and over the odd inputs
+    const float *const z = dense_smem + L::TILES + buf * F_ROWS * L::HS + (tid >> 1) * L::HS;
+    const int64_t r = t * F_ROWS + (tid >> 1);
+    for (int c0 = (tid & 1) * 4; c0 < a.cls; c0 += 8) {
+      float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+      for (int k = 0; k < HID_T; k += 4) {
+        float4 h = *reinterpret_cast<const float4 *>(z + k);
+        h = make_float4(fmaxf(h.x, 0.0f), fmaxf(h.y, 0.0f), fmaxf(h.z, 0.0f), fmaxf(h.w, 0.0f));
 #pragma unroll
-    for (int i = 0; i < RPT; ++i)
-#pragma unroll
-      for (int j = 0; j < NC; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
-#pragma unroll 2
-    for (int k = 0; k < IN_T; k += 4) {
-      float4 p[RPT];
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) p[i] = *reinterpret_cast<const float4 *>(tile + (ty + TY * i) * L::PS + k);
-#pragma unroll
-      for (int kk = 0; kk < 4; kk += 2) {
-        float2 w[NC];
-#pragma unroll
-        for (int j = 0; j < NC; j += 2)
-          *reinterpret_cast<float4 *>(w + j) = *reinterpret_cast<const float4 *>(w1 + (k + kk) * HID_T + 2 * (j / 2 * 32 + tx * 2));
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-          const float2 x = kk == 0 ? make_float2(p[i].x, p[i].y) : make_float2(p[i].z, p[i].w);
-#pragma unroll
-          for (int j = 0; j < NC; ++j) fma2(acc[i][j], x, w[j]);
+        for (int c = 0; c < 4; ++c) {
+          const float4 w = *reinterpret_cast<const float4 *>(w2 + (c0 + c) * L::HS + k);
+          u[c] = fmaf(h.x, w.x, fmaf(h.y, w.y, fmaf(h.z, w.z, fmaf(h.w, w.w, u[c]))));
         }
       }
-    }
-    __syncthreads();  // P of this tile is done with: its place takes H
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      const int r = ty + TY * i;
-      const float si = s[buf * F_ROWS + r];
-#pragma unroll
-      for (int jj = 0; jj < NC; ++jj) {
-        const int j = jj / 2 * 32 + tx * 2 + (jj & 1);
-        tile[r * L::HS + j] = fmaxf(fmaf(si, b1[j], acc[i][jj].x + acc[i][jj].y), 0.0f);
-      }
-    }
-    __syncthreads();
-    const int64_t r0 = t * F_ROWS;
-    for (int i = tid; i < F_ROWS * (HID_T / 4); i += F_THREADS) {
-      const int r = i / (HID_T / 4), c = (i % (HID_T / 4)) * 4;
-      if (r0 + r < a.n && c < a.hid)
-        __stcs(reinterpret_cast<float4 *>(a.H + (r0 + r) * a.hid + c), *reinterpret_cast<const float4 *>(tile + r * L::HS + c));
-    }
-    // U: two threads per row, every other group of four classes each
-    {
-      constexpr int TPR = F_THREADS / F_ROWS;
-      const int r = tid / TPR;
-      if (r0 + r < a.n) {
-        for (int c0 = tid % TPR * 4; c0 < a.cls; c0 += 4 * TPR) {
-          float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-          for (int k = 0; k < HID_T; k += 4) {
-            const float4 h = *reinterpret_cast<const float4 *>(tile + r * L::HS + k);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float4 w = *reinterpret_cast<const float4 *>(w2 + (c0 + c) * L::HS + k);
-              u[c] = fmaf(h.x, w.x, fmaf(h.y, w.y, fmaf(h.z, w.z, fmaf(h.w, w.w, u[c]))));
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (c0 + c < a.cls) a.U[(r0 + r) * a.cls + c0 + c] = u[c];
-        }
-      }
+      for (int c = 0; c < 4; ++c)
+        if (c0 + c < a.cls && r < a.n) a.U[r * a.cls + c0 + c] = u[c];
     }
     __syncthreads();  // the tile's place is free for the copies of the round after next
   }
@@ -225,7 +160,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
       float *const b = dense_smem + L::BUF + buf * L::BUF_FLOATS;
       const int64_t r0 = t * B_ROWS;
       stage_rows<B_ROWS, IN_T, D_THREADS>(b + L::P, a.P, r0, a.n, a.in);
-      stage_rows<B_ROWS, HID_T, D_THREADS>(b + L::H, a.H, r0, a.n, a.hid);
+      stage_rows<B_ROWS, HID_T, D_THREADS>(b + L::H, a.Z, r0, a.n, a.hid);
       for (int i = tid; i < B_ROWS * a.cls; i += D_THREADS) {
         const int r = i / a.cls, c = i % a.cls;
         const bool on = r0 + r < a.n;
@@ -277,7 +212,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int i = 0; i < NI / 2; ++i) fma2(acc[j][i], make_float2(dj[j], dj[j]), pi[i]);
-      const float hv = h[r * L::HS + hj];
+      const float hv = fmaxf(h[r * L::HS + hj], 0.0f);
 #pragma unroll
       for (int c = 0; c < PER; c += VC) {
         float gv[VC];
@@ -396,13 +331,13 @@ bool dense_smem_limit(Kernel kernel, size_t bytes) {
   return true;
 }
 
-template <int IN_T, int HID_T>
+template <int HID_T>
 bool forward_variant(Context &ctx, const DenseArgs &a) {
-  const size_t smem = sizeof(float) * ForwardShared<IN_T, HID_T>::FLOATS;
-  if (!dense_smem_limit(gcn_forward_kernel<IN_T, HID_T>, smem)) return false;
+  const size_t smem = sizeof(float) * ForwardShared<HID_T>::FLOATS;
+  if (!dense_smem_limit(gcn_forward_kernel<HID_T>, smem)) return false;
   const int64_t tiles = (static_cast<int64_t>(a.n) + F_ROWS - 1) / F_ROWS;
   const int grid = static_cast<int>(tiles < ctx.num_sms ? tiles : ctx.num_sms);
-  gcn_forward_kernel<IN_T, HID_T><<<grid, F_THREADS, smem, ctx.stream>>>(a);
+  gcn_forward_kernel<HID_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(1);
   return true;
@@ -430,17 +365,15 @@ bool check_dense(const DenseArgs &a) {
                   a.cls >= 1 && a.cls <= MAX_CLASSES,
               "gcn: expect in and hidden in multiples of 4 up to 128 and up to %d classes (got %d, %d, %d)", MAX_CLASSES,
               a.in, a.hid, a.cls);
-  const uintptr_t all = reinterpret_cast<uintptr_t>(a.P) | reinterpret_cast<uintptr_t>(a.H);
-  CSG_REQUIRE(all % 16 == 0, "gcn: P and H must be 16-byte aligned");
+  const uintptr_t all = reinterpret_cast<uintptr_t>(a.P) | reinterpret_cast<uintptr_t>(a.Z);
+  CSG_REQUIRE(all % 16 == 0, "gcn: P and Z must be 16-byte aligned");
   return true;
 }
 
 bool run_forward(Context &ctx, const DenseArgs &a) {
   if (!check_dense(a)) return false;
   CSG_CUDA(cudaSetDevice(ctx.device));
-  if (a.in <= 64)
-    return a.hid <= 32 ? forward_variant<64, 32>(ctx, a) : a.hid <= 64 ? forward_variant<64, 64>(ctx, a) : forward_variant<64, 128>(ctx, a);
-  return a.hid <= 32 ? forward_variant<128, 32>(ctx, a) : a.hid <= 64 ? forward_variant<128, 64>(ctx, a) : forward_variant<128, 128>(ctx, a);
+  return a.hid <= 32 ? forward_variant<32>(ctx, a) : a.hid <= 64 ? forward_variant<64>(ctx, a) : forward_variant<128>(ctx, a);
 }
 
 template <int CLS_T>
@@ -479,14 +412,13 @@ bool run_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *ptr, cons
 
 }  // namespace
 
-bool launch_gcn_forward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *P, const float *s,
-                        const float *W1, const float *b1, const float *W2, float *H, float *U) {
-  DenseArgs a = {n, in, hid, cls, P, s, W1, b1, W2, H, U, nullptr, nullptr, nullptr, nullptr, nullptr};
+bool launch_gcn_forward(Context &ctx, int32_t n, int32_t hid, int32_t cls, const float *Z, const float *W2, float *U) {
+  DenseArgs a = {n, 4, hid, cls, nullptr, nullptr, W2, Z, U, nullptr, nullptr, nullptr, nullptr, nullptr};
   return run_forward(ctx, a);
 }
-bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *G, const float *H,
+bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *G, const float *Z,
                          const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2) {
-  DenseArgs a = {n, in, hid, cls, P, s, nullptr, nullptr, W2, const_cast<float *>(H), nullptr, G, nullptr, dW1, db1, dW2};
+  DenseArgs a = {n, in, hid, cls, P, s, W2, Z, nullptr, G, nullptr, dW1, db1, dW2};
   return run_backward(ctx, a);
 }
 bool launch_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr, const float *d_val, float *d_out) {

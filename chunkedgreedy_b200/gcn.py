@@ -75,50 +75,53 @@ class GraphOperator:
         return self.spmm_ms
 
 
-class DenseFn(torch.autograd.Function):
-    """relu(P W1^T + s b1^T) W2^T, in one kernel forward and one backward; no gradient for P
-    and s."""
+class LayersFn(torch.autograd.Function):
+    """relu(op(x W1^T + b1)) W2^T for features that want no gradient.  The backward pass needs the
+    first layer's gradient D^T op(x) (op is symmetric: op(D)^T x), so it takes one sparse product
+    over the features and everything dense in one kernel."""
 
     @staticmethod
-    def forward(ctx, P, s, w1, b1, w2, lib_ctx):
-        n, hidden, classes = P.shape[0], w1.shape[0], w2.shape[0]
-        P, w1, b1, w2 = P.contiguous(), w1.contiguous(), b1.contiguous(), w2.contiguous()
-        H = torch.empty((n, hidden), dtype=torch.float32, device=P.device)
-        U = torch.empty((n, classes), dtype=torch.float32, device=P.device)
-        ctx.lib_ctx = _ctx(lib_ctx, P)
-        with torch.cuda.device(P.device):
-            _enter(ctx.lib_ctx, P)
-            if _lib.load().sporder_gcn_forward(ctx.lib_ctx.handle, n, P.shape[1], hidden, classes, P.data_ptr(),
-                                               s.data_ptr(), w1.data_ptr(), b1.data_ptr(), w2.data_ptr(),
-                                               H.data_ptr(), U.data_ptr()) != 0:
+    def forward(ctx, x, op, w1, b1, w2):
+        n, hidden, classes = x.shape[0], w1.shape[0], w2.shape[0]
+        x, w2 = x.contiguous(), w2.contiguous()
+        z = op(torch.mm(x, w1.t()).add_(b1))
+        u = torch.empty((n, classes), dtype=torch.float32, device=x.device)
+        ctx.lib_ctx = _ctx(getattr(op, "ctx", None), x)
+        with torch.cuda.device(x.device):
+            _enter(ctx.lib_ctx, x)
+            if _lib.load().sporder_gcn_forward(ctx.lib_ctx.handle, n, hidden, classes, z.data_ptr(), w2.data_ptr(),
+                                               u.data_ptr()) != 0:
                 _lib.check()
-        ctx.save_for_backward(P, s, H, w2)
-        return U
+        ctx.op = op
+        ctx.save_for_backward(x, z, w2)
+        return u
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, g):
-        P, s, H, w2 = ctx.saved_tensors
-        n, in_dim, hidden, classes = P.shape[0], P.shape[1], H.shape[1], w2.shape[0]
+        x, z, w2 = ctx.saved_tensors
+        op = ctx.op
+        n, in_dim, hidden, classes = x.shape[0], x.shape[1], z.shape[1], w2.shape[0]
         g = g.contiguous()
-        dw1 = torch.empty((hidden, in_dim), dtype=torch.float32, device=P.device)
-        db1 = torch.empty(hidden, dtype=torch.float32, device=P.device)
-        dw2 = torch.empty((classes, hidden), dtype=torch.float32, device=P.device)
-        with torch.cuda.device(P.device):
-            _enter(ctx.lib_ctx, P)
+        p = op(x)
+        s = op.row_sums() if hasattr(op, "row_sums") else op(torch.ones_like(x[:, :1]))[:, 0].contiguous()
+        dw1 = torch.empty((hidden, in_dim), dtype=torch.float32, device=x.device)
+        db1 = torch.empty(hidden, dtype=torch.float32, device=x.device)
+        dw2 = torch.empty((classes, hidden), dtype=torch.float32, device=x.device)
+        with torch.cuda.device(x.device):
+            _enter(ctx.lib_ctx, x)
             if _lib.load().sporder_gcn_backward(ctx.lib_ctx.handle, n, in_dim, hidden, classes, g.data_ptr(),
-                                                H.data_ptr(), P.data_ptr(), s.data_ptr(), w2.data_ptr(),
+                                                z.data_ptr(), p.data_ptr(), s.data_ptr(), w2.data_ptr(),
                                                 dw1.data_ptr(), db1.data_ptr(), dw2.data_ptr()) != 0:
                 _lib.check()
-        return None, None, dw1, db1, dw2, None
+        return None, None, dw1, db1, dw2
 
 
 class GCN(torch.nn.Module):
-    """Linear -> op -> ReLU -> op -> Linear.  The sparse products are taken where they are
-    narrowest, which does not change what is computed: op is linear in its columns, so
-    op(x W1^T + b1) = op(x) W1^T + op(1) b1^T and op(h) W2^T = op(h W2^T).  With the operator in front of
-    the first layer, training needs no product for that layer's gradient at all (features carry
-    none)."""
+    """Linear -> op -> ReLU -> op -> Linear, the second operator taken behind the linear layer
+    where that is narrower (op is linear in its columns: op(h) W2^T = op(h W2^T)).  The first layer
+    keeps its order: hidden units within a rounding of zero decide by their sign, and op(x) W1^T rounds
+    differently."""
 
     def __init__(self, in_dim, hidden, classes):
         super().__init__()
@@ -128,21 +131,13 @@ class GCN(torch.nn.Module):
     def forward(self, x, op):
         hidden, in_dim = self.w1.weight.shape
         classes = self.w2.weight.shape[0]
-        training = torch.is_grad_enabled()
-        # columns of sparse products, operator first against layer first, forward and backward
-        first = in_dim * (2 if training and x.requires_grad else 1)
-        if first <= hidden * (2 if training else 1) and self.w1.bias is not None:
-            p = SpMMFn.apply(x, op)
-            s = op.row_sums() if hasattr(op, "row_sums") else op(torch.ones_like(x[:, :1]))[:, 0].contiguous()
-            # limits of the fused kernels; others, and features that want a gradient, by torch
-            if (not p.requires_grad and in_dim % 4 == 0 and in_dim <= 128 and hidden % 4 == 0
-                    and hidden <= 128 and classes <= 48 and classes <= hidden
-                    and all(t.is_cuda and t.dtype == torch.float32 for t in (p, s, self.w1.weight, self.w2.weight))):
-                u = DenseFn.apply(p, s, self.w1.weight, self.w1.bias, self.w2.weight, getattr(op, "ctx", None))
-                return SpMMFn.apply(u, op) + self.w2.bias
-            h = F.relu(torch.addr(F.linear(p, self.w1.weight), s, self.w1.bias))
-        else:
-            h = F.relu(SpMMFn.apply(self.w1(x), op))
+        # limits of the fused kernels; others, and features that want a gradient, by torch
+        if (not x.requires_grad and in_dim % 4 == 0 and in_dim <= min(128, 2 * hidden) and hidden % 4 == 0
+                and hidden <= 128 and classes <= min(48, hidden) and self.w1.bias is not None
+                and all(t.is_cuda and t.dtype == torch.float32 for t in (x, self.w1.weight, self.w2.weight))):
+            u = LayersFn.apply(x, op, self.w1.weight, self.w1.bias, self.w2.weight)
+            return SpMMFn.apply(u, op) + self.w2.bias
+        h = F.relu(SpMMFn.apply(self.w1(x), op))
         if classes < hidden:
             return SpMMFn.apply(F.linear(h, self.w2.weight), op) + self.w2.bias
         return self.w2(SpMMFn.apply(h, op))

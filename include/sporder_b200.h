@@ -267,20 +267,19 @@ SPORDER_API int32_t sporder_spmm_static(int32_t n, int32_t nnz, int32_t w, const
 SPORDER_API int32_t sporder_row_sums(sporder_context_t ctx, int32_t n, int32_t nnz,
                                      const int32_t *d_ptr, const float *d_val, float *d_out);
 
-/* Dense part of a two-layer GCN between its two sparse products, fp32, row-major.  With
- * P = A x (n x in_dim) and s = A 1 (n):
- *   forward:  H = relu(P W1^T + s b1^T) (n x hidden), U = H W2^T (n x classes);
- *   backward, for G = dL/dU: with D = (G W2) masked by H > 0,
- *             dW1 = D^T P, db1 = D^T s, dW2 = G^T H (overwritten, not added to).
- * in_dim and hidden in multiples of 4 up to 128, classes up to 48, P and H 16-byte aligned.
+/* Dense parts of a two-layer GCN, fp32, row-major.  With Z the first sparse product
+ * (n x hidden), P = A x (n x in_dim) and s = A 1 (n):
+ *   forward:  U = relu(Z) W2^T (n x classes);
+ *   backward, for G = dL/dU: with D = (G W2) masked by Z > 0,
+ *             dW1 = D^T P, db1 = D^T s, dW2 = G^T relu(Z) (overwritten, not added to).
+ * in_dim and hidden in multiples of 4 up to 128, classes up to 48, P and Z 16-byte aligned.
  * The sums of the backward pass are taken in the same order on every call.  Return 0 or -1. */
-SPORDER_API int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t in_dim,
-                                        int32_t hidden, int32_t classes, const float *d_P,
-                                        const float *d_s, const float *d_W1, const float *d_b1,
-                                        const float *d_W2, float *d_H, float *d_U);
+SPORDER_API int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t hidden,
+                                        int32_t classes, const float *d_Z, const float *d_W2,
+                                        float *d_U);
 SPORDER_API int32_t sporder_gcn_backward(sporder_context_t ctx, int32_t n, int32_t in_dim,
                                          int32_t hidden, int32_t classes, const float *d_G,
-                                         const float *d_H, const float *d_P, const float *d_s,
+                                         const float *d_Z, const float *d_P, const float *d_s,
                                          const float *d_W2, float *d_dW1, float *d_db1,
                                          float *d_dW2);
 
