@@ -72,6 +72,7 @@ SYMBOLS = {
     "sporder_spmm_async": (C.c_int32, [_P, C.c_int32, C.c_int32, C.c_int32, _P, _P, _P, _P, _P]),
     "sporder_spmm_static": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P]),
     "sporder_row_sums": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P]),
+    "sporder_linear": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 4),
     "sporder_gcn_forward": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 3),
     "sporder_gcn_backward": (C.c_int32, [_P] + [C.c_int32] * 4 + [_P] * 8),
     "sporder_kernel_launches": (C.c_uint64, []),

@@ -869,6 +869,16 @@ int32_t sporder_row_sums(sporder_context_t ctx, int32_t n, int32_t nnz, const in
   return csg::launch_row_sums(ctx->c, n, nnz, d_ptr, d_val, d_out) ? 0 : -1;
 }
 
+int32_t sporder_linear(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t out_dim, const float *d_x,
+                       const float *d_W, const float *d_b, float *d_Y) {
+  csg::clear_error();
+  if (!ctx || !d_x || !d_W || !d_b || !d_Y) {
+    csg::set_error("linear: bad arguments");
+    return -1;
+  }
+  return csg::launch_linear(ctx->c, n, in_dim, out_dim, d_x, d_W, d_b, d_Y) ? 0 : -1;
+}
+
 int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, const float *d_Z,
                             const float *d_W2, float *d_U) {
   csg::clear_error();

@@ -83,11 +83,16 @@ class LayersFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, op, w1, b1, w2):
         n, hidden, classes = x.shape[0], w1.shape[0], w2.shape[0]
-        x, w2 = x.contiguous(), w2.contiguous()
-        z = op(torch.mm(x, w1.t()).add_(b1))
+        x, w1, b1, w2 = x.contiguous(), w1.contiguous(), b1.contiguous(), w2.contiguous()
+        y = torch.empty((n, hidden), dtype=torch.float32, device=x.device)
         u = torch.empty((n, classes), dtype=torch.float32, device=x.device)
         ctx.lib_ctx = _ctx(getattr(op, "ctx", None), x)
         with torch.cuda.device(x.device):
+            _enter(ctx.lib_ctx, x)
+            if _lib.load().sporder_linear(ctx.lib_ctx.handle, n, x.shape[1], hidden, x.data_ptr(), w1.data_ptr(),
+                                          b1.data_ptr(), y.data_ptr()) != 0:
+                _lib.check()
+            z = op(y)
             _enter(ctx.lib_ctx, x)
             if _lib.load().sporder_gcn_forward(ctx.lib_ctx.handle, n, hidden, classes, z.data_ptr(), w2.data_ptr(),
                                                u.data_ptr()) != 0:
@@ -133,7 +138,7 @@ class GCN(torch.nn.Module):
         classes = self.w2.weight.shape[0]
         # limits of the fused kernels; others, and features that want a gradient, by torch
         if (not x.requires_grad and in_dim % 4 == 0 and in_dim <= min(128, 2 * hidden) and hidden % 4 == 0
-                and hidden <= 128 and classes <= min(48, hidden) and self.w1.bias is not None
+                and hidden <= 128 and classes <= min(48, hidden) and self.w1.bias is not None and x.data_ptr() % 16 == 0
                 and all(t.is_cuda and t.dtype == torch.float32 for t in (x, self.w1.weight, self.w2.weight))):
             u = LayersFn.apply(x, op, self.w1.weight, self.w1.bias, self.w2.weight)
             return SpMMFn.apply(u, op) + self.w2.bias

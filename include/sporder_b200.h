@@ -267,6 +267,13 @@ SPORDER_API int32_t sporder_spmm_static(int32_t n, int32_t nnz, int32_t w, const
 SPORDER_API int32_t sporder_row_sums(sporder_context_t ctx, int32_t n, int32_t nnz,
                                      const int32_t *d_ptr, const float *d_val, float *d_out);
 
+/* Y = x W^T + b, fp32, row-major: x n x in_dim, W out_dim x in_dim, both dimensions in multiples
+ * of 4 up to 128, x and Y 16-byte aligned.  Inputs are summed in order, the bias added last.
+ * Queued without waiting.  Returns 0 or -1. */
+SPORDER_API int32_t sporder_linear(sporder_context_t ctx, int32_t n, int32_t in_dim,
+                                   int32_t out_dim, const float *d_x, const float *d_W,
+                                   const float *d_b, float *d_Y);
+
 /* Dense parts of a two-layer GCN, fp32, row-major.  With Z the first sparse product
  * (n x hidden), P = A x (n x in_dim) and s = A 1 (n):
  *   forward:  U = relu(Z) W2^T (n x classes);

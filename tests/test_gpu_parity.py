@@ -594,6 +594,30 @@ def test_gcn_model_against_fp64(n, sizes, want_x):
         assert float((got.double() - want).norm()) <= 2e-5 * float(want.norm()) + 1e-6
 
 
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 30_000])
+@pytest.mark.parametrize("in_dim,out_dim", [(4, 4), (64, 32), (64, 64), (64, 128), (100, 64), (128, 36), (128, 128)])
+def test_linear_rounds_like_the_plain_product(n, in_dim, out_dim):
+    # hidden units near zero decide by their sign, so the layer must round as torch's does
+    sp = _sp()
+    from chunkedgreedy_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((n, in_dim), device="cuda", generator=g)
+    w = torch.randn((out_dim, in_dim), device="cuda", generator=g)
+    b = torch.randn(out_dim, device="cuda", generator=g)
+    y = torch.full((n, out_dim), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    ctx = sp.Context()
+    assert _lib.load().sporder_linear(ctx.handle, n, in_dim, out_dim, x.data_ptr(), w.data_ptr(), b.data_ptr(),
+                                      y.data_ptr()) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    want = x.double() @ w.double().t() + b.double()
+    scale = x.abs() @ w.abs().t() + b.abs()
+    assert torch.all((y.double() - want).abs() <= 1e-6 * scale)
+    if n == 30_000 and in_dim >= 64 and out_dim in (32, 64, 128):
+        assert torch.equal(y, torch.nn.functional.linear(x, w, b))
+    ctx.close()
+
+
 @pytest.mark.parametrize("name", ["stencil1024", "road2m"])
 def test_full_size_streaming_workloads_bit_exact(name):
     # benchmark configurations 2 and 3 at their full sizes (1.05 M / 2 M rows): the oracle
