@@ -433,10 +433,14 @@ __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_rows_kernel(S
 // Second launch: the pieces (a.piece nonzeros each) of the queued long rows, spread over
 // all lane groups; piece number -> queue entry by binary search on the entries' first
 // piece numbers (ascending by construction).  Partial rows are added with atomics.
+// Twice as many gathers in flight as the first launch has: a piece is a plain run of them, and
+// what bounds it is the latency of memory (R-MAT scale 22, width 128: 1.21 ms with eight rows of B at
+// a time, 0.94 with sixteen; 0.96 with eight in four blocks per SM.  The first launch, which has
+// its walk in registers beside, slows down by a quarter either way).
 template <int G, int VEC, int PAN, bool MASK>
 __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(SpmmArgs a) {
   constexpr int PER_WARP = 32 / G;
-  constexpr int U = Step<PAN>::U;
+  constexpr int U = 2 * Step<PAN>::U;
   const int lane = threadIdx.x & 31;
   const int sub = lane / G, gl = lane % G;
   const int32_t group = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER_WARP + sub;
@@ -464,7 +468,7 @@ __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(S
       for (int pn = 0; pn < PAN; ++pn)
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[pn][v] = 0.0f;
-      for (int32_t p = pb; p < pe; p += U) fma_step<G, VEC, PAN, MASK>(a, p, pe - p < U ? pe - p : U, col0, acc);
+      for (int32_t p = pb; p < pe; p += U) fma_step<G, VEC, PAN, MASK, U>(a, p, pe - p < U ? pe - p : U, col0, acc);
 #pragma unroll
       for (int pn = 0; pn < PAN; ++pn)
         if (panel_on<G, VEC, MASK>(col0, pn, a.w))
