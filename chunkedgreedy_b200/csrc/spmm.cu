@@ -528,6 +528,9 @@ template <int G, int VEC, int PAN, bool MASK>
 __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(SpmmArgs a) {
   constexpr int PER_WARP = 32 / G;
   constexpr int U = 2 * Step<PAN>::U;
+  constexpr int LONG_PAIRS = 256;  // pairs staged per warp
+  __shared__ int2 spair[G == 32 ? M_WARPS : 1][G == 32 ? LONG_PAIRS : 1];
+  [[maybe_unused]] int2 *const sp = spair[G == 32 ? threadIdx.x >> 5 : 0];
   const int lane = threadIdx.x & 31;
   const int sub = lane / G, gl = lane % G;
   const int32_t group = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER_WARP + sub;
@@ -555,7 +558,22 @@ __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(S
       for (int pn = 0; pn < PAN; ++pn)
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[pn][v] = 0.0f;
-      for (int32_t p = pb; p < pe; p += U) fma_step<G, VEC, PAN, MASK, U>(a, p, pe - p < U ? pe - p : U, col0, acc);
+      if constexpr (G == 32) {  // the pairs through shared memory, as in whole_unit
+        const char *bcol = reinterpret_cast<const char *>(a.B + col0);
+        for (int32_t p = pb; p < pe; p += LONG_PAIRS) {
+          const int32_t part = pe - p < LONG_PAIRS ? pe - p : LONG_PAIRS;
+          __syncwarp();
+          for (int32_t k = lane; k < part; k += 32)
+            sp[k] = make_int2(__ldcs(a.ind + p + k), __float_as_int(__ldcs(a.val + p + k)));
+          __syncwarp();
+          int32_t k = 0;
+          for (; part - k >= U; k += U) short_slots<G, VEC, PAN, MASK, U>(sp + k, bcol, a.w * 4, col0, acc);
+          staged_row<G, VEC, PAN, MASK>(sp + k, part - k, bcol, a.w * 4, col0, acc);
+        }
+      } else {
+        for (int32_t p = pb; p < pe; p += U)
+          fma_step<G, VEC, PAN, MASK, U>(a, p, pe - p < U ? pe - p : U, col0, acc);
+      }
 #pragma unroll
       for (int pn = 0; pn < PAN; ++pn)
         if (panel_on<G, VEC, MASK>(col0, pn, a.w))
