@@ -424,6 +424,23 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
       if (count > 0) whole_unit<VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
     return;
   }
+  // Narrower, but with a column for each lane of a warp: units of short rows by lane groups, in the
+  // others a row to the whole warp.  Walked by lane groups, those took trips in turn for columns and
+  // gathers, and code for a remainder of each group's own.  At widths 32, 40 and 64: R-MAT scale
+  // 20 took 464, 866 and 666 us, now 384, 510 and 466; 65,536 Zipf rows 51, 104 and 75 us, now 48, 57 and
+  // 52.  At 16 half of each load would be idle, and the walk is faster.
+  if constexpr (G < 32 && G * VEC >= 32) {
+    static_assert(PAN == 1, "one panel covers the row");
+    int32_t first = 0, count = 0;
+    while (draw_unit(a, wp, lane, &first, &count)) {
+      if (count == 0) continue;
+      if (unit_is_short(wp, count, a.nnz, lane))
+        short_rows<G, VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
+      else
+        whole_unit<G * VEC / 32, 1, MASK>(a, wp, spair[warp], first, count, lane);
+    }
+    return;
+  }
   const int panels = (a.w + G * VEC - 1) / (G * VEC);
   // warp-uniform: the rows in hand [bfirst, bfirst + bcount) and how many of them are given out
   int32_t bfirst = 0, bcount = 0, bnext = 0;
@@ -601,7 +618,9 @@ bool launch_variant(Context &ctx, SpmmArgs a) {
   a.piece = a.split / 4;
   spmm_rows_kernel<G, VEC, PAN, MASK><<<ctx.num_sms * (G == 32 ? 4 : M_BLOCKS_PER_SM), M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
-  spmm_long_kernel<G, VEC, PAN, MASK><<<grid, M_THREADS, 0, ctx.stream>>>(a);
+  // (a piece goes to a whole warp wherever each of its lanes has a column)
+  constexpr int LG = G * VEC >= 32 ? 32 : G;
+  spmm_long_kernel<LG, G * VEC / LG, PAN, MASK><<<grid, M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
   return true;

@@ -331,7 +331,7 @@ def test_spmm_on_units_of_short_rows(w, longest):
     assert np.array_equal(C, C2)
 
 
-@pytest.mark.parametrize("w", [3, 5, 6, 9, 12, 31, 33, 41, 66, 100, 130, 260])
+@pytest.mark.parametrize("w", [3, 5, 6, 9, 12, 31, 33, 34, 36, 41, 62, 66, 100, 130, 260])
 def test_spmm_ragged_widths_and_rows_at_the_split(w):
     # widths that fill their lane groups in part (one, two and four columns per lane, one and
     # two panels per walk), rows of both sides of the limit a group walks alone, and operands
