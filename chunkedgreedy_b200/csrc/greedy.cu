@@ -201,8 +201,8 @@ __global__ void __launch_bounds__(G_WARPS * 32) greedy_kernel(GreedyArgs a) {
 //    that needs the one before it, and written without care the step takes 460 cycles instead of 135.
 // On a B200, per call: power-law band of 65,536 rows 320 -> 74 us (64 chains, the longest of 900
 // steps), R-MAT scale 22 646 -> 258 us (4096 chains).
-// A candidate without a list of its own (only a false promise of symmetry makes one) would let
-// the chain reach bare rows: such a chunk runs on the table.
+// A candidate without a list of its own (a caller's own table can hold one) would let the
+// chain reach bare rows: such a chunk runs on the table.
 constexpr int GS_MAX_SPAN = 32768;   // rows of a chunk: their numbers must fit 15 bits
 constexpr uint32_t BARE = 0x8000u;   // in `place`: a bare row's place in the chunk, else a numbered row
 constexpr int GS_WINDOW = 32;        // flags behind the last row that read as visited

@@ -1892,9 +1892,9 @@ __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
 template <int CELLS>
 bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_rows) {
   // A call that runs one chunk ahead has two of these sequences in flight: the chunk ahead on
-  // the side stream with a quarter of the SMs for its chains, the rest on the context's stream
-  // with the other three quarters (a chain block takes a whole SM, and the kernel of the other
-  // rows starts only when every chain block has one).
+  // the side stream, the rest on the context's stream.  Where a chain block takes a whole SM
+  // (sketches beyond ROUND_CELLS) the two share the SMs, since the kernel of the other rows starts
+  // only when every chain block has one.
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
   constexpr bool in_rounds = CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
@@ -1935,7 +1935,9 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
       CSG_CUDA(cudaFuncSetAttribute(heavy_consume_kernel<CELLS>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
-      heavy_consume_kernel<CELLS><<<phase == PHASE_PRIO ? prio_chain_blocks(ctx.num_sms) : phase == PHASE_REST ? ctx.num_sms - prio_chain_blocks(ctx.num_sms) : ctx.num_sms, S_THREADS, pad, st>>>(a);
+      const int ahead = prio_chain_blocks(ctx.num_sms);
+      const int blocks = phase == PHASE_PRIO ? ahead : phase == PHASE_REST ? ctx.num_sms - ahead : ctx.num_sms;
+      heavy_consume_kernel<CELLS><<<blocks, S_THREADS, pad, st>>>(a);
       CSG_CUDA(cudaGetLastError());
     }
   }

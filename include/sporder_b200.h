@@ -21,11 +21,9 @@
  *     thread succeeded).
  *   - `is_symmetric` is the reference's promise that the pattern equals its
  *     transpose (sporder/src/common/csr2csc.h:49-59, where the CSR arrays are then
- *     read as the CSC).  With it the library reads the column groups straight off
- *     the CSR arrays instead of sorting; results are the same as without it on a
- *     symmetric pattern.  On a pattern that is not symmetric a true promise gives a
- *     different, still valid permutation (as in the reference) and never an
- *     out-of-range access.  Row shards (sporder_csg_shard) have no such parameter.
+ *     read as the CSC).  The library accepts it and does not depend on it: results
+ *     and times are the same with and without, and a false promise has no effect.
+ *     Row shards (sporder_csg_shard) have no such parameter.
  */
 #ifndef SPORDER_B200_H
 #define SPORDER_B200_H
