@@ -339,7 +339,12 @@ __device__ __forceinline__ void queue_long_row(const SpmmArgs &a, int32_t r, int
 // itself, the gathers of every eight nonzeros waited for the trip that fetched their columns
 // first, as long as their own.  Without the walk's state there is room for four blocks per SM.
 // R-MAT scale 22 at width 128: 3.03 ms walking, 2.37 staged, 2.18 staged with four blocks per SM.
-template <int VEC, int PAN, bool MASK>
+//
+// MG > 0, a product of one panel of MG lanes with MVEC columns each: rows of up to GROUP_MAX nonzeros
+// go to lane groups of MG lanes, several rows at a time (most rows of a power-law graph: width 64,
+// R-MAT scale 22, 1.98 ms without, 1.90 with), the longer ones to the whole warp, VEC columns a lane.
+constexpr int GROUP_MAX = 2;
+template <int VEC, int PAN, bool MASK, int MG = 0, int MVEC = 1>
 __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp, int2 *sp, int32_t bfirst, int32_t bcount,
                                            int lane) {
   constexpr int G = 32;
@@ -376,7 +381,29 @@ __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp,
       }
     }
     const int32_t rows = take > 0 ? take : 1;
-    for (int32_t i = 0; i < rows; ++i) {
+    unsigned whole = rows >= 32 ? FULL : (1u << rows) - 1u;  // the rows that the whole warp takes
+    if constexpr (MG > 0) {
+      const unsigned grouped = __ballot_sync(FULL, lane < take && wp[r0 + lane + 1] - wp[r0 + lane] <= GROUP_MAX);
+      whole &= ~grouped;
+      const int32_t col0 = (lane % MG) * MVEC;
+      unsigned mine = grouped;  // group k takes the rows k, k + 32 / MG, ... of them
+      for (int k = 0; k < lane / MG; ++k) mine &= mine - 1u;
+      while (mine) {
+        const int i = __ffs(static_cast<int>(mine)) - 1;
+        const int32_t b = wp[r0 + i] - p0, e = wp[r0 + i + 1] - p0;
+        float acc[1][MVEC];
+#pragma unroll
+        for (int v = 0; v < MVEC; ++v) acc[0][v] = 0.0f;
+        staged_row<MG, MVEC, 1, MASK>(sp + b, e - b, reinterpret_cast<const char *>(a.B + col0), wbytes, col0, acc);
+        if (panel_on<MG, MVEC, MASK>(col0, 0, a.w))
+          store_c<MVEC>(a.C + static_cast<size_t>(bfirst + r0 + i) * a.w + col0, acc[0], false);
+#pragma unroll
+        for (int k = 0; k < 32 / MG; ++k) mine &= mine - 1u;
+      }
+      __syncwarp();
+    }
+    for (; whole; whole &= whole - 1u) {
+      const int32_t i = __ffs(static_cast<int>(whole)) - 1;
       const int32_t b = wp[r0 + i] - p0, cnt = take > 0 ? wp[r0 + i + 1] - p0 - b : len0;
       float *out = a.C + static_cast<size_t>(bfirst + r0 + i) * a.w + lane * VEC;
       for (int pn0 = 0; pn0 < panels; pn0 += PAN) {
@@ -424,12 +451,13 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
       if (count > 0) whole_unit<VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
     return;
   }
-  // Narrower, but with a column for each lane of a warp: units of short rows by lane groups, in the
-  // others a row to the whole warp.  Walked by lane groups, those took trips in turn for columns and
-  // gathers, and code for a remainder of each group's own.  At widths 32, 40 and 64: R-MAT scale
-  // 20 took 464, 866 and 666 us, now 384, 510 and 466; 65,536 Zipf rows 51, 104 and 75 us, now 48, 57 and
-  // 52.  At 16 half of each load would be idle, and the walk is faster.
-  if constexpr (G < 32 && G * VEC >= 32) {
+  // Narrower, but with two columns for each lane of a warp: units of short rows by lane groups, in
+  // the others most nonzeros go to the whole warp.  Walked by lane groups, those took trips in turn
+  // for columns and gathers, and code for a remainder of each group's own.  At widths 40 and 64: R-MAT
+  // scale 22 took 3.09 and 2.34 ms, now 2.00 and 1.87; 65,536 Zipf rows 104 and 75 us, now 56 and 52.
+  // At 32 columns a warp has too few bytes in flight this way where B is far larger than the L2 (R-MAT
+  // scale 22: 1.42 ms walked, 1.51 by the warp).
+  if constexpr (G < 32 && G * VEC >= 64) {
     static_assert(PAN == 1, "one panel covers the row");
     int32_t first = 0, count = 0;
     while (draw_unit(a, wp, lane, &first, &count)) {
@@ -437,7 +465,7 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
       if (unit_is_short(wp, count, a.nnz, lane))
         short_rows<G, VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
       else
-        whole_unit<G * VEC / 32, 1, MASK>(a, wp, spair[warp], first, count, lane);
+        whole_unit<G * VEC / 32, 1, MASK, G, VEC>(a, wp, spair[warp], first, count, lane);
     }
     return;
   }
@@ -618,8 +646,8 @@ bool launch_variant(Context &ctx, SpmmArgs a) {
   a.piece = a.split / 4;
   spmm_rows_kernel<G, VEC, PAN, MASK><<<ctx.num_sms * (G == 32 ? 4 : M_BLOCKS_PER_SM), M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
-  // (a piece goes to a whole warp wherever each of its lanes has a column)
-  constexpr int LG = G * VEC >= 32 ? 32 : G;
+  // (a piece goes to a whole warp wherever a row may)
+  constexpr int LG = G * VEC >= 64 ? 32 : G;
   spmm_long_kernel<LG, G * VEC / LG, PAN, MASK><<<grid, M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
