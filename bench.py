@@ -402,7 +402,7 @@ def run_ours(args, rank, world, local_rank):
         "clocks": clocks.summary(),
         "stages_ms": stage,
         "roofline": {"bound": "hbm",
-                     "kernel": "sketch + top-k stage (heavy_expand, heavy_rounds, sketch_kernel)",
+                     "kernel": "sketch + top-k stage (heavy_expand, heavy_rounds, rows_in_lanes)",
                      "achieved": ach,
                      "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_src,
                      "algorithmic_bytes": int(b_sketch), "table_rows_written": int(rows_written),
@@ -452,9 +452,8 @@ def run_ours(args, rank, world, local_rank):
 # DRAM bytes (read + write) of the sketch stage's kernels per csg call at full size, from an
 # ncu capture of `bench.py --steps 1 --warmup 1 --no-ref-cuda --no-cpu-baseline --no-spmm`;
 # a number of the build it was captured on, not of this run
-TRAFFIC_RMAT22 = 4454053376
-TRAFFIC_NOTE = ("dram__bytes_read+write of heavy_expand + heavy_rounds + sketch_kernel + heavy_topk, "
-                "one ncu capture at N=1 on the scale-22 matrix; null for other sizes and N")
+TRAFFIC_RMAT22 = None
+TRAFFIC_NOTE = "dram__bytes_read+write of the stage's kernels: not captured for the present kernels"
 
 
 def order_digest(order_np):
