@@ -436,7 +436,8 @@ __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp,
 // the next row of its warp's unit as soon as its current row is finished, so the groups of
 // a warp never wait for the one with the longest row.  Longer rows are zeroed and
 // queued for the second launch.  A row is walked once per PAN panels (w = panels * G * VEC).
-template <int G, int VEC, int PAN, bool MASK>
+// BY_WARP: see whole_unit.
+template <int G, int VEC, int PAN, bool MASK, bool BY_WARP>
 __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm_rows_kernel(SpmmArgs a) {
   constexpr int U = Step<PAN>::U;
   __shared__ int32_t sptr[M_WARPS][BATCH_MAX + 1];
@@ -451,13 +452,11 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
       if (count > 0) whole_unit<VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
     return;
   }
-  // Narrower, but with two columns for each lane of a warp: units of short rows by lane groups, in
+  // Narrower, but with a column or two for each lane of a warp: units of short rows by lane groups, in
   // the others most nonzeros go to the whole warp.  Walked by lane groups, those took trips in turn
   // for columns and gathers, and code for a remainder of each group's own.  At widths 40 and 64: R-MAT
   // scale 22 took 3.09 and 2.34 ms, now 2.00 and 1.87; 65,536 Zipf rows 104 and 75 us, now 56 and 52.
-  // At 32 columns a warp has too few bytes in flight this way where B is far larger than the L2 (R-MAT
-  // scale 22: 1.42 ms walked, 1.51 by the warp).
-  if constexpr (G < 32 && G * VEC >= 64) {
+  if constexpr (G < 32 && BY_WARP) {
     static_assert(PAN == 1, "one panel covers the row");
     int32_t first = 0, count = 0;
     while (draw_unit(a, wp, lane, &first, &count)) {
@@ -627,7 +626,7 @@ __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(S
   }
 }
 
-template <int G, int VEC, int PAN, bool MASK>
+template <int G, int VEC, int PAN, bool MASK, bool BY_WARP = (G * VEC >= 64)>
 bool launch_variant(Context &ctx, SpmmArgs a) {
   // cost per unit: enough units that every warp of the grid draws several of them
   const int grid = ctx.num_sms * M_BLOCKS_PER_SM;
@@ -644,10 +643,10 @@ bool launch_variant(Context &ctx, SpmmArgs a) {
   a.split = SPLIT_MIN;
   while (a.split < SPLIT && (a.split < 2 * share || a.nnz / a.split + 1 > a.queue_cap)) a.split *= 2;
   a.piece = a.split / 4;
-  spmm_rows_kernel<G, VEC, PAN, MASK><<<ctx.num_sms * (G == 32 ? 4 : M_BLOCKS_PER_SM), M_THREADS, 0, ctx.stream>>>(a);
+  spmm_rows_kernel<G, VEC, PAN, MASK, BY_WARP><<<ctx.num_sms * (G == 32 ? 4 : M_BLOCKS_PER_SM), M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   // (a piece goes to a whole warp wherever a row may)
-  constexpr int LG = G * VEC >= 64 ? 32 : G;
+  constexpr int LG = BY_WARP ? 32 : G;
   spmm_long_kernel<LG, G * VEC / LG, PAN, MASK><<<grid, M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
@@ -679,6 +678,12 @@ bool dispatch_spmm(Context &ctx, const SpmmArgs &a) {
     if (w % 256 == 0) return launch_variant<32, 4, 2, false>(ctx, a);
     if (w % 128 == 0) return launch_variant<32, 4, 1, false>(ctx, a);
     if (w == 64) return launch_variant<16, 4, 1, false>(ctx, a);
+    // At 32 columns the whole warp has few bytes in flight, which tells once most of B is not in
+    // the L2.  R-MAT scale 20 (134 MB of B) 464 us walked, 409 by the warp; its symmetrised form 664
+    // and 643; 262,144 rows of that (34 MB) 239 and 152; scale 22 (537 MB) 1.42 and 1.51 ms.  Matrices of
+    // short rows gain nothing (9-point mesh 135 and 136 us).
+    const bool long_rows = a.nnz > 12ll * a.n, near_l2 = static_cast<long long>(a.n) * w * 4 <= (256ll << 20);
+    if (w == 32 && long_rows && near_l2) return launch_variant<8, 4, 1, false, true>(ctx, a);
     if (w == 32) return launch_variant<8, 4, 1, false>(ctx, a);
     if (w == 16) return launch_variant<4, 4, 1, false>(ctx, a);
     if (w == 8) return launch_variant<2, 4, 1, false>(ctx, a);

@@ -331,7 +331,7 @@ def test_spmm_on_units_of_short_rows(w, longest):
     assert np.array_equal(C, C2)
 
 
-@pytest.mark.parametrize("w", [3, 5, 6, 9, 12, 31, 33, 34, 36, 41, 62, 66, 100, 130, 260])
+@pytest.mark.parametrize("w", [3, 5, 6, 9, 12, 31, 32, 33, 34, 36, 41, 62, 66, 100, 130, 260])
 def test_spmm_ragged_widths_and_rows_at_the_split(w):
     # widths that fill their lane groups in part (one, two and four columns per lane, one and
     # two panels per walk), rows of both sides of the limit a group walks alone, and operands
@@ -339,7 +339,7 @@ def test_spmm_ragged_widths_and_rows_at_the_split(w):
     sp = _sp()
     n = 3000
     rng = np.random.default_rng(w)
-    lengths = rng.integers(0, 20, size=n)
+    lengths = rng.integers(0, 27, size=n)
     lengths[:8] = [127, 128, 129, 255, 1023, 1024, 1025, 2500]
     ptr, ind, val = _rows_of_given_lengths(lengths, n, 11)
     B = rng.standard_normal((n, w)).astype(np.float32)
