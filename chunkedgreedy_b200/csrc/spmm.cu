@@ -26,19 +26,11 @@
 
 #include "../../include/sporder_b200.h"
 #include "common.cuh"
+#include "spmm_plan.h"
 
 namespace csg {
 
 namespace {
-
-constexpr int M_THREADS = 256;
-constexpr int M_WARPS = M_THREADS / 32;
-constexpr int M_BLOCKS_PER_SM = 3;
-constexpr int SPLIT = 1024;      // longest row one lane group walks alone in a large product ...
-constexpr int SPLIT_MIN = 128;   // ... and in a small one (see launch_variant)
-constexpr int ROW_COST = 4;      // cost of a row beside its nonzeros, in nonzeros
-constexpr int UNIT_MAX = 2048;   // largest unit cost; a unit holds at most UNIT_MAX / ROW_COST rows
-constexpr int BATCH_MAX = UNIT_MAX / ROW_COST;
 
 // Columns of the lane's panel pn that exist: with MASK the last panel of a width that is not a
 // multiple of G * VEC is ragged, and the lanes behind the last column load and store nothing.
@@ -192,10 +184,10 @@ __device__ __forceinline__ void store_c(float *out, const float (&acc)[VEC], boo
 // rows (opcode counts of a profiler run: a third of them integer multiply-adds for
 // addresses, predicates and moves), and the kernel there is bound by instruction issue.
 constexpr int SHORT_MAX = 16;
-constexpr int S_PAIRS = 448;  // pairs staged per warp
 
 // The warp draws its next unit: rows [*first, *first + *count), their pointers in wp.  False: no
 // units are left.  (A unit may hold no row.)
+template <int BATCH>
 __device__ __forceinline__ bool draw_unit(const SpmmArgs &a, int32_t *wp, int lane, int32_t *first, int32_t *count) {
   uint32_t t = 0;
   if (lane == 0) t = atomicAdd(&a.ctrl[CTRL_TICKET], 1u);
@@ -207,8 +199,8 @@ __device__ __forceinline__ bool draw_unit(const SpmmArgs &a, int32_t *wp, int la
   unit_bounds(a, static_cast<long long>(t) * a.unit, (static_cast<long long>(t) + 1) * a.unit, first, &last);
   if (last > a.n) last = a.n;
   if (*first < last) {
-    *count = last - *first;  // at most unit / ROW_COST <= BATCH_MAX rows
-    if (*count > BATCH_MAX) *count = BATCH_MAX;  // (only with row pointers that decrease)
+    *count = last - *first;  // at most unit / ROW_COST <= BATCH rows
+    if (*count > BATCH) *count = BATCH;  // (only with row pointers that decrease)
     __syncwarp();
     for (int k = lane; k <= *count; k += 32) wp[k] = __ldg(a.ptr + *first + k);
     __syncwarp();
@@ -216,16 +208,25 @@ __device__ __forceinline__ bool draw_unit(const SpmmArgs &a, int32_t *wp, int la
   return true;
 }
 
-// true when every row of the staged unit is well-formed and has at most SHORT_MAX nonzeros
-__device__ __forceinline__ bool unit_is_short(const int32_t *wp, int32_t bcount, int32_t nnz, int lane) {
+// Longest row of the staged unit, SHORT_MAX + 1 when one is malformed (the general path deals with it)
+__device__ __forceinline__ int32_t unit_longest(const int32_t *wp, int32_t bcount, int32_t nnz, int lane) {
   int32_t worst = 0;
   for (int k = lane; k < bcount; k += 32) {
     const int32_t b = wp[k], e = wp[k + 1];
-    int32_t len = e - b;
-    if (b < 0 || e < b || e > nnz) len = SHORT_MAX + 1;  // malformed: the general path deals with it
+    const int32_t len = b < 0 || e < b || e > nnz ? SHORT_MAX + 1 : e - b;
     worst = len > worst ? len : worst;
   }
-  return __reduce_max_sync(FULL, worst) <= SHORT_MAX;
+  return __reduce_max_sync(FULL, worst);
+}
+
+// The rows of a short unit are of much the same length (on average 7/8 of the longest: the lane groups of
+// a warp then run the same cases), and not of few nonzeros.  A unit of short rows has many of them, and
+// by lane groups a row makes more trips than by the warp, which with two panels loses from six nonzeros
+// down (5-point mesh of 50,000 rows at width 192: 32 us by the warp, 36 by groups of 16), with one from four.
+template <int PAN>
+__device__ __forceinline__ bool unit_is_even(const int32_t *wp, int32_t bcount, int32_t longest) {
+  const int32_t nonzeros = wp[bcount] - wp[0];
+  return 7 * longest * bcount <= 8 * nonzeros && (PAN == 1 ? 4 : 6) * bcount <= nonzeros;
 }
 
 // N nonzeros of a row, pairs at sp[0 .. N): gather and FMA
@@ -258,10 +259,10 @@ __device__ __forceinline__ void short_slots(const int2 *sp, const char *bcol, in
 
 // The nonzeros sp[0 .. cnt) of one row into acc: pieces of UC while more than CAP are left, then
 // all the rest in one piece.
-template <int G, int VEC, int PAN, bool MASK>
+template <int G, int VEC, int PAN, bool MASK, int UC = Step<PAN>::U>
 __device__ __forceinline__ void staged_row(const int2 *sp, int32_t cnt, const char *bcol, int32_t wbytes, int32_t col0,
                                            float (&acc)[PAN][VEC]) {
-  constexpr int UC = Step<PAN>::U, CAP = UC + 1;
+  constexpr int CAP = UC + 1;
   int32_t q = 0;
   for (; cnt - q > CAP; q += UC) short_slots<G, VEC, PAN, MASK, UC>(sp + q, bcol, wbytes, col0, acc);
   switch (cnt - q) {
@@ -277,8 +278,8 @@ __device__ __forceinline__ void staged_row(const int2 *sp, int32_t cnt, const ch
 }
 
 // all rows [bfirst, bfirst + bcount) of a short unit; wp holds their row pointers, sp is the
-// warp's pair buffer
-template <int G, int VEC, int PAN, bool MASK>
+// warp's buffer of S_PAIRS pairs
+template <int G, int VEC, int PAN, bool MASK, int S_PAIRS, int UC = Step<PAN>::U>
 __device__ __forceinline__ void short_rows(const SpmmArgs &a, const int32_t *wp, int2 *sp, int32_t bfirst,
                                            int32_t bcount, int lane) {
   constexpr int PER_WARP = 32 / G;
@@ -315,7 +316,7 @@ __device__ __forceinline__ void short_rows(const SpmmArgs &a, const int32_t *wp,
         const char *bcol = reinterpret_cast<const char *>(a.B + col0);
         // (every gather of a piece is issued before its first FMA, so a row of nine costs one
         // trip to memory, not two)
-        staged_row<G, VEC, PAN, MASK>(sp + b, e - b, bcol, wbytes, col0, acc);
+        staged_row<G, VEC, PAN, MASK, UC>(sp + b, e - b, bcol, wbytes, col0, acc);
 #pragma unroll
         for (int pn = 0; pn < PAN; ++pn)
           if (panel_on<G, VEC, MASK>(col0, pn, a.w)) store_c<VEC>(out + (pn0 + pn) * (G * VEC), acc[pn], false);
@@ -338,13 +339,14 @@ __device__ __forceinline__ void queue_long_row(const SpmmArgs &a, int32_t r, int
 // buffer are staged with coalesced loads and the rows worked off from there.  Walking the row
 // itself, the gathers of every eight nonzeros waited for the trip that fetched their columns
 // first, as long as their own.  Without the walk's state there is room for four blocks per SM.
-// R-MAT scale 22 at width 128: 3.03 ms walking, 2.37 staged, 2.18 staged with four blocks per SM.
+// R-MAT scale 22 at width 128, this launch alone: 3.03 ms walking, 2.37 staged, 2.18 staged with four
+// blocks per SM; both launches 4.3 ms walking, 3.1 to 3.3 so.
 //
 // MG > 0, a product of one panel of MG lanes with MVEC columns each: rows of up to GROUP_MAX nonzeros
 // go to lane groups of MG lanes, several rows at a time (most rows of a power-law graph: width 64,
 // R-MAT scale 22, 1.98 ms without, 1.90 with), the longer ones to the whole warp, VEC columns a lane.
 constexpr int GROUP_MAX = 2;
-template <int VEC, int PAN, bool MASK, int MG = 0, int MVEC = 1>
+template <int VEC, int PAN, bool MASK, int S_PAIRS, int UC, int MG = 0, int MVEC = 1>
 __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp, int2 *sp, int32_t bfirst, int32_t bcount,
                                            int lane) {
   constexpr int G = 32;
@@ -415,12 +417,12 @@ __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp,
         const int32_t col0 = pn0 * (G * VEC) + lane * VEC;
         const char *bcol = reinterpret_cast<const char *>(a.B + col0);
         if (take > 0) {
-          staged_row<G, VEC, PAN, MASK>(sp + b, cnt, bcol, wbytes, col0, acc);
+          staged_row<G, VEC, PAN, MASK, UC>(sp + b, cnt, bcol, wbytes, col0, acc);
         } else {
           for (int32_t q = 0; q < cnt; q += S_PAIRS) {
             const int32_t part = cnt - q < S_PAIRS ? cnt - q : S_PAIRS;
             stage(p0 + q, part);
-            staged_row<G, VEC, PAN, MASK>(sp, part, bcol, wbytes, col0, acc);
+            staged_row<G, VEC, PAN, MASK, UC>(sp, part, bcol, wbytes, col0, acc);
           }
         }
 #pragma unroll
@@ -436,35 +438,51 @@ __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp,
 // the next row of its warp's unit as soon as its current row is finished, so the groups of
 // a warp never wait for the one with the longest row.  Longer rows are zeroed and
 // queued for the second launch.  A row is walked once per PAN panels (w = panels * G * VEC).
-// BY_WARP: see whole_unit.
-template <int G, int VEC, int PAN, bool MASK, bool BY_WARP>
-__global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm_rows_kernel(SpmmArgs a) {
+// WHOLE, EVEN, BLOCKS: see SpmmShape and whole_unit.
+template <int G, int VEC, int PAN, bool MASK, bool WHOLE, int EVEN, int BLOCKS>
+__global__ void __launch_bounds__(M_THREADS, BLOCKS) spmm_rows_kernel(SpmmArgs a) {
   constexpr int U = Step<PAN>::U;
-  __shared__ int32_t sptr[M_WARPS][BATCH_MAX + 1];
-  __shared__ int2 spair[M_WARPS][S_PAIRS];
+  constexpr int ROWS = batch_rows(G, VEC), PAIRS = batch_pairs(G, VEC, PAN, BLOCKS);
+  __shared__ int32_t sptr[M_WARPS][ROWS + 1];
+  __shared__ int2 spair[M_WARPS][PAIRS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gl = lane % G;
   const unsigned below_group = (1u << (lane - gl)) - 1u;  // lanes of the groups in front of mine
   int32_t *wp = sptr[warp];
+  // With four blocks per SM a lane has 64 registers: pieces of six nonzeros fit them, eight do not (R-MAT scale
+  // 22 at 128: 3.26 ms with eight, 3.13 with six).
+  constexpr int SIX = PAN == 1 ? 6 : U;
   if constexpr (G == 32) {
+    constexpr int SPAN = EVEN == G ? PAN : 1;
+    constexpr int UC = VEC == 4 && BLOCKS == 4 ? SIX : U, SUC = BLOCKS == 4 && Step<SPAN>::U > 6 ? 6 : Step<SPAN>::U;
     int32_t first = 0, count = 0;
-    while (draw_unit(a, wp, lane, &first, &count))
-      if (count > 0) whole_unit<VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
+    while (draw_unit<ROWS>(a, wp, lane, &first, &count)) {
+      if (count == 0) continue;
+      const int32_t longest = VEC == 4 ? unit_longest(wp, count, a.nnz, lane) : SHORT_MAX + 1;
+      if (longest <= SHORT_MAX && (EVEN == G || unit_is_even<PAN>(wp, count, longest)))
+        short_rows<EVEN, VEC, SPAN, EVEN == G && MASK, PAIRS, SUC>(a, wp, spair[warp], first, count, lane);
+      else
+        whole_unit<VEC, PAN, MASK, PAIRS, UC>(a, wp, spair[warp], first, count, lane);
+    }
     return;
   }
   // Narrower, but with a column or two for each lane of a warp: units of short rows by lane groups, in
   // the others most nonzeros go to the whole warp.  Walked by lane groups, those took trips in turn
   // for columns and gathers, and code for a remainder of each group's own.  At widths 40 and 64: R-MAT
   // scale 22 took 3.09 and 2.34 ms, now 2.00 and 1.87; 65,536 Zipf rows 104 and 75 us, now 56 and 52.
-  if constexpr (G < 32 && BY_WARP) {
+  if constexpr (G < 32 && WHOLE) {
     static_assert(PAN == 1, "one panel covers the row");
+    constexpr int UC = EVEN == G ? U : SIX;
     int32_t first = 0, count = 0;
-    while (draw_unit(a, wp, lane, &first, &count)) {
+    while (draw_unit<ROWS>(a, wp, lane, &first, &count)) {
       if (count == 0) continue;
-      if (unit_is_short(wp, count, a.nnz, lane))
-        short_rows<G, VEC, PAN, MASK>(a, wp, spair[warp], first, count, lane);
+      const int32_t longest = unit_longest(wp, count, a.nnz, lane);
+      if (EVEN != G && longest <= SHORT_MAX && unit_is_even<PAN>(wp, count, longest))
+        short_rows<EVEN, VEC, 1, false, PAIRS>(a, wp, spair[warp], first, count, lane);
+      else if (longest <= SHORT_MAX)
+        short_rows<G, VEC, PAN, MASK, PAIRS>(a, wp, spair[warp], first, count, lane);
       else
-        whole_unit<G * VEC / 32, 1, MASK, G, VEC>(a, wp, spair[warp], first, count, lane);
+        whole_unit<G * VEC / 32, 1, MASK, PAIRS, UC, G, VEC>(a, wp, spair[warp], first, count, lane);
     }
     return;
   }
@@ -500,8 +518,8 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
     if (want) {
       if (bnext >= bcount && !exhausted) {
         bnext = 0;
-        exhausted = !draw_unit(a, wp, lane, &bfirst, &bcount);
-        short_unit = bcount > 0 && unit_is_short(wp, bcount, a.nnz, lane);
+        exhausted = !draw_unit<ROWS>(a, wp, lane, &bfirst, &bcount);
+        short_unit = bcount > 0 && unit_longest(wp, bcount, a.nnz, lane) <= SHORT_MAX;
       }
       bool hold = false;  // a short unit in hand: no row of it is handed out one by one
       {
@@ -509,7 +527,7 @@ __global__ void __launch_bounds__(M_THREADS, G == 32 ? 4 : M_BLOCKS_PER_SM) spmm
           hold = true;
           // (groups still walking a row of the unit before finish it first)
           if (__ballot_sync(FULL, row >= 0) == 0u) {
-            short_rows<G, VEC, PAN, MASK>(a, wp, spair[warp], bfirst, bcount, lane);
+            short_rows<G, VEC, PAN, MASK, PAIRS>(a, wp, spair[warp], bfirst, bcount, lane);
             bnext = bcount;
             short_unit = false;
             // (no group holds a row here: saying so frees the walk's registers for short_rows)
@@ -626,76 +644,32 @@ __global__ void __launch_bounds__(M_THREADS, M_BLOCKS_PER_SM) spmm_long_kernel(S
   }
 }
 
-template <int G, int VEC, int PAN, bool MASK, bool BY_WARP = (G * VEC >= 64)>
-bool launch_variant(Context &ctx, SpmmArgs a) {
-  // cost per unit: enough units that every warp of the grid draws several of them
-  const int grid = ctx.num_sms * M_BLOCKS_PER_SM;
-  const long long total = static_cast<long long>(ROW_COST) * a.n + a.nnz;
-  long long unit = total / (static_cast<long long>(grid) * M_WARPS * 8);
-  if (unit < 128) unit = 128;
-  if (unit > UNIT_MAX) unit = UNIT_MAX;
-  a.unit = static_cast<int32_t>(unit);
-  // A row walked alone is a serial chain of gathers: it should not outlast what the other
-  // groups do meanwhile, twice the average share of a group here.  Large products keep the
-  // upper limit (fewer atomics), small ones would otherwise wait for their longest row: one
-  // of 1024 nonzeros is 128 dependent steps of gathers.
-  const long long share = static_cast<long long>(a.nnz) / (static_cast<long long>(grid) * M_WARPS * (32 / G));
-  a.split = SPLIT_MIN;
-  while (a.split < SPLIT && (a.split < 2 * share || a.nnz / a.split + 1 > a.queue_cap)) a.split *= 2;
-  a.piece = a.split / 4;
-  spmm_rows_kernel<G, VEC, PAN, MASK, BY_WARP><<<ctx.num_sms * (G == 32 ? 4 : M_BLOCKS_PER_SM), M_THREADS, 0, ctx.stream>>>(a);
+template <int G, int VEC, int PAN, bool MASK, bool WHOLE, int EVEN, int BLOCKS>
+bool launch_shape(Context &ctx, const SpmmArgs &a, const SpmmPlan &p) {
+  spmm_rows_kernel<G, VEC, PAN, MASK, WHOLE, EVEN, BLOCKS><<<p.rows_grid, M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   // (a piece goes to a whole warp wherever a row may)
-  constexpr int LG = BY_WARP ? 32 : G;
-  spmm_long_kernel<LG, G * VEC / LG, PAN, MASK><<<grid, M_THREADS, 0, ctx.stream>>>(a);
+  constexpr int LG = WHOLE ? 32 : G;
+  spmm_long_kernel<LG, G * VEC / LG, PAN, MASK><<<p.long_grid, M_THREADS, 0, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
   return true;
 }
 
-// Widths that fill their lane groups only in part (a task's class count, a feature dimension
-// such as 100): the smallest group that covers the row in one panel, or 32 lanes walking one
-// or two panels at a time, the last panel masked.
-template <int VEC>
-bool launch_masked(Context &ctx, const SpmmArgs &a) {
-  const int cols = a.w / VEC;
-  if (cols <= 4) return launch_variant<4, VEC, 1, true>(ctx, a);
-  if (cols <= 8) return launch_variant<8, VEC, 1, true>(ctx, a);
-  if (cols <= 16) return launch_variant<16, VEC, 1, true>(ctx, a);
-  if ((cols + 31) / 32 % 2 == 0) return launch_variant<32, VEC, 2, true>(ctx, a);
-  return launch_variant<32, VEC, 1, true>(ctx, a);
-}
-
-// Lane groups by dense width: four or two columns per lane where the width and the alignment
-// of B and C allow, single floats otherwise, and as many lanes as the row has such pieces (up
-// to 32); two panels per walk when the panel count is even.  (Groups of one to eight lanes for
-// widths without a power-of-two factor, one float per lane, left a group walking the row once
-// per column: 5.5 ms for 0.28 M nonzeros at width 41 on a B200, 0.095 ms with the masked panels.)
-bool dispatch_spmm(Context &ctx, const SpmmArgs &a) {
-  const int w = a.w;
+bool dispatch_spmm(Context &ctx, SpmmArgs a) {
   const uintptr_t both = reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C);
-  if (w % 4 == 0 && both % 16 == 0) {
-    if (w % 256 == 0) return launch_variant<32, 4, 2, false>(ctx, a);
-    if (w % 128 == 0) return launch_variant<32, 4, 1, false>(ctx, a);
-    if (w == 64) return launch_variant<16, 4, 1, false>(ctx, a);
-    // At 32 columns the whole warp has few bytes in flight, which tells once most of B is not in
-    // the L2.  R-MAT scale 20 (134 MB of B) 464 us walked, 409 by the warp; its symmetrised form 664
-    // and 643; 262,144 rows of that (34 MB) 239 and 152; scale 22 (537 MB) 1.42 and 1.51 ms.  Matrices of
-    // short rows gain nothing (9-point mesh 135 and 136 us).
-    const bool long_rows = a.nnz > 12ll * a.n, near_l2 = static_cast<long long>(a.n) * w * 4 <= (256ll << 20);
-    if (w == 32 && long_rows && near_l2) return launch_variant<8, 4, 1, false, true>(ctx, a);
-    if (w == 32) return launch_variant<8, 4, 1, false>(ctx, a);
-    if (w == 16) return launch_variant<4, 4, 1, false>(ctx, a);
-    if (w == 8) return launch_variant<2, 4, 1, false>(ctx, a);
-    if (w == 4) return launch_variant<1, 4, 1, false>(ctx, a);
-    return launch_masked<4>(ctx, a);
-  }
-  if (w % 2 == 0 && both % 8 == 0) {
-    if (w == 2) return launch_variant<1, 2, 1, false>(ctx, a);
-    return launch_masked<2>(ctx, a);
-  }
-  if (w == 1) return launch_variant<1, 1, 1, false>(ctx, a);
-  return launch_masked<1>(ctx, a);
+  const int align = both % 16 == 0 ? 16 : both % 8 == 0 ? 8 : 4;
+  const SpmmPlan p = spmm_plan(a.n, a.nnz, a.w, align, ctx.num_sms, a.queue_cap);
+  a.unit = p.unit;
+  a.split = p.split;
+  a.piece = p.piece;
+#define CSG_LAUNCH(G, VEC, PAN, MASK, WHOLE, EVEN, BLOCKS)         \
+  if (p.shape == SpmmShape{G, VEC, PAN, MASK, WHOLE, EVEN, BLOCKS}) \
+    return launch_shape<G, VEC, PAN, MASK != 0, WHOLE != 0, EVEN, BLOCKS>(ctx, a, p);
+  CSG_SPMM_SHAPES(CSG_LAUNCH)
+#undef CSG_LAUNCH
+  set_error("spmm: no kernel of the planned shape (width %d)", a.w);
+  return false;
 }
 
 }  // namespace
@@ -707,7 +681,6 @@ bool launch_spmm(Context &ctx, int32_t n, int32_t nnz, int32_t w, const int32_t 
   a.n = n;
   a.w = w;
   a.nnz = nnz;
-  a.unit = UNIT_MAX;
   a.ptr = d_ptr;
   a.ind = d_ind;
   a.val = d_val;
@@ -787,7 +760,6 @@ bool run_spmm_static(int32_t n, int32_t nnz, int32_t w, const int32_t *d_ptr, co
   a.n = n;
   a.w = w;
   a.nnz = nnz;
-  a.unit = UNIT_MAX;
   a.ptr = d_ptr;
   a.ind = d_ind;
   a.val = d_val;
