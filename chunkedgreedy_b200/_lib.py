@@ -75,6 +75,11 @@ SYMBOLS = {
     "sporder_linear": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 4),
     "sporder_gcn_forward": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 3),
     "sporder_gcn_backward": (C.c_int32, [_P] + [C.c_int32] * 4 + [_P] * 8),
+    "sporder_gcn_forward_padded": (C.c_int32, [_P] + [C.c_int32] * 4 + [_P] * 3),
+    "sporder_gcn_backward_padded": (C.c_int32, [_P] + [C.c_int32] * 5 + [_P] * 8),
+    "sporder_gcn_hidden_gradient": (C.c_int32, [_P] + [C.c_int32] * 4 + [_P] * 5),
+    "sporder_pad_columns": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 2),
+    "sporder_gcn_input_gradients": (C.c_int32, [_P] + [C.c_int32] * 3 + [_P] * 4),
     "sporder_kernel_launches": (C.c_uint64, []),
     "sporder_chunk_greedy": (None, [_P, C.c_int32, C.c_int32, _P, _P, C.c_bool, C.c_int32, C.c_float,
                                     C.c_int32, _P, C.POINTER(CsgTiming), C.POINTER(CgStats)]),

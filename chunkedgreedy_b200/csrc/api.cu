@@ -879,25 +879,67 @@ int32_t sporder_linear(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t
   return csg::launch_linear(ctx->c, n, in_dim, out_dim, d_x, d_W, d_b, d_Y) ? 0 : -1;
 }
 
-int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, const float *d_Z,
-                            const float *d_W2, float *d_U) {
+int32_t sporder_gcn_forward_padded(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, int32_t columns,
+                                   const float *d_Z, const float *d_W2, float *d_U) {
   csg::clear_error();
   if (!ctx || !d_Z || !d_W2 || !d_U) {
     csg::set_error("gcn_forward: bad arguments");
     return -1;
   }
-  return csg::launch_gcn_forward(ctx->c, n, hidden, classes, d_Z, d_W2, d_U) ? 0 : -1;
+  return csg::launch_gcn_forward(ctx->c, n, hidden, classes, columns, d_Z, d_W2, d_U) ? 0 : -1;
 }
 
-int32_t sporder_gcn_backward(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, int32_t classes,
-                             const float *d_G, const float *d_Z, const float *d_P, const float *d_s,
-                             const float *d_W2, float *d_dW1, float *d_db1, float *d_dW2) {
+int32_t sporder_gcn_forward(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, const float *d_Z,
+                            const float *d_W2, float *d_U) {
+  return sporder_gcn_forward_padded(ctx, n, hidden, classes, classes, d_Z, d_W2, d_U);
+}
+
+int32_t sporder_gcn_backward_padded(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, int32_t classes,
+                                    int32_t columns, const float *d_G, const float *d_Z, const float *d_P,
+                                    const float *d_s, const float *d_W2, float *d_dW1, float *d_db1, float *d_dW2) {
   csg::clear_error();
   if (!ctx || !d_G || !d_Z || !d_P || !d_s || !d_W2 || !d_dW1 || !d_db1 || !d_dW2) {
     csg::set_error("gcn_backward: bad arguments");
     return -1;
   }
-  return csg::launch_gcn_backward(ctx->c, n, in_dim, hidden, classes, d_G, d_Z, d_P, d_s, d_W2, d_dW1, d_db1, d_dW2) ? 0 : -1;
+  return csg::launch_gcn_backward(ctx->c, n, in_dim, hidden, classes, columns, d_G, d_Z, d_P, d_s, d_W2, d_dW1, d_db1,
+                                  d_dW2) ? 0 : -1;
+}
+
+int32_t sporder_gcn_backward(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, int32_t classes,
+                             const float *d_G, const float *d_Z, const float *d_P, const float *d_s,
+                             const float *d_W2, float *d_dW1, float *d_db1, float *d_dW2) {
+  return sporder_gcn_backward_padded(ctx, n, in_dim, hidden, classes, classes, d_G, d_Z, d_P, d_s, d_W2, d_dW1, d_db1,
+                                     d_dW2);
+}
+
+int32_t sporder_gcn_hidden_gradient(sporder_context_t ctx, int32_t n, int32_t hidden, int32_t classes, int32_t columns,
+                                    const float *d_G, const float *d_Z, const float *d_W2, float *d_D, float *d_dW2) {
+  csg::clear_error();
+  if (!ctx || !d_G || !d_Z || !d_W2 || !d_D || !d_dW2) {
+    csg::set_error("gcn_hidden_gradient: bad arguments");
+    return -1;
+  }
+  return csg::launch_gcn_hidden_gradient(ctx->c, n, hidden, classes, columns, d_G, d_Z, d_W2, d_D, d_dW2) ? 0 : -1;
+}
+
+int32_t sporder_pad_columns(sporder_context_t ctx, int32_t n, int32_t from, int32_t to, const float *d_src, float *d_dst) {
+  csg::clear_error();
+  if (!ctx || !d_src || !d_dst) {
+    csg::set_error("pad_columns: bad arguments");
+    return -1;
+  }
+  return csg::launch_pad_columns(ctx->c, n, from, to, d_src, d_dst) ? 0 : -1;
+}
+
+int32_t sporder_gcn_input_gradients(sporder_context_t ctx, int32_t n, int32_t in_dim, int32_t hidden, const float *d_E,
+                                    const float *d_x, float *d_dW1, float *d_db1) {
+  csg::clear_error();
+  if (!ctx || !d_E || !d_x || !d_dW1 || !d_db1) {
+    csg::set_error("gcn_input_gradients: bad arguments");
+    return -1;
+  }
+  return csg::launch_gcn_input_gradients(ctx->c, n, in_dim, hidden, d_E, d_x, d_dW1, d_db1) ? 0 : -1;
 }
 
 }  // extern "C"

@@ -191,9 +191,15 @@ size_t reorder_workspace_bytes(int32_t n, int32_t nnz, int mode);
 bool launch_spmm(Context &ctx, int32_t n, int32_t nnz, int32_t w, const int32_t *d_ptr,
                  const int32_t *d_ind, const float *d_val, const float *d_B, float *d_C);
 
-bool launch_gcn_forward(Context &ctx, int32_t n, int32_t hid, int32_t cls, const float *Z, const float *W2, float *U);
-bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *G, const float *Z,
-                         const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2);
+bool launch_gcn_forward(Context &ctx, int32_t n, int32_t hid, int32_t cls, int32_t ld, const float *Z, const float *W2,
+                        float *U);
+bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, int32_t ld, const float *G,
+                         const float *Z, const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2);
+bool launch_gcn_hidden_gradient(Context &ctx, int32_t n, int32_t hid, int32_t cls, int32_t ld, const float *G,
+                                const float *Z, const float *W2, float *D, float *dW2);
+bool launch_pad_columns(Context &ctx, int32_t n, int32_t from, int32_t to, const float *src, float *dst);
+bool launch_gcn_input_gradients(Context &ctx, int32_t n, int32_t in, int32_t hid, const float *E, const float *x,
+                                float *dW1, float *db1);
 bool launch_linear(Context &ctx, int32_t n, int32_t in, int32_t hid, const float *x, const float *W, const float *b, float *Y);
 bool launch_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr, const float *d_val, float *d_out);
 

@@ -4,8 +4,10 @@
 // (experiments/e2e_gcn.py:126-137).  With Z the first sparse product, P = A x and s = A 1 (the row
 // sums), and the second sparse product taken behind the second linear layer (it is narrower there):
 //   forward   U = relu(Z) W2^T
-//   backward  (G = dL/dU)  D = (G W2) * (Z > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T relu(Z).
-// One kernel each way; D never exists in memory.  The backward pass is bound by fp32 multiply-adds
+//   backward  (G = dL/dU)  D = (G W2) * (Z > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T relu(Z);
+// or, where the hidden layer is narrower than the inputs, with E = A D in place of P (A is symmetric):
+//             dW1 = E^T x,  db1 = E^T 1.
+// One kernel forward, one backward, where D never exists in memory, or two around E = A D.  The backward pass is bound by fp32 multiply-adds
 // (2 n in hidden of them, against three passes over n rows of 128 floats): blocks are persistent, one
 // per SM, operands staged with cp.async a tile ahead, 8 x 8 results per thread.  On 1.05 M rows,
 // 128 -> 128 -> 16, on a B200: 1.09 ms (53 % of the fp32 pipes; two warps per scheduler, and the
@@ -23,9 +25,9 @@ constexpr int B_ROWS = 32;   // ... and backward
 constexpr int MAX_CLASSES = 48;
 
 struct DenseArgs {
-  int32_t n, in, hid, cls;
+  int32_t n, in, hid, cls, ld;  // ld: floats per row of U and G, those behind the classes zero
   const float *P, *s, *W2, *Z;
-  float *U;
+  float *U, *D;
   const float *G;
   float *part;        // backward: a block's sums
   float *dW1, *db1, *dW2;
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) 
     __syncthreads();
     const float *const z = dense_smem + L::TILES + buf * F_ROWS * L::HS + (tid >> 1) * L::HS;
     const int64_t r = t * F_ROWS + (tid >> 1);
-    for (int c0 = (tid & 1) * 4; c0 < a.cls; c0 += 8) {
+    for (int c0 = (tid & 1) * 4; c0 < a.ld; c0 += 8) {
       float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 8
       for (int k = 0; k < HID_T; k += 4) {
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_forward_kernel(DenseArgs a) 
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        if (c0 + c < a.cls && r < a.n) a.U[r * a.cls + c0 + c] = u[c];
+        if (c0 + c < a.ld && r < a.n) a.U[r * a.ld + c0 + c] = u[c];
     }
     __syncthreads();  // the tile's place is free for the copies of the round after next
   }
@@ -203,22 +205,63 @@ struct PartLayout {
   static constexpr int W2 = HID_T * IN_T, B1 = W2 + CLS_T * HID_T, FLOATS = B1 + D_THREADS;
 };
 
+// B_ROWS rows of G from row r0 into dst, CLS_T apart, zeros behind the last row
+template <int CLS_T>
+__device__ __forceinline__ void stage_classes(float *dst, const DenseArgs &a, int64_t r0) {
+  for (int i = threadIdx.x; i < B_ROWS * a.cls; i += D_THREADS) {
+    const int r = i / a.cls, c = i % a.cls;
+    const bool on = r0 + r < a.n;
+    copy4(dst + r * CLS_T + c, a.G + (on ? (r0 + r) * a.ld + c : 0), on);
+  }
+}
+
+// (G W2) of one row and hidden unit, masked: w2 is the unit's column of W2, z its row's value of Z
+template <int CLS_T>
+__device__ __forceinline__ float hidden_gradient(const float *g, const float (&w2)[CLS_T], float z) {
+  float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int c = 0; c < CLS_T; c += 4) {
+    const float4 q = *reinterpret_cast<const float4 *>(g + c);
+    x[0] = fmaf(q.x, w2[c], x[0]);
+    x[1] = fmaf(q.y, w2[c + 1], x[1]);
+    x[2] = fmaf(q.z, w2[c + 2], x[2]);
+    x[3] = fmaf(q.w, w2[c + 3], x[3]);
+  }
+  return z > 0.0f ? (x[0] + x[1]) + (x[2] + x[3]) : 0.0f;
+}
+
+// acc2 += g * hv for PER classes
+template <int PER>
+__device__ __forceinline__ void add_classes(float (&acc2)[PER], const float *g, float hv) {
+  constexpr int VC = PER % 4 == 0 ? 4 : 2;
+#pragma unroll
+  for (int c = 0; c < PER; c += VC) {
+    float gv[VC];
+    if constexpr (VC == 4) *reinterpret_cast<float4 *>(gv) = *reinterpret_cast<const float4 *>(g + c);
+    else *reinterpret_cast<float2 *>(gv) = *reinterpret_cast<const float2 *>(g + c);
+#pragma unroll
+    for (int x = 0; x < VC; ++x) acc2[c + x] = fmaf(gv[x], hv, acc2[c + x]);
+  }
+}
+
+// CLS_T == 0: a.Z holds E, which takes the place of D; neither G nor s nor W2 is there, dW2 is not asked for
 template <int IN_T, int HID_T, int CLS_T>
 __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a) {
   using L = BackwardShared<IN_T, HID_T, CLS_T>;
   using O = PartLayout<IN_T, HID_T, CLS_T>;
   constexpr int NJ = HID_T / 16, VJ = NJ < 4 ? NJ : 4, QJ = NJ / VJ;  // hidden units per thread, QJ runs of VJ
   constexpr int NI = IN_T / 16, VI = 4, QI = NI / VI;   // inputs per thread, in fours
-  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS, VC = PER % 4 == 0 ? 4 : 2;  // dW2: PER classes of one hidden unit per thread
+  constexpr bool GIVEN = CLS_T == 0;
+  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS;  // dW2: PER classes of one hidden unit per thread
   extern __shared__ __align__(16) float dense_smem[];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int hj = tid % HID_T, group = tid / HID_T;
-  float w2[CLS_T];  // this thread's hidden unit's column of W2
+  float w2[GIVEN ? 1 : CLS_T];  // this thread's hidden unit's column of W2
 #pragma unroll
   for (int c = 0; c < CLS_T; ++c)
     w2[c] = c < a.cls && hj < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + hj] : 0.0f;
   float2 acc[NJ][NI / 2];
-  float acc2[PER], accb = 0.0f;
+  float acc2[GIVEN ? 1 : PER], accb = 0.0f;
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
 #pragma unroll
@@ -234,12 +277,10 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
       const int64_t r0 = t * B_ROWS;
       stage_rows<B_ROWS, IN_T, D_THREADS>(b + L::P, a.P, r0, a.n, a.in);
       stage_rows<B_ROWS, HID_T, D_THREADS>(b + L::H, a.Z, r0, a.n, a.hid);
-      for (int i = tid; i < B_ROWS * a.cls; i += D_THREADS) {
-        const int r = i / a.cls, c = i % a.cls;
-        const bool on = r0 + r < a.n;
-        copy4(b + L::G + r * CLS_T + c, a.G + (on ? r0 * a.cls + i : 0), on);
+      if constexpr (!GIVEN) {
+        stage_classes<CLS_T>(b + L::G, a, r0);
+        for (int i = tid; i < B_ROWS; i += D_THREADS) copy4(b + L::S + i, a.s + (r0 + i < a.n ? r0 + i : 0), r0 + i < a.n);
       }
-      for (int i = tid; i < B_ROWS; i += D_THREADS) copy4(b + L::S + i, a.s + (r0 + i < a.n ? r0 + i : 0), r0 + i < a.n);
     }
     copies_commit();
   };
@@ -251,23 +292,20 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
     __syncthreads();
     const float *const b = dense_smem + L::BUF + buf * L::BUF_FLOATS;
     const float *const p = b + L::P, *const h = b + L::H, *const g = b + L::G, *const s = b + L::S;
-    float *const d = dense_smem + L::D;
+    const float *d = h;
+    if constexpr (GIVEN) {
+      for (int r = group; r < B_ROWS; r += GROUPS) accb += h[r * L::HS + hj];
+    } else {
+      float *const own = dense_smem + L::D;
 #pragma unroll 4
-    for (int r = group; r < B_ROWS; r += GROUPS) {
-      float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int c = 0; c < CLS_T; c += 4) {
-        const float4 q = *reinterpret_cast<const float4 *>(g + r * CLS_T + c);
-        x[0] = fmaf(q.x, w2[c], x[0]);
-        x[1] = fmaf(q.y, w2[c + 1], x[1]);
-        x[2] = fmaf(q.z, w2[c + 2], x[2]);
-        x[3] = fmaf(q.w, w2[c + 3], x[3]);
+      for (int r = group; r < B_ROWS; r += GROUPS) {
+        const float y = hidden_gradient<CLS_T>(g + r * CLS_T, w2, h[r * L::HS + hj]);
+        own[r * L::HS + hj] = y;
+        accb = fmaf(y, s[r], accb);
       }
-      const float y = h[r * L::HS + hj] > 0.0f ? (x[0] + x[1]) + (x[2] + x[3]) : 0.0f;
-      d[r * L::HS + hj] = y;
-      accb = fmaf(y, s[r], accb);
+      d = own;
+      __syncthreads();
     }
-    __syncthreads();
 #pragma unroll 4
     for (int r = 0; r < B_ROWS; ++r) {
       float dj[NJ];
@@ -285,15 +323,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int i = 0; i < NI / 2; ++i) fma2(acc[j][i], make_float2(dj[j], dj[j]), pi[i]);
-      const float hv = fmaxf(h[r * L::HS + hj], 0.0f);
-#pragma unroll
-      for (int c = 0; c < PER; c += VC) {
-        float gv[VC];
-        if constexpr (VC == 4) *reinterpret_cast<float4 *>(gv) = *reinterpret_cast<const float4 *>(g + r * CLS_T + group * PER + c);
-        else *reinterpret_cast<float2 *>(gv) = *reinterpret_cast<const float2 *>(g + r * CLS_T + group * PER + c);
-#pragma unroll
-        for (int x = 0; x < VC; ++x) acc2[c + x] = fmaf(gv[x], hv, acc2[c + x]);
-      }
+      if constexpr (!GIVEN) add_classes<PER>(acc2, g + r * CLS_T + group * PER, fmaxf(h[r * L::HS + hj], 0.0f));
     }
     __syncthreads();
   }
@@ -311,11 +341,64 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
   out[O::B1 + tid] = accb;
 }
 
+// D written out, and dW2 = G^T relu(Z): the first half where the operator goes over D.  Bound by its three
+// passes (Z and G in, D out); two blocks per SM keep their copies in flight.
+template <int HID_T, int CLS_T>
+struct HiddenShared {
+  static constexpr int HS = HID_T + 4;
+  static constexpr int H = 0, G = H + B_ROWS * HS, BUF_FLOATS = G + B_ROWS * CLS_T, FLOATS = 2 * BUF_FLOATS;
+};
+template <int HID_T, int CLS_T>
+__global__ void __launch_bounds__(D_THREADS, 2) gcn_hidden_kernel(DenseArgs a) {
+  using L = HiddenShared<HID_T, CLS_T>;
+  using O = PartLayout<0, HID_T, CLS_T>;
+  constexpr int GROUPS = D_THREADS / HID_T, PER = CLS_T / GROUPS;
+  extern __shared__ __align__(16) float dense_smem[];
+  const int tid = threadIdx.x, hj = tid % HID_T, group = tid / HID_T;
+  float w2[CLS_T], acc2[PER];
+#pragma unroll
+  for (int c = 0; c < CLS_T; ++c)
+    w2[c] = c < a.cls && hj < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + hj] : 0.0f;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) acc2[c] = 0.0f;
+  for (int i = tid; i < L::FLOATS; i += D_THREADS) dense_smem[i] = 0.0f;  // classes behind the last
+  __syncthreads();
+  const int64_t tiles = (static_cast<int64_t>(a.n) + B_ROWS - 1) / B_ROWS;
+  auto stage = [&](int64_t t, int buf) {
+    if (t < tiles) {
+      float *const b = dense_smem + buf * L::BUF_FLOATS;
+      stage_rows<B_ROWS, HID_T, D_THREADS>(b + L::H, a.Z, t * B_ROWS, a.n, a.hid);
+      stage_classes<CLS_T>(b + L::G, a, t * B_ROWS);
+    }
+    copies_commit();
+  };
+  stage(blockIdx.x, 0);
+  int buf = 0;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, buf ^= 1) {
+    stage(t + gridDim.x, buf ^ 1);
+    copies_wait<1>();
+    __syncthreads();
+    const float *const h = dense_smem + buf * L::BUF_FLOATS + L::H, *const g = dense_smem + buf * L::BUF_FLOATS + L::G;
+#pragma unroll 4
+    for (int r = group; r < B_ROWS; r += GROUPS) {
+      const float y = hidden_gradient<CLS_T>(g + r * CLS_T, w2, h[r * L::HS + hj]);
+      if (t * B_ROWS + r < a.n && hj < a.hid) a.D[(t * B_ROWS + r) * a.hid + hj] = y;
+    }
+#pragma unroll 4
+    for (int r = 0; r < B_ROWS; ++r) add_classes<PER>(acc2, g + r * CLS_T + group * PER, fmaxf(h[r * L::HS + hj], 0.0f));
+    __syncthreads();
+  }
+  copies_wait<0>();
+  float *const out = a.part + static_cast<size_t>(blockIdx.x) * O::FLOATS;
+#pragma unroll
+  for (int c = 0; c < PER; ++c) out[O::W2 + (group * PER + c) * HID_T + hj] = acc2[c];
+}
+
 // the blocks' sums, always in the same order
 template <int IN_T, int HID_T, int CLS_T>
 __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) {
   using O = PartLayout<IN_T, HID_T, CLS_T>;
-  const int w1 = a.hid * a.in, w2 = a.cls * a.hid, total = w1 + w2 + a.hid;
+  const int w1 = a.hid * a.in, w2 = a.cls * a.hid, total = w1 + w2 + (a.db1 ? a.hid : 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     int at, times = 1;
     float *to;
@@ -398,6 +481,17 @@ __global__ void __launch_bounds__(256) row_pieces_kernel(const int32_t *__restri
   }
 }
 
+// dst: n rows of `to` floats, the first `from` of them src's, zeros behind
+__global__ void __launch_bounds__(256) pad_columns_kernel(int32_t n, int32_t from, int32_t to, const float *__restrict__ src,
+                                                          float *__restrict__ dst) {
+  const int64_t total = static_cast<int64_t>(n) * to, step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+    const int64_t r = i / to;
+    const int32_t c = static_cast<int32_t>(i - r * to);
+    dst[i] = c < from ? src[r * from + c] : 0.0f;
+  }
+}
+
 template <typename Kernel>
 bool dense_smem_limit(Kernel kernel, size_t bytes) {
   CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
@@ -433,6 +527,22 @@ bool backward_variant(Context &ctx, DenseArgs a) {
   return true;
 }
 
+template <int HID_T, int CLS_T>
+bool hidden_variant(Context &ctx, DenseArgs a) {
+  const size_t smem = sizeof(float) * HiddenShared<HID_T, CLS_T>::FLOATS;
+  if (!dense_smem_limit(gcn_hidden_kernel<HID_T, CLS_T>, smem)) return false;
+  const int64_t tiles = (static_cast<int64_t>(a.n) + B_ROWS - 1) / B_ROWS;
+  const int grid = static_cast<int>(tiles < 2 * ctx.num_sms ? tiles : 2 * ctx.num_sms);
+  if (!ensure_workspace(ctx, sizeof(float) * PartLayout<0, HID_T, CLS_T>::FLOATS * static_cast<size_t>(grid))) return false;
+  a.part = reinterpret_cast<float *>(ctx.ws);
+  gcn_hidden_kernel<HID_T, CLS_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
+  CSG_CUDA(cudaGetLastError());
+  gcn_sums_kernel<0, HID_T, CLS_T><<<(a.cls * a.hid + 255) / 256, 256, 0, ctx.stream>>>(a, grid);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(2);
+  return true;
+}
+
 template <int IN_T, int HID_T>
 bool linear_variant(Context &ctx, int32_t n, int32_t in, int32_t hid, const float *x, const float *W, const float *b, float *Y) {
   const size_t smem = sizeof(float) * LinearShared<IN_T, HID_T>::FLOATS;
@@ -445,13 +555,15 @@ bool linear_variant(Context &ctx, int32_t n, int32_t in, int32_t hid, const floa
   return true;
 }
 
+// Limits: the weights and two tiles of `linear_kernel` (200 KB for 128 x 128) and the sums that the backward
+// kernels hold in registers (64 per thread) fill an SM; wider layers take library products.
 bool check_dense(const DenseArgs &a) {
   CSG_REQUIRE(a.n >= 1 && a.in >= 4 && a.in <= 128 && a.in % 4 == 0 && a.hid >= 4 && a.hid <= 128 && a.hid % 4 == 0 &&
-                  a.cls >= 1 && a.cls <= MAX_CLASSES,
-              "gcn: expect in and hidden in multiples of 4 up to 128 and up to %d classes (got %d, %d, %d)", MAX_CLASSES,
-              a.in, a.hid, a.cls);
+                  a.cls >= 1 && a.cls <= a.ld && a.ld <= MAX_CLASSES,
+              "gcn: expect in and hidden in multiples of 4 up to 128 and up to %d classes (got %d, %d, %d in %d columns)",
+              MAX_CLASSES, a.in, a.hid, a.cls, a.ld);
   const uintptr_t all = reinterpret_cast<uintptr_t>(a.P) | reinterpret_cast<uintptr_t>(a.Z);
-  CSG_REQUIRE(all % 16 == 0, "gcn: P and Z must be 16-byte aligned");
+  CSG_REQUIRE(all % 16 == 0, "gcn: dense operands must be 16-byte aligned");
   return true;
 }
 
@@ -475,7 +587,30 @@ bool run_backward_classes(Context &ctx, const DenseArgs &a) {
 bool run_backward(Context &ctx, const DenseArgs &a) {
   if (!check_dense(a)) return false;
   CSG_CUDA(cudaSetDevice(ctx.device));
-  return a.cls <= 16 ? run_backward_classes<16>(ctx, a) : run_backward_classes<MAX_CLASSES>(ctx, a);
+  return a.cls <= 16   ? run_backward_classes<16>(ctx, a)
+         : a.cls <= 32 ? run_backward_classes<32>(ctx, a)
+                       : run_backward_classes<MAX_CLASSES>(ctx, a);
+}
+
+template <int CLS_T>
+bool run_hidden_classes(Context &ctx, const DenseArgs &a) {
+  return a.hid <= 32   ? hidden_variant<32, CLS_T>(ctx, a)
+         : a.hid <= 64 ? hidden_variant<64, CLS_T>(ctx, a)
+                       : hidden_variant<128, CLS_T>(ctx, a);
+}
+
+bool run_hidden(Context &ctx, DenseArgs a) {
+  if (!check_dense(a)) return false;
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  a.in = 0;  // (no input gradients among the sums)
+  return a.cls <= 16 ? run_hidden_classes<16>(ctx, a) : a.cls <= 32 ? run_hidden_classes<32>(ctx, a) : run_hidden_classes<MAX_CLASSES>(ctx, a);
+}
+
+bool run_inputs(Context &ctx, DenseArgs a) {
+  if (!check_dense(a)) return false;
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  a.cls = 0;
+  return run_backward_classes<0>(ctx, a);
 }
 
 bool run_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *ptr, const float *val, float *out) {
@@ -497,14 +632,39 @@ bool run_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *ptr, cons
 
 }  // namespace
 
-bool launch_gcn_forward(Context &ctx, int32_t n, int32_t hid, int32_t cls, const float *Z, const float *W2, float *U) {
-  DenseArgs a = {n, 4, hid, cls, nullptr, nullptr, W2, Z, U, nullptr, nullptr, nullptr, nullptr, nullptr};
+bool launch_gcn_forward(Context &ctx, int32_t n, int32_t hid, int32_t cls, int32_t ld, const float *Z, const float *W2,
+                        float *U) {
+  DenseArgs a = {};
+  a.n = n, a.in = 4, a.hid = hid, a.cls = cls, a.ld = ld, a.Z = Z, a.W2 = W2, a.U = U;
   return run_forward(ctx, a);
 }
-bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, const float *G, const float *Z,
-                         const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2) {
-  DenseArgs a = {n, in, hid, cls, P, s, W2, Z, nullptr, G, nullptr, dW1, db1, dW2};
+bool launch_gcn_backward(Context &ctx, int32_t n, int32_t in, int32_t hid, int32_t cls, int32_t ld, const float *G,
+                         const float *Z, const float *P, const float *s, const float *W2, float *dW1, float *db1, float *dW2) {
+  DenseArgs a = {};
+  a.n = n, a.in = in, a.hid = hid, a.cls = cls, a.ld = ld, a.G = G, a.Z = Z, a.P = P, a.s = s, a.W2 = W2;
+  a.dW1 = dW1, a.db1 = db1, a.dW2 = dW2;
   return run_backward(ctx, a);
+}
+bool launch_gcn_hidden_gradient(Context &ctx, int32_t n, int32_t hid, int32_t cls, int32_t ld, const float *G,
+                                const float *Z, const float *W2, float *D, float *dW2) {
+  DenseArgs a = {};
+  a.n = n, a.in = 4, a.hid = hid, a.cls = cls, a.ld = ld, a.G = G, a.Z = Z, a.W2 = W2, a.D = D, a.dW2 = dW2;
+  return run_hidden(ctx, a);
+}
+bool launch_gcn_input_gradients(Context &ctx, int32_t n, int32_t in, int32_t hid, const float *E, const float *x,
+                                float *dW1, float *db1) {
+  DenseArgs a = {};
+  a.n = n, a.in = in, a.hid = hid, a.cls = a.ld = 1, a.Z = E, a.P = x, a.dW1 = dW1, a.db1 = db1;
+  return run_inputs(ctx, a);
+}
+bool launch_pad_columns(Context &ctx, int32_t n, int32_t from, int32_t to, const float *src, float *dst) {
+  CSG_REQUIRE(n >= 1 && from >= 1 && to >= from, "pad_columns: bad sizes n=%d from=%d to=%d", n, from, to);
+  CSG_CUDA(cudaSetDevice(ctx.device));
+  const int64_t blocks = (static_cast<int64_t>(n) * to + 255) / 256;
+  pad_columns_kernel<<<static_cast<int>(blocks < ctx.num_sms * 8 ? blocks : ctx.num_sms * 8), 256, 0, ctx.stream>>>(n, from, to, src, dst);
+  CSG_CUDA(cudaGetLastError());
+  count_launches(1);
+  return true;
 }
 bool launch_linear(Context &ctx, int32_t n, int32_t in, int32_t hid, const float *x, const float *W, const float *b, float *Y) {
   CSG_REQUIRE(n >= 1 && in >= 4 && in <= 128 && in % 4 == 0 && hid >= 4 && hid <= 128 && hid % 4 == 0,

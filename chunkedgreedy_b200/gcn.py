@@ -75,29 +75,62 @@ class GraphOperator:
         return self.spmm_ms
 
 
+def moved_columns(width):
+    """Full width that a sparse product of ``width`` columns costs as much as, or more: a power of two up
+    to 32, a multiple of four beyond."""
+    return max(4, 1 << (width - 1).bit_length()) if width <= 32 else (width + 3) // 4 * 4
+
+
+def padded_columns(width):
+    """Columns to take a sparse product of ``width`` at where the caller may choose.  Symmetrised R-MAT scale 20, us: 3
+    columns 480 and 4 425, 7 651 and 8 416, 13 1,014 and 16 479, 20 850, 30 1,058 and 32 634.  An odd width from 17 on
+    has a lane per column (17 628, 47 880 and 48 832), beyond 32 the rest is small."""
+    return width if width > 32 or (width > 16 and width % 2) else moved_columns(width)
+
+
+def step_widths(rows, in_dim, hidden, classes, fused):
+    """Widths of a training step's four sparse products, (first layer forward, second forward, second
+    backward, first backward).  The second operator goes behind the second linear layer (op(h) W2^T =
+    op(h W2^T)) where that moves no more columns, on the fused route, which saves besides; on torch's where the
+    columns saved are worth a bias and a padding of their own (300 inputs, 64 hidden units, 10 classes: 4,096 rows 0.67 ms
+    as it stands and 0.70 behind, 1.05 M rows 6.7 and 6.1).  Logits are padded from 32,768 rows on: below, a step
+    is its launches (4,096 rows 0.58 ms, 0.60 padded).  The first layer keeps its order: hidden units within a rounding
+    of zero decide by their sign, and op(x) W1^T rounds differently.  Backward, the fused route takes op(x)
+    or op(D), whichever moves fewer columns (128 inputs, 64 hidden units, 16 classes, 1.05 M rows: 4.8 and 4.2 ms)."""
+    saved = hidden - moved_columns(classes)
+    behind = saved >= 0 if fused else rows * saved >= 1 << 22
+    second = hidden if not behind else padded_columns(classes) if rows >= 1 << 15 else classes
+    first = in_dim if fused and moved_columns(in_dim) <= moved_columns(hidden) else hidden
+    return hidden, second, second, first
+
+
+def _call(fn, *args):
+    if fn(*args) != 0:
+        _lib.check()
+
+
 class LayersFn(torch.autograd.Function):
-    """relu(op(x W1^T + b1)) W2^T for features that want no gradient.  The backward pass needs the
-    first layer's gradient D^T op(x) (op is symmetric: op(D)^T x), so it takes one sparse product
-    over the features and everything dense in one kernel."""
+    """relu(op(x W1^T + b1)) W2^T for features that want no gradient, in ``out`` columns, those
+    behind the classes zero.  The backward pass needs the first layer's gradient D^T op(x) = op(D)^T x (op
+    is symmetric): one sparse product over whichever is narrower, and everything dense in one or two kernels."""
 
     @staticmethod
-    def forward(ctx, x, op, w1, b1, w2):
+    def forward(ctx, x, op, w1, b1, w2, out, first):
         n, hidden, classes = x.shape[0], w1.shape[0], w2.shape[0]
         x, w1, b1, w2 = x.contiguous(), w1.contiguous(), b1.contiguous(), w2.contiguous()
         y = torch.empty((n, hidden), dtype=torch.float32, device=x.device)
-        u = torch.empty((n, classes), dtype=torch.float32, device=x.device)
+        u = torch.empty((n, out), dtype=torch.float32, device=x.device)
         ctx.lib_ctx = _ctx(getattr(op, "ctx", None), x)
+        lib, handle = _lib.load(), ctx.lib_ctx.handle
         with torch.cuda.device(x.device):
             _enter(ctx.lib_ctx, x)
-            if _lib.load().sporder_linear(ctx.lib_ctx.handle, n, x.shape[1], hidden, x.data_ptr(), w1.data_ptr(),
-                                          b1.data_ptr(), y.data_ptr()) != 0:
-                _lib.check()
+            _call(lib.sporder_linear, handle, n, x.shape[1], hidden, x.data_ptr(), w1.data_ptr(), b1.data_ptr(),
+                  y.data_ptr())
             z = op(y)
             _enter(ctx.lib_ctx, x)
-            if _lib.load().sporder_gcn_forward(ctx.lib_ctx.handle, n, hidden, classes, z.data_ptr(), w2.data_ptr(),
-                                               u.data_ptr()) != 0:
-                _lib.check()
-        ctx.op = op
+            _call(lib.sporder_gcn_forward_padded, handle, n, hidden, classes, out, z.data_ptr(), w2.data_ptr(),
+                  u.data_ptr())
+        ctx.op, ctx.first = op, first
         ctx.save_for_backward(x, z, w2)
         return u
 
@@ -106,27 +139,66 @@ class LayersFn(torch.autograd.Function):
     def backward(ctx, g):
         x, z, w2 = ctx.saved_tensors
         op = ctx.op
-        n, in_dim, hidden, classes = x.shape[0], x.shape[1], z.shape[1], w2.shape[0]
+        n, in_dim, hidden, classes, out = x.shape[0], x.shape[1], z.shape[1], w2.shape[0], g.shape[1]
         g = g.contiguous()
-        p = op(x)
-        s = op.row_sums() if hasattr(op, "row_sums") else op(torch.ones_like(x[:, :1]))[:, 0].contiguous()
         dw1 = torch.empty((hidden, in_dim), dtype=torch.float32, device=x.device)
         db1 = torch.empty(hidden, dtype=torch.float32, device=x.device)
         dw2 = torch.empty((classes, hidden), dtype=torch.float32, device=x.device)
+        lib, handle = _lib.load(), ctx.lib_ctx.handle
         with torch.cuda.device(x.device):
-            _enter(ctx.lib_ctx, x)
-            if _lib.load().sporder_gcn_backward(ctx.lib_ctx.handle, n, in_dim, hidden, classes, g.data_ptr(),
-                                                z.data_ptr(), p.data_ptr(), s.data_ptr(), w2.data_ptr(),
-                                                dw1.data_ptr(), db1.data_ptr(), dw2.data_ptr()) != 0:
-                _lib.check()
-        return None, None, dw1, db1, dw2
+            if ctx.first == in_dim:
+                p = op(x)
+                s = op.row_sums() if hasattr(op, "row_sums") else op(torch.ones_like(x[:, :1]))[:, 0].contiguous()
+                _enter(ctx.lib_ctx, x)
+                _call(lib.sporder_gcn_backward_padded, handle, n, in_dim, hidden, classes, out, g.data_ptr(),
+                      z.data_ptr(), p.data_ptr(), s.data_ptr(), w2.data_ptr(), dw1.data_ptr(), db1.data_ptr(),
+                      dw2.data_ptr())
+            else:
+                d = torch.empty_like(z)
+                _enter(ctx.lib_ctx, x)
+                _call(lib.sporder_gcn_hidden_gradient, handle, n, hidden, classes, out, g.data_ptr(), z.data_ptr(),
+                      w2.data_ptr(), d.data_ptr(), dw2.data_ptr())
+                e = op(d)
+                _enter(ctx.lib_ctx, x)
+                _call(lib.sporder_gcn_input_gradients, handle, n, in_dim, hidden, e.data_ptr(), x.data_ptr(),
+                      dw1.data_ptr(), db1.data_ptr())
+        return None, None, dw1, db1, dw2, None, None
+
+
+def _pad_columns(g, width, ctx):
+    if not (g.is_cuda and g.dtype == torch.float32):
+        return F.pad(g, (0, width - g.shape[1]))
+    g = g.contiguous()
+    padded = torch.empty((g.shape[0], width), dtype=torch.float32, device=g.device)
+    ctx = _ctx(ctx, g)
+    with torch.cuda.device(g.device):
+        _enter(ctx, g)
+        _call(_lib.load().sporder_pad_columns, ctx.handle, g.shape[0], g.shape[1], width, g.data_ptr(),
+              padded.data_ptr())
+    return padded
+
+
+class LogitsFn(torch.autograd.Function):
+    """op(u) + b over the first ``classes`` columns of u."""
+
+    @staticmethod
+    def forward(ctx, u, op, b, classes):
+        ctx.op, ctx.width, ctx.biased = op, u.shape[1], b is not None
+        z = op(u.contiguous())
+        if ctx.width != classes:
+            z = z[:, :classes]
+        return z + b if ctx.biased else z.contiguous()
+
+    @staticmethod
+    def backward(ctx, g):
+        db = g.sum(0) if ctx.biased else None
+        if ctx.width != g.shape[1]:
+            g = _pad_columns(g, ctx.width, getattr(ctx.op, "ctx", None))
+        return ctx.op(g.contiguous()), None, db, None
 
 
 class GCN(torch.nn.Module):
-    """Linear -> op -> ReLU -> op -> Linear, the second operator taken behind the linear layer
-    where that is narrower (op is linear in its columns: op(h) W2^T = op(h W2^T)).  The first layer
-    keeps its order: hidden units within a rounding of zero decide by their sign, and op(x) W1^T rounds
-    differently."""
+    """Linear -> op -> ReLU -> op -> Linear; `step_widths` says where the operators go."""
 
     def __init__(self, in_dim, hidden, classes):
         super().__init__()
@@ -137,15 +209,19 @@ class GCN(torch.nn.Module):
         hidden, in_dim = self.w1.weight.shape
         classes = self.w2.weight.shape[0]
         # limits of the fused kernels; others, and features that want a gradient, by torch
-        if (not x.requires_grad and in_dim % 4 == 0 and in_dim <= min(128, 2 * hidden) and hidden % 4 == 0
-                and hidden <= 128 and classes <= min(48, hidden) and self.w1.bias is not None and x.data_ptr() % 16 == 0
-                and all(t.is_cuda and t.dtype == torch.float32 for t in (x, self.w1.weight, self.w2.weight))):
-            u = LayersFn.apply(x, op, self.w1.weight, self.w1.bias, self.w2.weight)
-            return SpMMFn.apply(u, op) + self.w2.bias
+        fused = (not x.requires_grad and in_dim % 4 == 0 and in_dim <= 128 and hidden % 4 == 0 and hidden <= 128
+                 and classes <= 48 and moved_columns(classes) <= hidden and self.w1.bias is not None
+                 and x.data_ptr() % 16 == 0
+                 and all(t.is_cuda and t.dtype == torch.float32 for t in (x, self.w1.weight, self.w2.weight)))
+        _, out, _, first = step_widths(x.shape[0], in_dim, hidden, classes, fused)
+        if fused:
+            u = LayersFn.apply(x, op, self.w1.weight, self.w1.bias, self.w2.weight, out, first)
+            return LogitsFn.apply(u, op, self.w2.bias, classes)
         h = F.relu(SpMMFn.apply(self.w1(x), op))
-        if classes < hidden:
-            return SpMMFn.apply(F.linear(h, self.w2.weight), op) + self.w2.bias
-        return self.w2(SpMMFn.apply(h, op))
+        if out == hidden:
+            return self.w2(SpMMFn.apply(h, op))
+        w2 = self.w2.weight if out == classes else F.pad(self.w2.weight, (0, 0, 0, out - classes))
+        return LogitsFn.apply(F.linear(h, w2), op, self.w2.bias, classes)
 
 
 def normalised_values(ptr, ind):

@@ -288,6 +288,35 @@ SPORDER_API int32_t sporder_gcn_backward(sporder_context_t ctx, int32_t n, int32
                                          const float *d_W2, float *d_dW1, float *d_db1,
                                          float *d_dW2);
 
+/* The same with U and G in rows of `columns` floats (classes <= columns <= 48): forward writes
+ * zeros behind the classes, backward does not read there.  sporder_pad_columns brings a matrix of
+ * `from` columns into that form.  (A sparse product of a ragged width costs more than the next
+ * full one.) */
+SPORDER_API int32_t sporder_gcn_forward_padded(sporder_context_t ctx, int32_t n, int32_t hidden,
+                                               int32_t classes, int32_t columns, const float *d_Z,
+                                               const float *d_W2, float *d_U);
+SPORDER_API int32_t sporder_gcn_backward_padded(sporder_context_t ctx, int32_t n, int32_t in_dim,
+                                                int32_t hidden, int32_t classes, int32_t columns,
+                                                const float *d_G, const float *d_Z,
+                                                const float *d_P, const float *d_s,
+                                                const float *d_W2, float *d_dW1, float *d_db1,
+                                                float *d_dW2);
+SPORDER_API int32_t sporder_pad_columns(sporder_context_t ctx, int32_t n, int32_t from, int32_t to,
+                                        const float *d_src, float *d_dst);
+
+/* The same gradients in two halves around a sparse product at the hidden width, for layers whose
+ * inputs are wider (the operator is symmetric, E = A D):
+ *   hidden_gradient: D as above (n x hidden) and dW2;
+ *   input_gradients: dW1 = E^T x, db1 = column sums of E, x n x in_dim.
+ * Limits as above, Z, D, E and x 16-byte aligned.  Return 0 or -1. */
+SPORDER_API int32_t sporder_gcn_hidden_gradient(sporder_context_t ctx, int32_t n, int32_t hidden,
+                                                int32_t classes, int32_t columns,
+                                                const float *d_G, const float *d_Z,
+                                                const float *d_W2, float *d_D, float *d_dW2);
+SPORDER_API int32_t sporder_gcn_input_gradients(sporder_context_t ctx, int32_t n, int32_t in_dim,
+                                                int32_t hidden, const float *d_E,
+                                                const float *d_x, float *d_dW1, float *d_db1);
+
 /* Number of kernels this library has launched in this process (all contexts). */
 SPORDER_API uint64_t sporder_kernel_launches(void);
 
