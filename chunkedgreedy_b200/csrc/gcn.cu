@@ -7,9 +7,10 @@
 //   backward  (G = dL/dU)  D = (G W2) * (Z > 0),  dW1 = D^T P,  db1 = D^T s,  dW2 = G^T relu(Z);
 // or, where the hidden layer is narrower than the inputs, with E = A D in place of P (A is symmetric):
 //             dW1 = E^T x,  db1 = E^T 1.
-// One kernel forward, one backward, where D never exists in memory, or two around E = A D.  The backward pass is bound by fp32 multiply-adds
-// (2 n in hidden of them, against three passes over n rows of 128 floats): blocks are persistent, one
-// per SM, operands staged with cp.async a tile ahead, 8 x 8 results per thread.  On 1.05 M rows,
+// One kernel forward, one backward, where D never exists in memory, or two around E = A D.  The
+// backward pass is bound by fp32 multiply-adds (2 n in hidden of them, against three passes over n
+// rows of 128 floats): blocks are persistent, one per SM, operands staged with cp.async a tile ahead,
+// 8 x 8 results per thread.  On 1.05 M rows,
 // 128 -> 128 -> 16, on a B200: 1.09 ms (53 % of the fp32 pipes; two warps per scheduler, and the
 // phases of a tile do not overlap); one torch kernel per operation took 2.4 ms.
 #include "../../include/sporder_b200.h"
@@ -262,10 +263,14 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
     w2[c] = c < a.cls && hj < a.hid ? a.W2[static_cast<size_t>(c) * a.hid + hj] : 0.0f;
   float2 acc[NJ][NI / 2];
   float acc2[GIVEN ? 1 : PER], accb = 0.0f;
+  [[maybe_unused]] float lost = 0.0f;
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int i = 0; i < NI / 2; ++i) acc[j][i] = make_float2(0.0f, 0.0f);
+  // (E is read where it lies, so there are registers for a tile's sums apart from the sums of all tiles: these
+  // largely cancel, and a chain over all rows of a block loses more)
+  [[maybe_unused]] float2 all[GIVEN ? NJ : 1][GIVEN ? NI / 2 : 1] = {};
 #pragma unroll
   for (int c = 0; c < PER; ++c) acc2[c] = 0.0f;
   for (int i = tid; i < 2 * L::BUF_FLOATS; i += D_THREADS) dense_smem[L::BUF + i] = 0.0f;  // classes behind the last
@@ -294,7 +299,12 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
     const float *const p = b + L::P, *const h = b + L::H, *const g = b + L::G, *const s = b + L::S;
     const float *d = h;
     if constexpr (GIVEN) {
-      for (int r = group; r < B_ROWS; r += GROUPS) accb += h[r * L::HS + hj];
+      // (the sum over all rows largely cancels: the tile's rows first, then compensated)
+      float tile = 0.0f;
+      for (int r = group; r < B_ROWS; r += GROUPS) tile += h[r * L::HS + hj];
+      const float y = tile - lost, sum = accb + y;
+      lost = (sum - accb) - y;
+      accb = sum;
     } else {
       float *const own = dense_smem + L::D;
 #pragma unroll 4
@@ -325,9 +335,24 @@ __global__ void __launch_bounds__(D_THREADS, 1) gcn_backward_kernel(DenseArgs a)
         for (int i = 0; i < NI / 2; ++i) fma2(acc[j][i], make_float2(dj[j], dj[j]), pi[i]);
       if constexpr (!GIVEN) add_classes<PER>(acc2, g + r * CLS_T + group * PER, fmaxf(h[r * L::HS + hj], 0.0f));
     }
+    if constexpr (GIVEN) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI / 2; ++i) {
+          all[j][i] = make_float2(all[j][i].x + acc[j][i].x, all[j][i].y + acc[j][i].y);
+          acc[j][i] = make_float2(0.0f, 0.0f);
+        }
+    }
     __syncthreads();
   }
   copies_wait<0>();
+  if constexpr (GIVEN) {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int i = 0; i < NI / 2; ++i) acc[j][i] = all[j][i];
+  }
   float *const out = a.part + static_cast<size_t>(blockIdx.x) * O::FLOATS;
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
@@ -394,7 +419,7 @@ __global__ void __launch_bounds__(D_THREADS, 2) gcn_hidden_kernel(DenseArgs a) {
   for (int c = 0; c < PER; ++c) out[O::W2 + (group * PER + c) * HID_T + hj] = acc2[c];
 }
 
-// the blocks' sums, always in the same order
+// the blocks' sums, always in the same order, in 64 bits (some hundred terms that largely cancel)
 template <int IN_T, int HID_T, int CLS_T>
 __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) {
   using O = PartLayout<IN_T, HID_T, CLS_T>;
@@ -414,7 +439,7 @@ __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) 
       to = a.db1 + (i - w1 - w2);
       times = D_THREADS / HID_T;
     }
-    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
     for (int g = 0; g < times; ++g) {
       const float *src = a.part + at + g * HID_T;
       int b = 0;
@@ -423,7 +448,7 @@ __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) 
         for (int u = 0; u < 4; ++u) sum[u] += src[static_cast<size_t>(b + u) * O::FLOATS];
       for (; b < blocks; ++b) sum[0] += src[static_cast<size_t>(b) * O::FLOATS];
     }
-    *to = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    *to = static_cast<float>((sum[0] + sum[1]) + (sum[2] + sum[3]));
   }
 }
 
