@@ -32,6 +32,40 @@ def test_columns():
         4, 4, 8, 16, 16, 17, 32, 32, 32, 31, 32, 33, 47]
 
 
+def test_layers_with_hooks_and_other_layers_are_called():
+    # a pre-hook that sets the weight (as weight normalisation does), a hook that sees the output, a layer
+    # of another kind; sizes at which plain layers would have their weights taken out of them
+    n = 1 << 17
+    x = torch.randn((n, 4), generator=torch.Generator().manual_seed(0))
+    op = lambda t: 0.5 * t  # noqa: E731 (stands for the sparse product)
+    model = gcn.GCN(4, 64, 3)
+    with torch.no_grad():
+        want = op(torch.relu(op(model.w1(x)))) @ (2.0 * model.w2.weight).t() + model.w2.bias
+        assert torch.allclose(model(x, op), op(torch.relu(op(model.w1(x)))) @ model.w2.weight.t() + model.w2.bias, atol=1e-5)
+        weight, seen = model.w2.weight.clone(), []
+
+        def set_weight(layer, value):
+            layer.weight.copy_(value)
+
+        pre = model.w2.register_forward_pre_hook(lambda m, _: set_weight(m, 2.0 * weight))
+        post = model.w2.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+        assert torch.allclose(model(x, op), want, atol=1e-5) and seen == [(n, 3)]
+        pre.remove()
+        post.remove()
+        model.w2 = torch.nn.Sequential(torch.nn.Linear(64, 8), torch.nn.ReLU(), torch.nn.Linear(8, 3))
+        assert torch.allclose(model(x, op), model.w2(op(torch.relu(op(model.w1(x))))), atol=1e-5)
+
+
+def test_logits_without_a_bias():
+    model = gcn.GCN(4, 64, 3)
+    model.w2.bias = None
+    x = torch.randn((1 << 17, 4))
+    z = model(x, lambda t: 0.5 * t)
+    assert torch.allclose(z, 0.5 * torch.relu(0.5 * model.w1(x)) @ model.w2.weight.t(), atol=1e-5)
+    z.sum().backward()
+    assert model.w2.weight.grad.shape == (3, 64)
+
+
 def _signs(model, x, op):
     """Which hidden units the model takes as positive.  One within a rounding of zero may fall on the other side in
     64 bits, and its whole gradient with it, so the reference below takes the model's own decisions."""
