@@ -229,6 +229,14 @@ __device__ __forceinline__ bool unit_is_even(const int32_t *wp, int32_t bcount, 
   return 7 * longest * bcount <= 8 * nonzeros && (PAN == 1 ? 4 : 6) * bcount <= nonzeros;
 }
 
+// Rows of up to 32 nonzeros, on average a third of the longest or more: at 32 columns, where a lane of the whole
+// warp loads a single float, lane groups are still the faster way (24 nonzeros in each of 1.05 M rows: 786 us by
+// the warp, 395 by groups; 1 to 31: 607 and 431).  Power-law graphs have few such units (R-MAT scale 20 425 and 421).
+constexpr int MILD_MAX = 32;
+__device__ __forceinline__ bool unit_is_mild(const int32_t *wp, int32_t bcount, int32_t longest) {
+  return longest <= MILD_MAX && longest * bcount <= 3 * (wp[bcount] - wp[0]);
+}
+
 // N nonzeros of a row, pairs at sp[0 .. N): gather and FMA
 template <int G, int VEC, int PAN, bool MASK, int N>
 __device__ __forceinline__ void short_slots(const int2 *sp, const char *bcol, int32_t wbytes, int32_t col0,
@@ -343,8 +351,10 @@ __device__ __forceinline__ void queue_long_row(const SpmmArgs &a, int32_t r, int
 // blocks per SM; both launches 4.3 ms walking, 3.1 to 3.3 so.
 //
 // MG > 0, a product of one panel of MG lanes with MVEC columns each: rows of up to GROUP_MAX nonzeros
-// go to lane groups of MG lanes, several rows at a time (most rows of a power-law graph: width 64,
-// R-MAT scale 22, 1.98 ms without, 1.90 with), the longer ones to the whole warp, VEC columns a lane.
+// go to lane groups of MG lanes, several rows at a time, the longer ones to the whole warp, VEC columns
+// a lane.  Two is where the widths and graphs measured agree best, within a few percent of 1 to 4: symmetrised R-MAT
+// scale 20 (half the edges) at 64, 594 us with 0, 537, 534, 536, 537 with 4; R-MAT scale 22 1,942, 1,929, 1,922, 1,916,
+// 1,904; scale 20 with 4 edges a row at 40, 237, 246, 246, 253, 252; 131,072 Zipf rows at 48, 118, 117, 118, 123, 124.
 constexpr int GROUP_MAX = 2;
 template <int VEC, int PAN, bool MASK, int S_PAIRS, int UC, int MG = 0, int MVEC = 1>
 __device__ __forceinline__ void whole_unit(const SpmmArgs &a, const int32_t *wp, int2 *sp, int32_t bfirst, int32_t bcount,
@@ -479,7 +489,7 @@ __global__ void __launch_bounds__(M_THREADS, BLOCKS) spmm_rows_kernel(SpmmArgs a
       const int32_t longest = unit_longest(wp, count, a.nnz, lane);
       if (EVEN != G && longest <= SHORT_MAX && unit_is_even<PAN>(wp, count, longest))
         short_rows<EVEN, VEC, 1, false, PAIRS>(a, wp, spair[warp], first, count, lane);
-      else if (longest <= SHORT_MAX)
+      else if (longest <= SHORT_MAX || (G == 8 && unit_is_mild(wp, count, longest)))
         short_rows<G, VEC, PAN, MASK, PAIRS>(a, wp, spair[warp], first, count, lane);
       else
         whole_unit<G * VEC / 32, 1, MASK, PAIRS, UC, G, VEC>(a, wp, spair[warp], first, count, lane);

@@ -62,10 +62,11 @@ inline SpmmShape spmm_shape(int32_t n, int32_t nnz, int32_t w, int align) {
   const int cols = w / vec;
   auto narrow = [&](int lanes, int masked, int whole) { return SpmmShape{lanes, vec, 1, masked, whole, lanes, M_BLOCKS_PER_SM}; };
   if (vec == 4) {
-    // At 32 columns the whole warp has few bytes in flight, which tells once most of B is not in
-    // the L2.  R-MAT scale 20 (134 MB of B) 464 us walked, 409 by the warp; its symmetrised form 664
-    // and 643; 262,144 rows of that (34 MB) 239 and 152; scale 22 (537 MB) 1.42 and 1.51 ms.  Matrices of
-    // short rows gain nothing (9-point mesh 135 and 136 us).
+    // At 32 columns a lane of the whole warp has a single float per gather, which saves power-law graphs the
+    // idle lanes of groups that wait for the longest row, and tells against it once most of B is not in the L2.
+    // By the warp over walked, R-MAT of 9 to 16 edges a row: 0.78 to 0.97 with 8 MiB of B, 0.62 to 0.87 with 32, 0.87
+    // to 0.98 with 128, 0.87 to 0.94 with 183, 0.91 to 0.95 with 256, 0.92 to 1.00 with 366, 0.93 to 1.07 with 512.  (4 edges
+    // would gain as well, but their lengths on average are those of meshes, which lose a percent.)
     if (w == 32) return narrow(8, 0, nnz > 12ll * n && b_bytes <= (256ll << 20));
     if (w == 64) return narrow(16, 0, 1);
     if (w == 16 || w == 8 || w == 4) return narrow(cols, 0, 0);

@@ -85,13 +85,17 @@ torch = pytest.importorskip("torch")
 
 def _rows(kind, n):
     """Row lengths: `even` 9 for all; `mixed` 1 to 16, no two neighbours alike; `edge` 16 and 17 (the longest short
-    row and one more); `late` short rows with one of 300 in the middle."""
+    row and one more); `late` short rows with one of 300 in the middle; `mild` 1 to 31, `over` 32 and 33."""
     if kind == "even":
         length = torch.full((n,), 9, device="cuda")
     elif kind == "mixed":
         length = torch.arange(n, device="cuda") * 7 % 16 + 1
     elif kind == "edge":
         length = 16 + (torch.arange(n, device="cuda") % 40 == 39).long()
+    elif kind == "mild":
+        length = torch.arange(n, device="cuda") * 7 % 31 + 1
+    elif kind == "over":
+        length = 32 + (torch.arange(n, device="cuda") % 40 == 39).long()
     else:
         length = torch.full((n,), 6, device="cuda")
         length[n // 2] = 300
@@ -139,10 +143,46 @@ def test_shapes_of_large_products(kind, n, w):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["even", "mixed", "edge", "mild", "over", "late"])
+@pytest.mark.parametrize("n", [1, 33, 30_011, 300_007])
+def test_32_columns(kind, n):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    _check(_rows(kind, n), 32, g)
+
+
+def _best_of(ptr, ind, val, widths):
+    import chunkedgreedy_b200 as sp
+    n, best = ptr.numel() - 1, {}
+    for w in widths:
+        B, C = torch.randn((n, w), device="cuda"), torch.empty((n, w), device="cuda")
+        times = []
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(5):
+                sp.spmm(ptr, ind, val, B, out=C, sync=False)
+            e1.record()
+            e1.synchronize()
+            times.append(e0.elapsed_time(e1))
+        best[w] = min(times)
+    return best
+
+
+@pytest.mark.gpu
+def test_rows_of_24_at_32_columns_cost_half_of_64():
+    # 24 nonzeros anywhere in each of 2^20 rows: half the bytes of 64 columns.  With a warp to a row of 32 columns
+    # the ratio was 0.81, by lane groups it is 0.41.
+    n = 1 << 20
+    ptr = torch.arange(0, 24 * n + 1, 24, device="cuda", dtype=torch.int32)
+    ind = torch.randint(0, n, (24 * n,), device="cuda", dtype=torch.int32)
+    best = _best_of(ptr, ind, torch.randn(24 * n, device="cuda"), (32, 64))
+    assert best[32] <= 0.65 * best[64], best
+
+
+@pytest.mark.gpu
 def test_a_mesh_costs_no_more_per_column_at_a_wide_width():
     # 9-point mesh in grid order, 2^20 rows: the gathers of 96 columns are 1.5 times those of 64.
     # With a warp to a row and a quarter of its lanes idle the ratio was 2.4, by lane groups it is 1.4.
-    import chunkedgreedy_b200 as sp
     a = 1024
     v = torch.arange(a * a, device="cuda")
     y, x = v // a, v % a
@@ -156,17 +196,5 @@ def test_a_mesh_costs_no_more_per_column_at_a_wide_width():
     ptr[1:] = torch.cumsum(ok.sum(1), 0)
     ind = cols[ok].int()
     val = torch.randn(ind.numel(), device="cuda")
-    best = {}
-    for w in (64, 96):
-        B, C = torch.randn((a * a, w), device="cuda"), torch.empty((a * a, w), device="cuda")
-        times = []
-        for _ in range(12):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            for _ in range(5):
-                sp.spmm(ptr, ind, val, B, out=C, sync=False)
-            e1.record()
-            e1.synchronize()
-            times.append(e0.elapsed_time(e1))
-        best[w] = min(times)
+    best = _best_of(ptr, ind, val, (64, 96))
     assert best[96] <= 1.9 * best[64], best
