@@ -24,7 +24,7 @@
 // A permutation that keeps every row and column inside its block of 1024 (every csg order
 // with the default chunk size does) needs none of this: the old row is sorted by column, so the
 // new row is already sorted block by block and only the entries of one block have to be ordered
-// among themselves.  ptr_new_kernel notices such a permutation and tells the host, which then
+// among themselves.  len_block_sums_kernel notices such a permutation and tells the host, which then
 // launches apply_flat_kernel instead of the kernels above.  That one, which also does the copy
 // of the rows-only mode, cuts the output into tiles of 2048 entries whatever rows they belong to.
 #include <cstddef>
@@ -66,18 +66,35 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *tota
   return base + incl - v;
 }
 
+// Entries of the rows that each block of new rows takes.  With `outcome`, the last block also tells the host
+// whether any row leaves its block of 1024: here and not in ptr_new_kernel, so that the host reads it and
+// launches the rest while the scan still runs (a random order of a 65,536-row mesh: 90 us with the
+// wait behind ptr_new_kernel, 84 here).
 __global__ void __launch_bounds__(R_THREADS) len_block_sums_kernel(
     int32_t n, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
-    int32_t *__restrict__ block_sums) {
+    int32_t *__restrict__ block_sums, uint32_t *__restrict__ leaves_block, volatile uint32_t *outcome, uint32_t ticket) {
   __shared__ int32_t sm[R_THREADS / 32];
   const int32_t base = blockIdx.x * R_SCAN_TILE;
   int32_t s = 0;
+  int moved = 0;
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
     const int32_t p = base + i * R_THREADS + threadIdx.x;
     if (p < n) {
       const int32_t src = new_order[p];
       s += ptr_old[src + 1] - ptr_old[src];
+      moved |= (src >> LOCAL_BITS) != (p >> LOCAL_BITS);
+    }
+  }
+  moved = __syncthreads_or(moved);
+  if (outcome && threadIdx.x == 0) {
+    if (moved) atomicExch(leaves_block, 1u);
+    __threadfence();
+    if (atomicAdd(leaves_block + 1, 1u) == gridDim.x - 1) {
+      __threadfence();
+      outcome[1] = atomicAdd(leaves_block, 0u);
+      __threadfence_system();
+      outcome[0] = ticket;
     }
   }
   int32_t tot;
@@ -120,15 +137,10 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32
 __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     int32_t n, int32_t nnz, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
     const int32_t *__restrict__ block_sums, int32_t *__restrict__ ptr_new,
-    int32_t *__restrict__ old2new, uint32_t *__restrict__ leaves_block, int32_t *__restrict__ tile_row,
-    int32_t *__restrict__ row_delta,
-    volatile uint32_t *outcome, uint32_t ticket) {
+    int32_t *__restrict__ old2new, int32_t *__restrict__ tile_row, int32_t *__restrict__ row_delta) {
   constexpr int WARPS = R_THREADS / 32;
   __shared__ int32_t sums[R_SCAN_IPT * WARPS];  // of 32 rows each, in row order
-  __shared__ int moved;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) moved = 0;
-  __syncthreads();
   const int32_t first = blockIdx.x * R_SCAN_TILE + threadIdx.x;
   int32_t len[R_SCAN_IPT], from[R_SCAN_IPT], incl[R_SCAN_IPT];
 #pragma unroll
@@ -140,7 +152,6 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
       from[i] = ptr_old[src];
       len[i] = ptr_old[src + 1] - from[i];
       if (old2new) old2new[src] = p;
-      if ((src >> LOCAL_BITS) != (p >> LOCAL_BITS)) moved = 1;  // leaves its block of 1024
     }
     incl[i] = len[i];
   }
@@ -156,7 +167,6 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
   for (int i = 0; i < R_SCAN_IPT; ++i)
     if (lane == 31) sums[i * WARPS + warp] = incl[i];
   __syncthreads();
-  if (threadIdx.x == 0 && moved) atomicExch(leaves_block, 1u);
   if (warp == 0) {  // sums -> what lies in front of each 32 rows
     static_assert(R_SCAN_IPT * WARPS == 64, "two per lane");
     const int32_t x = sums[2 * lane], y = sums[2 * lane + 1];
@@ -183,15 +193,6 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     if (p < n) {
       row_delta[p] = from[i] - run;
       ptr_new[p + 1] = run + len[i];
-    }
-  }
-  if (outcome) {  // the last block tells the host whether any row left its block of 1024
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(leaves_block + 1, 1u) == gridDim.x - 1) {
-      outcome[1] = atomicAdd(leaves_block, 0u);
-      __threadfence_system();
-      outcome[0] = ticket;
     }
   }
 }
@@ -262,8 +263,10 @@ __device__ __forceinline__ void apply_class(const ApplyArgs &a, unsigned mask, i
 }
 
 // One warp per 32 consecutive new rows: descriptors with coalesced loads, rows of up to 32
-// entries finished here, longer rows queued for the kernels behind.
-__global__ void __launch_bounds__(R_THREADS) apply_short_kernel(ApplyArgs a) {
+// entries finished here, longer rows queued for the kernels behind.  Latency of its gathers: eight
+// blocks per SM, 32 registers (road network of 2.1 M rows, random order: 162 us with 40 registers and
+// six blocks, 136 with eight).
+__global__ void __launch_bounds__(R_THREADS, 8) apply_short_kernel(ApplyArgs a) {
   const int lane = threadIdx.x & 31;
   const int32_t warps = (gridDim.x * blockDim.x) >> 5;
   const int32_t batches = (a.n + 31) / 32;
@@ -848,15 +851,15 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
     a.tmp_val = reinterpret_cast<float *>(ctx.ws + ar.take(sizeof(float) * static_cast<size_t>(nnz > 0 ? nnz : 1)));
   }
   CSG_CUDA(cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), ctx.stream));
-  len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums);
+  uint32_t *const outcome = reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  ++ctx.outcome_ticket;
+  len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, a.counters + CNT_MOVED,
+                                                          symmetric ? outcome : nullptr, ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
   scan_block_sums_kernel<<<1, 1024, 0, ctx.stream>>>(nb, block_sums);
   CSG_CUDA(cudaGetLastError());
-  uint32_t *const outcome = reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
-  ++ctx.outcome_ticket;
   ptr_new_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, nnz, d_ptr_old, d_new_order, block_sums, d_ptr_new,
-                                                   old2new, a.counters + CNT_MOVED, tile_row, row_delta,
-                                                   symmetric ? outcome : nullptr, ctx.outcome_ticket);
+                                                   old2new, tile_row, row_delta);
   CSG_CUDA(cudaGetLastError());
   count_launches(3);
   if (nnz == 0) return true;
