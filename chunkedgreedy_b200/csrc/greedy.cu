@@ -42,7 +42,7 @@ struct ChainStats {  // lives at ctrl[CTRL_STATS ...]
 };
 
 // The chain of rows [start, end), run by one warp on the table itself.
-__device__ __noinline__ void chain_chunk(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited) {
+__device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited) {
   const int lane = lane_id();
   const int32_t size = end - start;
   const int32_t words = (size + 31) >> 5;
@@ -248,6 +248,12 @@ __device__ __forceinline__ void sts_u16(uint32_t at, uint32_t v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(static_cast<uint16_t>(v)));
 }
 
+// Out of line, for the one chunk in a million: inlined it would cost greedy_lists_kernel registers.  (Where the
+// table is all there is it is inlined: called, it reads its arguments from memory at every step.)
+__device__ __noinline__ void chain_chunk_rare(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited) {
+  chain_chunk(a, start, end, visited);
+}
+
 // LONG: lists of more than 32 entries.
 template <bool STATS, bool LONG>
 __global__ void greedy_lists_kernel(GreedyArgs a) {
@@ -352,7 +358,7 @@ __global__ void greedy_lists_kernel(GreedyArgs a) {
   }
   __syncthreads();
   if (odd) {
-    if (warp == 0) chain_chunk(a, start, end, has);  // (its two bitmaps fit the words)
+    if (warp == 0) chain_chunk_rare(a, start, end, has);  // (its two bitmaps fit the words)
     return;
   }
   if (warp == 0 && m > 0) {
