@@ -33,6 +33,8 @@ constexpr int T_IPT = 8;
 constexpr int T_TILE = T_THREADS * T_IPT;  // 4096
 constexpr int C_NNZ = 65536;               // largest chunk (nonzeros) that compact_kernel looks at ...
 constexpr int C_ROWS = 2048;               // ... and its rows
+constexpr int C_TALL_ROWS = 4096;          // ... where chunks have more,
+constexpr int C_TALL_NNZ = 28672;          // with so many nonzeros
 
 struct TransposeArgs {
   int32_t n, nnz, chunk, num_chunks, passes;
@@ -99,35 +101,38 @@ __device__ __forceinline__ int32_t row_of(const int32_t *p, int32_t lo, int32_t 
 //     of the group: its place.  (That is one comparison per candidate the sketch stage will have to
 //     work through, so it never dominates.)
 //  5. members go out with their groups in CSR order, which is the order seg[] wants.
-// Two sizes: blocks of 512 threads, two to an SM, for up to 6144 numbered nonzeros (in up to 3072 columns); chunks with
-// more go on to blocks of 1024 threads for up to 22,528 (in up to 6144 columns), those with more
-// again to the tiled sort.
+// Chunks of up to 2,048 rows: blocks of 512 threads, two to an SM, for up to 6144 numbered nonzeros (in up to 3072
+// columns); chunks with more go on to blocks of 1024 threads for up to 22,528 (in up to 6144 columns), those with
+// more again to the tiled sort.  Taller ones: blocks of 1024 threads for up to 16,384 (launch_compact).
 // On a B200, 1.05 M rows of the shuffled mesh: 227 us with the groups read off the promised
 // symmetry, 115 without any promise; 65,536 rows of the power-law band: 173 -> 84 us.
-template <int THREADS_, int CAP_, int TABLE_BITS_, int FILTER_BITS_>
+template <int THREADS_, int CAP_, int TABLE_BITS_, int FILTER_BITS_, int ROWS_>
 struct CompactSize {
+  static constexpr int ROWS = ROWS_, NNZ = ROWS_ == C_ROWS ? C_NNZ : C_TALL_NNZ, GROUP_BITS = ROWS_ < 4096 ? 12 : 13;
+  static constexpr uint32_t GROUP = (1u << GROUP_BITS) - 1u;  // rows of a column
   static constexpr int THREADS = THREADS_, WARPS = THREADS / 32, CAP = CAP_, TABLE_BITS = TABLE_BITS_, FILTER_BITS = FILTER_BITS_;
   static constexpr int TABLE = 1 << TABLE_BITS, FILTER = (1 << FILTER_BITS) / 32;  // entries; words of each map
   // columns from which on a thread gives up: they cannot fill the table, however many are on their way
   static constexpr int COLUMNS = TABLE - 2 * THREADS;
   struct Shared {
     uint32_t key[TABLE];          // columns, then how many members wrote their row
-    uint32_t cnt[TABLE];          // rows per column, then (place << 12) | rows, 0 for a column with one
+    uint32_t cnt[TABLE];          // rows per column, then (place << GROUP_BITS) | rows, 0 for a column with one
     union {
       uint32_t filter[2][FILTER];
       uint16_t member[CAP];       // rows of the groups
     };
     uint16_t slot[CAP];           // table entry of each numbered nonzero
     uint16_t row[CAP];            // its position, then its row
-    int32_t sptr[C_ROWS + 1];
-    uint32_t work[C_ROWS];
-    uint32_t cols[C_ROWS / 2];    // 16 bits a row
+    int32_t sptr[ROWS + 1];
+    uint32_t work[ROWS];
+    uint32_t cols[ROWS / 2];      // 16 bits a row
     int32_t warp_sum[32];
     int32_t ticket, columns;
   };
 };
-using CompactSmall = CompactSize<512, 6144, 12, 17>;
-using CompactLarge = CompactSize<1024, 22528, 13, 17>;
+using CompactSmall = CompactSize<512, 6144, 12, 17, C_ROWS>;
+using CompactLarge = CompactSize<1024, 22528, 13, 17, C_ROWS>;
+using CompactTall = CompactSize<1024, 16384, 13, 17, C_TALL_ROWS>;
 
 // exclusive sum over the block's threads; *total is the sum of all
 template <int WARPS>
@@ -156,9 +161,9 @@ __device__ __forceinline__ int32_t block_sum(int32_t v, int32_t *warp_sum, int32
 
 __device__ __forceinline__ uint32_t column_hash(uint32_t c) { return c * 0x9E3779B1u; }
 
-// LARGE: the chunks that the small form left (ctrl[CTRL_NEXT_COUNT] of them); what does not fit
+// NEXT: the chunks that the form before left (ctrl[CTRL_NEXT_COUNT] of them).  LAST: what does not fit
 // goes to the tiled sort.
-template <typename S, bool LARGE>
+template <typename S, bool NEXT, bool LAST>
 __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename S::Shared &sh = *reinterpret_cast<typename S::Shared *>(smem_raw);
@@ -166,15 +171,15 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
   const int tid = threadIdx.x, lane = tid & 31;
   for (;;) {
     __syncthreads();
-    if (tid == 0) sh.ticket = static_cast<int32_t>(atomicAdd(&a.ctrl[LARGE ? CTRL_NEXT_TICKET : CTRL_CHUNK_TICKET], 1u));
+    if (tid == 0) sh.ticket = static_cast<int32_t>(atomicAdd(&a.ctrl[NEXT ? CTRL_NEXT_TICKET : CTRL_CHUNK_TICKET], 1u));
     __syncthreads();
-    if (sh.ticket >= (LARGE ? static_cast<int32_t>(a.ctrl[CTRL_NEXT_COUNT]) : a.num_chunks)) break;
-    const int32_t q = LARGE ? a.next_chunk[sh.ticket] : sh.ticket;
+    if (sh.ticket >= (NEXT ? static_cast<int32_t>(a.ctrl[CTRL_NEXT_COUNT]) : a.num_chunks)) break;
+    const int32_t q = NEXT ? a.next_chunk[sh.ticket] : sh.ticket;
     if (a.skip_prio && static_cast<uint32_t>(q) == a.ctrl_main[CTRL_PRIO]) continue;
     const ChunkSpan c = chunk_span(a, q);
     const int32_t b = c.b, rows = c.rows;
     const int L = c.L;
-    if (L > C_NNZ || rows > C_ROWS) {
+    if (L > S::NNZ || rows > S::ROWS) {
       if (tid == 0) a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
       for (int i = tid; i < rows; i += THREADS) a.row_work[c.cs + i] = 0;  // (the tiled sort adds to it)
       continue;
@@ -187,7 +192,7 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
       if (i == rows - 1) sh.sptr[rows] = y;
       ordered &= x <= y;
       sh.work[i] = 0;
-      if (i < C_ROWS / 2) sh.cols[i] = 0;
+      if (i < S::ROWS / 2) sh.cols[i] = 0;
     }
     if (!ordered) atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
     for (int i = tid * 4; i < S::TABLE; i += THREADS * 4) {
@@ -259,12 +264,12 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
     __syncthreads();
     if (numbered > S::CAP || sh.columns > S::COLUMNS) {  // (the same in all threads)
       if (tid == 0) {
-        if (LARGE)
+        if (LAST)
           a.heavy_chunk[atomicAdd(&a.ctrl[CTRL_HEAVY_COUNT], 1u)] = q;
         else
           a.next_chunk[atomicAdd(&a.ctrl[CTRL_NEXT_COUNT], 1u)] = q;
       }
-      if (LARGE)
+      if (LAST)
         for (int i = tid; i < rows; i += THREADS) a.row_work[c.cs + i] = 0;  // (the tiled sort adds to it)
       continue;
     }
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         v[i] = sh.cnt[i * THREADS + tid];
-        if (v[i] > 4095u) {  // (only with columns repeated inside rows)
+        if (v[i] > S::GROUP) {  // (only with columns repeated inside rows)
           atomicExch(&a.ctrl[CTRL_BAD_INPUT], 1u);
           v[i] = 0;
         }
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const uint32_t n = v[i];
-        sh.cnt[i * THREADS + tid] = n >= 2 ? (static_cast<uint32_t>(run) << 12) | n : 0u;
+        sh.cnt[i * THREADS + tid] = n >= 2 ? (static_cast<uint32_t>(run) << S::GROUP_BITS) | n : 0u;
         sh.key[i * THREADS + tid] = 0u;
         run += n >= 2 ? static_cast<int32_t>(n) : 0;
       }
@@ -305,9 +310,9 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
       if (g == 0u) continue;
       const int32_t r = row_of(sh.sptr, 0, rows, b + sh.row[s]);
       sh.row[s] = static_cast<uint16_t>(r);
-      const uint32_t at = (g >> 12) + atomicAdd(&sh.key[t], 1u);
+      const uint32_t at = (g >> S::GROUP_BITS) + atomicAdd(&sh.key[t], 1u);
       if (index_ok(a.ctrl, CHK_GROUP, at, S::CAP)) sh.member[at] = static_cast<uint16_t>(r);
-      atomicAdd(&sh.work[r], (g & 4095u) - 1u);
+      atomicAdd(&sh.work[r], (g & S::GROUP) - 1u);
     }
     __syncthreads();
     int32_t written = 0;
@@ -319,7 +324,7 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
         g = sh.cnt[sh.slot[s]];
         r = sh.row[s];
       }
-      const int32_t start = static_cast<int32_t>(g >> 12), len = static_cast<int32_t>(g & 4095u);
+      const int32_t start = static_cast<int32_t>(g >> S::GROUP_BITS), len = static_cast<int32_t>(g & S::GROUP);
       for (int32_t i = 0; i < len; ++i) rank += sh.member[start + i] < r ? 1 : 0;
       int32_t tile_total;
       const int32_t at = written + block_sum<S::WARPS>(g ? 1 : 0, sh.warp_sum, &tile_total);
@@ -910,8 +915,18 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
     CSG_CUDA(cudaGetLastError());
     return true;
   };
-  if (!launch(compact_kernel<CompactSmall, false>, CompactSmall::THREADS, sizeof(CompactSmall::Shared), 2)) return false;
-  if (!launch(compact_kernel<CompactLarge, true>, CompactLarge::THREADS, sizeof(CompactLarge::Shared), 1)) return false;
+  const int32_t rows = a.chunk < a.n ? a.chunk : a.n;
+  // Taller chunks, if there are enough of them for a block each to keep the chip busy: 64 chunks of 4,096
+  // rows of a road network 355 -> 159 us, 88 of 3,000 rows of a mesh 567 -> 276.  One chunk of 3,500 rows
+  // by itself took 763 us with it and 713 without; 4,096 rows of a mesh (36,800 nonzeros) are looked at only
+  // to find that they do not fit, 723 and 595: C_TALL_NNZ.
+  if (rows > C_ROWS && rows <= C_TALL_ROWS && a.num_chunks >= ctx.num_sms / 4) {
+    if (!launch(compact_kernel<CompactTall, false, true>, CompactTall::THREADS, sizeof(CompactTall::Shared), 1)) return false;
+    count_launches(1);
+    return true;
+  }
+  if (!launch(compact_kernel<CompactSmall, false, false>, CompactSmall::THREADS, sizeof(CompactSmall::Shared), 2)) return false;
+  if (!launch(compact_kernel<CompactLarge, true, true>, CompactLarge::THREADS, sizeof(CompactLarge::Shared), 1)) return false;
   count_launches(2);
   return true;
 }

@@ -1,0 +1,49 @@
+"""Chunks of more than 1,024 rows take kernels of their own: bit-exact tables and orders against
+the CPU oracle at the sizes where they change hands."""
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _check(ptr, ind, limits=(0,), **params):
+    import chunkedgreedy_b200 as sp
+    order, table = oracle.csg(ptr, ind, False, with_table=True, **params)
+    dp, di = torch.from_numpy(ptr).cuda(), torch.from_numpy(ind).cuda()
+    ctx = sp.Context()
+    for limit in limits:
+        ctx.set_stream_limit(limit)
+        got_order, got = sp.csg_table(dp, di, ctx=ctx, **params)
+        assert np.array_equal(got.cpu().numpy().view(np.uint64), table)
+        assert np.array_equal(got_order.cpu().numpy(), order)
+    ctx.close()
+
+
+def _csr(rows, n):
+    rows = [np.unique(np.asarray(r, dtype=np.int32)) for r in rows]
+    rows += [np.empty(0, dtype=np.int32)] * (n - len(rows))
+    ptr = np.zeros(n + 1, dtype=np.int32)
+    ptr[1:] = np.cumsum([r.size for r in rows])
+    return ptr, np.concatenate(rows)
+
+
+@pytest.mark.parametrize("chunk", [2048, 2049, 4095, 4096, 4097])
+def test_tall_chunks_grouped_by_a_block_each(chunk):
+    # enough chunks for a block each; among them a column that holds every row of its chunk, and one in all
+    # rows but one (13 bits of a group's length), a chunk with more members of groups than the block has
+    # places for, one with more nonzeros than it looks at, empty rows, and a last chunk of one row
+    rng = np.random.default_rng(chunk)
+    n = 40 * chunk + 1
+    count = rng.integers(0, 4, n)
+    count[3 * chunk:4 * chunk] = 6     # 16,384 members and more in groups
+    count[4 * chunk:5 * chunk] = 8     # 28,672 nonzeros and more
+    rows = [rng.integers(0, 9000, c) + 1 for c in count]
+    for i in range(chunk):
+        rows[chunk + i] = [0] + list(rows[chunk + i][:1])
+        if i != 17:
+            rows[2 * chunk + i] = [0, 1 + i % 3000]
+    ptr, ind = _csr(rows, n)
+    _check(ptr, ind, k=16, chunk_size=chunk)
