@@ -134,7 +134,7 @@ enum {
   CTRL_HEAVY_NEED = 10,    // and the word after it: stream elements of all rows of heavy weight (64-bit)
   CTRL_STREAM_OVERRUN = 12,  // set by heavy_expand_kernel when a slice would pass the stream buffer
   CTRL_CHECK = 13,         // checked build: site of the first index out of bounds, then the index (64-bit)
-  CTRL_MID_END = 16,       // end of the rows of heavy weight in row_list (those past CTRL_HEAVY_ROWS did not fit)
+  CTRL_MID_END = 16,       // end of the rows in row_list that are not run by a lane (those past CTRL_HEAVY_ROWS: by a warp)
   CTRL_LANE_TICKET = 17,   // next row for the kernel that runs a row per lane
   CTRL_NEXT_COUNT = 18,    // chunks compact_kernel's small form left to the large one, and that one's ticket
   CTRL_NEXT_TICKET = 19,
@@ -165,6 +165,11 @@ constexpr int SKETCH_PART_COLS = 128;   // columns of a heavy row whose stream o
 constexpr uint32_t HEAVY_WORK = 1u << 16;
 constexpr uint32_t CHAIN_ROWS = 296;
 constexpr uint32_t CHAIN_WORK_MIN = 64;
+constexpr int32_t LANE_TABLE_ROWS = 1024;  // largest chunk whose keys the row-per-lane kernel finds in a byte table
+// Larger chunks: rows of at least this many candidates and in the longest octaves go to a warp each, more octaves
+// up to this many rows (bucket_scan_kernel)
+constexpr uint32_t WARP_WORK_MIN = 1024;
+constexpr int32_t WARP_FEW_ROWS = 32768;
 
 // stage launchers; all enqueue on ctx.stream and return false after set_error()
 bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,

@@ -771,7 +771,15 @@ __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint
 // CHAIN_ROWS = two rows on each of 148 SMs: beyond one wave of them the chains only queue, and
 // what they do the lanes do with a sixth of the SM time (R-MAT scale 22 took 42 ms with 1184 rows
 // here).
-__global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, uint32_t ticket) {
+// `octaves` > 0: the lanes find their keys by a chained hash table and take some 680 cycles per candidate.
+// Of the rows that are left, those within so many octaves of the longest go to a warp each first; the
+// lanes' longest row then takes about as long as the chain of the longest of all (52 cycles per
+// candidate, 90 with a large key table: four octaves and three).  R-MAT scale 19 with chunks of 2,048:
+// 30.0 ms without, 16.9 with three, 13.4 with four, 14.2 with five; symmetrised scale 20, where the
+// chain is longer than any lane's row, 47.3, 47.4, 47.6 and 53.9; scale 16 as one chunk 29.3 with none
+// or three, 32.4 with five.
+__global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, uint32_t ticket, int octaves,
+                                   const uint32_t *ctrl_ahead) {
   const int lane = threadIdx.x;
   uint32_t c[4], sum = 0;
 #pragma unroll
@@ -786,7 +794,16 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     if (lane >= off) incl += t;
   }
   uint32_t run = incl - sum;
-  uint32_t heavy = 0;
+  uint32_t heavy = 0, mid = 0;
+  int longest = 0;
+#pragma unroll
+  for (int j = 3; j >= 0; --j)
+    if (c[j]) longest = WORK_BUCKETS - 1 - (4 * lane + j);
+  longest = __reduce_max_sync(FULL, longest);
+  // (the chunk ahead lists its rows down to a quarter of its longest)
+  if (ctrl_ahead && ctrl_ahead[CTRL_PRIO] != PRIO_NONE && ctrl_ahead[CTRL_PRIO_WORK] > 0)
+    longest = max(longest, work_bucket(4u * ctrl_ahead[CTRL_PRIO_WORK]));
+  const int least = max(work_bucket(WARP_WORK_MIN), longest - 4 * octaves);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int b = WORK_BUCKETS - 1 - (4 * lane + j);
@@ -794,14 +811,17 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     run += c[j];
     ctrl[CTRL_BUCKET_FILL + b] = 0;
     if (b >= work_bucket(HEAVY_WORK) || (b >= work_bucket(CHAIN_WORK_MIN) && run <= CHAIN_ROWS)) heavy = run;
+    if (octaves > 0 && b >= least) mid = run;
   }
   heavy = __reduce_max_sync(FULL, heavy);
+  mid = __reduce_max_sync(FULL, mid);
+  if (mid < heavy) mid = heavy;
   const uint32_t listed = __shfl_sync(FULL, run, 31);
   if (lane == 0) {
     ctrl[CTRL_ROWS_LISTED] = listed;
     ctrl[CTRL_HEAVY_ROWS] = heavy;
-    ctrl[CTRL_MID_END] = heavy;
-    ctrl[CTRL_LANE_TICKET] = heavy;
+    ctrl[CTRL_MID_END] = mid;
+    ctrl[CTRL_LANE_TICKET] = mid;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
     // for the host (wait_outcome)
@@ -937,8 +957,10 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
   if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
   bucket_count_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
+  const int32_t span = chunk < n ? chunk : n;
+  const int octaves = span <= LANE_TABLE_ROWS ? 0 : span <= WARP_FEW_ROWS ? 4 : 3;
   bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl, reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD,
-                                               ++ctx.outcome_ticket);
+                                               ++ctx.outcome_ticket, octaves, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
   row_list_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());

@@ -47,3 +47,15 @@ def test_tall_chunks_grouped_by_a_block_each(chunk):
             rows[2 * chunk + i] = [0, 1 + i % 3000]
     ptr, ind = _csr(rows, n)
     _check(ptr, ind, k=16, chunk_size=chunk)
+
+
+@pytest.mark.parametrize("k", [8, 16, 40])
+@pytest.mark.parametrize("chunk,skew", [(1024, 10), (1025, 10), (5000, 5), (40_000, 4)])
+def test_rows_by_warp_before_the_lanes(chunk, skew, k):
+    # streams from a few to tens of thousands of candidates: how many octaves below the longest
+    # go to a warp each changes with the rows of a chunk
+    rng = np.random.default_rng(chunk + k)
+    n = 40_000
+    rows = [list((n * rng.random(c) ** skew).astype(np.int64)) for c in 1 + rng.geometric(0.2, n) % 60]
+    ptr, ind = _csr(rows, n)
+    _check(ptr, ind, limits=(0, 3000), k=k, chunk_size=chunk)
