@@ -538,7 +538,7 @@ constexpr int L_RING = 32;         // candidates produced per row and phase, one
 constexpr int L_PRODUCERS = 4;     // producing warps ...
 constexpr int L_WARPS = 1 + L_PRODUCERS;
 constexpr int L_ROWS = 32 / L_PRODUCERS;  // ... and rows of each
-constexpr int L_TABLE_MAX = 1024;  // largest chunk (rows) indexed by a byte table
+constexpr int L_TABLE_MAX = LANE_TABLE_ROWS;
 
 // Key -> slot by one byte per row of the chunk (0 = not there, else slot + 1).  Keys travel as
 // the byte's place in the lane's column of the table; those of the slots, 16 bits each, are
@@ -741,10 +741,11 @@ struct LaneSketch {
   }
 };
 
-// The rows that did not fit the stream buffer, before the lanes' own (rare: a first call on
-// much larger rows than the context has seen, or a caller's bound on the buffer).
+// The rows between the chain kernel's and the lanes' own, before those: the long ones of chunks without a
+// byte table (bucket_scan_kernel says which), and rows that did not fit the stream buffer (rare: a first call
+// on much larger rows than the context has seen, or a caller's bound on the buffer).
 template <int CELLS>
-__device__ __noinline__ void rows_that_did_not_fit(const SketchArgs &a, uint32_t end, uint32_t *mem) {
+__device__ __noinline__ void rows_before_the_lanes(const SketchArgs &a, uint32_t end, uint32_t *mem) {
   mem += (threadIdx.x >> 5) * 2 * S_RING;
   rows_by_warp<CELLS>(a, end, reinterpret_cast<int32_t *>(mem), reinterpret_cast<float *>(mem + S_RING));
 }
@@ -975,7 +976,7 @@ __global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchAr
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   const uint32_t listed = a.ctrl[CTRL_ROWS_LISTED], mid_end = a.ctrl[CTRL_MID_END];
   const uint32_t span = static_cast<uint32_t>(a.chunk < a.n ? a.chunk : a.n);
-  if (a.ctrl[CTRL_HEAVY_ROWS] < mid_end) rows_that_did_not_fit<CELLS>(a, mid_end, lanes_mem);
+  if (a.ctrl[CTRL_HEAVY_ROWS] < mid_end) rows_before_the_lanes<CELLS>(a, mid_end, lanes_mem);
   __syncthreads();
   LaneShared &sh = *reinterpret_cast<LaneShared *>(lanes_mem + L::SHARED_OFF);
   uint32_t *const ring = lanes_mem + L::RING_OFF;
@@ -1304,7 +1305,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_consume_kernel(SketchArgs 
 // the dependent steps of the first warp are the bound and the order comes in their shadow.
 constexpr int H_RING = 512;      // stream elements staged per batch
 constexpr int ROUND_CELLS = 4;   // largest sketch (cells per lane) resolved in rounds
-constexpr int WINDOW_CELLS = 2;  // smallest sketch with whole-window rounds: with 32 slots a window of 32 can take every entry
+constexpr int WINDOW_CELLS = 2;  // smallest sketch with whole-window rounds (and with helping warps): with 32 slots a
+                                 // window of 32 can take every entry (heavy_rounds_32_kernel)
 constexpr int MATES = 1024;      // words of the duplicate detector
 constexpr int ROUND_TAB_MAX = 65536;  // largest chunk (rows) with a key -> slot table
 constexpr int TRIAL_ROUNDS = 8;     // rounds of each kind a row times before it settles on one ...
@@ -1759,48 +1761,44 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, const Ro
     __syncwarp();
     int p = 0;
     while (p < cnt && filled < M) p += round_fill<CELLS, TAB>(row, buf, p, cnt, lane, filled);
-    if constexpr (CELLS >= WINDOW_CELLS) {
-      // Which kind of round is faster depends on the row: a whole-window round costs more and
-      // pays where it resolves (nearly) the whole window - rows whose own length dominates their
-      // Dice terms.  Where the terms vary widely, entries put back light are taken again at
-      // once, either kind ends after a few elements and the cheaper one wins; and how often a
-      // strict round is cut short depends on the sketch size.  So the row measures: a few
-      // rounds of each kind against the clock, then a long stretch of the kind that resolved
-      // more elements per cycle, and again.
-      while (p < cnt) {
-        const int before = p;
-        const long long t0 = clock64();
-        const int2 at = mode == 0 ? window_rounds<CELLS, TAB>(row, buf, p, cnt, left)
-                                  : strict_rounds<CELLS, TAB>(row, buf, p, cnt, left);
-        p = at.x;
-        left = at.y;
-        if (trial >= 0) {  // a trial stretch: book it
-          got[trial] += p - before;
-          took[trial] += clock64() - t0;
-        }
-        if (left == 0) {
-          if (trial == 0) {  // window tried: now the strict kind
-            trial = 1;
-            mode = 1;
-            left = TRIAL_ROUNDS;
-          } else if (trial == 1) {  // both tried: elements per cycle, compared without dividing
-            mode = got[0] * took[1] >= got[1] * took[0] ? 0 : 1;
-            // the stretch grows while the same kind keeps winning (up to 16 times as long)
-            streak = mode == last_mode ? (streak < 4 ? streak + 1 : 4) : 0;
-            last_mode = mode;
-            trial = -1;
-            left = COMMIT_ROUNDS << streak;
-          } else {  // a committed stretch is over: measure again
-            trial = 0;
-            mode = 0;
-            left = TRIAL_ROUNDS;
-            got[0] = got[1] = 0;
-            took[0] = took[1] = 0;
-          }
+    // Which kind of round is faster depends on the row: a whole-window round costs more and
+    // pays where it resolves (nearly) the whole window - rows whose own length dominates their
+    // Dice terms.  Where the terms vary widely, entries put back light are taken again at
+    // once, either kind ends after a few elements and the cheaper one wins; and how often a
+    // strict round is cut short depends on the sketch size.  So the row measures: a few
+    // rounds of each kind against the clock, then a long stretch of the kind that resolved
+    // more elements per cycle, and again.
+    while (p < cnt) {
+      const int before = p;
+      const long long t0 = clock64();
+      const int2 at = mode == 0 ? window_rounds<CELLS, TAB>(row, buf, p, cnt, left)
+                                : strict_rounds<CELLS, TAB>(row, buf, p, cnt, left);
+      p = at.x;
+      left = at.y;
+      if (trial >= 0) {  // a trial stretch: book it
+        got[trial] += p - before;
+        took[trial] += clock64() - t0;
+      }
+      if (left == 0) {
+        if (trial == 0) {  // window tried: now the strict kind
+          trial = 1;
+          mode = 1;
+          left = TRIAL_ROUNDS;
+        } else if (trial == 1) {  // both tried: elements per cycle, compared without dividing
+          mode = got[0] * took[1] >= got[1] * took[0] ? 0 : 1;
+          // the stretch grows while the same kind keeps winning (up to 16 times as long)
+          streak = mode == last_mode ? (streak < 4 ? streak + 1 : 4) : 0;
+          last_mode = mode;
+          trial = -1;
+          left = COMMIT_ROUNDS << streak;
+        } else {  // a committed stretch is over: measure again
+          trial = 0;
+          mode = 0;
+          left = TRIAL_ROUNDS;
+          got[0] = got[1] = 0;
+          took[0] = took[1] = 0;
         }
       }
-    } else {
-      strict_rounds<CELLS, TAB>(row, buf, p, cnt, 1 << 30);
     }
     buf ^= 1;
   }
@@ -1869,6 +1867,228 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
   }
 }
 
+// ---- 32 slots ------------------------------------------------------------------------------
+// A warp per row: a lane orders its own slot while the look-ups of the window are under way, in
+// fewer cycles than a group's barriers take.  Strict rounds only.  Longest row of R-MAT scale 16
+// (101,366 candidates): 9.9 ms by a group of three warps, 7.7 this way, 145 cycles per candidate;
+// bound by the dependent steps of a round, as the larger sketches are.  Rows are drawn as warps ask,
+// so that the longest share an SM: spread one to an SM (the others empty), the same rounds took 10.9 ms of a
+// whole call that takes 8.1; with eight warps to a block 9.8.  What a round costs also hangs on how the
+// compiler orders it: with a row's places in a struct a call took 12.1 ms, as arguments 8.1.
+constexpr int T_RING = 1024;
+struct State32 {
+  __align__(16) uint32_t w[32];  // as in RoundState
+  __align__(16) int32_t key[32];
+  uint32_t sw[32];
+  int32_t si[32], sk[32], rank[32], miss_pos[32];
+  uint32_t fence_sink;
+};
+// Keeps the phases of a round apart in the instruction schedule: left alone, ptxas interleaves the
+// look-ups, the count and the limits, and a round takes a tenth longer than with a read of %clock
+// between them (which it does not move code across, as long as the value is used).
+__device__ __forceinline__ void phase_fence(uint32_t &sink) {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+  sink ^= t;
+}
+
+// the key of element e, with a table relative to the chunk (one outside the chunk only comes from rows that are
+// not sorted: kept in bounds)
+template <bool TAB>
+__device__ __forceinline__ int32_t key_32(uint32_t *ctrl, int32_t e, int32_t cbase, int32_t span) {
+  const uint32_t rel = static_cast<uint32_t>(key_in_chunk(ctrl, e, cbase, span) - cbase);
+  return static_cast<int32_t>(min(rel, static_cast<uint32_t>(span) - 1u)) + (TAB ? 0 : cbase);
+}
+template <bool TAB>
+__device__ __forceinline__ int slot_32(const State32 &st, const uint8_t *tab, int32_t s) {
+  if (TAB) return static_cast<int>(tab[s]) - 1;
+  int q = -1;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int4 kk = reinterpret_cast<const int4 *>(st.key)[i];
+    q = kk.x == s ? 4 * i : q;
+    q = kk.y == s ? 4 * i + 1 : q;
+    q = kk.z == s ? 4 * i + 2 : q;
+    q = kk.w == s ? 4 * i + 3 : q;
+  }
+  return q;
+}
+
+// round_strict and round_fill on 32 slots (the slot code is the lane)
+template <bool TAB>
+__device__ __forceinline__ int strict_32(State32 &st, uint8_t *tab, int32_t cbase, int32_t span, uint32_t *ctrl,
+                                         const int2 *ring, int p, int cnt, int lane, uint32_t &sink) {
+  const uint32_t below = (1u << lane) - 1u;
+  phase_fence(sink);
+  const bool valid = p + lane < cnt;
+  const int2 elem = valid ? ring[p + lane] : make_int2(cbase, 0);
+  const int32_t s = key_32<TAB>(ctrl, elem.x, cbase, span);
+  const float al = __int_as_float(elem.y);
+  const uint32_t mine = st.w[lane];
+  const int32_t mykey = st.key[lane];
+  const int q = valid ? slot_32<TAB>(st, tab, s) : 0;
+  const bool miss = valid && q < 0, hit = valid && q >= 0;
+  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
+  const uint32_t wq = st.w[hit ? q : 0];
+  const uint32_t missing = __ballot_sync(FULL, miss);
+  const int mtot = __popc(missing), mrank = __popc(missing & below);
+  phase_fence(sink);
+  // entries (x, i) below (mine, lane): weight bits are below 2^31, so x < y is the sign of x - y
+  int32_t acc[4] = {0, 0, 0, 0};
+  uint4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = reinterpret_cast<const uint4 *>(st.w)[i];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += static_cast<int32_t>(x[e] - mine - ((below >> (4 * i + e)) & 1u)) >> 31;
+  }
+  const int pos = -((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  st.sw[pos] = mine;
+  st.si[pos] = lane;
+  st.sk[pos] = mykey;
+  st.rank[lane] = pos;
+  phase_fence(sink);
+  if (miss) st.miss_pos[mrank] = lane;
+  __syncwarp();
+  phase_fence(sink);
+  const int rho = st.rank[hit ? q : 0];
+  const int tgt = st.si[mrank];
+  const uint32_t base = st.sw[mrank];
+  const int32_t old_key = st.sk[mrank];
+  const uint32_t top = st.sw[mtot > 0 ? mtot - 1 : 0];
+  const int at_hit = st.miss_pos[rho];
+  const int at_next = st.miss_pos[(mrank + 1) & 31];
+  const uint32_t nb = __float_as_uint(__uint_as_float(base) + al);
+  int lim = valid ? 32 : lane;
+  if (hit) {
+    const int at = rho < mtot ? at_hit : 32;
+    lim = at > lane ? at : lane;
+  }
+  if (miss) {
+    if (nb <= top) lim = nb > base ? (mrank + 1 < mtot ? at_next : 32) : lane;
+    if (same & below) lim = lane;
+  }
+  phase_fence(sink);
+  int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
+  L = L < 1 ? 1 : L;
+  const bool applies = lane < L;
+  const unsigned mates = same & (L >= 32 ? FULL : (1u << L) - 1u);
+  const int times = __popc(mates);
+  float wv = __uint_as_float(wq) + al;
+  if (times > 1) wv += al;  // (most of the repeats there are, without a loop)
+  if (times > 2)
+    for (int t = 2; t < times; ++t) wv += al;
+  if (applies && miss) {
+    if (TAB) tab[old_key] = 0;
+    st.key[tgt] = s;
+    st.w[tgt] = nb;
+    if (TAB) tab[s] = static_cast<uint8_t>(tgt + 1);
+  }
+  if (applies && hit && (mates & below) == 0u) st.w[q] = __float_as_uint(wv);
+  __syncwarp();
+  return L;
+}
+template <bool TAB>
+__device__ __forceinline__ int fill_32(State32 &st, uint8_t *tab, int32_t cbase, int32_t span, uint32_t *ctrl,
+                                       const int2 *ring, int p, int cnt, int lane, int &filled) {
+  const uint32_t below = (1u << lane) - 1u;
+  const bool valid = p + lane < cnt;
+  const int2 elem = valid ? ring[p + lane] : make_int2(cbase, 0);
+  const int32_t s = key_32<TAB>(ctrl, elem.x, cbase, span);
+  const float al = __int_as_float(elem.y);
+  const int q = valid ? slot_32<TAB>(st, tab, s) : 0;
+  const bool miss = valid && q < 0, hit = valid && q >= 0;
+  const uint32_t missing = __ballot_sync(FULL, miss);
+  const int mrank = __popc(missing & below);
+  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
+  int lim = valid ? 32 : lane;
+  if (miss && ((same & below) || mrank >= 32 - filled)) lim = lane;
+  const int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
+  const unsigned prefix = L >= 32 ? FULL : (1u << L) - 1u;
+  if (lane < L) {
+    if (miss) {
+      const int j = filled + mrank;
+      st.key[j] = s;
+      st.w[j] = __float_as_uint(al);
+      if (TAB) tab[s] = static_cast<uint8_t>(j + 1);
+    } else if (hit && ((same & prefix) & below) == 0u) {
+      float wv = __uint_as_float(st.w[q]);
+      for (int t = __popc(same & prefix); t > 0; --t) wv += al;
+      st.w[q] = __float_as_uint(wv);
+    }
+  }
+  filled += __popc(missing & prefix);
+  __syncwarp();
+  return L;
+}
+
+template <bool TAB>
+__device__ __noinline__ void row_32(const int2 *in, uint32_t total, State32 &st, uint8_t *tab, int32_t cbase, int32_t span,
+                                    uint32_t *ctrl, int2 *ring0, int2 *ring1, int32_t *out) {
+  const int lane = lane_id();
+  st.key[lane] = -1;
+  st.w[lane] = 0u;
+  int filled = 0, buf = 0;
+  uint32_t sink = 0;
+  __syncwarp();
+  stage_batch(ring0, in, static_cast<int>(total < T_RING ? total : T_RING), lane);
+  for (uint32_t base = 0; base < total; base += T_RING) {
+    const int cnt = static_cast<int>(total - base < T_RING ? total - base : T_RING);
+    const uint32_t next = base + T_RING;
+    if (next < total)
+      stage_batch(buf ? ring0 : ring1, in + next, static_cast<int>(total - next < T_RING ? total - next : T_RING), lane);
+    else
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest group: this batch is in
+    __syncwarp();
+    const int2 *const ring = buf ? ring1 : ring0;
+    int p = 0;
+    while (p < cnt && filled < 32) p += fill_32<TAB>(st, tab, cbase, span, ctrl, ring, p, cnt, lane, filled);
+    while (p < cnt) p += strict_32<TAB>(st, tab, cbase, span, ctrl, ring, p, cnt, lane, sink);
+    buf ^= 1;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  const int32_t kk = st.key[lane];
+  out[lane] = TAB && kk >= 0 ? kk + cbase : kk;
+  out[32 + lane] = static_cast<int32_t>(st.w[lane]);
+  if (TAB && kk >= 0) tab[kk] = 0;  // the table is empty again for the next row
+  if (lane == 0) st.fence_sink = sink;
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(S_THREADS, 1) heavy_rounds_32_kernel(SketchArgs a, int tab_bytes) {
+  int2(*const rings)[2][T_RING] = reinterpret_cast<int2(*)[2][T_RING]>(heavy_dyn);
+  __shared__ State32 state[S_WARPS];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
+  uint8_t *const tab = heavy_dyn + sizeof(int2) * S_WARPS * 2 * T_RING + static_cast<size_t>(warp) * tab_bytes;
+  for (int i = lane * 16; i < tab_bytes; i += 32 * 16) *reinterpret_cast<uint4 *>(tab + i) = make_uint4(0, 0, 0, 0);
+  __syncwarp();
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(&a.ctrl[CTRL_HEAVY_TICKET + 1], 1u);
+    item = __shfl_sync(FULL, item, 0);
+    if (item >= heavy) break;
+    const int32_t r = a.row_list[item];
+    // checked build: the row, its place in the state array and its stream's extent
+    if (!index_ok(a.ctrl, CHK_LIST, r, a.n) || !index_ok(a.ctrl, CHK_STATE, item, a.heavy_max) ||
+        !index_ok(a.ctrl, CHK_STREAM, static_cast<long long>(a.heavy_off[item]) + a.row_work[r],
+                  static_cast<long long>(a.stream_cap) + 1))
+      continue;
+    const int32_t cbase = (r / a.chunk) * a.chunk, span = a.chunk < a.n ? a.chunk : a.n;
+    int32_t *const out = a.heavy_state + static_cast<size_t>(item) * (2 * 32);
+    if (tab_bytes > 0)
+      row_32<true>(a.hstream + a.heavy_off[item], a.row_work[r], state[warp], tab, cbase, span, a.ctrl, rings[warp][0],
+                   rings[warp][1], out);
+    else  // chunk too large for key tables in shared memory
+      row_32<false>(a.hstream + a.heavy_off[item], a.row_work[r], state[warp], tab, cbase, span, a.ctrl, rings[warp][0],
+                    rings[warp][1], out);
+  }
+}
+
 template <int CELLS>
 __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
   const int lane = lane_id();
@@ -1896,7 +2116,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   // (sketches beyond ROUND_CELLS) the two share the SMs, since the kernel of the other rows starts
   // only when every chain block has one.
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
-  constexpr bool in_rounds = CELLS <= ROUND_CELLS;
+  constexpr bool in_rounds = CELLS >= WINDOW_CELLS && CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
     // (up to a million nonzeros there are a few thousand parts at most, less than a launch's worth)
     const bool one_kernel = a.nnz <= 1 << 20;
@@ -1916,6 +2136,17 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
     // settle on them first)
     if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
     // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a group of warps per row.
+    if constexpr (CELLS == 1) {
+      const int64_t tab = (static_cast<int64_t>(a.chunk < a.n ? a.chunk : a.n) + 15) / 16 * 16;
+      const int ring_bytes = static_cast<int>(sizeof(int2)) * S_WARPS * 2 * T_RING;
+      const int room = ctx.smem_optin - 1024 - static_cast<int>(sizeof(State32)) * S_WARPS;
+      const int tab_bytes = ring_bytes + tab * S_WARPS <= room ? static_cast<int>(tab) : 0;
+      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    cudaSharedmemCarveoutMaxShared));
+      heavy_rounds_32_kernel<<<ctx.num_sms, S_THREADS, ring_bytes + tab_bytes * S_WARPS, st>>>(a, tab_bytes);
+      CSG_CUDA(cudaGetLastError());
+    }
     if constexpr (in_rounds) {
       const int64_t span = a.chunk < a.n ? a.chunk : a.n;
       const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
@@ -1931,7 +2162,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       heavy_rounds_kernel<CELLS><<<ctx.num_sms, Helpers<CELLS>::THREADS * groups, groups * group_bytes, st>>>(a, tab_bytes);
       CSG_CUDA(cudaGetLastError());
     }
-    if constexpr (!in_rounds) {
+    if constexpr (CELLS > ROUND_CELLS) {
       const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
       CSG_CUDA(cudaFuncSetAttribute(heavy_consume_kernel<CELLS>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, pad));

@@ -1,5 +1,5 @@
-"""Chunks of more than 1,024 rows take kernels of their own: bit-exact tables and orders against
-the CPU oracle at the sizes where they change hands."""
+"""Chunks of more than 1,024 rows and sketches of 32 slots take kernels of their own: bit-exact
+tables and orders against the CPU oracle at the sizes where they change hands."""
 import numpy as np
 import pytest
 
@@ -47,6 +47,26 @@ def test_tall_chunks_grouped_by_a_block_each(chunk):
             rows[2 * chunk + i] = [0, 1 + i % 3000]
     ptr, ind = _csr(rows, n)
     _check(ptr, ind, k=16, chunk_size=chunk)
+
+
+def _hubs(n, hubs, members, seed):
+    """rows of two entries that lie in no hub or one or two, and eight that lie in all hubs"""
+    rng = np.random.default_rng(seed)
+    rows = [list(rng.integers(hubs, n, 2)) for _ in range(n)]
+    for h in range(hubs):
+        for r in rng.integers(0, n, members):
+            rows[r].append(h)
+    for r in range(0, n, n // 8):
+        rows[r] += range(hubs)
+    return _csr(rows, n)
+
+
+@pytest.mark.parametrize("k", [1, 4, 8])
+@pytest.mark.parametrize("n,hubs,members", [(1000, 120, 800), (9000, 40, 2000), (45_000, 32, 2300)])
+def test_rows_of_32_slots_against_oracle(n, hubs, members, k):
+    # the key table in shared memory and, for 45,000 rows, none; rows on either side of a warp each
+    ptr, ind = _hubs(n, hubs, members, n)
+    _check(ptr, ind, limits=(0, 1), k=k, chunk_size=n)
 
 
 @pytest.mark.parametrize("k", [8, 16, 40])
