@@ -47,6 +47,9 @@ def test_tall_chunks_grouped_by_a_block_each(chunk):
             rows[2 * chunk + i] = [0, 1 + i % 3000]
     ptr, ind = _csr(rows, n)
     _check(ptr, ind, k=16, chunk_size=chunk)
+    import chunkedgreedy_b200 as sp
+    got = sp.count_pillars(torch.from_numpy(ptr).cuda(), torch.from_numpy(ind).cuda(), chunk)
+    assert got == oracle.count_pillars(ptr, ind, chunk)
 
 
 def _hubs(n, hubs, members, seed):

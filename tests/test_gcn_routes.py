@@ -111,7 +111,7 @@ def _model_against_fp64(n, sizes, want_x):
         pairs.append((x.grad, xr.grad))
     for got, want in pairs:
         # (the bound of the fused kernels' other tests: sums of n terms that largely cancel)
-        assert float((got.double() - want).norm()) <= 2e-5 * float(want.norm()) + 1e-6
+        assert float((got.detach().double() - want).norm()) <= 2e-5 * float(want.norm()) + 1e-6
 
 
 @pytest.mark.gpu
