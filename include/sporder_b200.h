@@ -183,7 +183,8 @@ SPORDER_API void sporder_context_set_stream_limit(sporder_context_t ctx, uint64_
  * on a row shard) with many nonzeros run the chunk that holds the most of them ahead of the
  * rest, on a second stream of the context: that chunk's transposition first, then the
  * chains of its heaviest rows, while everything else is still being transposed.  min_nnz
- * = 0: the built-in rule (2^24 nonzeros and 64 chunks or more); > 0: every call of at least
+ * = 0: the built-in rule (2^24 nonzeros and 64 chunks or more, and by slots of the sketch where it
+ * gains); > 0: every call of at least
  * min_nnz nonzeros and two chunks; < 0: never.  Results are the same either way.  No
  * reference counterpart. */
 SPORDER_API void sporder_context_set_ahead_threshold(sporder_context_t ctx, int64_t min_nnz);
