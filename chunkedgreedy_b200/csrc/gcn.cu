@@ -419,9 +419,12 @@ __global__ void __launch_bounds__(D_THREADS, 2) gcn_hidden_kernel(DenseArgs a) {
   for (int c = 0; c < PER; ++c) out[O::W2 + (group * PER + c) * HID_T + hj] = acc2[c];
 }
 
-// the blocks' sums, always in the same order, in 64 bits (some hundred terms that largely cancel)
+// The blocks' sums, always in the same order, in 64 bits (some hundred terms that largely cancel).
+// Bound by the latency of its reads: 128 -> 128 -> 16 in small blocks, sixteen reads in flight 18 us,
+// 28.5 in blocks of 256 with four.
+constexpr int SUMS_THREADS = 64;
 template <int IN_T, int HID_T, int CLS_T>
-__global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) {
+__global__ void __launch_bounds__(SUMS_THREADS) gcn_sums_kernel(DenseArgs a, int blocks) {
   using O = PartLayout<IN_T, HID_T, CLS_T>;
   const int w1 = a.hid * a.in, w2 = a.cls * a.hid, total = w1 + w2 + (a.db1 ? a.hid : 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -443,6 +446,13 @@ __global__ void __launch_bounds__(256) gcn_sums_kernel(DenseArgs a, int blocks) 
     for (int g = 0; g < times; ++g) {
       const float *src = a.part + at + g * HID_T;
       int b = 0;
+      for (; b + 16 <= blocks; b += 16) {
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = src[static_cast<size_t>(b + u) * O::FLOATS];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) sum[u & 3] += v[u];
+      }
       for (; b + 4 <= blocks; b += 4)
 #pragma unroll
         for (int u = 0; u < 4; ++u) sum[u] += src[static_cast<size_t>(b + u) * O::FLOATS];
@@ -546,7 +556,7 @@ bool backward_variant(Context &ctx, DenseArgs a) {
   gcn_backward_kernel<IN_T, HID_T, CLS_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
   const int total = a.hid * a.in + a.cls * a.hid + a.hid;
-  gcn_sums_kernel<IN_T, HID_T, CLS_T><<<(total + 255) / 256, 256, 0, ctx.stream>>>(a, grid);
+  gcn_sums_kernel<IN_T, HID_T, CLS_T><<<(total + SUMS_THREADS - 1) / SUMS_THREADS, SUMS_THREADS, 0, ctx.stream>>>(a, grid);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
   return true;
@@ -562,7 +572,7 @@ bool hidden_variant(Context &ctx, DenseArgs a) {
   a.part = reinterpret_cast<float *>(ctx.ws);
   gcn_hidden_kernel<HID_T, CLS_T><<<grid, D_THREADS, smem, ctx.stream>>>(a);
   CSG_CUDA(cudaGetLastError());
-  gcn_sums_kernel<0, HID_T, CLS_T><<<(a.cls * a.hid + 255) / 256, 256, 0, ctx.stream>>>(a, grid);
+  gcn_sums_kernel<0, HID_T, CLS_T><<<(a.cls * a.hid + SUMS_THREADS - 1) / SUMS_THREADS, SUMS_THREADS, 0, ctx.stream>>>(a, grid);
   CSG_CUDA(cudaGetLastError());
   count_launches(2);
   return true;
