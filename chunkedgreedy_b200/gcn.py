@@ -93,13 +93,13 @@ def step_widths(rows, in_dim, hidden, classes, fused):
     backward, first backward).  The second operator goes behind the second linear layer (op(h) W2^T =
     op(h W2^T)) where that moves no more columns, on the fused route, which saves besides; on torch's where the
     columns saved are worth a bias and a padding of their own (300 inputs, 64 hidden units, 10 classes: 4,096 rows 0.67 ms
-    as it stands and 0.70 behind, 1.05 M rows 6.7 and 6.1).  Logits are padded from 32,768 rows on: below, a step
-    is its launches (4,096 rows 0.58 ms, 0.60 padded).  The first layer keeps its order: hidden units within a rounding
+    as it stands and 0.70 behind, 1.05 M rows 6.7 and 6.1).  Logits are padded from 131,072 rows on: below, a step
+    is its launches (4,096 rows 0.58 ms, 0.60 padded; 60,000 rows 0.62 and 0.65).  The first layer keeps its order: hidden units within a rounding
     of zero decide by their sign, and op(x) W1^T rounds differently.  Backward, the fused route takes op(x)
     or op(D), whichever moves fewer columns (128 inputs, 64 hidden units, 16 classes, 1.05 M rows: 4.8 and 4.2 ms)."""
     saved = hidden - moved_columns(classes)
     behind = saved >= 0 if fused else rows * saved >= 1 << 22
-    second = hidden if not behind else padded_columns(classes) if rows >= 1 << 15 else classes
+    second = hidden if not behind else padded_columns(classes) if rows >= 1 << 17 else classes
     first = in_dim if fused and moved_columns(in_dim) <= moved_columns(hidden) else hidden
     return hidden, second, second, first
 
@@ -184,17 +184,21 @@ class LogitsFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u, op, b, classes):
         ctx.op, ctx.width, ctx.biased = op, u.shape[1], b is not None
-        z = op(u.contiguous())
-        if ctx.width != classes:
-            z = z[:, :classes]
+        z = op(u.contiguous())[:, :classes]
         return z + b if ctx.biased else z.contiguous()
 
     @staticmethod
     def backward(ctx, g):
         db = g.sum(0) if ctx.biased else None
-        if ctx.width != g.shape[1]:
-            g = _pad_columns(g, ctx.width, getattr(ctx.op, "ctx", None))
+        g = _pad_columns(g, ctx.width, getattr(ctx.op, "ctx", None))
         return ctx.op(g.contiguous()), None, db, None
+
+
+def _logits(u, op, b, classes):
+    if u.shape[1] != classes:
+        return LogitsFn.apply(u, op, b, classes)
+    z = SpMMFn.apply(u, op)  # (the bias by torch's own autograd: a small step is its host work)
+    return z if b is None else z + b
 
 
 def _plain(layer):
@@ -213,24 +217,24 @@ class GCN(torch.nn.Module):
         self.w2 = torch.nn.Linear(hidden, classes)
 
     def forward(self, x, op):
-        if not (_plain(self.w1) and _plain(self.w2)):
-            return self.w2(SpMMFn.apply(F.relu(SpMMFn.apply(self.w1(x), op)), op))
-        hidden, in_dim = self.w1.weight.shape
-        classes = self.w2.weight.shape[0]
+        # (a small step is its host work, and a module's attributes are looked up one by one)
+        l1, l2 = self.w1, self.w2
+        if not (_plain(l1) and _plain(l2)):
+            return l2(SpMMFn.apply(F.relu(SpMMFn.apply(l1(x), op)), op))
+        w1, b1, w2, b2 = l1.weight, l1.bias, l2.weight, l2.bias
+        (hidden, in_dim), classes = w1.shape, w2.shape[0]
         # limits of the fused kernels; others, and features that want a gradient, by torch
         fused = (not x.requires_grad and in_dim % 4 == 0 and in_dim <= 128 and hidden % 4 == 0 and hidden <= 128
-                 and classes <= 48 and moved_columns(classes) <= hidden and self.w1.bias is not None
+                 and classes <= 48 and moved_columns(classes) <= hidden and b1 is not None
                  and x.data_ptr() % 16 == 0
-                 and all(t.is_cuda and t.dtype == torch.float32 for t in (x, self.w1.weight, self.w2.weight)))
+                 and all(t.is_cuda and t.dtype == torch.float32 for t in (x, w1, w2)))
         _, out, _, first = step_widths(x.shape[0], in_dim, hidden, classes, fused)
         if fused:
-            u = LayersFn.apply(x, op, self.w1.weight, self.w1.bias, self.w2.weight, out, first)
-            return LogitsFn.apply(u, op, self.w2.bias, classes)
-        h = F.relu(SpMMFn.apply(self.w1(x), op))
+            return _logits(LayersFn.apply(x, op, w1, b1, w2, out, first), op, b2, classes)
+        h = F.relu(SpMMFn.apply(l1(x), op))
         if out == hidden:
-            return self.w2(SpMMFn.apply(h, op))
-        w2 = self.w2.weight if out == classes else F.pad(self.w2.weight, (0, 0, 0, out - classes))
-        return LogitsFn.apply(F.linear(h, w2), op, self.w2.bias, classes)
+            return l2(SpMMFn.apply(h, op))
+        return _logits(F.linear(h, w2 if out == classes else F.pad(w2, (0, 0, 0, out - classes))), op, b2, classes)
 
 
 def normalised_values(ptr, ind):

@@ -7,7 +7,7 @@ torch = pytest.importorskip("torch")
 
 from chunkedgreedy_b200 import gcn  # noqa: E402
 
-ROWS = [1, 4096, 32_768, 65_536, 1 << 20]
+ROWS = [1, 4096, 65_536, 131_071, 131_072, 1 << 20]
 
 
 @pytest.mark.parametrize("in_dim", [4, 16, 64, 100, 128])
@@ -115,7 +115,7 @@ def _model_against_fp64(n, sizes, want_x):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 32_768, 40_001])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 40_001, 131_073])
 @pytest.mark.parametrize("sizes", [(128, 32, 17), (128, 32, 30), (100, 36, 9), (128, 64, 3), (128, 64, 48), (128, 128, 30),
                                    (100, 64, 47), (12, 8, 5), (128, 16, 7), (68, 4, 2), (128, 124, 33)])
 def test_fused_routes_against_fp64(n, sizes):
@@ -124,7 +124,7 @@ def test_fused_routes_against_fp64(n, sizes):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,sizes", [(100_000, (300, 64, 10)), (100_000, (36, 256, 30)), (4096, (300, 64, 10)),
+@pytest.mark.parametrize("n,sizes", [(131_072, (300, 64, 10)), (131_072, (36, 256, 30)), (4096, (300, 64, 10)),
                                      (100_000, (128, 64, 13))])
 @pytest.mark.parametrize("want_x", [False, True])
 def test_library_products_behind_and_in_front(n, sizes, want_x):
