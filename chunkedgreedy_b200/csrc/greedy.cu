@@ -248,8 +248,9 @@ __device__ __forceinline__ void sts_u16(uint32_t at, uint32_t v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(static_cast<uint16_t>(v)));
 }
 
-// Out of line, for the one chunk in a million: inlined it would cost greedy_lists_kernel registers.  (Where the
-// table is all there is it is inlined: called, it reads its arguments from memory at every step.)
+// Out of line for greedy_lists_kernel, whose registers it would cost and which hardly ever calls it.  greedy_kernel,
+// which does nothing else, has it inlined: called, it read its arguments from memory at every step (mesh of
+// 262,144 rows in chunks of 8,192, k = 16: 3.95 ms per csg call, 3.72 inlined).
 __device__ __noinline__ void chain_chunk_rare(const GreedyArgs &a, int32_t start, int32_t end, uint32_t *visited) {
   chain_chunk(a, start, end, visited);
 }
