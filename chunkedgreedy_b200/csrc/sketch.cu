@@ -17,7 +17,7 @@
 //    stream is an order-dependent chain;
 //  * the longest rows (65536 candidates or more, and shorter ones while they are few) set the
 //    run time.  Their streams are written out to memory by the whole grid (heavy_expand_kernel,
-//    one warp per 128 columns); then a group of warps works on each row and resolves up to 32
+//    one warp per 128 columns); then a group of warps works on each row and resolves up to 64
 //    candidates per round (see "the chains in rounds" below);
 //  * all other rows run side by side, one per LANE: the container of a row is a column of
 //    shared memory, a step of 32 rows costs a warp little more than a step of one row did, and
@@ -1282,34 +1282,43 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_consume_kernel(SketchArgs 
 // A full sketch behaves like a queue ordered by (weight, slot code): a miss takes the
 // least entry and puts it back heavier, so within a short stretch of the stream the i-th
 // miss takes the i-th entry of the order as it stood at the start of the stretch.  A round
-// looks at the next 32 stream elements, one per lane, and resolves the longest prefix for
-// which that holds, all lanes at once.  With the sketch state S0 at the start of the round,
-// m(L) misses among the first L elements and E_0 < E_1 < ... the entries of S0 in order,
-// the prefix of length L is resolved exactly as the sequential container would when
-//   (1) no two of its misses carry the same key (the second would be a hit on the first),
-//   (2) no hit of the prefix lands on one of E_0 .. E_{m(L)-1} (taken before or after the
-//       hit, the sequential outcome would differ from the one read off S0), and
-//   (3) every entry put back, E_i with weight w(E_i) + alpha, stays above E_{m(L)-1}, so it
-//       is not taken again inside the prefix.
-// All three only get harder as L grows, so every lane computes the longest prefix its own
-// element allows and one redux.sync takes the minimum; L >= 1 always.  Then miss number i
-// rewrites slot E_i, hits add their alpha (hits on one key all add the same alpha, so
-// their order is immaterial), and the next round starts L elements further on.  While the
-// sketch still has empty slots only (1) applies and miss number i fills the next i-th slot.
+// looks at the next 32 or 64 stream elements, one or two per lane, and resolves the whole window:
+//   * the misses take the entries of the order S0 at the start of the round one after the other, but skip an
+//     entry that a hit has made heavier before they reached it ("held");
+//   * an element whose key S0 holds in an entry that was taken before the element's turn is
+//     a miss, not a hit ("gone"), and takes the next entry like any other miss;
+//   * a second element with the key of an earlier one is a hit on the entry the first one ("leader")
+//     left, whichever kind the first one was.
+// Only leaders with their entry among the window's lightest ("open") can go either way.  Let r be an open element's
+// entry's place in the order, P the leaders in front of it that S0 does not hold and A the open elements in front of
+// it with places below r.  The entry is gone iff P + A > r: of the entries below, A are taken or held for certain, and
+// an open element in front with a place above r counts only if it is gone itself - but then
+// P' + A' > r' for it, at most r' - r - 1 of its A' lie between r and r', so P + A >= P' + A' - (r' - r - 1) > r.
+// P alone, and P plus all leaders in front that S0 holds, settle most open elements; the others count A by a ballot
+// each (1.5 a window of the longest row of R-MAT scale 20).
+// All this holds as long as no entry put back or made heavier is light enough to be taken again: the window ends
+// before the first miss whose entry is not below the least weight the window has left in any ("least"; equal weights
+// count as not below).  One element alone is always resolved exactly.  Of 64 elements, a round resolves 59.2 on the
+// longest row of R-MAT scale 20 (64 slots), 64.0 on that of its symmetrised form (128 slots); 20 to 30 where the
+// Dice terms vary widely, as a window of 32 does: rounds_row times both widths on every row.
+// While the sketch has empty slots, miss number i fills the next i-th slot, and the window ends at the second
+// element of a key.
 // A group of warps works on one row: its first warp walks the stream and decides the rounds, the other
-// warps order the slots for it (rank_slots), which is most of the instructions of a round and
-// none of its dependent steps; meanwhile the first warp looks the window up.  State lives in
+// warps order the slots for it (rank_slots); meanwhile the first warp looks the window up.  State lives in
 // shared memory: weights and keys by slot code, a key -> slot table over the chunk's rows, and
-// the order of the round.  Cycles per candidate of the longest rows of R-MAT scale 20, symmetrised
-// (128 slots): 105 with one warp per row, 64 this way; of R-MAT scale 22 (64 slots) 53 and 52 - there
-// the dependent steps of the first warp are the bound and the order comes in their shadow.
-constexpr int H_RING = 512;      // stream elements staged per batch
+// the order of the round.  What bounds it is the dependent instructions of the first warp, some 450 a round of 64
+// (1,850 cycles) and 300 a round of 32 (1,090): no pipe is busy.  ns per candidate with windows of 32 and strict
+// rounds that ended at the first open element that is not held, and now: R-MAT scale 20, 64 slots, longest row
+// 23.4 -> 15.9, rows of 166,000 / 76,000 / 30,000 candidates 51 -> 20.8, 89 -> 27.0, 184 -> 39.2; symmetrised scale 19,
+// 128 slots, longest 29.4 -> 18.2, 146,000 / 61,000 candidates 41 -> 26.5, 78 -> 31.7; power-law band of 4,096 rows
+// 26.7 -> 16.4.
+constexpr int H_RING = 1024;     // stream elements in a row's ring ...
+constexpr int H_SEG = 256;       // ... staged this many at a time
 constexpr int ROUND_CELLS = 4;   // largest sketch (cells per lane) resolved in rounds
-constexpr int WINDOW_CELLS = 2;  // smallest sketch with whole-window rounds (and with helping warps): with 32 slots a
-                                 // window of 32 can take every entry (heavy_rounds_32_kernel)
-constexpr int MATES = 1024;      // words of the duplicate detector
+constexpr int WINDOW_CELLS = 2;  // smallest sketch resolved by a group of warps (32 slots: heavy_rounds_32_kernel)
+constexpr int MATES = 1024;      // words of the duplicate detector (two for 64 elements)
 constexpr int ROUND_TAB_MAX = 65536;  // largest chunk (rows) with a key -> slot table
-constexpr int TRIAL_ROUNDS = 8;     // rounds of each kind a row times before it settles on one ...
+constexpr int TRIAL_ROUNDS = 8;     // rounds of each width a row times before it settles on one ...
 constexpr int COMMIT_ROUNDS = 160;  // ... for this many rounds
 template <int CELLS>
 struct Helpers {
@@ -1325,21 +1334,19 @@ constexpr int BAR_ROW = 1, BAR_STATE = 2, BAR_ORDER = 3;
 template <int CELLS>
 struct RoundState {
   static constexpr int M = 32 * CELLS;
-  __align__(16) uint32_t w[M];   // weight bits by slot code (cell * 32 + lane)
-  __align__(16) int32_t key[M];
+  static constexpr int W = M < 64 ? M : 64;  // widest window, and entries of the order that are kept
+  __align__(16) uint32_t w[M + 4];   // weight bits by slot code (cell * 32 + lane); the last for who has none
+  __align__(16) int32_t key[M + 4];
   int32_t rank[M];               // position of each slot in ascending (weight, code) order
-  uint32_t sw[32];               // the 32 lightest in that order: weights ...
-  int32_t si[32];                // ... slot codes ...
-  int32_t sk[32];                // ... and keys
-  uint32_t cw[32];               // the same without the entries that hits hold back
-  int32_t ci[32], ck[32], cr[32];
-  int32_t miss_pos[32];          // lane of the i-th miss of the window
+  uint2 order[W];                // the lightest in that order: weight bits, key << 8 | slot code
+  uint2 takes[W + 2];            // the same without the entries that hits hold back
   int32_t row_done;              // tells the other warps that the row is through
   uint32_t item;                 // the row in hand (place in the list)
+  uint32_t spare;                // where stores of lanes without one go
 };
 
-// A group's shared memory: state, two stream buffers (the next batch lands while this one is
-// consumed), the duplicate detector (all zero between rounds), then the key -> slot table (slot
+// A group's shared memory: state, the ring of stream elements (a segment lands while the ones before it are
+// consumed), the duplicate detector (all zero between windows), then the key -> slot table (slot
 // + 1, one byte per row of the chunk; none for very large chunks).  The rounds are functions of
 // their own; they get an offset and build their pointers from the array itself, so that the
 // compiler sees shared memory and not a generic address (slower by some ten cycles a load).
@@ -1347,25 +1354,27 @@ extern __shared__ __align__(16) unsigned char heavy_dyn[];
 template <int CELLS>
 struct GroupMemory {
   static constexpr int RING = (sizeof(RoundState<CELLS>) + 15) / 16 * 16;
-  static constexpr int MATE = RING + 2 * H_RING * 8;
-  static constexpr int TAB = MATE + MATES * 4;
+  static constexpr int MATE = RING + H_RING * 8;
+  // (chunks of more than MATES rows share half as many words: their tables are the larger part)
+  static constexpr __host__ __device__ int tab_offset(bool hash) { return MATE + (hash ? MATES / 2 : MATES) * 8; }
+  static constexpr int SPARE = static_cast<int>(offsetof(RoundState<CELLS>, spare));
   static __device__ __forceinline__ RoundState<CELLS> &state(int base) {
     return *reinterpret_cast<RoundState<CELLS> *>(heavy_dyn + base);
   }
-  static __device__ __forceinline__ int2 *ring(int base, int buffer) {
-    return reinterpret_cast<int2 *>(heavy_dyn + base + RING) + buffer * H_RING;
+  static __device__ __forceinline__ int2 *ring(int base) {
+    return reinterpret_cast<int2 *>(heavy_dyn + base + RING);
   }
-  static __device__ __forceinline__ uint32_t *mates(int base) {
-    return reinterpret_cast<uint32_t *>(heavy_dyn + base + MATE);
+  static __device__ __forceinline__ uint2 *mates(int base) {
+    return reinterpret_cast<uint2 *>(heavy_dyn + base + MATE);
   }
-  static __device__ __forceinline__ uint8_t *tab(int base) { return heavy_dyn + base + TAB; }
+  template <bool HASH>
+  static __device__ __forceinline__ uint8_t *tab(int base) { return heavy_dyn + base + tab_offset(HASH); }
 };
 
 // what the rounds of a row need to know
 struct RoundRow {
   int base;           // the group's place in shared memory
   int32_t cbase;      // first row of the chunk
-  bool mates_hashed;  // the chunk has more than MATES rows: words are shared
   uint32_t *ctrl;     // checked build: where a key outside its chunk is recorded ...
   int32_t span;       // ... and the rows of a chunk
   int bars;           // the group's named barriers are bars + BAR_*
@@ -1382,9 +1391,9 @@ __device__ __forceinline__ void bar_wait(int id) {
 
 // Slot that holds key s (relative to the chunk), or -1.  With TAB from the key -> slot table;
 // without it by comparing s with every slot's key (unique in a sketch, empty slots hold -1).
-template <int CELLS, bool TAB>
+template <int CELLS, bool TAB, bool HASH>
 __device__ __forceinline__ int slot_of(const RoundRow &row, int32_t s) {
-  if (TAB) return static_cast<int>(GroupMemory<CELLS>::tab(row.base)[s]) - 1;
+  if (TAB) return static_cast<int>(GroupMemory<CELLS>::template tab<HASH>(row.base)[s]) - 1;
   const RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
   int q = -1;
 #pragma unroll
@@ -1399,284 +1408,376 @@ __device__ __forceinline__ int slot_of(const RoundRow &row, int32_t s) {
 }
 
 // One of the other warps: the place of its sixteen slots in the (weight, code) order, the
-// number of entries (x, i) below (mine, slot).  Two lanes per slot, half of the entries each.
+// number of entries (x, i) below (mine, slot).  GROUP lanes to GROUP / 2 slots, as many parts of the entries.
 // "x < mine" is counted as sat((mine - x) * 2^90), one fused multiply-add that is exactly 1 or 0:
 // weights lie in [2^-31, 2^32], so two different ones are at least 2^-54 apart.  An equal entry
-// is below for a smaller code; that choice is made per block of four entries (mine or the next
-// float above it), and the slot's own block is put right afterwards.
+// is below for a smaller code: then the bar is the next float above.
+// Returns false once the row is through.
 template <int CELLS>
-__device__ __forceinline__ void rank_slots(int base, int helper, int lane) {
+__device__ __forceinline__ bool rank_slots(int base, int helper, int lane) {
   RoundState<CELLS> &st = GroupMemory<CELLS>::state(base);
-  constexpr int M = 32 * CELLS, QUADS = M / 8;  // blocks of four entries per half
   constexpr float BIG = 1.2379400392853803e27f;  // 2^90
-  const int slot = helper * 16 + (lane & 15), half = lane >> 4, own = slot >> 2;
+  constexpr float ZERO = 8388608.0f;             // 2^23: counts are read off its last bits
+  constexpr int GROUP = 8, SLOTS = GROUP / 2, QUADS = 8 * CELLS / GROUP;
+  const int sub = lane % GROUP, first = helper * 16 + lane / GROUP * SLOTS, slot = first + sub % SLOTS, own = first / 4;
   const float4 *const v4 = reinterpret_cast<const float4 *>(st.w);
+  float4 all[QUADS];  // (loaded in one go: left to itself the compiler waits for every load)
+  float m[SLOTS];
+#pragma unroll
+  for (int b = 0; b < QUADS; ++b) all[b] = v4[b * GROUP + sub];
+#pragma unroll
+  for (int i = 0; i < SLOTS; ++i) m[i] = __uint_as_float(st.w[first + i]);
   const uint32_t bits = st.w[slot];
   const int32_t key = st.key[slot];
-  const float mine = __uint_as_float(bits);
-  const float lt = mine * BIG, le = __uint_as_float(bits + 1u) * BIG;
-  const float4 mates = v4[own];
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  float4 all[QUADS];  // (loaded in one go: left to itself the compiler waits for every load)
+  const bool done = *static_cast<volatile int32_t *>(&st.row_done);
+  float acc[SLOTS];
 #pragma unroll
-  for (int b = 0; b < QUADS; ++b) all[b] = v4[half * QUADS + b];
+  for (int i = 0; i < SLOTS; ++i) {
+    const float lt = m[i] * BIG, le = __uint_as_float(__float_as_uint(m[i]) + 1u) * BIG;
+    acc[i] = ZERO;
 #pragma unroll
-  for (int b = 0; b < QUADS; ++b) {
-    const float bar = half * QUADS + b < own ? le : lt;
-    acc[0] += __saturatef(fmaf(all[b].x, -BIG, bar));
-    acc[1] += __saturatef(fmaf(all[b].y, -BIG, bar));
-    acc[2] += __saturatef(fmaf(all[b].z, -BIG, bar));
-    acc[3] += __saturatef(fmaf(all[b].w, -BIG, bar));
-  }
-  int pos = static_cast<int>((acc[0] + acc[1]) + (acc[2] + acc[3]));
-  if (own / QUADS == half) {
-    const int e = slot & 3;
-    pos += (e > 0 && mates.x == mine ? 1 : 0) + (e > 1 && mates.y == mine ? 1 : 0) + (e > 2 && mates.z == mine ? 1 : 0);
-  }
-  pos += __shfl_xor_sync(FULL, pos, 16);
-  if (half == 0) {
-    st.rank[slot] = pos;
-    if (pos < 32) st.sw[pos] = bits;
-  } else if (pos < 32) {
-    st.si[pos] = slot;
-    st.sk[pos] = key;
-  }
-}
-
-// The window of a round, one element per lane, as looked up before the order is known.
-template <int CELLS>
-struct Window {
-  bool valid;
-  int32_t s;      // key, relative to the chunk
-  float al;       // Dice term
-  int q;          // slot that holds the key, or -1
-  int32_t mate;   // word of the duplicate detector
-};
-
-template <int CELLS, bool TAB>
-__device__ __forceinline__ Window<CELLS> look_up(const RoundRow &row, int buf, int p, int cnt, int lane) {
-  const int2 *const ring = GroupMemory<CELLS>::ring(row.base, buf);
-  Window<CELLS> w;
-  w.valid = p + lane < cnt;
-  const int2 elem = w.valid ? ring[p + lane] : make_int2(row.cbase, 0);
-  // (a key outside the chunk only comes from rows that are not sorted: kept in bounds)
-  w.s = static_cast<int32_t>(min(static_cast<uint32_t>(key_in_chunk(row.ctrl, elem.x, row.cbase, row.span) - row.cbase),
-                                 static_cast<uint32_t>(row.span) - 1u));
-  w.al = __int_as_float(elem.y);
-  // Lanes that carry the same key: every lane sets its bit in a word of shared memory under its
-  // key, and reads the word back later.  match.any, the instruction made for this, takes some
-  // 380 cycles here.
-  w.mate = row.mates_hashed ? static_cast<int32_t>((static_cast<uint32_t>(w.s) * 0x9E3779B1u) >> 22) : w.s;
-  if (w.valid) atomicOr(&GroupMemory<CELLS>::mates(row.base)[w.mate], 1u << lane);
-  w.q = w.valid ? slot_of<CELLS, TAB>(row, w.s) : -1;
-  return w;
-}
-
-// lanes of the window with this lane's key; clears the detector
-template <int CELLS>
-__device__ __forceinline__ unsigned same_key(const RoundRow &row, const Window<CELLS> &w, int lane) {
-  uint32_t *const mates = GroupMemory<CELLS>::mates(row.base);
-  __syncwarp();
-  unsigned same = w.valid ? mates[w.mate] : 0u;
-  if (row.mates_hashed) {  // a word may stand for several keys: rare, then the slow instruction
-    const int32_t first = __shfl_sync(FULL, w.s, same ? __ffs(static_cast<int>(same)) - 1 : lane);
-    if (__any_sync(FULL, w.valid && first != w.s)) same = __match_any_sync(FULL, w.valid ? w.s : -1 - lane);
-    if (!w.valid) same = 0u;
-  }
-  __syncwarp();
-  if (w.valid) mates[w.mate] = 0u;
-  return same;
-}
-
-// One strict round on a full sketch; returns the number of stream elements resolved (>= 1).
-template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_strict(const RoundRow &row, int buf, int p, int cnt, int lane) {
-  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
-  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
-  const uint32_t below = (1u << lane) - 1u;
-  bar_arrive<CELLS>(row.bars + BAR_STATE);
-  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
-  const bool miss = w.valid && w.q < 0, hit = w.valid && w.q >= 0;
-  const int q = hit ? w.q : 0;
-  const uint32_t wq = st.w[q];
-  const uint32_t missing = __ballot_sync(FULL, miss);
-  const int mtot = __popc(missing), mrank = __popc(missing & below);
-  if (miss) st.miss_pos[mrank] = lane;
-  const unsigned same = same_key<CELLS>(row, w, lane);
-  bar_wait<CELLS>(row.bars + BAR_ORDER);
-  // every lane reads what either kind of element needs, then selects
-  const int rho = st.rank[q];
-  const int tgt = st.si[mrank & 31];
-  const uint32_t base = st.sw[mrank & 31];
-  const int32_t old_key = st.sk[mrank & 31];
-  const uint32_t top = st.sw[mtot > 0 ? mtot - 1 : 0];
-  const int at_hit = st.miss_pos[rho & 31];
-  const int at_next = st.miss_pos[(mrank + 1) & 31];
-  const uint32_t nb = __float_as_uint(__uint_as_float(base) + w.al);
-  int lim = w.valid ? 32 : lane;
-  if (hit) {  // (2): this hit and the miss that takes its slot cannot share a prefix
-    const int at = rho < mtot ? at_hit : 32;
-    lim = at > lane ? at : lane;
-  }
-  if (miss) {
-    // (3): above the heaviest entry any miss of this window can take, the weight put back
-    // is safe.  Otherwise (rare) the prefix ends before the next miss, or before this one
-    // if the sum did not even grow.
-    if (nb <= top) lim = nb > base ? (mrank + 1 < mtot ? at_next : 32) : lane;
-    if (same & below) lim = lane;  // (1)
-  }
-  int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
-  L = L < 1 ? 1 : L;  // one element alone is always resolved exactly
-  const bool applies = lane < L;
-  const unsigned mates = same & (L >= 32 ? FULL : (1u << L) - 1u);
-  const int times = __popc(mates);
-  float wv = __uint_as_float(wq) + w.al;
-  for (int t = 1; t < times; ++t) wv += w.al;
-  if (applies && miss) {
-    if (TAB) tab[old_key] = 0;
-    st.key[tgt] = w.s;
-    st.w[tgt] = nb;
-    if (TAB) tab[w.s] = static_cast<uint8_t>(tgt + 1);
-  }
-  if (applies && hit && (mates & below) == 0u) st.w[q] = __float_as_uint(wv);  // first hit of its key
-  __syncwarp();
-  return L;
-}
-
-// One round on a full sketch of 64 slots or more that resolves the WHOLE window.  The three
-// conditions of the strict round end a prefix at the first element whose outcome cannot be read
-// off the order of S0 directly.  Almost all of those are hits on an entry that the misses of the
-// window are about to take, and their outcome still follows from S0 by a little bookkeeping:
-//   * the misses take the entries of S0 in order, but skip an entry that a hit has made
-//     heavier before they reached it (put back one Dice term heavier, an entry lands behind
-//     everything a window of 32 can take: checked below, not assumed);
-//   * an element whose key S0 holds in an entry that was taken before the element's turn is
-//     a miss, not a hit, and takes the next entry like any other miss;
-//   * a second element with the key of an earlier one is a hit on the entry the first one
-//     left, whichever kind the first one was.
-// Only the first element of each key ("leader") with its entry among the 32 lightest can go
-// either way: with P misses before element j and b skipped entries below its entry's rank r,
-// the entry is gone iff P + b > r.  Bounds on P + b settle most of them without looking at
-// the others (see "slack" below); a window where one stays undecided walks them in stream
-// order (a handful per window, state in two 32-bit masks, every lane computing the same).
-// The miss with i misses before it then takes the (i+1)-th entry that no hit holds back.  The
-// read-off is exact as long as nothing put back or made heavier is light enough to be taken
-// again inside the window; an element whose new weight does not clear the heaviest entry taken
-// ends the prefix before the next miss behind it (before itself, if its weight did not grow at
-// all).  On the heaviest R-MAT rows that happens in one window of 32,000 (the row's own Dice
-// terms dominate) to one in ten (rows whose terms vary more), and a round resolves 32.0 resp.
-// 29.3 elements where a strict one resolves 16.4 on the former; on rows whose terms vary widely
-// either kind ends after 6 to 13 and the strict round is the cheaper one, which is why
-// rounds_row times both kinds on every row and keeps the one that resolves more per cycle.
-template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_window(const RoundRow &row, int buf, int p, int cnt, int lane) {
-  RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
-  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
-  constexpr int M = 32 * CELLS;
-  static_assert(CELLS >= WINDOW_CELLS, "a window of 32 needs more than 32 slots");
-  const uint32_t below = (1u << lane) - 1u;
-  bar_arrive<CELLS>(row.bars + BAR_STATE);
-  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
-  const bool present = w.valid && w.q >= 0;  // S0 holds the key
-  const int q = present ? w.q : 0;
-  const uint32_t wq = st.w[q];
-  const unsigned same = same_key<CELLS>(row, w, lane);
-  const bool leader = w.valid && (same & below) == 0u;  // first element of its key in the window
-  const uint32_t absent = __ballot_sync(FULL, leader && !present);
-  const int absent_before = __popc(absent & below);
-  bar_wait<CELLS>(row.bars + BAR_ORDER);
-  const int rho = present ? st.rank[q] : M;
-  const uint32_t my_w = st.sw[lane];  // the entry of rank `lane`
-  const int32_t my_i = st.si[lane], my_k = st.sk[lane];
-  // Which leaders miss: those S0 does not hold, and those whose entry is gone by their turn.
-  // An open element (leader, entry among the 32 lightest) with `before` certain misses and
-  // `nth` open elements in front of it: at least `before`, at most `before + nth` entries
-  // below its own are taken or skipped by its turn, so rank < before means gone and
-  // rank >= before + nth means still there, whatever the open elements in front did.  Most
-  // windows have only such elements; the others are walked in stream order.
-  const bool open = leader && present && rho < 32;
-  uint32_t open_set = __ballot_sync(FULL, open);
-  const int slack = rho - absent_before;
-  const bool sure_gone = open && slack < 0;
-  const bool sure_held = open && slack >= __popc(open_set & below);
-  uint32_t flipped = __ballot_sync(FULL, sure_gone);  // lanes whose entry was taken before their turn
-  uint32_t held = __reduce_or_sync(FULL, sure_held ? 1u << (rho & 31) : 0u);  // ranks a hit holds back
-  if (__any_sync(FULL, open && !sure_gone && !sure_held)) {
-    flipped = 0u;
-    held = 0u;
-    while (open_set) {
-      const int j = __ffs(open_set) - 1;
-      open_set &= open_set - 1u;
-      const int r = __shfl_sync(FULL, rho, j);
-      const int before = __popc((absent | flipped) & ((1u << j) - 1u));
-      const int skipped = __popc(held & ((1u << r) - 1u));
-      if (before + skipped > r)
-        flipped |= 1u << j;
-      else
-        held |= 1u << r;
+    for (int b = 0; b < QUADS; ++b) {
+      // entries of the slots' own block of four in front of this slot, and others, have the bar of their block
+      const bool before = b * GROUP + sub < own, upto = b * GROUP + sub <= own;
+      const float bar = before ? le : lt, front = upto ? le : lt;
+      const int e = (first + i) & 3;
+      const float x[4] = {all[b].x, all[b].y, all[b].z, all[b].w};
+      float c[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[k] = __saturatef(fmaf(x[k], -BIG, k < (SLOTS == 4 ? i : e) ? front : bar));
+      acc[i] += (c[0] + c[1]) + (c[2] + c[3]);
     }
   }
-  const uint32_t missing = absent | flipped;
-  const int mtot = __popc(missing);
-  const bool miss = (missing >> lane) & 1u;
-  // the i-th miss takes the i-th entry of the order that no hit holds back
-  if (((held >> lane) & 1u) == 0u) {
-    const int at = lane - __popc(held & below);
-    st.cw[at] = my_w;
-    st.ci[at] = my_i;
-    st.ck[at] = my_k;
-    st.cr[at] = lane;
+  // counts of the slots in the bytes of one word
+  uint32_t counts = __byte_perm(__float_as_uint(acc[0]), __float_as_uint(acc[1]), 0x0040) & 0xFFFFu;
+  if (SLOTS == 4)
+    counts = __byte_perm(counts, __byte_perm(__float_as_uint(acc[SLOTS - 2]), __float_as_uint(acc[SLOTS - 1]), 0x0040), 0x5410);
+#pragma unroll
+  for (int d = 1; d < GROUP; d <<= 1) counts += __shfl_xor_sync(FULL, counts, d);
+  const int pos = static_cast<int>(counts >> (8 * (sub % SLOTS)) & 255u);
+  if (done) return false;
+  if (sub < SLOTS)
+    st.rank[slot] = pos;
+  else if (pos < RoundState<CELLS>::W)
+    st.order[pos] = make_uint2(bits, static_cast<uint32_t>(key) << 8 | static_cast<uint32_t>(slot));
+  return true;
+}
+
+// The window of a round, E elements per lane (element 32 e + lane of the window in place e).
+template <int E>
+struct Window {
+  bool valid[E];
+  int32_t s[E];   // key, relative to the chunk
+  float al[E];    // Dice term
+};
+
+// bits of a mask over the window (32 to a word) in front of this lane's element e
+template <int E>
+__device__ __forceinline__ int count_before(const uint32_t (&mask)[E], int e, uint32_t below) {
+  int c = __popc(mask[e] & below);
+#pragma unroll
+  for (int f = 0; f < E; ++f)
+    if (f < e) c += __popc(mask[f]);
+  return c;
+}
+
+// elements of `same` among the first L of the window
+template <int E>
+__device__ __forceinline__ int count_prefix(const uint32_t (&same)[E], int L) {
+  int c = 0;
+#pragma unroll
+  for (int f = 0; f < E; ++f) {
+    const int l = L - 32 * f;
+    c += __popc(same[f] & (l >= 32 ? FULL : l <= 0 ? 0u : (1u << l) - 1u));
   }
-  const int mine_i = miss ? __popc(missing & below) : 0;
-  const int last_i = mtot > 0 ? mtot - 1 : 0;
-  const uint32_t behind = missing & ~(below | (1u << lane));
-  const int next_miss = behind ? __ffs(static_cast<int>(behind)) - 1 : 32;
-  const uint32_t hv = __float_as_uint(__uint_as_float(wq) + w.al);
+  return c;
+}
+
+template <int CELLS, int E>
+__device__ __forceinline__ void window_load(const RoundRow &row, uint32_t p, uint32_t end, int lane, Window<E> &w) {
+  const int2 *const ring = GroupMemory<CELLS>::ring(row.base);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int2 elem = ring[(p + e * 32 + lane) & (H_RING - 1)];
+    w.valid[e] = p + e * 32 + lane < end;
+    const int32_t key = w.valid[e] ? elem.x : row.cbase;
+    // (a key outside the chunk only comes from rows that are not sorted: kept in bounds)
+    w.s[e] = static_cast<int32_t>(min(static_cast<uint32_t>(key_in_chunk(row.ctrl, key, row.cbase, row.span) - row.cbase),
+                                      static_cast<uint32_t>(row.span) - 1u));
+    w.al[e] = __int_as_float(elem.y);
+  }
+}
+
+// Elements with the same key, part one: every lane sets its bit in a word of shared memory under its key.
+// match.any, the instruction made for this, takes some 380 cycles here.
+template <bool HASH>
+__device__ __forceinline__ int mate_word(int32_t s) {
+  return HASH ? static_cast<int>((static_cast<uint32_t>(s) * 0x9E3779B1u) >> 23) : s;
+}
+template <int CELLS, int E, bool HASH>
+__device__ __forceinline__ void window_mark(const RoundRow &row, int lane, const Window<E> &w) {
+  uint2 *const mates = GroupMemory<CELLS>::mates(row.base);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    uint2 &word = mates[mate_word<HASH>(w.s[e])];
+    if (w.valid[e]) atomicOr(e == 0 ? &word.x : &word.y, 1u << lane);
+  }
+}
+// Part two (after a __syncwarp): the marks, 32 elements of the window to a word; the words are clear again.
+template <int CELLS, int E, bool HASH>
+__device__ __forceinline__ void window_collect(const RoundRow &row, uint32_t p, int lane, const Window<E> &w,
+                                               uint32_t (&same)[E][E]) {
+  uint2 *const mates = GroupMemory<CELLS>::mates(row.base);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const uint2 both = mates[mate_word<HASH>(w.s[e])];
+    same[e][0] = w.valid[e] ? both.x : 0u;
+    if (E > 1) same[e][E - 1] = w.valid[e] ? both.y : 0u;
+  }
+  if (HASH) {  // a word may stand for several keys: the others are taken out one by one
+    const int2 *const ring = GroupMemory<CELLS>::ring(row.base);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+#pragma unroll
+      for (int f = 0; f < E; ++f)
+        for (uint32_t rest = same[e][f] & (e == f ? ~(1u << lane) : FULL); rest; rest &= rest - 1u) {
+          const int b = __ffs(static_cast<int>(rest)) - 1;
+          if (ring[(p + f * 32 + b) & (H_RING - 1)].x - row.cbase != w.s[e]) same[e][f] &= ~(1u << b);
+        }
+  }
   __syncwarp();
-  const uint32_t base = st.cw[mine_i];
-  const uint32_t top = st.cw[last_i];
-  const int t_last = mtot > 0 ? st.cr[last_i] : -1;  // rank of the heaviest entry taken
-  const int tgt = st.ci[mine_i];
-  const int32_t old_key = st.ck[mine_i];
-  const uint32_t nb = __float_as_uint(__uint_as_float(base) + w.al);
-  int lim = w.valid ? 32 : lane;
-  if (mtot > 0) {
-    if (miss && nb <= top) lim = nb > base ? next_miss : lane;
-    if (leader && present && !miss && rho <= t_last && hv <= top) lim = hv > wq ? next_miss : lane;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (w.valid[e]) mates[mate_word<HASH>(w.s[e])] = make_uint2(0u, 0u);
+}
+
+// One more Dice term for a key that comes again in the window; the element of `rest` (later elements of the key) that
+// brought it is taken out.
+template <int E>
+__device__ __forceinline__ void add_later(uint32_t (&rest)[E], float al, uint32_t &weight) {
+  uint32_t any = rest[0];
+#pragma unroll
+  for (int f = 1; f < E; ++f) any |= rest[f];
+  weight = any ? __float_as_uint(__uint_as_float(weight) + al) : weight;
+  if (E > 1) rest[E - 1] = rest[0] ? rest[E - 1] : rest[E - 1] & (rest[E - 1] - 1u);
+  rest[0] &= rest[0] - 1u;  // (0 stays 0)
+}
+
+// One round on a full sketch: resolves the window at p (loaded and marked), moves p on and loads and marks the next
+// one.  Lanes without a store write to a spare place instead of branching around it, and a window's look-ups by key
+// are made while the other warps order the slots: a branch costs the lone warp some 25 cycles.
+template <int CELLS, int E, bool TAB, bool HASH>
+__device__ __forceinline__ void round_window(const RoundRow &row, uint32_t &p, uint32_t end, int lane, Window<E> &w) {
+  using G = GroupMemory<CELLS>;
+  RoundState<CELLS> &st = G::state(row.base);
+  constexpr int M = 32 * CELLS, W = 32 * E;
+  static_assert(W <= RoundState<CELLS>::W, "a window takes entries of the order");
+  const uint32_t below = (1u << lane) - 1u;
+  bar_arrive<CELLS>(row.bars + BAR_STATE);
+  // while the other warps order the slots: what S0 says about the window
+  int q[E], absent_before[E], kept_before[E];
+  bool present[E], leader[E];
+  uint32_t absent[E], kept[E], same[E][E];
+  uint32_t one[E], all[E];  // weight with the first, with every Dice term of the key in the window
+#pragma unroll
+  for (int e = 0; e < E; ++e) q[e] = w.valid[e] ? slot_of<CELLS, TAB, HASH>(row, w.s[e]) : -1;
+  window_collect<CELLS, E, HASH>(row, p, lane, w, same);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    present[e] = q[e] >= 0;  // S0 holds the key
+    q[e] = present[e] ? q[e] : 0;
+    one[e] = st.w[q[e]];
+    leader[e] = w.valid[e] && (same[e][e] & below) == 0u && (e == 0 || same[e][0] == 0u);  // first element of its key
+    absent[e] = __ballot_sync(FULL, leader[e] && !present[e]);
+    kept[e] = __ballot_sync(FULL, leader[e] && present[e]);
   }
-  int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
-  L = L < 1 ? 1 : L;  // one element alone is always resolved exactly
-  const bool applies = lane < L && leader;
-  const int times = __popc(same & (L >= 32 ? FULL : (1u << L) - 1u));
-  float wv = miss ? __uint_as_float(nb) : __uint_as_float(hv);
-  for (int k = 1; k < times; ++k) wv += w.al;  // later elements of the key, in stream order
-  if (TAB && applies && miss) tab[old_key] = 0;
+  Window<E> nx;
+  window_load<CELLS, E>(row, p + W, end, lane, nx);
+  uint32_t rest[E][E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    absent_before[e] = count_before<E>(absent, e, below);
+    kept_before[e] = count_before<E>(kept, e, below);
+    one[e] = all[e] = __float_as_uint(__uint_as_float(one[e]) + w.al[e]);
+#pragma unroll
+    for (int f = 0; f < E; ++f) rest[e][f] = f == e ? same[e][f] & ~(below | 1u << lane) : f > e ? same[e][f] : 0u;
+    add_later<E>(rest[e], w.al[e], all[e]);
+  }
+  for (;;) {
+    bool later = false;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+#pragma unroll
+      for (int f = 0; f < E; ++f) later |= present[e] && rest[e][f];
+    if (!__any_sync(FULL, later)) break;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      add_later<E>(rest[e], w.al[e], all[e]);
+      add_later<E>(rest[e], w.al[e], all[e]);
+    }
+  }
+  bar_wait<CELLS>(row.bars + BAR_ORDER);
+  int rho[E];
+  uint2 mine[E];  // the entries of rank 32 e + lane
+#pragma unroll
+  for (int e = 0; e < E; ++e) rho[e] = st.rank[q[e]];
+#pragma unroll
+  for (int e = 0; e < E; ++e) mine[e] = st.order[e * 32 + lane];
+  bool open[E], gone[E], unsure[E], either = false;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    open[e] = leader[e] && present[e] && rho[e] < W;
+    gone[e] = open[e] && absent_before[e] > rho[e];
+    unsure[e] = open[e] && !gone[e] && absent_before[e] + kept_before[e] > rho[e];
+    either |= unsure[e];
+  }
+  if (__any_sync(FULL, either)) {  // count the open elements in front with lower places, one such element per word at a time
+    uint32_t left[E], any = 0u;
+#pragma unroll
+    for (int e = 0; e < E; ++e) any |= left[e] = __ballot_sync(FULL, unsure[e]);
+    while (any) {
+      int j[E], r[E], lower[E];
+      any = 0u;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        j[e] = 31 - __clz(static_cast<int>(left[e] | 1u));
+        r[e] = __shfl_sync(FULL, rho[e], j[e]);
+        lower[e] = 0;
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+#pragma unroll
+        for (int f = 0; f <= e; ++f) {
+          const uint32_t front = __ballot_sync(FULL, open[f] && rho[f] < r[e]);
+          lower[e] += __popc(f == e ? front & ((1u << j[e]) - 1u) : front);
+        }
+        if (lane == j[e]) gone[e] = open[e] && absent_before[e] + lower[e] > r[e];
+        left[e] &= ~(1u << j[e]);
+        any |= left[e];
+      }
+    }
+  }
+  // the elements that miss, and the entries that hits hold back
+  uint32_t missing[E], held[E], flipped = 0u;
+  bool miss[E];
+  int turn[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    uint32_t h = 0u;
+#pragma unroll
+    for (int f = 0; f < E; ++f) h |= open[f] && !gone[f] && (E == 1 || rho[f] >> 5 == e) ? 1u << (rho[f] & 31) : 0u;
+    held[e] = __reduce_or_sync(FULL, h);
+    const uint32_t f = __ballot_sync(FULL, gone[e]);
+    missing[e] = absent[e] | f;
+    flipped |= f;
+    miss[e] = (leader[e] && !present[e]) || gone[e];
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    st.takes[(held[e] >> lane) & 1u ? W : e * 32 + lane - count_before<E>(held, e, below)] = mine[e];
+#pragma unroll
+  for (int e = 0; e < E; ++e) turn[e] = flipped ? count_before<E>(missing, e, below) : absent_before[e];
+  __syncwarp();
+  uint2 take[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) take[e] = st.takes[miss[e] ? turn[e] : 0];
+  // the least weight that the window leaves in an entry: a miss whose entry is not below may have to
+  // take that one instead
+  uint32_t least = 0xFFFFFFFFu;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    one[e] = miss[e] ? __float_as_uint(__uint_as_float(take[e].x) + w.al[e]) : one[e];
+    least = miss[e] || open[e] ? min(least, one[e]) : least;
+  }
+  least = __reduce_min_sync(FULL, least);
+  int L = W;
+#pragma unroll
+  for (int e = E - 1; e >= 0; --e) {
+    const uint32_t again = __ballot_sync(FULL, miss[e] && take[e].x >= least);
+    L = again ? e * 32 + __ffs(static_cast<int>(again)) - 1 : L;
+  }
+  L = max(1, min(L, static_cast<int>(end - p)));  // one element alone is always resolved exactly
+  bool later = false;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    all[e] = miss[e] ? one[e] : all[e];
+#pragma unroll
+    for (int f = 0; f < E; ++f) {
+      rest[e][f] = miss[e] ? (f == e ? same[e][f] & ~(below | 1u << lane) : f > e ? same[e][f] : 0u) : 0u;
+      later |= rest[e][f] != 0u;
+    }
+  }
+  p += L;
+  if (L < W) {
+    window_load<CELLS, E>(row, p, end, lane, nx);
+    later = false;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      bool cut = false;
+      leader[e] = leader[e] && e * 32 + lane < L;
+#pragma unroll
+      for (int f = 0; f < E; ++f) {
+        const int l = L - 32 * f;
+        const uint32_t in = l >= 32 ? FULL : l <= 0 ? 0u : (1u << l) - 1u;
+        const uint32_t whole = f == e ? same[e][f] & ~(below | 1u << lane) : f > e ? same[e][f] : 0u;
+        cut |= (whole & ~in) != 0u;
+        rest[e][f] = whole & in;
+      }
+      all[e] = cut ? one[e] : all[e];
+#pragma unroll
+      for (int f = 0; f < E; ++f) {
+        rest[e][f] = leader[e] && (cut || miss[e]) ? rest[e][f] : 0u;
+        later |= rest[e][f] != 0u;
+      }
+    }
+  }
+  window_mark<CELLS, E, HASH>(row, lane, nx);
+  while (__any_sync(FULL, later)) {
+    later = false;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      add_later<E>(rest[e], w.al[e], all[e]);
+#pragma unroll
+      for (int f = 0; f < E; ++f) later |= rest[e][f] != 0u;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (TAB) heavy_dyn[row.base + (leader[e] && miss[e] ? G::tab_offset(HASH) + static_cast<int>(take[e].y >> 8) : G::SPARE)] = 0;
   // (a key taken by one miss may be put back by a later one, which then is a flipped lane:
   // clear first, then set)
-  if (flipped) __syncwarp();
-  if (applies && miss) {
-    st.key[tgt] = w.s;
-    st.w[tgt] = __float_as_uint(wv);
-    if (TAB) tab[w.s] = static_cast<uint8_t>(tgt + 1);
-  }
-  if (applies && !miss) st.w[q] = __float_as_uint(wv);
   __syncwarp();
-  return L;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const bool put = leader[e] && miss[e];
+    const int slot = static_cast<int>(take[e].y & 255u);
+    st.key[put ? slot : M] = w.s[e];
+    if (TAB) heavy_dyn[row.base + (put ? G::tab_offset(HASH) + w.s[e] : G::SPARE)] = static_cast<uint8_t>(slot + 1);
+    st.w[leader[e] ? (miss[e] ? slot : q[e]) : M] = all[e];
+  }
+  __syncwarp();
+  w = nx;
 }
 
 // One round while the sketch has empty slots; `filled` is updated.  (No order needed.)
-template <int CELLS, bool TAB>
-__device__ __forceinline__ int round_fill(const RoundRow &row, int buf, int p, int cnt, int lane, int &filled) {
+template <int CELLS, bool TAB, bool HASH>
+__device__ __forceinline__ int round_fill(const RoundRow &row, uint32_t p, uint32_t end, int lane, int &filled) {
   RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
-  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
+  uint8_t *const tab = GroupMemory<CELLS>::template tab<HASH>(row.base);
   constexpr int M = 32 * CELLS;
   const uint32_t below = (1u << lane) - 1u;
-  const Window<CELLS> w = look_up<CELLS, TAB>(row, buf, p, cnt, lane);
-  const bool miss = w.valid && w.q < 0, hit = w.valid && w.q >= 0;
+  Window<1> w;
+  window_load<CELLS, 1>(row, p, end, lane, w);
+  window_mark<CELLS, 1, HASH>(row, lane, w);
+  __syncwarp();
+  uint32_t mates[1][1];
+  window_collect<CELLS, 1, HASH>(row, p, lane, w, mates);
+  const int q = w.valid[0] ? slot_of<CELLS, TAB, HASH>(row, w.s[0]) : -1;
+  const bool miss = w.valid[0] && q < 0, hit = w.valid[0] && q >= 0;
   const uint32_t missing = __ballot_sync(FULL, miss);
   const int mrank = __popc(missing & below);
-  const unsigned same = same_key<CELLS>(row, w, lane);
-  int lim = w.valid ? 32 : lane;
+  const unsigned same = mates[0][0];
+  int lim = w.valid[0] ? 32 : lane;
   if (miss && ((same & below) || mrank >= M - filled)) lim = lane;
   const int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
   const unsigned prefix = L >= 32 ? FULL : (1u << L) - 1u;
@@ -1684,13 +1785,13 @@ __device__ __forceinline__ int round_fill(const RoundRow &row, int buf, int p, i
     if (miss) {
       const int j = filled + mrank;  // j-th slot to be filled: lane j / CELLS, cell j % CELLS
       const int code = (j % CELLS) * 32 + j / CELLS;
-      st.key[code] = w.s;
-      st.w[code] = __float_as_uint(w.al);
-      if (TAB) tab[w.s] = static_cast<uint8_t>(code + 1);
+      st.key[code] = w.s[0];
+      st.w[code] = __float_as_uint(w.al[0]);
+      if (TAB) tab[w.s[0]] = static_cast<uint8_t>(code + 1);
     } else if (hit && ((same & prefix) & below) == 0u) {
-      float wv = __uint_as_float(st.w[w.q]);
-      for (int t = __popc(same & prefix); t > 0; --t) wv += w.al;
-      st.w[w.q] = __float_as_uint(wv);
+      float wv = __uint_as_float(st.w[q]);
+      for (int t = __popc(same & prefix); t > 0; --t) wv += w.al[0];
+      st.w[q] = __float_as_uint(wv);
     }
   }
   filled += __popc(missing & prefix);
@@ -1707,34 +1808,67 @@ __device__ __forceinline__ void stage_batch(int2 *ring, const int2 *in, int cnt,
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Rounds of one kind on [p, cnt) of a batch, at most `left` of them; returns where they got to
-// and how many are left.  Functions of their own:
-// compiled into one body each kind loses speed to the other's registers and schedule.
-template <int CELLS, bool TAB>
-__device__ __noinline__ int2 window_rounds(const RoundRow row, int buf, int p, int cnt, int left) {
-  const int lane = lane_id();
-  while (p < cnt && left > 0) {
-    p += round_window<CELLS, TAB>(row, buf, p, cnt, lane);
-    --left;
-  }
-  return make_int2(p, left);
+// copies the H_SEG stream elements from `from` on (those in front of `total`) into the ring without passing
+// through registers
+__device__ __forceinline__ void stage_segment(int2 *ring, const int2 *in, uint32_t from, uint32_t total, int lane) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ring + (from & (H_RING - 1)))) + lane * 8;
+  const int2 *src = in + from + lane;
+  const int left = static_cast<int>(min(total - min(from, total), static_cast<uint32_t>(H_SEG))) - lane;
+#pragma unroll
+  for (int i = 0; i < H_SEG / 32; ++i)
+    if (i * 32 < left)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + i * 256), "l"(src + i * 32) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
 }
-template <int CELLS, bool TAB>
-__device__ __noinline__ int2 strict_rounds(const RoundRow row, int buf, int p, int cnt, int left) {
+
+// where a row's stream has got to: [p, ...), elements in front of `seg` + 2 H_SEG are in the ring or on their way
+struct RowStream {
+  const int2 *in;
+  uint32_t total, p, seg;
+};
+
+// Windows that start in a segment may reach into the next, so that one has to be here; the one behind it is
+// on its way meanwhile.
+__device__ __forceinline__ void next_segment(int2 *ring, RowStream &s, int lane) {
+  stage_segment(ring, s.in, s.seg + 2 * H_SEG, s.total, lane);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncwarp();
+}
+
+// At most `left` rounds of one width.  Functions of their own:
+// compiled into one body each kind loses speed to the other's registers and schedule.
+template <int CELLS, int E, bool TAB, bool HASH>
+__device__ __noinline__ uint2 window_rounds(const RoundRow row, RowStream s, int left) {
+  int2 *const ring = GroupMemory<CELLS>::ring(row.base);
   const int lane = lane_id();
-  while (p < cnt && left > 0) {
-    p += round_strict<CELLS, TAB>(row, buf, p, cnt, lane);
+  uint32_t end = min(s.total, s.seg + 2 * H_SEG);
+  Window<E> w;
+  window_load<CELLS, E>(row, s.p, end, lane, w);
+  window_mark<CELLS, E, HASH>(row, lane, w);
+  __syncwarp();
+  while (s.p < s.total && left > 0) {
+    if (s.p >= s.seg + H_SEG) {
+      s.seg += H_SEG;
+      next_segment(ring, s, lane);
+      end = min(s.total, s.seg + 2 * H_SEG);
+    }
+    round_window<CELLS, E, TAB, HASH>(row, s.p, end, lane, w);
     --left;
   }
-  return make_int2(p, left);
+  {  // the marks of the window that does not come here
+    uint32_t same[E][E];
+    window_collect<CELLS, E, HASH>(row, s.p, lane, w, same);
+    __syncwarp();
+  }
+  return make_uint2(s.p, s.seg);
 }
 
 // One heavy row, start to finish, by the first warp: stream batches in, rounds, final sketch out.
-template <int CELLS, bool TAB>
+template <int CELLS, bool TAB, bool HASH>
 __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, const RoundRow row, int32_t *out) {
   RoundState<CELLS> &st = GroupMemory<CELLS>::state(row.base);
-  uint8_t *const tab = GroupMemory<CELLS>::tab(row.base);
-  int2 *const ring0 = GroupMemory<CELLS>::ring(row.base, 0), *const ring1 = GroupMemory<CELLS>::ring(row.base, 1);
+  uint8_t *const tab = GroupMemory<CELLS>::template tab<HASH>(row.base);
+  int2 *const ring = GroupMemory<CELLS>::ring(row.base);
   constexpr int M = 32 * CELLS;
   const int lane = lane_id();
 #pragma unroll
@@ -1742,65 +1876,50 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, const Ro
     st.key[c * 32 + lane] = -1;
     st.w[c * 32 + lane] = 0u;
   }
-  int filled = 0, buf = 0;
-  // (see the loop below) kind of round in use (0 window, 1 strict), rounds left in the stretch,
-  // the trial being booked (-1 none), and what the trials resolved in how many cycles
-  int mode = 0, left = TRIAL_ROUNDS, trial = 0;
-  long long got[2] = {0, 0}, took[2] = {0, 0};
-  int streak = 0, last_mode = -1;
+  int filled = 0;
   __syncwarp();
-  stage_batch(ring0, in, static_cast<int>(total < H_RING ? total : H_RING), lane);
-  for (uint32_t base = 0; base < total; base += H_RING) {
-    const int cnt = static_cast<int>(total - base < H_RING ? total - base : H_RING);
-    const uint32_t next = base + H_RING;
-    if (next < total)
-      stage_batch(buf ? ring0 : ring1, in + next, static_cast<int>(total - next < H_RING ? total - next : H_RING), lane);
-    else
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest group: this batch is in
-    __syncwarp();
-    int p = 0;
-    while (p < cnt && filled < M) p += round_fill<CELLS, TAB>(row, buf, p, cnt, lane, filled);
-    // Which kind of round is faster depends on the row: a whole-window round costs more and
-    // pays where it resolves (nearly) the whole window - rows whose own length dominates their
-    // Dice terms.  Where the terms vary widely, entries put back light are taken again at
-    // once, either kind ends after a few elements and the cheaper one wins; and how often a
-    // strict round is cut short depends on the sketch size.  So the row measures: a few
-    // rounds of each kind against the clock, then a long stretch of the kind that resolved
-    // more elements per cycle, and again.
-    while (p < cnt) {
-      const int before = p;
-      const long long t0 = clock64();
-      const int2 at = mode == 0 ? window_rounds<CELLS, TAB>(row, buf, p, cnt, left)
-                                : strict_rounds<CELLS, TAB>(row, buf, p, cnt, left);
-      p = at.x;
-      left = at.y;
-      if (trial >= 0) {  // a trial stretch: book it
-        got[trial] += p - before;
-        took[trial] += clock64() - t0;
-      }
-      if (left == 0) {
-        if (trial == 0) {  // window tried: now the strict kind
-          trial = 1;
-          mode = 1;
-          left = TRIAL_ROUNDS;
-        } else if (trial == 1) {  // both tried: elements per cycle, compared without dividing
-          mode = got[0] * took[1] >= got[1] * took[0] ? 0 : 1;
-          // the stretch grows while the same kind keeps winning (up to 16 times as long)
-          streak = mode == last_mode ? (streak < 4 ? streak + 1 : 4) : 0;
-          last_mode = mode;
-          trial = -1;
-          left = COMMIT_ROUNDS << streak;
-        } else {  // a committed stretch is over: measure again
-          trial = 0;
-          mode = 0;
-          left = TRIAL_ROUNDS;
-          got[0] = got[1] = 0;
-          took[0] = took[1] = 0;
-        }
-      }
+  RowStream s = {in, total, 0u, 0u};
+  stage_segment(ring, in, 0, total, lane);
+  stage_segment(ring, in, H_SEG, total, lane);
+  next_segment(ring, s, lane);
+  while (s.p < total && filled < M) {
+    if (s.p >= s.seg + H_SEG) {
+      s.seg += H_SEG;
+      next_segment(ring, s, lane);
     }
-    buf ^= 1;
+    s.p += round_fill<CELLS, TAB, HASH>(row, s.p, min(total, s.seg + 2 * H_SEG), lane, filled);
+  }
+  // Which width is faster depends on the row: windows of 64 cost more and pay where most of them are resolved
+  // whole - rows whose own length dominates their Dice terms.  Where the terms vary widely, entries put back light
+  // are taken again soon and either width ends after the same few elements.  So the row measures: a few rounds of
+  // each width against the clock, then a long stretch of the one that resolved more elements per cycle, and again.
+  int wide = 1, left = TRIAL_ROUNDS, trial = 1;  // width in use, rounds of the stretch, width on trial (-1 none)
+  long long got[2] = {0, 0}, took[2] = {0, 0};
+  int streak = 0, last = -1;
+  while (s.p < total) {
+    const uint32_t from = s.p;
+    const long long t0 = clock64();
+    const uint2 at = wide ? window_rounds<CELLS, 2, TAB, HASH>(row, s, left) : window_rounds<CELLS, 1, TAB, HASH>(row, s, left);
+    s.p = at.x;
+    s.seg = at.y;
+    if (trial >= 0) {
+      got[trial] = s.p - from;
+      took[trial] = clock64() - t0;
+    }
+    if (trial == 1) {  // wide windows tried: now the others
+      trial = wide = 0;
+      left = TRIAL_ROUNDS;
+    } else if (trial == 0) {  // both tried: elements per cycle, compared without dividing
+      wide = got[1] * took[0] >= got[0] * took[1] ? 1 : 0;
+      // the stretch grows while the same width keeps winning (up to 16 times as long)
+      streak = wide == last ? (streak < 4 ? streak + 1 : 4) : 0;
+      last = wide;
+      trial = -1;
+      left = COMMIT_ROUNDS << streak;
+    } else {  // a stretch is over: measure again
+      trial = wide = 1;
+      left = TRIAL_ROUNDS;
+    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -1822,14 +1941,14 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
   constexpr int THREADS = Helpers<CELLS>::THREADS;
   using G = GroupMemory<CELLS>;
   const int group = threadIdx.x / THREADS, in_group = threadIdx.x % THREADS;
-  const int base = group * (G::TAB + tab_bytes);
+  const int32_t span = a.chunk < a.n ? a.chunk : a.n;
+  const int base = group * (G::tab_offset(span > MATES) + tab_bytes);
   RoundState<CELLS> &st = G::state(base);
   const int lane = lane_id(), warp = in_group >> 5, bars = 3 * group;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
-  for (int i = in_group * 16; i < MATES * 4 + tab_bytes; i += THREADS * 16)
-    *reinterpret_cast<uint4 *>(heavy_dyn + base + G::MATE + i) = make_uint4(0, 0, 0, 0);
-  const int32_t span = a.chunk < a.n ? a.chunk : a.n;
+  for (int i = G::MATE + in_group * 16; i < G::tab_offset(span > MATES) + tab_bytes; i += THREADS * 16)
+    *reinterpret_cast<uint4 *>(heavy_dyn + base + i) = make_uint4(0, 0, 0, 0);
   for (;;) {
     if (in_group == 0) {
       st.item = atomicAdd(&a.ctrl[CTRL_HEAVY_TICKET + 1], 1u);
@@ -1846,18 +1965,20 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
     if (warp > 0) {
       for (;;) {
         bar_wait<CELLS>(bars + BAR_STATE);
-        if (*static_cast<volatile int32_t *>(&st.row_done)) break;
-        rank_slots<CELLS>(base, warp - 1, lane);
+        if (!rank_slots<CELLS>(base, warp - 1, lane)) break;
         bar_arrive<CELLS>(bars + BAR_ORDER);
       }
     } else {
       if (ok) {
-        const RoundRow row = {base, (r / a.chunk) * a.chunk, span > MATES, a.ctrl, span, bars};
+        const RoundRow row = {base, (r / a.chunk) * a.chunk, a.ctrl, span, bars};
         int32_t *out = a.heavy_state + static_cast<size_t>(item) * (2 * CELLS * 32);
-        if (tab_bytes > 0)
-          rounds_row<CELLS, true>(a.hstream + a.heavy_off[item], a.row_work[r], row, out);
+        const int2 *in = a.hstream + a.heavy_off[item];
+        if (tab_bytes > 0 && span <= MATES)
+          rounds_row<CELLS, true, false>(in, a.row_work[r], row, out);
+        else if (tab_bytes > 0)
+          rounds_row<CELLS, true, true>(in, a.row_work[r], row, out);
         else
-          rounds_row<CELLS, false>(a.hstream + a.heavy_off[item], a.row_work[r], row, out);
+          rounds_row<CELLS, false, true>(in, a.row_work[r], row, out);
       }
       if (lane == 0) st.row_done = 1;
       __syncwarp();
@@ -1869,7 +1990,7 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
 
 // ---- 32 slots ------------------------------------------------------------------------------
 // A warp per row: a lane orders its own slot while the look-ups of the window are under way, in
-// fewer cycles than a group's barriers take.  Strict rounds only.  Longest row of R-MAT scale 16
+// fewer cycles than a group's barriers take.  Longest row of R-MAT scale 16
 // (101,366 candidates): 9.9 ms by a group of three warps, 7.7 this way, 145 cycles per candidate;
 // bound by the dependent steps of a round, as the larger sketches are.  Rows are drawn as warps ask,
 // so that the longest share an SM: spread one to an SM (the others empty), the same rounds took 10.9 ms of a
@@ -1914,7 +2035,9 @@ __device__ __forceinline__ int slot_32(const State32 &st, const uint8_t *tab, in
   return q;
 }
 
-// round_strict and round_fill on 32 slots (the slot code is the lane)
+// One round on a full sketch of 32 slots (the slot code is the lane): the longest prefix of the window for which
+// (1) no two of its misses carry the same key, (2) no hit lands on an entry that a miss of the prefix takes, and
+// (3) every entry put back stays above the last one taken - then the i-th miss takes the i-th entry of the order.
 template <bool TAB>
 __device__ __forceinline__ int strict_32(State32 &st, uint8_t *tab, int32_t cbase, int32_t span, uint32_t *ctrl,
                                          const int2 *ring, int p, int cnt, int lane, uint32_t &sink) {
@@ -2151,7 +2274,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       const int64_t span = a.chunk < a.n ? a.chunk : a.n;
       const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
       // (groups per block: as many as their tables leave room for)
-      const int group_bytes = GroupMemory<CELLS>::TAB + tab_bytes;
+      const int group_bytes = GroupMemory<CELLS>::tab_offset(span > MATES) + tab_bytes;
       const int room = ctx.smem_optin - 1024;
       int groups = Helpers<CELLS>::ROWS;
       while (groups > 1 && groups * group_bytes > room) --groups;

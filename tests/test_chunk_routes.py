@@ -1,5 +1,5 @@
-"""Chunks of more than 1,024 rows and sketches of 32 slots take kernels of their own: bit-exact
-tables and orders against the CPU oracle at the sizes where they change hands."""
+"""Chunks of more than 1,024 rows, sketches of 32 slots and the longest rows of a call take kernels of their own:
+bit-exact tables and orders against the CPU oracle at the sizes where they change hands."""
 import numpy as np
 import pytest
 
@@ -82,3 +82,32 @@ def test_rows_by_warp_before_the_lanes(chunk, skew, k):
     rows = [list((n * rng.random(c) ** skew).astype(np.int64)) for c in 1 + rng.geometric(0.2, n) % 60]
     ptr, ind = _csr(rows, n)
     _check(ptr, ind, limits=(0, 3000), k=k, chunk_size=chunk)
+
+
+@pytest.mark.parametrize("spread", [0, 30])
+@pytest.mark.parametrize("k", [16, 24, 32])
+@pytest.mark.parametrize("chunk", [1024, 1025, 66_000])
+def test_windows_of_the_chains(chunk, k, spread):
+    # 64, 96 and 128 slots; keys found by a word each, by hashed words, and without a table of slots.  Streams that end
+    # at the edges of a window (32, 64), a staged segment (256) and the ring (1,024); columns of 40 rows drawn from few
+    # (most candidates hit) and many; Dice terms all but equal (whole windows) and of rows with 1 to 30 more entries
+    rng = np.random.default_rng(chunk + k + spread)
+    lengths = [e + d for e in (32, 64, 256, 512, 768, 1024, 1280, 2048) for d in (-1, 0, 1, 33)] + [6000, 9001]
+    rows = [[] for _ in range(chunk)]
+    col = 0
+    for i, length in enumerate(lengths):
+        left = length
+        while left > 0:
+            take = min(left, 40)
+            pool = 150 if i % 2 else chunk - 100
+            for r in 100 + rng.choice(pool, take, replace=False):
+                rows[r].append(col)
+            rows[i].append(col)
+            left -= take
+            col += 1
+    for r in range(100, chunk):  # (columns of its own: they bring no candidates)
+        extra = rng.integers(0, spread + 1)
+        rows[r] += range(col, col + extra)
+        col += extra
+    ptr, ind = _csr(rows, max(col, chunk))
+    _check(ptr, ind, k=k, chunk_size=chunk)
