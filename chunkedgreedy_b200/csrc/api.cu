@@ -111,11 +111,10 @@ size_t greedy_bitmap_words(int32_t n, int32_t chunk) {
   return chunks * 2 * words;
 }
 
-constexpr uint64_t STREAM_CAP_MAX = uint64_t(1) << 27;  // 2^27 elements = 1 GiB
 constexpr int32_t AHEAD_MIN_NNZ = 1 << 24;  // smaller calls do not pay for a second pipeline's launches
 
 // Stream elements the buffer of the heaviest rows gets for this call: never more than the
-// rows could stream at all (nnz * chunk span), than 1 GiB or than the caller's limit; at
+// rows could stream at all (nnz * chunk span), than 2 GiB or than the caller's limit; at
 // least what the largest earlier call of the context asked for, and for a first call eight
 // elements per nonzero (at least 2^20: 8 MiB).
 uint64_t stream_capacity(const Context &ctx, size_t nnz, size_t span) {
@@ -161,7 +160,8 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   // streams of the heaviest rows
   const size_t span = static_cast<size_t>(p.chunk < n ? p.chunk : n);
   const size_t cap = transpose_only ? 1 : static_cast<size_t>(stream_capacity(ctx, z, span));
-  const size_t hmax = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
+  size_t hmax = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
+  if (hmax > static_cast<size_t>(n)) hmax = static_cast<size_t>(n);
   const size_t o_hs = ar.take(8 * cap), o_ho = ar.take(4 * (hmax + 1));
   const size_t o_hst = ar.take(4 * hmax * 2 * (p.M / 32) * 32);
   const size_t pmax = transpose_only ? 1 : z / SKETCH_PART_COLS + hmax + 1;  // column slices of the heavy rows
@@ -213,6 +213,7 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   s->part_off = reinterpret_cast<uint32_t *>(ctx.ws + o_po);
   s->stream_cap = static_cast<uint32_t>(cap);
   s->heavy_max = static_cast<uint32_t>(hmax);
+  s->slots = p.M;
   s->heavy_chunk = reinterpret_cast<int32_t *>(ctx.ws + o_hc);
   s->heavy_tile_base = reinterpret_cast<int32_t *>(ctx.ws + o_htb);
   s->tile_hist = reinterpret_cast<uint32_t *>(ctx.ws + o_th);

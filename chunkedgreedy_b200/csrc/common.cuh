@@ -115,6 +115,7 @@ struct CsgScratch {
   uint32_t *heavy_off;
   int32_t *heavy_state;
   uint32_t stream_cap, heavy_max;
+  int32_t slots;  // of a row's sketch
   uint32_t *part_base, *part_off;
   bool no_heavy_rows = false;  // known on the host already: nothing for the chain kernel
   // compact_kernel's second list, tiled sort of heavy chunks (see transpose.cu)
@@ -141,10 +142,11 @@ enum {
   CTRL_PRIO = 50,          // chunk whose heavy rows run ahead of the rest (PRIO_NONE: no such chunk)
   CTRL_PRIO_WORK = 51,     // shortest candidate stream among the rows the chunk ahead lists
   CTRL_STATS = 56,         // see greedy.cu (8-byte aligned)
-  CTRL_BUCKET_COUNT = 128,  // WORK_BUCKETS entries each
-  CTRL_BUCKET_BASE = 256,
-  CTRL_BUCKET_FILL = 384,
-  CTRL_WORDS = 512
+  CTRL_BUCKET_COUNT = 128,  // WORK_BUCKETS entries each: rows,
+  CTRL_BUCKET_WORK = 256,   // their candidates (64-bit),
+  CTRL_BUCKET_BASE = 512,   // first place in the list, places taken
+  CTRL_BUCKET_FILL = 640,
+  CTRL_WORDS = 768
 };
 
 // Rows are listed by the length of their candidate stream, in quarter octaves (bucket 4 e + f
@@ -158,12 +160,14 @@ enum CallPhase { PHASE_ALL = 0, PHASE_PRIO = 1, PHASE_REST = 2 };
 // SMs the chains of the chunk ahead may hold (the other chains get the remaining ones)
 inline int prio_chain_blocks(int num_sms) { return num_sms / 4 > 0 ? num_sms / 4 : 1; }
 
+constexpr uint64_t STREAM_CAP_MAX = uint64_t(1) << 28;  // largest stream buffer: 2^28 elements = 2 GiB
 constexpr int SKETCH_PART_COLS = 128;   // columns of a heavy row whose stream one warp writes out
-// Rows that stream at least HEAVY_WORK candidates are "heavy": a warp of the chain kernel each.
-// Shorter rows join them, longest first, while the list of heavy rows stays within CHAIN_ROWS
-// and the stream has at least CHAIN_WORK_MIN elements (bucket_scan_kernel).
+// Rows that stream at least HEAVY_WORK candidates are "heavy": a group of warps of the chain kernel each.
+// Shorter rows of CHAIN_WORK_MIN candidates or more join them, longest first, up to CHAIN_ROWS rows: as many as the
+// times of ChainCosts say (bucket_scan_kernel), in sketches without such times while there are FEW_CHAIN_ROWS.
 constexpr uint32_t HEAVY_WORK = 1u << 16;
-constexpr uint32_t CHAIN_ROWS = 296;
+constexpr uint32_t CHAIN_ROWS = 4096;
+constexpr uint32_t FEW_CHAIN_ROWS = 296;
 constexpr uint32_t CHAIN_WORK_MIN = 64;
 constexpr int32_t LANE_TABLE_ROWS = 1024;  // largest chunk whose keys the row-per-lane kernel finds in a byte table
 // Larger chunks: rows of at least this many candidates and in the longest octaves go to a warp each, more octaves
@@ -273,6 +277,11 @@ __device__ __forceinline__ unsigned match_digit(uint32_t d) {
 __device__ __forceinline__ int work_bucket(uint32_t t) {
   const int e = 31 - __clz(t);
   return 4 * e + static_cast<int>((e >= 2 ? t >> (e - 2) : t << (2 - e)) & 3u);
+}
+
+// least length that falls into bucket b (from 8 candidates on)
+__device__ __forceinline__ float bucket_floor(int b) {
+  return static_cast<float>(1ull << (b >> 2)) * (1.0f + 0.25f * static_cast<float>(b & 3));
 }
 
 // packed entry of the top-k table; wire format of the reference

@@ -61,7 +61,7 @@ struct SketchArgs {
   int32_t *heavy_state;
   uint32_t stream_cap, heavy_max;
   uint32_t *part_base;  // first part of each heavy row, plus the total
-  uint32_t *part_off;   // per part: entries it produces, then its offset in hstream
+  uint32_t *part_off;   // per part: entries it produces
 };
 
 // The sketch of one row: CELLS slots per lane, all in registers.  Slot (lane, cell) is
@@ -1038,7 +1038,7 @@ __global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchAr
 // ---- heavy rows through materialised streams ------------------------------------------
 // part -> (heavy row, column range).  Uniform over the warp.
 struct PartRef {
-  uint32_t item;
+  uint32_t item, first;  // heavy row, and its first part
   int32_t r, pb, pe, row_size;
 };
 __device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, uint32_t heavy) {
@@ -1052,68 +1052,21 @@ __device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, 
   }
   PartRef p;
   p.item = lo;
+  p.first = a.part_base[lo];
   p.r = a.row_list[lo];
   const int32_t rb = a.row_seg[p.r], re = rb + a.row_cols[p.r];
   p.row_size = a.ptr[p.r + 1] - a.ptr[p.r];
-  p.pb = rb + static_cast<int32_t>(part - a.part_base[lo]) * H_PART;
+  p.pb = rb + static_cast<int32_t>(part - p.first) * H_PART;
   p.pe = p.pb + H_PART < re ? p.pb + H_PART : re;
   return p;
 }
 
-// stream entries a part (H_PART columns of a heavy row) will produce; one warp
-__device__ __forceinline__ void count_part(const SketchArgs &a, uint32_t part, uint32_t heavy) {
-  const int lane = lane_id();
-  const PartRef p = part_ref(a, part, heavy);
-  uint32_t cnt = 0;
-  for (int32_t q = p.pb + lane; q < p.pe; q += 32) {
-    const int32_t len = a.seg[q].y;
-    cnt += len >= 2 ? static_cast<uint32_t>(len - 1) : 0u;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) cnt += __shfl_down_sync(FULL, cnt, off);
-  if (lane == 0) a.part_off[part] = cnt;
-}
-
-// counts -> offsets (exclusive scan in place, one block of 1024)
-__device__ __forceinline__ void scan_parts(const SketchArgs &a, uint32_t parts) {
-  __shared__ uint32_t sm[32];
-  __shared__ uint32_t carry_s;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < parts; base += 1024) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < parts ? a.part_off[i] : 0u;
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (lane == 31) sm[warp] = incl;
-    __syncthreads();
-    uint32_t wbase = 0, tot = 0;
-    for (int w = 0; w < 32; ++w) {
-      const uint32_t t = sm[w];
-      if (w < warp) wbase += t;
-      tot += t;
-    }
-    const uint32_t carry = carry_s;
-    if (i < parts) a.part_off[i] = carry + wbase + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + tot;
-    __syncthreads();
-  }
-}
-
-// Offsets of the heavy rows' streams in hstream; trims the heavy set to what fits.  with_parts:
-// the parts' offsets as well, which kernels of their own do in calls with many.
-__global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a, int with_parts) {
+// Offsets of the heavy rows' streams in hstream; trims the heavy set to what fits.
+__global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
   __shared__ unsigned long long sm[32];
   __shared__ unsigned long long carry_s;
   __shared__ uint32_t count_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long lighter = 0;  // stream elements of the rows below HEAVY_WORK (the others are counted already)
   uint32_t H = a.ctrl[CTRL_HEAVY_ROWS];
   if (H > a.heavy_max) H = a.heavy_max;
   if (threadIdx.x == 0) {
@@ -1128,7 +1081,6 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a, int w
       const int32_t r = a.row_list[i];
       v = a.row_work[r];
       np = static_cast<uint32_t>((a.row_cols[r] + H_PART - 1) / H_PART);
-      if (v < HEAVY_WORK) lighter += v;
     }
     // parts first (same scan, second value packed in the high half of 64 bits)
     unsigned long long pk = (static_cast<unsigned long long>(np) << 43) | v;  // sums: < 2^21 parts, < 2^43 entries
@@ -1160,10 +1112,6 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a, int w
     if (threadIdx.x == 0) carry_s = carry + tot;
     __syncthreads();
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) lighter += __shfl_down_sync(FULL, lighter, off);
-  if (lane == 0 && lighter)
-    atomicAdd(reinterpret_cast<unsigned long long *>(a.ctrl + CTRL_HEAVY_NEED), lighter);
   if (threadIdx.x == 0) {
     const uint32_t Hc = count_s;
     // parts of the rows that stay heavy: part_base[Hc] closes the table
@@ -1176,22 +1124,26 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a, int w
     a.ctrl[CTRL_HEAVY_TICKET] = 0;
     a.ctrl[CTRL_HEAVY_TICKET + 1] = 0;
   }
-  if (!with_parts) return;
-  __syncthreads();
-  const uint32_t heavy = count_s, parts = a.ctrl[CTRL_HEAVY_PARTS];
-  for (uint32_t part = warp; part < parts; part += 32) count_part(a, part, heavy);
-  __syncthreads();
-  scan_parts(a, parts);
 }
 
+// stream entries each part (H_PART columns of a heavy row) will produce; one warp per part.  Whoever expands a part
+// adds up the parts of the row in front of it: one block that scanned all counts took 18 us of a call of
+// 360 (65,536 rows, some 300 parts) and 48 of one of 28 ms, the parts' own sums nothing that shows.
 __global__ void __launch_bounds__(256) heavy_part_count_kernel(SketchArgs a) {
+  const int lane = lane_id();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS], parts = a.ctrl[CTRL_HEAVY_PARTS];
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; part < parts; part += warps)
-    count_part(a, part, heavy);
+  for (uint32_t part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; part < parts; part += warps) {
+    const PartRef p = part_ref(a, part, heavy);
+    uint32_t cnt = 0;
+    for (int32_t q = p.pb + lane; q < p.pe; q += 32) {
+      const int32_t len = a.seg[q].y;
+      cnt += len >= 2 ? static_cast<uint32_t>(len - 1) : 0u;
+    }
+    cnt = __reduce_add_sync(FULL, cnt);
+    if (lane == 0) a.part_off[part] = cnt;
+  }
 }
-
-__global__ void __launch_bounds__(1024) heavy_part_scan_kernel(SketchArgs a) { scan_parts(a, a.ctrl[CTRL_HEAVY_PARTS]); }
 
 // one warp per part: its slice of the row's stream, written out in order
 __global__ void __launch_bounds__(S_THREADS) heavy_expand_kernel(SketchArgs a) {
@@ -1210,7 +1162,9 @@ __global__ void __launch_bounds__(S_THREADS) heavy_expand_kernel(SketchArgs a) {
     const PartRef p = part_ref(a, part, heavy);
     if (p.pe <= p.pb) continue;
     if (!index_ok(a.ctrl, CHK_LIST, p.r, a.n)) continue;
-    uint32_t at = a.part_off[part];
+    uint32_t before = 0;
+    for (uint32_t q = p.first + lane; q < part; q += 32) before += a.part_off[q];
+    uint32_t at = a.heavy_off[p.item] + __reduce_add_sync(FULL, before);
     int2 *out = a.hstream + at;
     prod.begin(p.r, p.pb, p.pe, p.row_size);
     for (;;) {
@@ -2241,17 +2195,10 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
   constexpr bool in_rounds = CELLS >= WINDOW_CELLS && CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
-    // (up to a million nonzeros there are a few thousand parts at most, less than a launch's worth)
-    const bool one_kernel = a.nnz <= 1 << 20;
-    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a, one_kernel ? 1 : 0);
+    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
-    if (!one_kernel) {
-      heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
-      CSG_CUDA(cudaGetLastError());
-      heavy_part_scan_kernel<<<1, 1024, 0, st>>>(a);
-      CSG_CUDA(cudaGetLastError());
-      count_launches(2);
-    }
+    heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
+    CSG_CUDA(cudaGetLastError());
     heavy_expand_kernel<<<ctx.num_sms * 8, S_THREADS, 0, st>>>(a);
     CSG_CUDA(cudaGetLastError());
     // (the rest of the call starts its own chains only behind this point: by then the chains
@@ -2341,7 +2288,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   if (no_heavy_rows) return true;
   heavy_topk_kernel<CELLS><<<ctx.num_sms, S_THREADS, 0, st>>>(a);
   CSG_CUDA(cudaGetLastError());
-  count_launches(4);
+  count_launches(5);
   return true;
 }
 

@@ -738,13 +738,15 @@ __device__ __forceinline__ bool taken_ahead(uint32_t prio, uint32_t least, int32
   return prio != PRIO_NONE && work >= least && static_cast<uint32_t>(r / chunk) == prio;
 }
 
-// rows per bucket of row_work
+// rows and candidates per bucket of row_work
 __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint32_t *row_work,
                                                            uint32_t *ctrl, int32_t chunk, const uint32_t *ctrl_ahead) {
   __shared__ uint32_t bucket[WORK_BUCKETS];
-  __shared__ unsigned long long need;
-  if (threadIdx.x < WORK_BUCKETS) bucket[threadIdx.x] = 0;
-  if (threadIdx.x == 0) need = 0;
+  __shared__ unsigned long long work[WORK_BUCKETS];  // (of rows that may get a chain)
+  if (threadIdx.x < WORK_BUCKETS) {
+    bucket[threadIdx.x] = 0;
+    work[threadIdx.x] = 0;
+  }
   __syncthreads();
   const uint32_t prio = ctrl_ahead ? ctrl_ahead[CTRL_PRIO] : PRIO_NONE;
   const uint32_t least = ctrl_ahead ? ctrl_ahead[CTRL_PRIO_WORK] : 0u;
@@ -752,34 +754,59 @@ __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint
     uint32_t t = __ldcg(row_work + r);
     if (taken_ahead(prio, least, chunk, r, t)) t = 0;
     if (t) atomicAdd(&bucket[work_bucket(t)], 1u);
-    // stream elements of the rows heavy enough for a materialised stream: what the stream
-    // buffer would have to hold for all of them (the host sizes the next call's buffer by it)
-    if (t >= HEAVY_WORK) atomicAdd(&need, static_cast<unsigned long long>(t));
+    if (t >= CHAIN_WORK_MIN) atomicAdd(&work[work_bucket(t)], static_cast<unsigned long long>(t));
   }
   __syncthreads();
-  if (threadIdx.x < WORK_BUCKETS && bucket[threadIdx.x])
+  if (threadIdx.x < WORK_BUCKETS && bucket[threadIdx.x]) {
     atomicAdd(&ctrl[CTRL_BUCKET_COUNT + threadIdx.x], bucket[threadIdx.x]);
-  if (threadIdx.x == 0 && need)
-    atomicAdd(reinterpret_cast<unsigned long long *>(ctrl + CTRL_HEAVY_NEED), need);
+    if (work[threadIdx.x])
+      atomicAdd(reinterpret_cast<unsigned long long *>(ctrl + CTRL_BUCKET_WORK) + threadIdx.x, work[threadIdx.x]);
+  }
+}
+
+// What the two kernels take, in microseconds: `groups` chains at a time with `chain` per candidate each when all are
+// busy, `alone` for the longest, `row` for every row; a lane `lane` per candidate of its row, all of them together
+// `lanes`; `start` for the launches that a call without chains leaves out, `list` and `expand` for what they do per row and
+// candidate.  chain = 0: no such times, FEW_CHAIN_ROWS rows.
+struct ChainCosts {
+  float groups, chain, alone, row, lane, lanes, start, list, expand;
+  uint32_t rows_max, stream_cap;
+};
+
+// Measured: csg and top-k graphs of R-MAT matrices and their symmetrised forms, rows listed down to 2^12 .. 2^17
+// candidates, times of both kernels; chains as their own benchmark has them.  A call's time with the rule below
+// and with chains for rows of 2^16 candidates or 296 rows, ms: R-MAT scale 22 21.4 and 23.5, top-k graph of scale 16
+// 22.8 and 27.3, scale 19 in chunks of 2,048 10.7 and 12.9; symmetrised R-MAT of scale 20 27.9 and 28.0, of 262,144
+// rows 12.2 and 16.2, of 65,536 rows 3.3 and 4.1.
+ChainCosts chain_costs(const Context &ctx, int slots, bool key_table, uint32_t rows_max, uint32_t stream_cap) {
+  ChainCosts c = {};
+  c.rows_max = rows_max;
+  c.stream_cap = stream_cap;
+  if (slots < 64 || slots > 128) return c;
+  c.groups = 2.0f * static_cast<float>(ctx.num_sms);
+  c.chain = slots == 64 ? 0.030f : slots == 96 ? 0.035f : 0.052f;
+  c.alone = slots == 64 ? 0.018f : 0.021f;
+  c.row = 3.0f;
+  c.lane = key_table ? 0.24f : 0.40f;
+  c.lanes = (key_table ? (slots == 64 ? 5.5e-5f : 7.5e-5f) : 1.0e-4f) * 148.0f / static_cast<float>(ctx.num_sms);
+  c.start = 30.0f;
+  c.list = 0.015f;
+  c.expand = 6.0e-6f;
+  return c;
 }
 
 // Longest bucket first (one warp, lane l counts the buckets 127 - 4 l .. 124 - 4 l).
-// Which rows get a warp of the chain kernel each: all rows of HEAVY_WORK candidates or more,
-// and below that the longest buckets that keep the list within CHAIN_ROWS rows.  A row resolved
-// in rounds takes 40 to 200 cycles per candidate and half an SM; run by one lane among 32 it takes
-// about 600, so in a call with few long rows the lanes would be waiting for the longest one.
-// CHAIN_ROWS = two rows on each of 148 SMs: beyond one wave of them the chains only queue, and
-// what they do the lanes do with a sixth of the SM time (R-MAT scale 22 took 42 ms with 1184 rows
-// here).
+// Which rows get a group of warps of the chain kernel each: all rows of HEAVY_WORK candidates or more,
+// and below that as many buckets as make the later of the two kernels end soonest (a tenth of the other's time, which
+// runs beside it, added).  A chain takes 40 to 80 cycles per candidate and a good part of an SM, a lane among 32 some
+// 500 and a sixth of the SM time: too few chains and the lanes wait for their longest row, too many and the chains
+// queue.  Without times: the longest buckets that keep the list within FEW_CHAIN_ROWS rows.
 // `octaves` > 0: the lanes find their keys by a chained hash table and take some 680 cycles per candidate.
-// Of the rows that are left, those within so many octaves of the longest go to a warp each first; the
-// lanes' longest row then takes about as long as the chain of the longest of all (52 cycles per
-// candidate, 90 with a large key table: four octaves and three).  R-MAT scale 19 with chunks of 2,048:
-// 30.0 ms without, 16.9 with three, 13.4 with four, 14.2 with five; symmetrised scale 20, where the
-// chain is longer than any lane's row, 47.3, 47.4, 47.6 and 53.9; scale 16 as one chunk 29.3 with none
-// or three, 32.4 with five.
+// Of the rows that are left, those within so many octaves of the longest go to a warp each first (four octaves, three
+// in very large chunks).  R-MAT scale 19 with chunks of 2,048, chains for 296 rows: 30.0 ms without, 16.9 with three, 13.4
+// with four, 14.2 with five.
 __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, uint32_t ticket, int octaves,
-                                   const uint32_t *ctrl_ahead) {
+                                   const uint32_t *ctrl_ahead, ChainCosts cost) {
   const int lane = threadIdx.x;
   uint32_t c[4], sum = 0;
 #pragma unroll
@@ -794,29 +821,83 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     if (lane >= off) incl += t;
   }
   uint32_t run = incl - sum;
-  uint32_t heavy = 0, mid = 0;
+  const uint32_t listed = __shfl_sync(FULL, incl, 31);
   int longest = 0;
 #pragma unroll
   for (int j = 3; j >= 0; --j)
     if (c[j]) longest = WORK_BUCKETS - 1 - (4 * lane + j);
   longest = __reduce_max_sync(FULL, longest);
+  const float top = bucket_floor(longest + 1);
   // (the chunk ahead lists its rows down to a quarter of its longest)
   if (ctrl_ahead && ctrl_ahead[CTRL_PRIO] != PRIO_NONE && ctrl_ahead[CTRL_PRIO_WORK] > 0)
     longest = max(longest, work_bucket(4u * ctrl_ahead[CTRL_PRIO_WORK]));
   const int least = max(work_bucket(WARP_WORK_MIN), longest - 4 * octaves);
+  uint32_t heavy = 0, mid = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int b = WORK_BUCKETS - 1 - (4 * lane + j);
     ctrl[CTRL_BUCKET_BASE + b] = run;
     run += c[j];
     ctrl[CTRL_BUCKET_FILL + b] = 0;
-    if (b >= work_bucket(HEAVY_WORK) || (b >= work_bucket(CHAIN_WORK_MIN) && run <= CHAIN_ROWS)) heavy = run;
+    if (b >= work_bucket(HEAVY_WORK) || (cost.chain == 0.0f && b >= work_bucket(CHAIN_WORK_MIN) && run <= FEW_CHAIN_ROWS))
+      heavy = run;
     if (octaves > 0 && b >= least) mid = run;
   }
   heavy = __reduce_max_sync(FULL, heavy);
+  // (where the lanes end their longest row before a chain kernel would have begun, there is nothing to weigh)
+  const bool weigh = cost.chain > 0.0f && top * cost.lane > cost.start;
+  unsigned long long need = 0;
+  if (weigh || heavy > 0) {
+    const unsigned long long *const bucket_work = reinterpret_cast<const unsigned long long *>(ctrl + CTRL_BUCKET_WORK);
+    unsigned long long work[4], work_sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      work[j] = bucket_work[WORK_BUCKETS - 1 - (4 * lane + j)];
+      work_sum += work[j];
+    }
+    unsigned long long work_run = work_sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned long long u = __shfl_up_sync(FULL, work_run, off);
+      if (lane >= off) work_run += u;
+    }
+    const float all = static_cast<float>(__shfl_sync(FULL, work_run, 31));
+    work_run -= work_sum;
+    run = incl - sum;
+    // time with the chains down to this bucket, and the least of them: of all choices (what the stream buffer should
+    // hold the next time), and of those that fit the buffer as it is
+    float best = 3.0e38f, best_fit = 3.0e38f;
+    uint32_t rows_fit = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int b = WORK_BUCKETS - 1 - (4 * lane + j);
+      run += c[j];
+      work_run += work[j];
+      if (c[j] && run <= heavy) need = work_run;
+      if (!weigh || c[j] == 0 || b < work_bucket(CHAIN_WORK_MIN) || run > cost.rows_max) continue;
+      const float s = static_cast<float>(work_run), r = static_cast<float>(run);
+      const float chains = fmaxf(top * cost.alone, (s * cost.chain + r * cost.row) / cost.groups);
+      const float lanes = run < listed ? fmaxf(bucket_floor(b) * cost.lane, (all - s) * cost.lanes) : 0.0f;
+      const float time = fmaxf(chains, lanes) + 0.1f * fminf(chains, lanes) + r * cost.list + s * cost.expand;
+      if (work_run <= STREAM_CAP_MAX && time < best) {
+        best = time;
+        need = max(need, work_run);
+      }
+      if (work_run <= cost.stream_cap && time < best_fit) {
+        best_fit = time;
+        rows_fit = run;
+      }
+    }
+    if (weigh) {
+      const uint32_t time = __reduce_min_sync(FULL, __float_as_uint(best)), fit = __reduce_min_sync(FULL, __float_as_uint(best_fit));
+      if (__float_as_uint(best) != time && run > heavy) need = 0;
+      heavy = max(heavy, __reduce_max_sync(FULL, __float_as_uint(best_fit) == fit ? rows_fit : 0u));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) need = max(need, __shfl_xor_sync(FULL, need, off));
+  }
   mid = __reduce_max_sync(FULL, mid);
   if (mid < heavy) mid = heavy;
-  const uint32_t listed = __shfl_sync(FULL, run, 31);
   if (lane == 0) {
     ctrl[CTRL_ROWS_LISTED] = listed;
     ctrl[CTRL_HEAVY_ROWS] = heavy;
@@ -824,6 +905,7 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     ctrl[CTRL_LANE_TICKET] = mid;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
+    *reinterpret_cast<unsigned long long *>(ctrl + CTRL_HEAVY_NEED) = need;
     // for the host (wait_outcome)
     outcome[1] = heavy;
     outcome[2] = ctrl[CTRL_HEAVY_COUNT];
@@ -832,26 +914,47 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
   }
 }
 
-__global__ void row_list_kernel(int32_t n, const uint32_t *__restrict__ row_work, uint32_t *ctrl,
-                                int32_t *__restrict__ row_list, int32_t chunk,
-                                const uint32_t *ctrl_ahead) {
+// The list itself.  A block draws the places of a step's rows bucket by bucket: with an atomic per warp and bucket
+// on the few counters that all rows share, the kernel took 15.3 us at 1,048,576 rows of a mesh, now 9.5.
+constexpr int LIST_ROWS = 4;  // rows per thread and step
+__global__ void __launch_bounds__(256) row_list_kernel(int32_t n, const uint32_t *__restrict__ row_work, uint32_t *ctrl,
+                                                       int32_t *__restrict__ row_list, int32_t chunk,
+                                                       const uint32_t *ctrl_ahead) {
+  __shared__ uint32_t bucket[WORK_BUCKETS];  // rows of the step, then the place of its first
   const int lane = threadIdx.x & 31;
-  const int32_t total = gridDim.x * blockDim.x;
+  const int32_t step = blockDim.x * LIST_ROWS;
   const uint32_t prio = ctrl_ahead ? ctrl_ahead[CTRL_PRIO] : PRIO_NONE;
   const uint32_t least = ctrl_ahead ? ctrl_ahead[CTRL_PRIO_WORK] : 0u;
-  for (int32_t base = blockIdx.x * blockDim.x; base < n; base += total) {
-    const int32_t r = base + threadIdx.x;
-    uint32_t t = r < n ? row_work[r] : 0u;
-    if (r < n && taken_ahead(prio, least, chunk, r, t)) t = 0;
-    const int bkt = t ? work_bucket(t) : -1;
-    const unsigned peers = match_digit(t ? static_cast<uint32_t>(bkt) : 256u);
-    if (t) {
-      const int leader = __ffs(peers) - 1;
-      uint32_t pre = 0;
-      if (lane == leader) pre = atomicAdd(&ctrl[CTRL_BUCKET_FILL + bkt], __popc(peers));
-      pre = __shfl_sync(peers, pre, leader);
-      row_list[ctrl[CTRL_BUCKET_BASE + bkt] + pre + __popc(peers & ((1u << lane) - 1u))] = r;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * step; base < n; base += static_cast<int64_t>(gridDim.x) * step) {
+    if (threadIdx.x < WORK_BUCKETS) bucket[threadIdx.x] = 0;
+    __syncthreads();
+    int bkt[LIST_ROWS];
+    uint32_t at[LIST_ROWS];
+#pragma unroll
+    for (int i = 0; i < LIST_ROWS; ++i) {
+      const int64_t r = base + i * blockDim.x + threadIdx.x;
+      uint32_t t = r < n ? row_work[r] : 0u;
+      if (r < n && taken_ahead(prio, least, chunk, static_cast<int32_t>(r), t)) t = 0;
+      bkt[i] = t ? work_bucket(t) : -1;
     }
+#pragma unroll
+    for (int i = 0; i < LIST_ROWS; ++i) {
+      const unsigned peers = match_digit(bkt[i] >= 0 ? static_cast<uint32_t>(bkt[i]) : 256u);
+      if (bkt[i] >= 0) {
+        const int leader = __ffs(peers) - 1;
+        uint32_t pre = 0;
+        if (lane == leader) pre = atomicAdd(&bucket[bkt[i]], __popc(peers));
+        at[i] = __shfl_sync(peers, pre, leader) + __popc(peers & ((1u << lane) - 1u));
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < WORK_BUCKETS && bucket[threadIdx.x])
+      bucket[threadIdx.x] = ctrl[CTRL_BUCKET_BASE + threadIdx.x] + atomicAdd(&ctrl[CTRL_BUCKET_FILL + threadIdx.x], bucket[threadIdx.x]);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < LIST_ROWS; ++i)
+      if (bkt[i] >= 0) row_list[bucket[bkt[i]] + at[i]] = static_cast<int32_t>(base + i * blockDim.x + threadIdx.x);
+    __syncthreads();
   }
 }
 
@@ -960,9 +1063,12 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
   const int32_t span = chunk < n ? chunk : n;
   const int octaves = span <= LANE_TABLE_ROWS ? 0 : span <= WARP_FEW_ROWS ? 4 : 3;
   bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl, reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD,
-                                               ++ctx.outcome_ticket, octaves, ctrl_ahead);
+                                               ++ctx.outcome_ticket, octaves, ctrl_ahead,
+                                               chain_costs(ctx, s.slots, span <= LANE_TABLE_ROWS, s.heavy_max, s.stream_cap));
   CSG_CUDA(cudaGetLastError());
-  row_list_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
+  int steps = static_cast<int>((static_cast<int64_t>(n) + 256 * LIST_ROWS - 1) / (256 * LIST_ROWS));
+  if (steps > ctx.num_sms * 32) steps = ctx.num_sms * 32;
+  row_list_kernel<<<steps, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
   CSG_CUDA(cudaGetLastError());
   count_launches(3);
   return true;
@@ -1011,8 +1117,7 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   if (outcome[2] != 0) {
     s.no_heavy_rows = false;
     if (!launch_heavy(ctx, a, false, st)) return false;
-    CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, sizeof(uint32_t) * WORK_BUCKETS, st));
-    CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_HEAVY_NEED, 0, 2 * sizeof(uint32_t), st));
+    CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, 3 * sizeof(uint32_t) * WORK_BUCKETS, st));
     return launch_lists(ctx, n, chunk, s, nullptr);
   }
   return true;

@@ -172,8 +172,8 @@ SPORDER_API const char *sporder_last_error(void);
 SPORDER_API void sporder_context_set_stream(sporder_context_t ctx, void *stream);
 
 /* Upper bound, in stream elements of 8 bytes, on the buffer that holds the materialised
- * candidate streams of the heaviest rows (rows that stream 65536 candidates or more are
- * computed fastest from such a copy).  0 = no bound beyond the built-in 2^27 elements (1 GiB).
+ * candidate streams of the heaviest rows (rows that stream tens of thousands of candidates are
+ * computed fastest from such a copy).  0 = no bound beyond the built-in 2^28 elements (2 GiB).
  * Without a bound a call plans max(8 * nnz, 2^20) elements, or what the largest earlier
  * call of this context needed, never more than nnz * chunk_size.  Rows that do not fit are
  * computed by the kernel of the lighter rows; results are the same for every bound. */

@@ -111,3 +111,17 @@ def test_windows_of_the_chains(chunk, k, spread):
         col += extra
     ptr, ind = _csr(rows, max(col, chunk))
     _check(ptr, ind, k=k, chunk_size=chunk)
+
+
+@pytest.mark.parametrize("k", [12, 24, 32])
+def test_many_rows_with_a_chain_each(k):
+    # 5,000 rows of some 2,500 candidates and fewer: more rows than one block scans at a time, more than the list of
+    # chains takes, and, with little room for their streams, only the first of them
+    rng = np.random.default_rng(k)
+    rows = [[] for _ in range(5000)]
+    for c in range(9000):
+        base = c % 5 * 1000
+        for r in base + (1000 * rng.random(33) ** 2).astype(np.int64):
+            rows[r].append(c)
+    ptr, ind = _csr(rows, 9000)
+    _check(ptr, ind, limits=(0, 200_000, 0), k=k, chunk_size=1000)
