@@ -217,6 +217,12 @@ bool launch_row_sums(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr,
 constexpr unsigned FULL = 0xFFFFFFFFu;
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
+// Programmatic dependent launches: the blocks of a kernel may be placed while the kernel in front of it in its stream
+// still runs, once all of that one's blocks run or are through.  Such a kernel waits before it touches anything an
+// earlier one of the call writes; each of them waits, so that the end of one means the end of all before it.
+__device__ __forceinline__ void wait_for_kernels_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- checked build ----------------------------------------------------------------------
 // Compiled with -DSPORDER_CHECKED (python -m chunkedgreedy_b200.build --checked) every index
 // that a kernel derives from data another kernel wrote - positions in the transposed chunk,
@@ -295,6 +301,24 @@ __device__ __forceinline__ int32_t entry_index(uint64_t e) {
 }
 __device__ __forceinline__ uint32_t entry_weight_bits(uint64_t e) {
   return static_cast<uint32_t>(e >> 32);
+}
+#endif
+
+#ifdef __CUDACC__
+// launch of a kernel that calls wait_for_kernels_before()
+template <typename... Params, typename... Args>
+cudaError_t launch_behind(void (*kernel)(Params...), int grid, int threads, int smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 #endif
 

@@ -26,7 +26,7 @@
 // new row is already sorted block by block and only the entries of one block have to be ordered
 // among themselves.  len_block_sums_kernel notices such a permutation and tells the host, which then
 // launches apply_flat_kernel instead of the kernels above.  That one, which also does the copy
-// of the rows-only mode, cuts the output into tiles of 2048 entries whatever rows they belong to.
+// of the rows-only mode, cuts the output into tiles of 128 entries whatever rows they belong to.
 #include <cstddef>
 
 #include "common.cuh"
@@ -39,7 +39,7 @@ constexpr int R_THREADS = 256;
 constexpr int R_SCAN_IPT = 8;
 constexpr int R_SCAN_TILE = R_THREADS * R_SCAN_IPT;  // rows per scan block
 constexpr int LOCAL_BITS = 10;                       // blocks of 1024 rows / columns: the default csg chunk
-constexpr int FLAT_TILE = 2048;                      // output entries per tile of apply_flat_kernel
+constexpr int FLAT_TILE = 128;                       // output entries per tile of apply_flat_kernel
 constexpr int R_WARP = 256;                          // longest row sorted by one warp in registers
 constexpr int R_MED = 4096;                          // longest row (and tile of a longer row) sorted in shared memory
 
@@ -69,10 +69,11 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *tota
 // Entries of the rows that each block of new rows takes.  With `outcome`, the last block also tells the host
 // whether any row leaves its block of 1024: here and not in ptr_new_kernel, so that the host reads it and
 // launches the rest while the scan still runs (a random order of a 65,536-row mesh: 90 us with the
-// wait behind ptr_new_kernel, 84 here).
+// wait behind ptr_new_kernel, 84 here).  The kernels behind it are programmatic dependent launches: 8 us less a call.
 __global__ void __launch_bounds__(R_THREADS) len_block_sums_kernel(
     int32_t n, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
     int32_t *__restrict__ block_sums, uint32_t *__restrict__ leaves_block, volatile uint32_t *outcome, uint32_t ticket) {
+  let_next_kernel_start();
   __shared__ int32_t sm[R_THREADS / 32];
   const int32_t base = blockIdx.x * R_SCAN_TILE;
   int32_t s = 0;
@@ -103,6 +104,8 @@ __global__ void __launch_bounds__(R_THREADS) len_block_sums_kernel(
 }
 
 __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32_t *block_sums) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   // exclusive scan in place, one block, any nb
   __shared__ int32_t sm[32];
   __shared__ int32_t carry_s;
@@ -138,6 +141,7 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     int32_t n, int32_t nnz, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
     const int32_t *__restrict__ block_sums, int32_t *__restrict__ ptr_new,
     int32_t *__restrict__ old2new, int32_t *__restrict__ tile_row, int32_t *__restrict__ row_delta) {
+  let_next_kernel_start();
   constexpr int WARPS = R_THREADS / 32;
   __shared__ int32_t sums[R_SCAN_IPT * WARPS];  // of 32 rows each, in row order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -167,6 +171,7 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
   for (int i = 0; i < R_SCAN_IPT; ++i)
     if (lane == 31) sums[i * WARPS + warp] = incl[i];
   __syncthreads();
+  wait_for_kernels_before();  // (the row lengths are the caller's)
   if (warp == 0) {  // sums -> what lies in front of each 32 rows
     static_assert(R_SCAN_IPT * WARPS == 64, "two per lane");
     const int32_t x = sums[2 * lane], y = sums[2 * lane + 1];
@@ -373,234 +378,302 @@ __device__ __forceinline__ void warp_row(const ApplyArgs &a, int32_t src, int32_
 }
 
 // ---- tiles of the output ---------------------------------------------------------------------
-// A block per tile of FLAT_TILE consecutive output entries, rows in order.  ROWS: a copy of the
+// A warp per tile of FLAT_TILE consecutive output entries, rows in order.  ROWS: a copy of the
 // old rows in their new order.  Otherwise (a permutation that keeps rows and columns in their
 // blocks of 1024) an entry's place is the start of its run - the entries of its row in its column's
 // block - plus the number of smaller entries in the run, found by comparing where the run is
 // short and in a bit map of the block where it is long.  Runs belong to the tile that holds their
 // first entry; a tile reads on behind its end as far as its last run goes.
-// All rows cost the same per entry this way.  By kinds of rows (bitonic networks up to 32 entries,
-// run scans by a warp and by a block above) the reordered R-MAT scale 22 took 1.17 ms here, 0.95 this
-// way; bound by instructions (some 270 per entry, the passes over the tile in shared memory) at four blocks per SM.
-constexpr int FLAT_HALO = 1 << LOCAL_BITS;  // a run holds at most 1024 entries
-constexpr int FLAT_LONG = 48;               // shortest run that gets a bit map
-constexpr int FLAT_MAX = FLAT_TILE + FLAT_HALO;
-struct FlatShared {
-  int32_t delta[FLAT_TILE];               // at the first entry of a row: where it comes from, relative
-  uint32_t row_head[FLAT_TILE / 32];      // bit per entry: first of its row
-  int16_t row_before[FLAT_TILE / 32];     // last such entry in the words in front, -1: none in the tile
-  // (the copy of the rows-only mode needs no more than this)
-  uint32_t run_head[FLAT_MAX / 32];       // the same for runs
-  int16_t run_before[FLAT_MAX / 32];
-  int32_t key[FLAT_MAX];
-  float val[FLAT_TILE];
-  uint16_t run_end[FLAT_MAX];             // at the first entry of a run; FLAT_MAPPED + its bit map for a long one
-  uint32_t map[FLAT_MAX / FLAT_LONG][32];
-  uint16_t map_before[FLAT_MAX / FLAT_LONG][32];
-  int32_t maps;
+// All rows cost the same per entry this way.  By blocks of 256 threads on tiles of 2048 entries, with ten barriers a
+// tile, the reordered R-MAT scale 22 took 955 us here, now 522; mesh of 1,048,576 rows 94 and 48.  Bound by the
+// latency of the gathers at 48 warps per SM (40 registers; 11 KB of shared memory a block leave the L1 its space: with
+// 27 KB 677 us).  Tiles of 64 / 96 / 256 entries: 10 / 4 / 30 % slower.
+constexpr int FLAT_PER = FLAT_TILE / 32;    // windows of 32 entries
+// longest run ranked by comparing: 20 took 624 us for the whole call, 28 606, 48 581, 72 579, 128 585 (a bit map costs a
+// warp two trips over the run and a scan)
+constexpr int FLAT_LONG = 72;
+constexpr int FLAT_WARPS = R_THREADS / 32;
+// whether a run is ranked by comparing: short, and its last entries no further behind the tile than one window
+__device__ __forceinline__ bool flat_short(int32_t s, int32_t end) {
+  return end - s <= FLAT_LONG && end <= FLAT_TILE + 32;
+}
+
+struct FlatWarp {
+  uint32_t row_head[FLAT_PER];    // entries that begin a row
+  int32_t delta[FLAT_TILE];       // at these: where the row was less where it is
+  int32_t key[FLAT_TILE + 32];    // new columns, and those behind the tile as far as its last run goes
+  uint32_t map[32];               // a long run's columns, and how many lie in front of each word
+  uint16_t map_before[32];
 };
-constexpr uint32_t FLAT_MAPPED = 0x8000u;
 
-// last set bit at or below lane `lane` of word w, or what the words in front say
-__device__ __forceinline__ int32_t last_head(const uint32_t *heads, const int16_t *before, int w, int lane) {
-  const uint32_t m = heads[w] & (FULL >> (31 - lane));
-  return m ? w * 32 + 31 - __clz(static_cast<int>(m)) : before[w];
-}
-// `before` of `words` words, by one warp
-__device__ __forceinline__ void heads_before(const uint32_t *heads, int16_t *before, int words) {
-  const int lane = lane_id();
-  int carry = -1;
-  for (int w0 = 0; w0 < words; w0 += 32) {
-    const int w = w0 + lane;
-    const uint32_t h = w < words ? heads[w] : 0u;
-    const int mine = h ? w * 32 + 31 - __clz(static_cast<int>(h)) : -1;
-    int incl = mine;
+// Runs of more than FLAT_DEFER entries wait until the block is through with its tiles and are then ranked by all its
+// warps, eight runs at a time (a warp by itself needed 9 us for 1,000 entries, nearly half of a small call's kernel).
+constexpr int FLAT_DEFER = 128, FLAT_QUEUE = 64, FLAT_BATCH = 4;
+struct FlatRun {
+  int32_t at, len, delta;  // first entry of the output, entries, where they were less where they go
+};
+struct FlatBlock {
+  int32_t queued;
+  FlatRun run[FLAT_QUEUE];
+};
+
+__device__ __forceinline__ void flat_mark(FlatWarp &sh, int32_t k) { atomicOr(&sh.map[(k >> 5) & 31], 1u << (k & 31)); }
+// columns in front of each word of the map, by one warp
+__device__ __forceinline__ void flat_count(FlatWarp &sh, int lane) {
+  const int c = __popc(sh.map[lane]);
+  int incl = c;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int t = __shfl_up_sync(FULL, incl, off);
-      if (lane >= off) incl = max(incl, t);
-    }
-    int prev = __shfl_up_sync(FULL, incl, 1);
-    if (lane == 0) prev = -1;
-    if (w < words) before[w] = static_cast<int16_t>(max(prev, carry));
-    carry = max(carry, __shfl_sync(FULL, incl, 31));
+  for (int off = 1; off < 32; off <<= 1) {
+    const int x = __shfl_up_sync(FULL, incl, off);
+    if (lane >= off) incl += x;
   }
+  sh.map_before[lane] = static_cast<uint16_t>(incl - c);
+}
+__device__ __forceinline__ void flat_put(const ApplyArgs &a, const FlatWarp &sh, const FlatRun &run, int32_t i, int32_t k) {
+  const int32_t w = (k >> 5) & 31;
+  const int32_t at = run.at + sh.map_before[w] + __popc(sh.map[w] & ((1u << (k & 31)) - 1u));
+  a.ind_new[at] = k;
+  if (a.val_new) a.val_new[at] = a.val_old[run.at + run.delta + i];
 }
 
-template <bool ROWS>
-__global__ void __launch_bounds__(R_THREADS, 4) apply_flat_kernel(ApplyArgs a) {
-  extern __shared__ __align__(16) unsigned char flat_smem[];
-  FlatShared &sh = *reinterpret_cast<FlatShared *>(flat_smem);
-  constexpr int PER = FLAT_TILE / R_THREADS;  // entries per thread: 32 consecutive ones per warp and turn
-  const int tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  const int32_t nnz = min(a.ptr_new[a.n], a.nnz);
-  const int32_t tiles = nnz / FLAT_TILE + (nnz % FLAT_TILE ? 1 : 0);
-  for (int32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int32_t t0 = t * FLAT_TILE, cnt = nnz - t0 < FLAT_TILE ? nnz - t0 : FLAT_TILE, t1 = t0 + cnt;
-    const int32_t ra = a.tile_row[t], rb = t + 1 < tiles ? a.tile_row[t + 1] : a.n - 1;
-    __syncthreads();
-    if (tid < FLAT_TILE / 32) sh.row_head[tid] = 0;
-    if (!ROWS && tid == 0) sh.maps = 0;
-    __syncthreads();
-    const int32_t delta0 = a.row_delta[ra];
-    const int32_t rb_start = a.ptr_new[rb], rb_end = a.ptr_new[rb + 1];  // (rb holds entry t1, if there is one)
-    for (int32_t p = ra + tid; p <= rb; p += R_THREADS) {
-      const int32_t b = a.ptr_new[p], e = a.ptr_new[p + 1], d = a.row_delta[p];
-      if (b >= t1) break;  // (behind the last row with entries there may be many without)
-      if (b >= t0 && e > b) {
-        sh.delta[b - t0] = d;
-        atomicOr(&sh.row_head[(b - t0) >> 5], 1u << ((b - t0) & 31));
+// A run that begins at entry s of the tile, by one warp.
+__device__ __forceinline__ void flat_run_by_warp(const ApplyArgs &a, FlatWarp &sh, const FlatRun &run, int32_t s, int lane) {
+  auto key = [&](int32_t i) {
+    return s + i < FLAT_TILE ? sh.key[s + i] : a.old2new[a.ind_old[run.at + run.delta + i]];
+  };
+  sh.map[lane] = 0u;
+  __syncwarp();
+  for (int32_t i = lane; i < run.len; i += 32) flat_mark(sh, key(i));
+  __syncwarp();
+  flat_count(sh, lane);
+  __syncwarp();
+  for (int32_t i = lane; i < run.len; i += 32) flat_put(a, sh, run, i, key(i));
+  __syncwarp();
+}
+
+// The runs that waited, by all warps: a map each, the entries of all of them side by side.
+__device__ __forceinline__ void flat_runs_by_block(const ApplyArgs &a, FlatWarp *shared, const FlatRun *run, int runs) {
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  int32_t total = 0;
+  for (int r = 0; r < runs; ++r) total += run[r].len;
+  shared[warp].map[lane] = 0u;
+  __syncthreads();
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int32_t i0 = 0; i0 < total; i0 += FLAT_BATCH * R_THREADS) {
+      int32_t key[FLAT_BATCH], at[FLAT_BATCH], of[FLAT_BATCH];
+#pragma unroll
+      for (int b = 0; b < FLAT_BATCH; ++b) {
+        at[b] = i0 + b * R_THREADS + threadIdx.x;
+        of[b] = 0;
+        if (at[b] >= total) {
+          of[b] = -1;
+          continue;
+        }
+        while (at[b] >= run[of[b]].len) at[b] -= run[of[b]++].len;
+        key[b] = a.ind_old[run[of[b]].at + run[of[b]].delta + at[b]];
+      }
+#pragma unroll
+      for (int b = 0; b < FLAT_BATCH; ++b)
+        if (of[b] >= 0) key[b] = a.old2new[key[b]];
+#pragma unroll
+      for (int b = 0; b < FLAT_BATCH; ++b) {
+        if (of[b] < 0) continue;
+        if (pass == 0)
+          flat_mark(shared[of[b]], key[b]);
+        else
+          flat_put(a, shared[of[b]], run[of[b]], at[b], key[b]);
       }
     }
     __syncthreads();
-    if (warp == 0) heads_before(sh.row_head, sh.row_before, FLAT_TILE / 32);
+    if (pass == 0) {
+      flat_count(shared[warp], lane);
+      __syncthreads();
+    }
+  }
+}
+
+template <bool ROWS, bool VALUES>
+__global__ void __launch_bounds__(R_THREADS, 6) apply_flat_kernel(ApplyArgs a) {
+  __shared__ FlatWarp shared[FLAT_WARPS];
+  __shared__ FlatBlock later;
+  constexpr int PER = FLAT_PER;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  FlatWarp &sh = shared[warp];
+  const uint32_t upto = FULL >> (31 - lane);
+  wait_for_kernels_before();
+  const int32_t nnz = min(a.ptr_new[a.n], a.nnz);
+  const int32_t tiles = nnz / FLAT_TILE + (nnz % FLAT_TILE ? 1 : 0);
+  if (!ROWS) {
+    if (threadIdx.x == 0) later.queued = 0;
     __syncthreads();
-    int32_t from[PER], key[PER];
+  }
+  for (int32_t t = blockIdx.x * FLAT_WARPS + warp; t < tiles; t += gridDim.x * FLAT_WARPS) {
+    const int32_t t0 = t * FLAT_TILE, cnt = nnz - t0 < FLAT_TILE ? nnz - t0 : FLAT_TILE, t1 = t0 + cnt;
+    const int32_t ra = a.tile_row[t];
+    if (lane < PER) sh.row_head[lane] = 0u;
+    __syncwarp();
+    const int32_t delta0 = a.row_delta[ra];
+    int32_t row_end;  // of the row that holds the tile's last entry
+    for (int32_t p0 = ra;; p0 += 32) {
+      const int32_t r = p0 + lane;
+      int32_t b = nnz, e = nnz, d = 0;
+      if (r < a.n) {
+        b = a.ptr_new[r];
+        e = a.ptr_new[r + 1];
+        d = a.row_delta[r];
+      }
+      if (b >= t0 && b < t1 && e > b) {
+        sh.delta[b - t0] = d;
+        atomicOr(&sh.row_head[(b - t0) >> 5], 1u << ((b - t0) & 31));
+      }
+      const unsigned behind = __ballot_sync(FULL, e >= t1);
+      if (behind) {
+        row_end = __shfl_sync(FULL, e, __ffs(static_cast<int>(behind)) - 1);
+        break;
+      }
+    }
+    __syncwarp();
+    int32_t key[PER], from[PER];
+    uint32_t rows[PER];
+    int32_t last = -1;  // entry that begins the row in hand
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int w = warp * PER + u, e = w * 32 + lane;
-      const int32_t h = last_head(sh.row_head, sh.row_before, w, lane);
+      const int e = u * 32 + lane;
+      rows[u] = sh.row_head[u];
+      const uint32_t m = rows[u] & upto;
+      const int32_t h = m ? u * 32 + 31 - __clz(static_cast<int>(m)) : last;
       from[u] = t0 + e + (h >= 0 ? sh.delta[h] : delta0);
       key[u] = e < cnt ? a.ind_old[from[u]] : 0;
+      if (rows[u]) last = u * 32 + 31 - __clz(static_cast<int>(rows[u]));
+    }
+    float val[PER];
+    if (VALUES) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) val[u] = u * 32 + lane < cnt ? a.val_old[from[u]] : 0.0f;
     }
     if (ROWS) {
 #pragma unroll
       for (int u = 0; u < PER; ++u) {
-        const int e = (warp * PER + u) * 32 + lane;
+        const int e = u * 32 + lane;
         if (e < cnt) {
           a.ind_new[t0 + e] = key[u];
-          if (a.val_new) a.val_new[t0 + e] = a.val_old[from[u]];
+          if (VALUES) a.val_new[t0 + e] = val[u];
         }
       }
+      __syncwarp();
       continue;
     }
-    // In the same trip: the values, straight to shared memory; the entry in front of the tile, if
-    // its row goes on here; and the entries behind the tile, if the row that ends it goes on there.
-    if (a.val_new) {
-#pragma unroll
-      for (int u = 0; u < PER; ++u) {
-        const int e = (warp * PER + u) * 32 + lane;
-        if (e < cnt) {
-          const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(&sh.val[e]));
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(a.val_old + from[u]) : "memory");
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    const int32_t last = last_head(sh.row_head, sh.row_before, (cnt - 1) >> 5, (cnt - 1) & 31);
+    // in the same trip: the entry in front of the tile, if its row goes on here, and 32 behind it, as far as its
+    // last row goes
     const int32_t last_delta = last >= 0 ? sh.delta[last] : delta0;
-    const bool goes_on = t1 < nnz && rb_start < t1, comes_in = (sh.row_head[0] & 1u) == 0u;
+    const bool comes_in = (rows[0] & 1u) == 0u, in = t1 + lane < row_end;
     int32_t prev = comes_in ? a.ind_old[t0 - 1 + delta0] : 0;
-    bool in = goes_on && t1 + tid < rb_end;
-    int32_t more = in ? a.ind_old[t1 + tid + last_delta] : 0;
+    int32_t more = in ? a.ind_old[t1 + lane + last_delta] : 0;
+    float more_val = 0.0f;
+    if (VALUES && in) more_val = a.val_old[t1 + lane + last_delta];
 #pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int e = (warp * PER + u) * 32 + lane;
-      key[u] = e < cnt ? a.old2new[key[u]] : 0x7FFFFFFF;
-    }
+    for (int u = 0; u < PER; ++u) key[u] = u * 32 + lane < cnt ? a.old2new[key[u]] : 0;
     if (comes_in) prev = a.old2new[prev];
     if (in) more = a.old2new[more];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) sh.key[(warp * PER + u) * 32 + lane] = key[u];
-    __syncthreads();
-    const bool joined = comes_in && (prev >> LOCAL_BITS) == (sh.key[0] >> LOCAL_BITS);  // a run of the tile before
-    int32_t ext = 0;  // entries of the last run behind the tile's end
-    if (goes_on) {
-      const int32_t blk = sh.key[cnt - 1] >> LOCAL_BITS;
-      for (;;) {
-        const bool same = in && (more >> LOCAL_BITS) == blk;
-        if (same) sh.key[cnt + ext + tid] = more;
-        const int got = __syncthreads_count(same);
-        ext += got;
-        if (got < R_THREADS || ext >= FLAT_HALO) break;
-        in = t1 + ext + tid < rb_end && ext + tid < FLAT_HALO;
-        if (in) more = a.old2new[a.ind_old[t1 + ext + tid + last_delta]];
-      }
-    }
-    const int32_t total = cnt + ext;
+    // first entries of runs; entries behind the matrix count as such
+    uint32_t heads[PER];
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int w = warp * PER + u, e = w * 32 + lane;
-      bool head = false;
-      if (e < cnt)
-        head = e == 0 ? !joined
-                      : ((sh.row_head[w] >> lane) & 1u) != 0u || (sh.key[e - 1] >> LOCAL_BITS) != (key[u] >> LOCAL_BITS);
-      const unsigned m = __ballot_sync(FULL, head);
-      if (lane == 0) sh.run_head[w] = m;
+      const int e = u * 32 + lane;
+      int32_t front = __shfl_up_sync(FULL, key[u], 1);
+      const int32_t across = u > 0 ? __shfl_sync(FULL, key[u > 0 ? u - 1 : 0], 31) : prev;
+      if (lane == 0) front = across;
+      const bool head = (front >> LOCAL_BITS) != (key[u] >> LOCAL_BITS) || (u == 0 && lane == 0 && !comes_in) || e >= cnt;
+      heads[u] = __ballot_sync(FULL, head) | rows[u];
+      sh.key[e] = key[u];
     }
-    if (tid < FLAT_HALO / 32) sh.run_head[FLAT_TILE / 32 + tid] = 0;
-    __syncthreads();
-    if (warp == 0) heads_before(sh.run_head, sh.run_before, FLAT_MAX / 32);
-    __syncthreads();
-    // ends of the runs.  (A tile that is not full is the last one and has nothing behind it.)
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int w = warp * PER + u, e = w * 32 + lane;
-      if (e > 0 && e < cnt && ((sh.run_head[w] >> lane) & 1u)) {
-        const int32_t s = last_head(sh.run_head, sh.run_before, (e - 1) >> 5, (e - 1) & 31);
-        if (s >= 0) sh.run_end[s] = static_cast<uint16_t>(e);
+    // the last run's entries behind the tile
+    int32_t ext = 0;
+    if (row_end > t1) {  // (only a full tile has something behind it)
+      const int32_t blk = __shfl_sync(FULL, key[PER - 1], 31) >> LOCAL_BITS;
+      unsigned other = __ballot_sync(FULL, !in || (more >> LOCAL_BITS) != blk);
+      ext = other ? __ffs(static_cast<int>(other)) - 1 : 32;
+      sh.key[FLAT_TILE + lane] = more;
+      while (other == 0u) {
+        const int32_t at = t1 + ext + lane;
+        other = __ballot_sync(FULL, at >= row_end || (a.old2new[a.ind_old[at + last_delta]] >> LOCAL_BITS) != blk);
+        ext += other ? __ffs(static_cast<int>(other)) - 1 : 32;
       }
     }
-    if (tid == 0) {
-      const int32_t s = last_head(sh.run_head, sh.run_before, (cnt - 1) >> 5, (cnt - 1) & 31);
-      if (s >= 0) sh.run_end[s] = static_cast<uint16_t>(total);
-    }
-    __syncthreads();
-    // bit maps of the long runs
+    __syncwarp();
+    int32_t next[PER];  // first head behind each window
+    next[PER - 1] = FLAT_TILE + ext;
+#pragma unroll
+    for (int u = PER - 2; u >= 0; --u)
+      next[u] = heads[u + 1] ? (u + 1) * 32 + __ffs(static_cast<int>(heads[u + 1])) - 1 : next[u + 1];
+    int32_t run = -1;  // first entry of the run in hand; -1: the tile before does it
     bool any_long = false;
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int w = warp * PER + u, e = w * 32 + lane;
-      if (e < cnt && ((sh.run_head[w] >> lane) & 1u) && sh.run_end[e] - e >= FLAT_LONG) {
-        const int32_t id = atomicAdd(&sh.maps, 1);
-        sh.run_end[e] = static_cast<uint16_t>(FLAT_MAPPED + id);
-        any_long = true;
-      }
-    }
-    if (__syncthreads_or(any_long)) {
-      for (int i = tid; i < sh.maps * 32; i += R_THREADS) sh.map[i >> 5][i & 31] = 0u;
-      __syncthreads();
-      for (int e = tid; e < total; e += R_THREADS) {
-        const int32_t s = last_head(sh.run_head, sh.run_before, e >> 5, e & 31);
-        const uint32_t end = s >= 0 ? sh.run_end[s] : 0u;
-        if (end >= FLAT_MAPPED) {
-          const int32_t k = sh.key[e];
-          atomicOr(&sh.map[end - FLAT_MAPPED][(k >> 5) & 31], 1u << (k & 31));
+      const int e = u * 32 + lane;
+      const uint32_t m = heads[u] & upto, after = heads[u] & ~upto;
+      const int32_t s = m ? u * 32 + 31 - __clz(static_cast<int>(m)) : run;
+      const int32_t end = after ? u * 32 + __ffs(static_cast<int>(after)) - 1 : next[u];
+      if (heads[u]) run = u * 32 + 31 - __clz(static_cast<int>(heads[u]));
+      if (s >= 0 && e < cnt) {
+        if (flat_short(s, end)) {
+          int32_t at = t0 + s;
+          for (int32_t j = s; j < end; ++j) at += sh.key[j] < key[u] ? 1 : 0;
+          a.ind_new[at] = key[u];
+          if (VALUES) a.val_new[at] = val[u];
+        } else {
+          any_long = true;
         }
       }
-      __syncthreads();
-      for (int m = warp; m < sh.maps; m += R_THREADS / 32) {
-        const int c = __popc(sh.map[m][lane]);
-        int incl = c;
+    }
+    if (run >= 0 && lane < ext && flat_short(run, FLAT_TILE + ext)) {
+      int32_t at = t0 + run;
+      for (int32_t j = run; j < FLAT_TILE + ext; ++j) at += sh.key[j] < more ? 1 : 0;
+      a.ind_new[at] = more;
+      if (VALUES) a.val_new[at] = more_val;
+    }
+    if (__any_sync(FULL, any_long)) {
+#pragma unroll 1
+      for (int u = 0; u < PER; ++u) {
+        uint32_t h = 0u;
+        int32_t behind = 0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const int x = __shfl_up_sync(FULL, incl, off);
-          if (lane >= off) incl += x;
+        for (int v = 0; v < PER; ++v)
+          if (v == u) {
+            h = heads[v];
+            behind = next[v];
+          }
+        while (h) {
+          const int32_t s = u * 32 + __ffs(static_cast<int>(h)) - 1;
+          h &= h - 1u;
+          const int32_t end = h ? u * 32 + __ffs(static_cast<int>(h)) - 1 : behind;
+          if (s >= cnt || flat_short(s, end)) continue;
+          int32_t row = -1;  // where the run's row begins in the tile
+          for (int v = 0; v <= u; ++v) {
+            const uint32_t m = v < u ? sh.row_head[v] : sh.row_head[v] & (FULL >> (31 - (s & 31)));
+            if (m) row = v * 32 + 31 - __clz(static_cast<int>(m));
+          }
+          const FlatRun long_run = {t0 + s, end - s, row >= 0 ? sh.delta[row] : delta0};
+          int32_t place = FLAT_QUEUE;
+          if (long_run.len > FLAT_DEFER) {
+            if (lane == 0) place = atomicAdd(&later.queued, 1);
+            place = __shfl_sync(FULL, place, 0);
+          }
+          if (place < FLAT_QUEUE) {
+            if (lane == 0) later.run[place] = long_run;
+          } else {
+            flat_run_by_warp(a, sh, long_run, s, lane);
+          }
         }
-        sh.map_before[m][lane] = static_cast<uint16_t>(incl - c);
       }
-      __syncthreads();
     }
-    if (a.val_new) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();
-    }
-#pragma unroll 2
-    for (int e = tid; e < total; e += R_THREADS) {
-      const int32_t s = last_head(sh.run_head, sh.run_before, e >> 5, e & 31), k = sh.key[e];
-      if (s < 0) continue;  // the tile before does it
-      const uint32_t end = sh.run_end[s];
-      int32_t rank = 0;
-      if (end >= FLAT_MAPPED) {
-        const uint32_t m = end - FLAT_MAPPED, w = (k >> 5) & 31;
-        rank = sh.map_before[m][w] + __popc(sh.map[m][w] & ((1u << (k & 31)) - 1u));
-      } else if (end - s > 1) {
-        for (int32_t j = s; j < static_cast<int32_t>(end); ++j) rank += sh.key[j] < k ? 1 : 0;
-      }
-      a.ind_new[t0 + s + rank] = k;
-      if (a.val_new) a.val_new[t0 + s + rank] = e < cnt ? sh.val[e] : a.val_old[t0 + e + last_delta];
-    }
+    __syncwarp();
   }
+  if (ROWS) return;
+  __syncthreads();
+  const int queued = min(later.queued, FLAT_QUEUE);
+  for (int i = 0; i < queued; i += FLAT_WARPS)
+    flat_runs_by_block(a, shared, later.run + i, min(queued - i, FLAT_WARPS));
 }
 
 // One warp per queued row of 33..R_WARP entries.
@@ -856,11 +929,9 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, a.counters + CNT_MOVED,
                                                           symmetric ? outcome : nullptr, ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
-  scan_block_sums_kernel<<<1, 1024, 0, ctx.stream>>>(nb, block_sums);
-  CSG_CUDA(cudaGetLastError());
-  ptr_new_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, nnz, d_ptr_old, d_new_order, block_sums, d_ptr_new,
-                                                   old2new, tile_row, row_delta);
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(scan_block_sums_kernel, 1, 1024, 0, ctx.stream, nb, block_sums));
+  CSG_CUDA(launch_behind(ptr_new_kernel, nb, R_THREADS, 0, ctx.stream, n, nnz, d_ptr_old, d_new_order, block_sums,
+                         d_ptr_new, old2new, tile_row, row_delta));
   count_launches(3);
   if (nnz == 0) return true;
   bool local = false;
@@ -869,13 +940,12 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
     local = reinterpret_cast<volatile uint32_t *>(outcome)[1] == 0u;
   }
   if (!symmetric || local) {
-    int64_t grid = (static_cast<int64_t>(nnz) + FLAT_TILE - 1) / FLAT_TILE;
+    constexpr int64_t block = static_cast<int64_t>(FLAT_TILE) * FLAT_WARPS;
+    int64_t grid = (static_cast<int64_t>(nnz) + block - 1) / block;
     if (grid > ctx.num_sms * 32) grid = ctx.num_sms * 32;
-    const int smem = symmetric ? static_cast<int>(sizeof(FlatShared)) : static_cast<int>(offsetof(FlatShared, run_head));
-    auto kernel = symmetric ? apply_flat_kernel<false> : apply_flat_kernel<true>;
-    CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kernel<<<static_cast<int>(grid), R_THREADS, smem, ctx.stream>>>(a);
-    CSG_CUDA(cudaGetLastError());
+    auto kernel = symmetric ? (with_vals ? apply_flat_kernel<false, true> : apply_flat_kernel<false, false>)
+                            : (with_vals ? apply_flat_kernel<true, true> : apply_flat_kernel<true, false>);
+    CSG_CUDA(launch_behind(kernel, static_cast<int>(grid), R_THREADS, 0, ctx.stream, a));
     count_launches(1);
     return true;
   }
