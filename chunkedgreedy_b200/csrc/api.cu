@@ -339,6 +339,7 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
   }
   CsgScratch s, sp;
   if (!plan_scratch(ctx, n, nnz, p, d_table, &s, 0, false, ahead ? &sp : nullptr)) return false;
+  s.one_stream = sp.one_stream = !ahead;
   cudaStream_t st = ctx.stream;
   const bool zero_table = d_table != nullptr || stats != nullptr;
 

@@ -118,6 +118,7 @@ struct CsgScratch {
   int32_t slots;  // of a row's sketch
   uint32_t *part_base, *part_off;
   bool no_heavy_rows = false;  // known on the host already: nothing for the chain kernel
+  bool one_stream = true;      // the call runs on one stream: its kernels may be programmatic dependent launches
   // compact_kernel's second list, tiled sort of heavy chunks (see transpose.cu)
   int32_t *next_chunk, *heavy_chunk, *heavy_tile_base;
   uint32_t *tile_hist, *digit_base;
@@ -305,9 +306,10 @@ __device__ __forceinline__ uint32_t entry_weight_bits(uint64_t e) {
 #endif
 
 #ifdef __CUDACC__
-// launch of a kernel that calls wait_for_kernels_before()
+// launch of a kernel that calls wait_for_kernels_before(), as a programmatic dependent one or like any other
 template <typename... Params, typename... Args>
-cudaError_t launch_behind(void (*kernel)(Params...), int grid, int threads, int smem, cudaStream_t st, Args... args) {
+cudaError_t launch_behind(bool dependent, void (*kernel)(Params...), int grid, int threads, int smem, cudaStream_t st,
+                          Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -317,7 +319,7 @@ cudaError_t launch_behind(void (*kernel)(Params...), int grid, int threads, int 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 #endif

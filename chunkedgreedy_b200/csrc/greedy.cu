@@ -171,6 +171,7 @@ __device__ __forceinline__ void chain_chunk(const GreedyArgs &a, int32_t start, 
 
 // Chunks whose lists do not fit shared memory: a warp each.
 __global__ void __launch_bounds__(G_WARPS * 32) greedy_kernel(GreedyArgs a) {
+  wait_for_kernels_before();
   extern __shared__ uint32_t g_smem[];
   const int warp = threadIdx.x >> 5;
   const int32_t q = blockIdx.x * G_WARPS + warp;
@@ -258,6 +259,7 @@ __device__ __noinline__ void chain_chunk_rare(const GreedyArgs &a, int32_t start
 // LONG: lists of more than 32 entries.
 template <bool STATS, bool LONG>
 __global__ void greedy_lists_kernel(GreedyArgs a) {
+  wait_for_kernels_before();
   extern __shared__ __align__(16) unsigned char gl_smem[];
   __shared__ int32_t odd, count;
   const int lane = lane_id(), warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -543,15 +545,13 @@ bool launch_greedy(Context &ctx, int32_t n, const CsgParams &p, CsgScratch &s,
       CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
       // many chunks: several blocks to an SM; few: more warps to write the lists of each
       const int threads = a.num_chunks <= 2 * ctx.num_sms ? 512 : 256;
-      kernel<<<a.num_chunks, threads, bytes, ctx.stream>>>(a);
-      CSG_CUDA(cudaGetLastError());
+      CSG_CUDA(launch_behind(s.one_stream, kernel, a.num_chunks, threads, bytes, ctx.stream, a));
       count_launches(1);
       return true;
     }
   }
   const int grid = (a.num_chunks + G_WARPS - 1) / G_WARPS;
-  greedy_kernel<<<grid, G_WARPS * 32, smem, ctx.stream>>>(a);
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(s.one_stream, greedy_kernel, grid, G_WARPS * 32, static_cast<int>(smem), ctx.stream, a));
   count_launches(1);
   return true;
 }

@@ -929,8 +929,8 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, a.counters + CNT_MOVED,
                                                           symmetric ? outcome : nullptr, ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
-  CSG_CUDA(launch_behind(scan_block_sums_kernel, 1, 1024, 0, ctx.stream, nb, block_sums));
-  CSG_CUDA(launch_behind(ptr_new_kernel, nb, R_THREADS, 0, ctx.stream, n, nnz, d_ptr_old, d_new_order, block_sums,
+  CSG_CUDA(launch_behind(true, scan_block_sums_kernel, 1, 1024, 0, ctx.stream, nb, block_sums));
+  CSG_CUDA(launch_behind(true, ptr_new_kernel, nb, R_THREADS, 0, ctx.stream, n, nnz, d_ptr_old, d_new_order, block_sums,
                          d_ptr_new, old2new, tile_row, row_delta));
   count_launches(3);
   if (nnz == 0) return true;
@@ -945,7 +945,7 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
     if (grid > ctx.num_sms * 32) grid = ctx.num_sms * 32;
     auto kernel = symmetric ? (with_vals ? apply_flat_kernel<false, true> : apply_flat_kernel<false, false>)
                             : (with_vals ? apply_flat_kernel<true, true> : apply_flat_kernel<true, false>);
-    CSG_CUDA(launch_behind(kernel, static_cast<int>(grid), R_THREADS, 0, ctx.stream, a));
+    CSG_CUDA(launch_behind(true, kernel, static_cast<int>(grid), R_THREADS, 0, ctx.stream, a));
     count_launches(1);
     return true;
   }

@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(S_THREADS) sketch_kernel(SketchArgs a, int all
   rows_by_warp<CELLS>(a, a.ctrl[all ? CTRL_ROWS_LISTED : CTRL_MID_END], ring_s[warp], ring_a[warp]);
   // Launched as the programmatic dependent of the heavy-chain kernel, this kernel starts
   // while that one is still running; it must not be seen as finished before it.
-  if (after_primary) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (after_primary) wait_for_kernels_before();
 }
 
 // ---- a row per lane -----------------------------------------------------------------------
@@ -970,7 +970,9 @@ __device__ __forceinline__ void select_phase(const SketchArgs &a, uint32_t *mem,
 
 template <int CELLS, typename Index>
 // (four blocks per SM by registers, so that one also fits beside the 18 warps of a chain block at 128 slots)
-__global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchArgs a) {
+__global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchArgs a, int wait_first) {
+  if (wait_first) wait_for_kernels_before();
+  let_next_kernel_start();
   using L = LaneLayout<CELLS>;
   extern __shared__ __align__(16) uint32_t lanes_mem[];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -1032,7 +1034,7 @@ __global__ void __launch_bounds__(32 * L_WARPS, 4) rows_in_lanes_kernel(SketchAr
   }
   // Launched as the programmatic dependent of the heavy-chain kernel (see launch_cells): it must
   // not be seen as finished before that one.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_kernels_before();
 }
 
 // ---- heavy rows through materialised streams ------------------------------------------
@@ -1063,6 +1065,8 @@ __device__ __forceinline__ PartRef part_ref(const SketchArgs &a, uint32_t part, 
 
 // Offsets of the heavy rows' streams in hstream; trims the heavy set to what fits.
 __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   __shared__ unsigned long long sm[32];
   __shared__ unsigned long long carry_s;
   __shared__ uint32_t count_s;
@@ -1130,6 +1134,8 @@ __global__ void __launch_bounds__(1024) heavy_offsets_kernel(SketchArgs a) {
 // adds up the parts of the row in front of it: one block that scanned all counts took 18 us of a call of
 // 360 (65,536 rows, some 300 parts) and 48 of one of 28 ms, the parts' own sums nothing that shows.
 __global__ void __launch_bounds__(256) heavy_part_count_kernel(SketchArgs a) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   const int lane = lane_id();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS], parts = a.ctrl[CTRL_HEAVY_PARTS];
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -1147,6 +1153,8 @@ __global__ void __launch_bounds__(256) heavy_part_count_kernel(SketchArgs a) {
 
 // one warp per part: its slice of the row's stream, written out in order
 __global__ void __launch_bounds__(S_THREADS) heavy_expand_kernel(SketchArgs a) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   __shared__ int32_t ring_s[S_WARPS][S_RING];
   __shared__ float ring_a[S_WARPS][S_RING];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -1197,7 +1205,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_consume_kernel(SketchArgs 
   if (heavy_pad[0] == 255 && a.n < 0) return;  // keeps the padding referenced
   // every block of this grid is resident now (one per SM): let the kernel of the other
   // rows, launched behind this one in the same stream, start on whatever is left
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_kernels_before();  // (first: the kernel of the other rows, which starts now, does not wait for the ones before)
+  let_next_kernel_start();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
   int32_t *bs = ring_s[warp];
   float *ba = ring_a[warp];
@@ -1899,7 +1908,8 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
   const int base = group * (G::tab_offset(span > MATES) + tab_bytes);
   RoundState<CELLS> &st = G::state(base);
   const int lane = lane_id(), warp = in_group >> 5, bars = 3 * group;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_kernels_before();  // (first: the kernel of the other rows, which starts now, does not wait for the ones before)
+  let_next_kernel_start();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
   for (int i = G::MATE + in_group * 16; i < G::tab_offset(span > MATES) + tab_bytes; i += THREADS * 16)
     *reinterpret_cast<uint4 *>(heavy_dyn + base + i) = make_uint4(0, 0, 0, 0);
@@ -2139,7 +2149,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_rounds_32_kernel(SketchArg
   int2(*const rings)[2][T_RING] = reinterpret_cast<int2(*)[2][T_RING]>(heavy_dyn);
   __shared__ State32 state[S_WARPS];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_kernels_before();  // (first: the kernel of the other rows, which starts now, does not wait for the ones before)
+  let_next_kernel_start();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
   uint8_t *const tab = heavy_dyn + sizeof(int2) * S_WARPS * 2 * T_RING + static_cast<size_t>(warp) * tab_bytes;
   for (int i = lane * 16; i < tab_bytes; i += 32 * 16) *reinterpret_cast<uint4 *>(tab + i) = make_uint4(0, 0, 0, 0);
@@ -2168,6 +2179,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_rounds_32_kernel(SketchArg
 
 template <int CELLS>
 __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
+  wait_for_kernels_before();
+  let_next_kernel_start();
   const int lane = lane_id();
   const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -2193,14 +2206,12 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   // (sketches beyond ROUND_CELLS) the two share the SMs, since the kernel of the other rows starts
   // only when every chain block has one.
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
+  const bool behind = phase == PHASE_ALL;
   constexpr bool in_rounds = CELLS >= WINDOW_CELLS && CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
-    heavy_offsets_kernel<<<1, 1024, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
-    heavy_part_count_kernel<<<ctx.num_sms * 4, 256, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
-    heavy_expand_kernel<<<ctx.num_sms * 8, S_THREADS, 0, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
+    CSG_CUDA(launch_behind(behind, heavy_offsets_kernel, 1, 1024, 0, st, a));
+    CSG_CUDA(launch_behind(behind, heavy_part_count_kernel, ctx.num_sms * 4, 256, 0, st, a));
+    CSG_CUDA(launch_behind(behind, heavy_expand_kernel, ctx.num_sms * 8, S_THREADS, 0, st, a));
     // (the rest of the call starts its own chains only behind this point: by then the chains
     // ahead, next in their stream, hold their SMs, and the kernel of the other rows cannot
     // settle on them first)
@@ -2214,8 +2225,8 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
       CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared));
-      heavy_rounds_32_kernel<<<ctx.num_sms, S_THREADS, ring_bytes + tab_bytes * S_WARPS, st>>>(a, tab_bytes);
-      CSG_CUDA(cudaGetLastError());
+      CSG_CUDA(launch_behind(false, heavy_rounds_32_kernel, ctx.num_sms, S_THREADS, ring_bytes + tab_bytes * S_WARPS, st, a,
+                             tab_bytes));
     }
     if constexpr (in_rounds) {
       const int64_t span = a.chunk < a.n ? a.chunk : a.n;
@@ -2229,8 +2240,10 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       // (all of an SM's memory as shared: a block of another split cannot move in beside this one)
       CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared));
-      heavy_rounds_kernel<CELLS><<<ctx.num_sms, Helpers<CELLS>::THREADS * groups, groups * group_bytes, st>>>(a, tab_bytes);
-      CSG_CUDA(cudaGetLastError());
+      // (a plain launch: started beside the end of the expansion, blocks gather on the SMs that are through first, and
+      // symmetrised R-MAT of scale 20 takes 29.4 ms instead of 27.7)
+      CSG_CUDA(launch_behind(false, heavy_rounds_kernel<CELLS>, ctx.num_sms, Helpers<CELLS>::THREADS * groups,
+                             groups * group_bytes, st, a, tab_bytes));
     }
     if constexpr (CELLS > ROUND_CELLS) {
       const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
@@ -2238,8 +2251,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, pad));
       const int ahead = prio_chain_blocks(ctx.num_sms);
       const int blocks = phase == PHASE_PRIO ? ahead : phase == PHASE_REST ? ctx.num_sms - ahead : ctx.num_sms;
-      heavy_consume_kernel<CELLS><<<blocks, S_THREADS, pad, st>>>(a);
-      CSG_CUDA(cudaGetLastError());
+      CSG_CUDA(launch_behind(false, heavy_consume_kernel<CELLS>, blocks, S_THREADS, pad, st, a));
     }
   }
   // The other rows run beside the heavy chains: their kernel follows in the same stream
@@ -2276,7 +2288,8 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
       return false;
   } else if constexpr (CELLS <= LANE_CELLS) {
     auto lanes = [&](auto kernel, int index_words) {
-      return launch_light(kernel, 32 * L_WARPS, (LaneLayout<CELLS>::I_OFF + index_words) * 4, !no_heavy_rows);
+      return launch_light(kernel, 32 * L_WARPS, (LaneLayout<CELLS>::I_OFF + index_words) * 4, behind || !no_heavy_rows,
+                          no_heavy_rows ? 1 : 0);
     };
     if (span <= L_TABLE_MAX) {
       if (!lanes(rows_in_lanes_kernel<CELLS, TableIndex<CELLS>>, TableIndex<CELLS>::words(span))) return false;
@@ -2286,8 +2299,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   }
   count_launches(1);
   if (no_heavy_rows) return true;
-  heavy_topk_kernel<CELLS><<<ctx.num_sms, S_THREADS, 0, st>>>(a);
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(behind, heavy_topk_kernel<CELLS>, ctx.num_sms, S_THREADS, 0, st, a));
   count_launches(5);
   return true;
 }

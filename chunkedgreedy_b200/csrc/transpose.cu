@@ -165,6 +165,8 @@ __device__ __forceinline__ uint32_t column_hash(uint32_t c) { return c * 0x9E377
 // goes to the tiled sort.
 template <typename S, bool NEXT, bool LAST>
 __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename S::Shared &sh = *reinterpret_cast<typename S::Shared *>(smem_raw);
   constexpr int THREADS = S::THREADS, U = 8;
@@ -741,6 +743,8 @@ __device__ __forceinline__ bool taken_ahead(uint32_t prio, uint32_t least, int32
 // rows and candidates per bucket of row_work
 __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint32_t *row_work,
                                                            uint32_t *ctrl, int32_t chunk, const uint32_t *ctrl_ahead) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   __shared__ uint32_t bucket[WORK_BUCKETS];
   __shared__ unsigned long long work[WORK_BUCKETS];  // (of rows that may get a chain)
   if (threadIdx.x < WORK_BUCKETS) {
@@ -807,6 +811,8 @@ ChainCosts chain_costs(const Context &ctx, int slots, bool key_table, uint32_t r
 // with four, 14.2 with five.
 __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, uint32_t ticket, int octaves,
                                    const uint32_t *ctrl_ahead, ChainCosts cost) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   const int lane = threadIdx.x;
   uint32_t c[4], sum = 0;
 #pragma unroll
@@ -920,6 +926,8 @@ constexpr int LIST_ROWS = 4;  // rows per thread and step
 __global__ void __launch_bounds__(256) row_list_kernel(int32_t n, const uint32_t *__restrict__ row_work, uint32_t *ctrl,
                                                        int32_t *__restrict__ row_list, int32_t chunk,
                                                        const uint32_t *ctrl_ahead) {
+  let_next_kernel_start();
+  wait_for_kernels_before();
   __shared__ uint32_t bucket[WORK_BUCKETS];  // rows of the step, then the place of its first
   const int lane = threadIdx.x & 31;
   const int32_t step = blockDim.x * LIST_ROWS;
@@ -1034,8 +1042,7 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
   auto launch = [&](auto kernel, int threads, size_t smem, int per_sm) -> bool {
     CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const int grid = a.num_chunks < ctx.num_sms * per_sm ? a.num_chunks : ctx.num_sms * per_sm;
-    kernel<<<grid, threads, smem, st>>>(a);
-    CSG_CUDA(cudaGetLastError());
+    CSG_CUDA(launch_behind(!a.skip_prio, kernel, grid, threads, static_cast<int>(smem), st, a));
     return true;
   };
   const int32_t rows = a.chunk < a.n ? a.chunk : a.n;
@@ -1058,18 +1065,16 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
 bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead) {
   int grid = (n + 255) / 256;
   if (grid > ctx.num_sms * 8) grid = ctx.num_sms * 8;
-  bucket_count_kernel<<<grid, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, chunk, ctrl_ahead);
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(s.one_stream, bucket_count_kernel, grid, 256, 0, ctx.stream, n, s.row_work, s.ctrl, chunk, ctrl_ahead));
   const int32_t span = chunk < n ? chunk : n;
   const int octaves = span <= LANE_TABLE_ROWS ? 0 : span <= WARP_FEW_ROWS ? 4 : 3;
-  bucket_scan_kernel<<<1, 32, 0, ctx.stream>>>(s.ctrl, reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD,
-                                               ++ctx.outcome_ticket, octaves, ctrl_ahead,
-                                               chain_costs(ctx, s.slots, span <= LANE_TABLE_ROWS, s.heavy_max, s.stream_cap));
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(s.one_stream, bucket_scan_kernel, 1, 32, 0, ctx.stream, s.ctrl,
+                         reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD, ++ctx.outcome_ticket, octaves, ctrl_ahead,
+                         chain_costs(ctx, s.slots, span <= LANE_TABLE_ROWS, s.heavy_max, s.stream_cap)));
   int steps = static_cast<int>((static_cast<int64_t>(n) + 256 * LIST_ROWS - 1) / (256 * LIST_ROWS));
   if (steps > ctx.num_sms * 32) steps = ctx.num_sms * 32;
-  row_list_kernel<<<steps, 256, 0, ctx.stream>>>(n, s.row_work, s.ctrl, s.row_list, chunk, ctrl_ahead);
-  CSG_CUDA(cudaGetLastError());
+  CSG_CUDA(launch_behind(s.one_stream, row_list_kernel, steps, 256, 0, ctx.stream, n, s.row_work, s.ctrl, s.row_list, chunk,
+                         ctrl_ahead));
   count_launches(3);
   return true;
 }
