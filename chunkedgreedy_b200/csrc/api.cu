@@ -319,19 +319,19 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
   // there while the context's stream transposes everything else; the two meet before the
   // greedy stage.  Results do not depend on the split (the same kernels on the same rows).
   // By default for calls of 2^24 nonzeros in 64 chunks or more, whose chunk ahead must hold 2^17 nonzeros:
-  // smaller calls do not pay for the second pipeline's fifteen launches.  With 96 and 128 slots the chains
-  // of the two parts slow each other where rows are long, and with 32, where a chain is one warp, nearly
-  // everywhere.  Time ahead over time not, R-MAT and its symmetrised form of 19 to 65 M nonzeros: 32 slots
-  // 1.02 to 1.63 in chunks of 1024 (R-MAT scale 22 111 and 71 ms), 0.95 to 1.43 in other chunks; 64 slots
-  // 0.62 to 0.99 from ten nonzeros a row on (1.07 at five); 96 slots 0.90 to 0.99 up to 12 nonzeros a row,
-  // 1.00 at 16, 1.03 to 1.06 from 23 on; 128 slots 0.83 to 0.90 up to 16, 0.92 to 0.99 at 23, 1.05 to 1.11
-  // from 27 on; 160 and 256 slots (a warp per row) 0.97 to 0.99; in chunks of 4096, 64 to 128 slots 0.88 to
+  // smaller calls do not pay for the second pipeline's fifteen launches.  With 32 slots, where a chain is one warp,
+  // the chains of the two parts slow each other nearly everywhere, with 96 and 128 in tall chunks, and with 128
+  // where rows are long.  Time ahead over time not, R-MAT and its symmetrised form of 19 to 65 M nonzeros, chunks of
+  // 512 to 1024: 32 slots 1.57 (R-MAT scale 22 111 and 71 ms); 64 slots 0.90 to 0.95; 96 slots 0.81 to 0.95 at 10 to
+  // 31 nonzeros a row; 128 slots 0.84 to 0.96 up to 27, 1.02 to 1.07 from there on, 0.90 to 0.95 in chunks of 512;
+  // 160 and 256 slots (a warp per row) 0.97 to 0.99; in chunks of 4096, 96 slots 1.07, 128 slots 1.28, 64 slots 0.88 to
   // 1.15.  A caller's own threshold (sporder_context_set_ahead_threshold) applies to any call of two chunks.
   const int64_t chunks = (static_cast<int64_t>(n) + p.chunk - 1) / p.chunk;
   bool ahead = ctx.side_stream != nullptr && p.chunk <= 4096;
   int32_t ahead_chunk_nnz = 1 << 17;
   if (ctx.ahead_min_nnz == 0) {
-    const bool slowed = p.M == 32 || (p.M == 96 && nnz >= 14ll * n) || (p.M == 128 && nnz >= 25ll * n);
+    const bool slowed = p.M == 32 || (p.chunk > 2048 && (p.M == 96 || p.M == 128)) ||
+                        (p.chunk > 512 && p.M == 128 && nnz >= 27ll * n);
     ahead = ahead && nnz >= AHEAD_MIN_NNZ && chunks >= 64 && !slowed;
   } else {
     ahead = ahead && ctx.ahead_min_nnz > 0 && nnz >= ctx.ahead_min_nnz && chunks >= 2;
