@@ -543,8 +543,9 @@ bool launch_greedy(Context &ctx, int32_t n, const CsgParams &p, CsgScratch &s,
       auto kernel = with_stats ? (lng ? greedy_lists_kernel<true, true> : greedy_lists_kernel<true, false>)
                                : (lng ? greedy_lists_kernel<false, true> : greedy_lists_kernel<false, false>);
       CSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      // many chunks: several blocks to an SM; few: more warps to write the lists of each
-      const int threads = a.num_chunks <= 2 * ctx.num_sms ? 512 : 256;
+      // many chunks: several blocks to an SM; few: more warps to write the lists of each (64 chunks 83.8 us with 512
+      // threads, 81.6 with 1024; 4 chunks 91.6 and 87.4)
+      const int threads = a.num_chunks <= ctx.num_sms ? 1024 : a.num_chunks <= 2 * ctx.num_sms ? 512 : 256;
       CSG_CUDA(launch_behind(s.one_stream, kernel, a.num_chunks, threads, bytes, ctx.stream, a));
       count_launches(1);
       return true;
