@@ -1274,11 +1274,12 @@ __global__ void __launch_bounds__(S_THREADS, 1) heavy_consume_kernel(SketchArgs 
 // rounds that ended at the first open element that is not held, and now: R-MAT scale 20, 64 slots, longest row
 // 23.4 -> 15.9, rows of 166,000 / 76,000 / 30,000 candidates 51 -> 20.8, 89 -> 27.0, 184 -> 39.2; symmetrised scale 19,
 // 128 slots, longest 29.4 -> 18.2, 146,000 / 61,000 candidates 41 -> 26.5, 78 -> 31.7; power-law band of 4,096 rows
-// 26.7 -> 16.4.
+// 26.7 -> 16.4.  32 slots, by windows of 32, which had a warp per row and strict rounds: whole calls 33.5 -> 12.0 ms (R-MAT
+// scale 20, k = 8), 5.3 -> 2.1 (top-k graph of an R-MAT matrix of 13,400 rows), 71.6 -> 21.9 (symmetrised, 262,144 rows
+// in chunks of 4,096).
 constexpr int H_RING = 1024;     // stream elements in a row's ring ...
 constexpr int H_SEG = 256;       // ... staged this many at a time
 constexpr int ROUND_CELLS = 4;   // largest sketch (cells per lane) resolved in rounds
-constexpr int WINDOW_CELLS = 2;  // smallest sketch resolved by a group of warps (32 slots: heavy_rounds_32_kernel)
 constexpr int MATES = 1024;      // words of the duplicate detector (two for 64 elements)
 constexpr int ROUND_TAB_MAX = 65536;  // largest chunk (rows) with a key -> slot table
 constexpr int TRIAL_ROUNDS = 8;     // rounds of each width a row times before it settles on one ...
@@ -1288,7 +1289,7 @@ struct Helpers {
   static constexpr int N = 2 * CELLS;                    // warps that order the slots, sixteen slots each
   // Groups (rows) per block, one block per SM: with two the registers of an SM still hold two
   // blocks of rows_in_lanes_kernel (one at 96 slots and more), which does most of the work of a large call.
-  static constexpr int ROWS = 2;
+  static constexpr int ROWS = CELLS == 1 ? 4 : 2;
   static constexpr int THREADS = 32 * (1 + N);           // of a group
 };
 // named barriers of a group: row in hand, state is ready to be ordered, the order is ready
@@ -1762,15 +1763,6 @@ __device__ __forceinline__ int round_fill(const RoundRow &row, uint32_t p, uint3
   return L;
 }
 
-// copies `cnt` stream elements into a ring buffer without passing through registers
-__device__ __forceinline__ void stage_batch(int2 *ring, const int2 *in, int cnt, int lane) {
-  for (int i = lane; i < cnt; i += 32) {
-    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ring + i));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(in + i) : "memory");
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
 // copies the H_SEG stream elements from `from` on (those in front of `total`) into the ring without passing
 // through registers
 __device__ __forceinline__ void stage_segment(int2 *ring, const int2 *in, uint32_t from, uint32_t total, int lane) {
@@ -1862,7 +1854,11 @@ __device__ __noinline__ void rounds_row(const int2 *in, uint32_t total, const Ro
   while (s.p < total) {
     const uint32_t from = s.p;
     const long long t0 = clock64();
-    const uint2 at = wide ? window_rounds<CELLS, 2, TAB, HASH>(row, s, left) : window_rounds<CELLS, 1, TAB, HASH>(row, s, left);
+    uint2 at;
+    if constexpr (CELLS == 1)  // (a window of 64 would need more entries than there are)
+      at = window_rounds<CELLS, 1, TAB, HASH>(row, s, 1 << 20);
+    else
+      at = wide ? window_rounds<CELLS, 2, TAB, HASH>(row, s, left) : window_rounds<CELLS, 1, TAB, HASH>(row, s, left);
     s.p = at.x;
     s.seg = at.y;
     if (trial >= 0) {
@@ -1952,231 +1948,6 @@ __global__ void __launch_bounds__(Helpers<CELLS>::THREADS *Helpers<CELLS>::ROWS)
   }
 }
 
-// ---- 32 slots ------------------------------------------------------------------------------
-// A warp per row: a lane orders its own slot while the look-ups of the window are under way, in
-// fewer cycles than a group's barriers take.  Longest row of R-MAT scale 16
-// (101,366 candidates): 9.9 ms by a group of three warps, 7.7 this way, 145 cycles per candidate;
-// bound by the dependent steps of a round, as the larger sketches are.  Rows are drawn as warps ask,
-// so that the longest share an SM: spread one to an SM (the others empty), the same rounds took 10.9 ms of a
-// whole call that takes 8.1; with eight warps to a block 9.8.  What a round costs also hangs on how the
-// compiler orders it: with a row's places in a struct a call took 12.1 ms, as arguments 8.1.
-constexpr int T_RING = 1024;
-struct State32 {
-  __align__(16) uint32_t w[32];  // as in RoundState
-  __align__(16) int32_t key[32];
-  uint32_t sw[32];
-  int32_t si[32], sk[32], rank[32], miss_pos[32];
-  uint32_t fence_sink;
-};
-// Keeps the phases of a round apart in the instruction schedule: left alone, ptxas interleaves the
-// look-ups, the count and the limits, and a round takes a tenth longer than with a read of %clock
-// between them (which it does not move code across, as long as the value is used).
-__device__ __forceinline__ void phase_fence(uint32_t &sink) {
-  uint32_t t;
-  asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
-  sink ^= t;
-}
-
-// the key of element e, with a table relative to the chunk (one outside the chunk only comes from rows that are
-// not sorted: kept in bounds)
-template <bool TAB>
-__device__ __forceinline__ int32_t key_32(uint32_t *ctrl, int32_t e, int32_t cbase, int32_t span) {
-  const uint32_t rel = static_cast<uint32_t>(key_in_chunk(ctrl, e, cbase, span) - cbase);
-  return static_cast<int32_t>(min(rel, static_cast<uint32_t>(span) - 1u)) + (TAB ? 0 : cbase);
-}
-template <bool TAB>
-__device__ __forceinline__ int slot_32(const State32 &st, const uint8_t *tab, int32_t s) {
-  if (TAB) return static_cast<int>(tab[s]) - 1;
-  int q = -1;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int4 kk = reinterpret_cast<const int4 *>(st.key)[i];
-    q = kk.x == s ? 4 * i : q;
-    q = kk.y == s ? 4 * i + 1 : q;
-    q = kk.z == s ? 4 * i + 2 : q;
-    q = kk.w == s ? 4 * i + 3 : q;
-  }
-  return q;
-}
-
-// One round on a full sketch of 32 slots (the slot code is the lane): the longest prefix of the window for which
-// (1) no two of its misses carry the same key, (2) no hit lands on an entry that a miss of the prefix takes, and
-// (3) every entry put back stays above the last one taken - then the i-th miss takes the i-th entry of the order.
-template <bool TAB>
-__device__ __forceinline__ int strict_32(State32 &st, uint8_t *tab, int32_t cbase, int32_t span, uint32_t *ctrl,
-                                         const int2 *ring, int p, int cnt, int lane, uint32_t &sink) {
-  const uint32_t below = (1u << lane) - 1u;
-  phase_fence(sink);
-  const bool valid = p + lane < cnt;
-  const int2 elem = valid ? ring[p + lane] : make_int2(cbase, 0);
-  const int32_t s = key_32<TAB>(ctrl, elem.x, cbase, span);
-  const float al = __int_as_float(elem.y);
-  const uint32_t mine = st.w[lane];
-  const int32_t mykey = st.key[lane];
-  const int q = valid ? slot_32<TAB>(st, tab, s) : 0;
-  const bool miss = valid && q < 0, hit = valid && q >= 0;
-  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
-  const uint32_t wq = st.w[hit ? q : 0];
-  const uint32_t missing = __ballot_sync(FULL, miss);
-  const int mtot = __popc(missing), mrank = __popc(missing & below);
-  phase_fence(sink);
-  // entries (x, i) below (mine, lane): weight bits are below 2^31, so x < y is the sign of x - y
-  int32_t acc[4] = {0, 0, 0, 0};
-  uint4 v[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = reinterpret_cast<const uint4 *>(st.w)[i];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[e] += static_cast<int32_t>(x[e] - mine - ((below >> (4 * i + e)) & 1u)) >> 31;
-  }
-  const int pos = -((acc[0] + acc[1]) + (acc[2] + acc[3]));
-  st.sw[pos] = mine;
-  st.si[pos] = lane;
-  st.sk[pos] = mykey;
-  st.rank[lane] = pos;
-  phase_fence(sink);
-  if (miss) st.miss_pos[mrank] = lane;
-  __syncwarp();
-  phase_fence(sink);
-  const int rho = st.rank[hit ? q : 0];
-  const int tgt = st.si[mrank];
-  const uint32_t base = st.sw[mrank];
-  const int32_t old_key = st.sk[mrank];
-  const uint32_t top = st.sw[mtot > 0 ? mtot - 1 : 0];
-  const int at_hit = st.miss_pos[rho];
-  const int at_next = st.miss_pos[(mrank + 1) & 31];
-  const uint32_t nb = __float_as_uint(__uint_as_float(base) + al);
-  int lim = valid ? 32 : lane;
-  if (hit) {
-    const int at = rho < mtot ? at_hit : 32;
-    lim = at > lane ? at : lane;
-  }
-  if (miss) {
-    if (nb <= top) lim = nb > base ? (mrank + 1 < mtot ? at_next : 32) : lane;
-    if (same & below) lim = lane;
-  }
-  phase_fence(sink);
-  int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
-  L = L < 1 ? 1 : L;
-  const bool applies = lane < L;
-  const unsigned mates = same & (L >= 32 ? FULL : (1u << L) - 1u);
-  const int times = __popc(mates);
-  float wv = __uint_as_float(wq) + al;
-  if (times > 1) wv += al;  // (most of the repeats there are, without a loop)
-  if (times > 2)
-    for (int t = 2; t < times; ++t) wv += al;
-  if (applies && miss) {
-    if (TAB) tab[old_key] = 0;
-    st.key[tgt] = s;
-    st.w[tgt] = nb;
-    if (TAB) tab[s] = static_cast<uint8_t>(tgt + 1);
-  }
-  if (applies && hit && (mates & below) == 0u) st.w[q] = __float_as_uint(wv);
-  __syncwarp();
-  return L;
-}
-template <bool TAB>
-__device__ __forceinline__ int fill_32(State32 &st, uint8_t *tab, int32_t cbase, int32_t span, uint32_t *ctrl,
-                                       const int2 *ring, int p, int cnt, int lane, int &filled) {
-  const uint32_t below = (1u << lane) - 1u;
-  const bool valid = p + lane < cnt;
-  const int2 elem = valid ? ring[p + lane] : make_int2(cbase, 0);
-  const int32_t s = key_32<TAB>(ctrl, elem.x, cbase, span);
-  const float al = __int_as_float(elem.y);
-  const int q = valid ? slot_32<TAB>(st, tab, s) : 0;
-  const bool miss = valid && q < 0, hit = valid && q >= 0;
-  const uint32_t missing = __ballot_sync(FULL, miss);
-  const int mrank = __popc(missing & below);
-  const unsigned same = __match_any_sync(FULL, valid ? s : -1 - lane);
-  int lim = valid ? 32 : lane;
-  if (miss && ((same & below) || mrank >= 32 - filled)) lim = lane;
-  const int L = static_cast<int>(__reduce_min_sync(FULL, static_cast<uint32_t>(lim)));
-  const unsigned prefix = L >= 32 ? FULL : (1u << L) - 1u;
-  if (lane < L) {
-    if (miss) {
-      const int j = filled + mrank;
-      st.key[j] = s;
-      st.w[j] = __float_as_uint(al);
-      if (TAB) tab[s] = static_cast<uint8_t>(j + 1);
-    } else if (hit && ((same & prefix) & below) == 0u) {
-      float wv = __uint_as_float(st.w[q]);
-      for (int t = __popc(same & prefix); t > 0; --t) wv += al;
-      st.w[q] = __float_as_uint(wv);
-    }
-  }
-  filled += __popc(missing & prefix);
-  __syncwarp();
-  return L;
-}
-
-template <bool TAB>
-__device__ __noinline__ void row_32(const int2 *in, uint32_t total, State32 &st, uint8_t *tab, int32_t cbase, int32_t span,
-                                    uint32_t *ctrl, int2 *ring0, int2 *ring1, int32_t *out) {
-  const int lane = lane_id();
-  st.key[lane] = -1;
-  st.w[lane] = 0u;
-  int filled = 0, buf = 0;
-  uint32_t sink = 0;
-  __syncwarp();
-  stage_batch(ring0, in, static_cast<int>(total < T_RING ? total : T_RING), lane);
-  for (uint32_t base = 0; base < total; base += T_RING) {
-    const int cnt = static_cast<int>(total - base < T_RING ? total - base : T_RING);
-    const uint32_t next = base + T_RING;
-    if (next < total)
-      stage_batch(buf ? ring0 : ring1, in + next, static_cast<int>(total - next < T_RING ? total - next : T_RING), lane);
-    else
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest group: this batch is in
-    __syncwarp();
-    const int2 *const ring = buf ? ring1 : ring0;
-    int p = 0;
-    while (p < cnt && filled < 32) p += fill_32<TAB>(st, tab, cbase, span, ctrl, ring, p, cnt, lane, filled);
-    while (p < cnt) p += strict_32<TAB>(st, tab, cbase, span, ctrl, ring, p, cnt, lane, sink);
-    buf ^= 1;
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  const int32_t kk = st.key[lane];
-  out[lane] = TAB && kk >= 0 ? kk + cbase : kk;
-  out[32 + lane] = static_cast<int32_t>(st.w[lane]);
-  if (TAB && kk >= 0) tab[kk] = 0;  // the table is empty again for the next row
-  if (lane == 0) st.fence_sink = sink;
-  __syncwarp();
-}
-
-__global__ void __launch_bounds__(S_THREADS, 1) heavy_rounds_32_kernel(SketchArgs a, int tab_bytes) {
-  int2(*const rings)[2][T_RING] = reinterpret_cast<int2(*)[2][T_RING]>(heavy_dyn);
-  __shared__ State32 state[S_WARPS];
-  const int lane = lane_id(), warp = threadIdx.x >> 5;
-  wait_for_kernels_before();  // (first: the kernel of the other rows, which starts now, does not wait for the ones before)
-  let_next_kernel_start();
-  const uint32_t heavy = a.ctrl[CTRL_HEAVY_ROWS];
-  uint8_t *const tab = heavy_dyn + sizeof(int2) * S_WARPS * 2 * T_RING + static_cast<size_t>(warp) * tab_bytes;
-  for (int i = lane * 16; i < tab_bytes; i += 32 * 16) *reinterpret_cast<uint4 *>(tab + i) = make_uint4(0, 0, 0, 0);
-  __syncwarp();
-  for (;;) {
-    uint32_t item = 0;
-    if (lane == 0) item = atomicAdd(&a.ctrl[CTRL_HEAVY_TICKET + 1], 1u);
-    item = __shfl_sync(FULL, item, 0);
-    if (item >= heavy) break;
-    const int32_t r = a.row_list[item];
-    // checked build: the row, its place in the state array and its stream's extent
-    if (!index_ok(a.ctrl, CHK_LIST, r, a.n) || !index_ok(a.ctrl, CHK_STATE, item, a.heavy_max) ||
-        !index_ok(a.ctrl, CHK_STREAM, static_cast<long long>(a.heavy_off[item]) + a.row_work[r],
-                  static_cast<long long>(a.stream_cap) + 1))
-      continue;
-    const int32_t cbase = (r / a.chunk) * a.chunk, span = a.chunk < a.n ? a.chunk : a.n;
-    int32_t *const out = a.heavy_state + static_cast<size_t>(item) * (2 * 32);
-    if (tab_bytes > 0)
-      row_32<true>(a.hstream + a.heavy_off[item], a.row_work[r], state[warp], tab, cbase, span, a.ctrl, rings[warp][0],
-                   rings[warp][1], out);
-    else  // chunk too large for key tables in shared memory
-      row_32<false>(a.hstream + a.heavy_off[item], a.row_work[r], state[warp], tab, cbase, span, a.ctrl, rings[warp][0],
-                    rings[warp][1], out);
-  }
-}
-
 template <int CELLS>
 __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
   wait_for_kernels_before();
@@ -2207,7 +1978,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
   // only when every chain block has one.
   cudaStream_t st = phase == PHASE_PRIO ? ctx.side_stream : ctx.stream;
   const bool behind = phase == PHASE_ALL;
-  constexpr bool in_rounds = CELLS >= WINDOW_CELLS && CELLS <= ROUND_CELLS;
+  constexpr bool in_rounds = CELLS <= ROUND_CELLS;
   if (!no_heavy_rows) {
     CSG_CUDA(launch_behind(behind, heavy_offsets_kernel, 1, 1024, 0, st, a));
     CSG_CUDA(launch_behind(behind, heavy_part_count_kernel, ctx.num_sms * 4, 256, 0, st, a));
@@ -2217,17 +1988,6 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
     // settle on them first)
     if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
     // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a group of warps per row.
-    if constexpr (CELLS == 1) {
-      const int64_t tab = (static_cast<int64_t>(a.chunk < a.n ? a.chunk : a.n) + 15) / 16 * 16;
-      const int ring_bytes = static_cast<int>(sizeof(int2)) * S_WARPS * 2 * T_RING;
-      const int room = ctx.smem_optin - 1024 - static_cast<int>(sizeof(State32)) * S_WARPS;
-      const int tab_bytes = ring_bytes + tab * S_WARPS <= room ? static_cast<int>(tab) : 0;
-      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
-      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_32_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    cudaSharedmemCarveoutMaxShared));
-      CSG_CUDA(launch_behind(false, heavy_rounds_32_kernel, ctx.num_sms, S_THREADS, ring_bytes + tab_bytes * S_WARPS, st, a,
-                             tab_bytes));
-    }
     if constexpr (in_rounds) {
       const int64_t span = a.chunk < a.n ? a.chunk : a.n;
       const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;

@@ -786,13 +786,13 @@ ChainCosts chain_costs(const Context &ctx, int slots, bool key_table, uint32_t r
   ChainCosts c = {};
   c.rows_max = rows_max;
   c.stream_cap = stream_cap;
-  if (slots < 64 || slots > 128) return c;
-  c.groups = 2.0f * static_cast<float>(ctx.num_sms);
-  c.chain = slots == 64 ? 0.030f : slots == 96 ? 0.035f : 0.052f;
-  c.alone = slots == 64 ? 0.018f : 0.021f;
+  if (slots > 128) return c;
+  c.groups = (slots == 32 ? 4.0f : 2.0f) * static_cast<float>(ctx.num_sms);
+  c.chain = slots == 32 ? 0.050f : slots == 64 ? 0.030f : slots == 96 ? 0.035f : 0.052f;
+  c.alone = slots == 32 ? 0.028f : slots == 64 ? 0.018f : 0.021f;
   c.row = 3.0f;
   c.lane = key_table ? 0.24f : 0.40f;
-  c.lanes = (key_table ? (slots == 64 ? 5.5e-5f : 7.5e-5f) : 1.0e-4f) * 148.0f / static_cast<float>(ctx.num_sms);
+  c.lanes = (key_table ? (slots <= 64 ? 5.5e-5f : 7.5e-5f) : 1.0e-4f) * 148.0f / static_cast<float>(ctx.num_sms);
   c.start = 30.0f;
   c.list = 0.015f;
   c.expand = 6.0e-6f;
