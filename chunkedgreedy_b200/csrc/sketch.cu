@@ -15,8 +15,8 @@
 // What differs is the machinery:
 //  * rows come from a work list ordered by the length of their stream, longest first: a
 //    stream is an order-dependent chain;
-//  * the longest rows (65536 candidates or more, and shorter ones while they are few) set the
-//    run time.  Their streams are written out to memory by the whole grid (heavy_expand_kernel,
+//  * the longest rows (65536 candidates or more, and of the shorter ones as many as let both kernels end
+//    soonest) set the run time.  Their streams are written out to memory by the whole grid (heavy_expand_kernel,
 //    one warp per 128 columns); then a group of warps works on each row and resolves up to 64
 //    candidates per round (see "the chains in rounds" below);
 //  * all other rows run side by side, one per LANE: the container of a row is a column of
