@@ -221,6 +221,9 @@ __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 // Programmatic dependent launches: the blocks of a kernel may be placed while the kernel in front of it in its stream
 // still runs, once all of that one's blocks run or are through.  Such a kernel waits before it touches anything an
 // earlier one of the call writes; each of them waits, so that the end of one means the end of all before it.
+// Nothing an earlier kernel of the call writes may be read through a pointer to const that is __restrict__, or by
+// __ldg: both promise that the memory stays the same for as long as the kernel runs, the time before the wait included,
+// and the load may go through the read-only path or in front of the wait.  The caller's own arrays may.
 __device__ __forceinline__ void wait_for_kernels_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

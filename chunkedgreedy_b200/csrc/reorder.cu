@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32
 
 __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     int32_t n, int32_t nnz, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
-    const int32_t *__restrict__ block_sums, int32_t *__restrict__ ptr_new,
+    const int32_t *block_sums, int32_t *__restrict__ ptr_new,
     int32_t *__restrict__ old2new, int32_t *__restrict__ tile_row, int32_t *__restrict__ row_delta) {
   let_next_kernel_start();
   constexpr int WARPS = R_THREADS / 32;
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
       const int32_t t = __shfl_up_sync(FULL, run, off);
       if (lane >= off) run += t;
     }
-    run += block_sums[blockIdx.x];
+    run += __ldcg(block_sums + blockIdx.x);
     sums[2 * lane] = run - x - y;
     sums[2 * lane + 1] = run - y;
   }

@@ -923,8 +923,8 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
 // The list itself.  A block draws the places of a step's rows bucket by bucket: with an atomic per warp and bucket
 // on the few counters that all rows share, the kernel took 15.3 us at 1,048,576 rows of a mesh, now 9.5.
 constexpr int LIST_ROWS = 4;  // rows per thread and step
-__global__ void __launch_bounds__(256) row_list_kernel(int32_t n, const uint32_t *__restrict__ row_work, uint32_t *ctrl,
-                                                       int32_t *__restrict__ row_list, int32_t chunk,
+__global__ void __launch_bounds__(256) row_list_kernel(int32_t n, const uint32_t *row_work, uint32_t *ctrl,
+                                                       int32_t *row_list, int32_t chunk,
                                                        const uint32_t *ctrl_ahead) {
   let_next_kernel_start();
   wait_for_kernels_before();
@@ -941,7 +941,7 @@ __global__ void __launch_bounds__(256) row_list_kernel(int32_t n, const uint32_t
 #pragma unroll
     for (int i = 0; i < LIST_ROWS; ++i) {
       const int64_t r = base + i * blockDim.x + threadIdx.x;
-      uint32_t t = r < n ? row_work[r] : 0u;
+      uint32_t t = r < n ? __ldcg(row_work + r) : 0u;
       if (r < n && taken_ahead(prio, least, chunk, static_cast<int32_t>(r), t)) t = 0;
       bkt[i] = t ? work_bucket(t) : -1;
     }
