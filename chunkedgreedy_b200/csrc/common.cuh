@@ -196,7 +196,6 @@ bool launch_table_stats(Context &ctx, int32_t n, int32_t k, const uint64_t *tabl
 bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_old,
                     const int32_t *d_ind_old, const float *d_val_old, const int32_t *d_new_order,
                     int mode, int32_t *d_ptr_new, int32_t *d_ind_new, float *d_val_new);
-size_t reorder_workspace_bytes(int32_t n, int32_t nnz, int mode);
 
 bool launch_spmm(Context &ctx, int32_t n, int32_t nnz, int32_t w, const int32_t *d_ptr,
                  const int32_t *d_ind, const float *d_val, const float *d_B, float *d_C);

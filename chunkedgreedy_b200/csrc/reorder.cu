@@ -27,6 +27,7 @@
 // among themselves.  len_block_sums_kernel notices such a permutation and tells the host, which then
 // launches apply_flat_kernel instead of the kernels above.  That one, which also does the copy
 // of the rows-only mode, cuts the output into tiles of 128 entries whatever rows they belong to.
+#include <algorithm>
 #include <cstddef>
 
 #include "common.cuh"
@@ -43,47 +44,32 @@ constexpr int FLAT_TILE = 128;                       // output entries per tile 
 constexpr int R_WARP = 256;                          // longest row sorted by one warp in registers
 constexpr int R_MED = 4096;                          // longest row (and tile of a longer row) sorted in shared memory
 
-__device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *total, int32_t *sm) {
-  // sm: R_THREADS/32 ints of shared memory
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t incl = v;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int32_t t = __shfl_up_sync(FULL, incl, off);
-    if (lane >= off) incl += t;
-  }
-  __syncthreads();
-  if (lane == 31) sm[warp] = incl;
-  __syncthreads();
-  int32_t base = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < R_THREADS / 32; ++w) {
-    const int32_t t = sm[w];
-    if (w < warp) base += t;
-    tot += t;
-  }
-  *total = tot;
-  return base + incl - v;
+// What lies in front of a row: entries in the low half, rows that have any in the high one.
+using RowCount = unsigned long long;
+__device__ __forceinline__ RowCount row_count(uint32_t entries, uint32_t rows) {
+  return static_cast<RowCount>(rows) << 32 | entries;
 }
 
-// Entries of the rows that each block of new rows takes.  With `outcome`, the last block also tells the host
+// Entries and rows with entries that each block of new rows takes.  With `outcome`, the last block also tells the host
 // whether any row leaves its block of 1024: here and not in ptr_new_kernel, so that the host reads it and
 // launches the rest while the scan still runs (a random order of a 65,536-row mesh: 90 us with the
 // wait behind ptr_new_kernel, 84 here).  The kernels behind it are programmatic dependent launches: 8 us less a call.
 __global__ void __launch_bounds__(R_THREADS) len_block_sums_kernel(
     int32_t n, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
-    int32_t *__restrict__ block_sums, uint32_t *__restrict__ leaves_block, volatile uint32_t *outcome, uint32_t ticket) {
+    RowCount *__restrict__ block_sums, uint32_t *__restrict__ leaves_block, volatile uint32_t *outcome, uint32_t ticket) {
   let_next_kernel_start();
-  __shared__ int32_t sm[R_THREADS / 32];
+  __shared__ RowCount sm[R_THREADS / 32];
   const int32_t base = blockIdx.x * R_SCAN_TILE;
-  int32_t s = 0;
+  uint32_t s = 0, rows = 0;
   int moved = 0;
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
     const int32_t p = base + i * R_THREADS + threadIdx.x;
     if (p < n) {
       const int32_t src = new_order[p];
-      s += ptr_old[src + 1] - ptr_old[src];
+      const uint32_t len = static_cast<uint32_t>(ptr_old[src + 1] - ptr_old[src]);
+      s += len;
+      rows += len ? 1u : 0u;
       moved |= (src >> LOCAL_BITS) != (p >> LOCAL_BITS);
     }
   }
@@ -98,38 +84,45 @@ __global__ void __launch_bounds__(R_THREADS) len_block_sums_kernel(
       outcome[0] = ticket;
     }
   }
-  int32_t tot;
-  block_exclusive_scan(s, &tot, sm);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
+  s = __reduce_add_sync(FULL, s);
+  rows = __reduce_add_sync(FULL, rows);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = row_count(s, rows);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    RowCount total = 0;
+#pragma unroll
+    for (int w = 0; w < R_THREADS / 32; ++w) total += sm[w];
+    block_sums[blockIdx.x] = total;
+  }
 }
 
-__global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32_t *block_sums) {
+__global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, RowCount *block_sums) {
   let_next_kernel_start();
   wait_for_kernels_before();
   // exclusive scan in place, one block, any nb
-  __shared__ int32_t sm[32];
-  __shared__ int32_t carry_s;
+  __shared__ RowCount sm[32];
+  __shared__ RowCount carry_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry_s = 0;
   __syncthreads();
   for (int32_t base = 0; base < nb; base += 1024) {
     const int32_t i = base + threadIdx.x;
-    const int32_t v = i < nb ? block_sums[i] : 0;
-    int32_t incl = v;
+    const RowCount v = i < nb ? block_sums[i] : 0;
+    RowCount incl = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const int32_t t = __shfl_up_sync(FULL, incl, off);
+      const RowCount t = __shfl_up_sync(FULL, incl, off);
       if (lane >= off) incl += t;
     }
     if (lane == 31) sm[warp] = incl;
     __syncthreads();
-    int32_t wbase = 0, tot = 0;
+    RowCount wbase = 0, tot = 0;
     for (int w = 0; w < 32; ++w) {
-      const int32_t t = sm[w];
+      const RowCount t = sm[w];
       if (w < warp) wbase += t;
       tot += t;
     }
-    const int32_t carry = carry_s;
+    const RowCount carry = carry_s;
     if (i < nb) block_sums[i] = carry + wbase + incl - v;
     __syncthreads();
     if (threadIdx.x == 0) carry_s = carry + tot;
@@ -137,16 +130,23 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, int32
   }
 }
 
+// Up to this many blocks of rows, ptr_new_kernel adds up the sums in front of its own block itself: one kernel less in the
+// chain of launches (power-law band of 65,536 rows, rows only 58.2 and 53.4 us, mesh of 1,048,576 rows 88.7 and 83.1).
+constexpr int32_t SCAN_IN_PLACE = 2048;
+
+// Row pointers of the new matrix, and for the tiles of apply_flat_kernel the list of the rows that have entries (first
+// entry, where it was less where it is; one more entry behind the last) with the place in it that each tile begins at.
 __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     int32_t n, int32_t nnz, const int32_t *__restrict__ ptr_old, const int32_t *__restrict__ new_order,
-    const int32_t *block_sums, int32_t *__restrict__ ptr_new,
-    int32_t *__restrict__ old2new, int32_t *__restrict__ tile_row, int32_t *__restrict__ row_delta) {
+    const RowCount *block_sums, int32_t *__restrict__ ptr_new,
+    int32_t *__restrict__ old2new, int32_t *__restrict__ tile_row, int2 *__restrict__ row_at, uint32_t rows_max) {
   let_next_kernel_start();
   constexpr int WARPS = R_THREADS / 32;
-  __shared__ int32_t sums[R_SCAN_IPT * WARPS];  // of 32 rows each, in row order
+  __shared__ RowCount sums[R_SCAN_IPT * WARPS];  // of 32 rows each, in row order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t first = blockIdx.x * R_SCAN_TILE + threadIdx.x;
   int32_t len[R_SCAN_IPT], from[R_SCAN_IPT], incl[R_SCAN_IPT];
+  uint32_t filled[R_SCAN_IPT];  // rows of the 32 that have entries
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
     const int32_t p = first + i * R_THREADS;
@@ -168,38 +168,79 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     }
   }
 #pragma unroll
-  for (int i = 0; i < R_SCAN_IPT; ++i)
-    if (lane == 31) sums[i * WARPS + warp] = incl[i];
+  for (int i = 0; i < R_SCAN_IPT; ++i) {
+    filled[i] = __ballot_sync(FULL, len[i] != 0);
+    if (lane == 31) sums[i * WARPS + warp] = row_count(static_cast<uint32_t>(incl[i]), __popc(filled[i]));
+  }
   __syncthreads();
-  wait_for_kernels_before();  // (the row lengths are the caller's)
-  if (warp == 0) {  // sums -> what lies in front of each 32 rows
+  if (warp == 0) {  // sums -> what lies in front of each 32 rows of the block
     static_assert(R_SCAN_IPT * WARPS == 64, "two per lane");
-    const int32_t x = sums[2 * lane], y = sums[2 * lane + 1];
-    int32_t run = x + y;
+    const RowCount x = sums[2 * lane], y = sums[2 * lane + 1];
+    RowCount run = x + y;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const int32_t t = __shfl_up_sync(FULL, run, off);
+      const RowCount t = __shfl_up_sync(FULL, run, off);
       if (lane >= off) run += t;
     }
-    run += __ldcg(block_sums + blockIdx.x);
     sums[2 * lane] = run - x - y;
     sums[2 * lane + 1] = run - y;
   }
   __syncthreads();
+  wait_for_kernels_before();  // (all so far is the caller's)
+  RowCount block_front;
+  if (gridDim.x > SCAN_IN_PLACE) {
+    block_front = __ldcg(block_sums + blockIdx.x);
+  } else {
+    constexpr int EACH = SCAN_IN_PLACE / R_THREADS;
+    RowCount part[EACH];
+#pragma unroll
+    for (int u = 0; u < EACH; ++u) {
+      const uint32_t b = u * R_THREADS + threadIdx.x;
+      part[u] = b < blockIdx.x ? __ldcg(block_sums + b) : 0;
+    }
+#pragma unroll
+    for (int u = 1; u < EACH; ++u) part[0] += part[u];
+    const uint32_t entries = __reduce_add_sync(FULL, static_cast<uint32_t>(part[0]));
+    const uint32_t rows = __reduce_add_sync(FULL, static_cast<uint32_t>(part[0] >> 32));
+    __shared__ RowCount front_of_block[WARPS];
+    if (lane == 0) front_of_block[warp] = row_count(entries, rows);
+    __syncthreads();
+    block_front = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) block_front += front_of_block[w];
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) ptr_new[0] = 0;
+  bool several = false;
+  uint32_t tile[R_SCAN_IPT], end[R_SCAN_IPT], place[R_SCAN_IPT];
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i) {
     const int32_t p = first + i * R_THREADS;
-    const int32_t run = sums[i * WARPS + warp] + incl[i] - len[i];
-    // the row that holds the first entry of a tile
-    for (int64_t t = (static_cast<int64_t>(run) + FLAT_TILE - 1) / FLAT_TILE;
-         t * FLAT_TILE < static_cast<int64_t>(run) + len[i] && t * FLAT_TILE < nnz; ++t)
-      tile_row[t] = p;
+    const RowCount front = block_front + sums[i * WARPS + warp];
+    const uint32_t run = static_cast<uint32_t>(front) + static_cast<uint32_t>(incl[i] - len[i]);
+    place[i] = static_cast<uint32_t>(front >> 32) + __popc(filled[i] & ((1u << lane) - 1u));
+    end[i] = run + static_cast<uint32_t>(len[i]);
     if (p < n) {
-      row_delta[p] = from[i] - run;
-      ptr_new[p + 1] = run + len[i];
+      ptr_new[p + 1] = static_cast<int32_t>(end[i]);
+      if (len[i] && place[i] < rows_max) row_at[place[i]] = make_int2(static_cast<int32_t>(run), from[i] - static_cast<int32_t>(run));
+      const uint32_t rows = place[i] + (len[i] ? 1u : 0u);
+      if (p == n - 1 && rows < rows_max) row_at[rows] = make_int2(static_cast<int32_t>(end[i]), 0);
     }
+    // the row that holds the first entry of a tile
+    end[i] = min(end[i], static_cast<uint32_t>(nnz));
+    tile[i] = (run + FLAT_TILE - 1) / FLAT_TILE;
+    if (tile[i] * FLAT_TILE < end[i]) tile_row[tile[i]] = static_cast<int32_t>(place[i]);
+    several |= (++tile[i]) * FLAT_TILE < end[i];
   }
+  // the further tiles of a row, by its warp (a row of 98,000 entries in front of R-MAT scale 22 has 768)
+  if (!__any_sync(FULL, several)) return;
+#pragma unroll
+  for (int i = 0; i < R_SCAN_IPT; ++i)
+    for (uint32_t more = __ballot_sync(FULL, tile[i] * FLAT_TILE < end[i]); more; more &= more - 1u) {
+      const int l = __ffs(static_cast<int>(more)) - 1;
+      const uint32_t last = __shfl_sync(FULL, end[i], l), at = __shfl_sync(FULL, place[i], l);
+      for (uint32_t t = __shfl_sync(FULL, tile[i], l) + lane; t * FLAT_TILE < last; t += 32)
+        tile_row[t] = static_cast<int32_t>(at);
+    }
 }
 
 struct ApplyArgs {
@@ -213,8 +254,9 @@ struct ApplyArgs {
   float *val_new;
   int32_t *queue_warp, *queue_block;  // new rows of 33..R_WARP entries / of up to R_MED
   int2 *queue_long;                   // longer rows: (new row, number of its first tile)
-  const int32_t *tile_row;            // per tile of the output: the row its first entry belongs to
-  const int32_t *row_delta;           // per new row: where it was less where it is
+  const int2 *row_at;                 // the rows that have entries: first entry, where it was less where it is
+  const int32_t *tile_row;            // per tile of the output: place in row_at of the row its first entry belongs to
+  int32_t rows_max;                   // entries of row_at
   uint32_t *counters;                 // [0] warp rows, [1] block rows, [2..3] packed (long rows, tiles),
                                       // [4] set when the permutation leaves blocks of 1024, [5] blocks that looked
   int32_t *tmp_key;                   // scratch copy of the long rows' sorted tiles, indexed like ind_new
@@ -388,6 +430,9 @@ __device__ __forceinline__ void warp_row(const ApplyArgs &a, int32_t src, int32_
 // tile, the reordered R-MAT scale 22 took 955 us here, now 522; mesh of 1,048,576 rows 94 and 48.  Bound by the
 // latency of the gathers at 48 warps per SM (40 registers; 11 KB of shared memory a block leave the L1 its space: with
 // 27 KB 677 us).  Tiles of 64 / 96 / 256 entries: 10 / 4 / 30 % slower.
+// A tile finds its rows in the list of those that have entries: at most 128, whatever lies between them.  Walked row by
+// row, 32 at a time, 4 M empty rows between two entries took one warp 88 ms (the whole call now 0.12), and half of the
+// rows of an R-MAT matrix are empty (scale 22 rows only 319 -> 276 us, scale 16 63 -> 55).
 constexpr int FLAT_PER = FLAT_TILE / 32;    // windows of 32 entries
 // longest run ranked by comparing: 20 took 624 us for the whole call, 28 606, 48 581, 72 579, 128 585 (a bit map costs a
 // warp two trips over the run and a scan)
@@ -512,23 +557,18 @@ __global__ void __launch_bounds__(R_THREADS, 6) apply_flat_kernel(ApplyArgs a) {
     const int32_t ra = a.tile_row[t];
     if (lane < PER) sh.row_head[lane] = 0u;
     __syncwarp();
-    const int32_t delta0 = a.row_delta[ra];
-    int32_t row_end;  // of the row that holds the tile's last entry
-    for (int32_t p0 = ra;; p0 += 32) {
-      const int32_t r = p0 + lane;
-      int32_t b = nnz, e = nnz, d = 0;
-      if (r < a.n) {
-        b = a.ptr_new[r];
-        e = a.ptr_new[r + 1];
-        d = a.row_delta[r];
+    int32_t row_end, delta0 = 0;  // end of the row that holds the tile's last entry; of the row that holds its first
+    for (int32_t p0 = ra;; p0 += 32) {  // (at most five times)
+      const int2 r = p0 < a.rows_max - lane ? a.row_at[p0 + lane] : make_int2(nnz, 0);
+      if (p0 == ra) delta0 = __shfl_sync(FULL, r.y, 0);
+      const unsigned behind = __ballot_sync(FULL, r.x >= t1);
+      const int rows = behind ? __ffs(static_cast<int>(behind)) - 1 : 32;
+      if (lane < rows && r.x >= t0) {
+        sh.delta[r.x - t0] = r.y;
+        atomicOr(&sh.row_head[(r.x - t0) >> 5], 1u << ((r.x - t0) & 31));
       }
-      if (b >= t0 && b < t1 && e > b) {
-        sh.delta[b - t0] = d;
-        atomicOr(&sh.row_head[(b - t0) >> 5], 1u << ((b - t0) & 31));
-      }
-      const unsigned behind = __ballot_sync(FULL, e >= t1);
       if (behind) {
-        row_end = __shfl_sync(FULL, e, __ffs(static_cast<int>(behind)) - 1);
+        row_end = min(__shfl_sync(FULL, r.x, rows), nnz);
         break;
       }
     }
@@ -566,7 +606,7 @@ __global__ void __launch_bounds__(R_THREADS, 6) apply_flat_kernel(ApplyArgs a) {
     // in the same trip: the entry in front of the tile, if its row goes on here, and 32 behind it, as far as its
     // last row goes
     const int32_t last_delta = last >= 0 ? sh.delta[last] : delta0;
-    const bool comes_in = (rows[0] & 1u) == 0u, in = t1 + lane < row_end;
+    const bool comes_in = (rows[0] & 1u) == 0u, in = lane < row_end - t1;
     int32_t prev = comes_in ? a.ind_old[t0 - 1 + delta0] : 0;
     int32_t more = in ? a.ind_old[t1 + lane + last_delta] : 0;
     float more_val = 0.0f;
@@ -596,7 +636,7 @@ __global__ void __launch_bounds__(R_THREADS, 6) apply_flat_kernel(ApplyArgs a) {
       sh.key[FLAT_TILE + lane] = more;
       while (other == 0u) {
         const int32_t at = t1 + ext + lane;
-        other = __ballot_sync(FULL, at >= row_end || (a.old2new[a.ind_old[at + last_delta]] >> LOCAL_BITS) != blk);
+        other = __ballot_sync(FULL, lane >= row_end - t1 - ext || (a.old2new[a.ind_old[at + last_delta]] >> LOCAL_BITS) != blk);
         ext += other ? __ffs(static_cast<int>(other)) - 1 : 32;
       }
     }
@@ -866,35 +906,42 @@ __global__ void __launch_bounds__(R_THREADS) apply_merge_kernel(ApplyArgs a) {
   }
 }
 
-}  // namespace
 
-size_t reorder_workspace_bytes(int32_t n, int32_t nnz, int mode) {
-  Arena ar;
-  const int32_t nb = (n + R_SCAN_TILE - 1) / R_SCAN_TILE;
-  ar.take(sizeof(int32_t) * (static_cast<size_t>(nb) + 1));
-  ar.take(256);                                         // queue counters
-  ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / 32 + 1));      // rows of 33..R_WARP entries
-  ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / R_WARP + 1));  // rows of up to R_MED
-  ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_MED + 1));      // longer rows
-  ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / FLAT_TILE + 2));  // first row of every output tile
-  ar.take(sizeof(int32_t) * static_cast<size_t>(n));                     // row_delta
-  if (mode == 1) {
-    ar.take(sizeof(int32_t) * static_cast<size_t>(n));  // old2new
-    ar.take(sizeof(int32_t) * static_cast<size_t>(nnz > 0 ? nnz : 1));  // sorted tiles: keys
-    ar.take(sizeof(float) * static_cast<size_t>(nnz > 0 ? nnz : 1));    // ... and values
+// Scratch of one call.  The list of rows that apply_flat_kernel reads and the sorted tiles of the other route share
+// their place: no call needs both.
+struct ReorderScratch {
+  size_t block_sums, counters, queue_warp, queue_block, queue_long, tile_row, old2new, row_at, tmp_key, tmp_val, bytes;
+  int32_t rows_max;
+  ReorderScratch(int32_t n, int32_t nnz, bool symmetric) {
+    const size_t rows = static_cast<size_t>(n), z = static_cast<size_t>(nnz > 0 ? nnz : 1);
+    rows_max = std::min(std::min(n, nnz), INT32_MAX - 1) + 1;  // and one behind the last
+    Arena ar;
+    block_sums = ar.take(sizeof(RowCount) * ((rows + R_SCAN_TILE - 1) / R_SCAN_TILE));
+    counters = ar.take(256);
+    queue_warp = ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / 32 + 1));       // rows of 33..R_WARP entries
+    queue_block = ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / R_WARP + 1));  // rows of up to R_MED
+    queue_long = ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_MED + 1));       // longer rows
+    tile_row = ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / FLAT_TILE + 2));
+    old2new = symmetric ? ar.take(sizeof(int32_t) * rows) : 0;
+    Arena tiles = ar;
+    tmp_key = symmetric ? tiles.take(sizeof(int32_t) * z) : 0;
+    tmp_val = symmetric ? tiles.take(sizeof(float) * z) : 0;
+    row_at = ar.take(sizeof(int2) * static_cast<size_t>(rows_max));
+    bytes = std::max(ar.off, tiles.off);
   }
-  return ar.off;
-}
+};
+
+}  // namespace
 
 bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_old,
                     const int32_t *d_ind_old, const float *d_val_old, const int32_t *d_new_order,
                     int mode, int32_t *d_ptr_new, int32_t *d_ind_new, float *d_val_new) {
   const bool symmetric = mode == 1;
   const bool with_vals = d_val_old != nullptr && d_val_new != nullptr;
-  if (!ensure_workspace(ctx, reorder_workspace_bytes(n, nnz, mode))) return false;
-  Arena ar;
+  const ReorderScratch lay(n, nnz, symmetric);
+  if (!ensure_workspace(ctx, lay.bytes)) return false;
   const int32_t nb = (n + R_SCAN_TILE - 1) / R_SCAN_TILE;
-  int32_t *block_sums = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nb) + 1)));
+  RowCount *block_sums = reinterpret_cast<RowCount *>(ctx.ws + lay.block_sums);
   ApplyArgs a;
   a.n = n;
   a.nnz = nnz;
@@ -905,34 +952,32 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   a.ptr_new = d_ptr_new;
   a.ind_new = d_ind_new;
   a.val_new = with_vals ? d_val_new : nullptr;
-  a.counters = reinterpret_cast<uint32_t *>(ctx.ws + ar.take(256));
-  a.queue_warp = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / 32 + 1)));
-  a.queue_block = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / R_WARP + 1)));
-  a.queue_long = reinterpret_cast<int2 *>(ctx.ws + ar.take(sizeof(int2) * (static_cast<size_t>(nnz) / R_MED + 1)));
-  int32_t *tile_row = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * (static_cast<size_t>(nnz) / FLAT_TILE + 2)));
+  a.counters = reinterpret_cast<uint32_t *>(ctx.ws + lay.counters);
+  a.queue_warp = reinterpret_cast<int32_t *>(ctx.ws + lay.queue_warp);
+  a.queue_block = reinterpret_cast<int32_t *>(ctx.ws + lay.queue_block);
+  a.queue_long = reinterpret_cast<int2 *>(ctx.ws + lay.queue_long);
+  int32_t *tile_row = reinterpret_cast<int32_t *>(ctx.ws + lay.tile_row);
+  int2 *row_at = reinterpret_cast<int2 *>(ctx.ws + lay.row_at);
   a.tile_row = tile_row;
-  int32_t *row_delta = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * static_cast<size_t>(n)));
-  a.row_delta = row_delta;
-  a.old2new = nullptr;
-  a.tmp_key = nullptr;
-  a.tmp_val = nullptr;
-  int32_t *old2new = nullptr;
-  if (symmetric) {
-    old2new = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * static_cast<size_t>(n)));
-    a.old2new = old2new;
-    a.tmp_key = reinterpret_cast<int32_t *>(ctx.ws + ar.take(sizeof(int32_t) * static_cast<size_t>(nnz > 0 ? nnz : 1)));
-    a.tmp_val = reinterpret_cast<float *>(ctx.ws + ar.take(sizeof(float) * static_cast<size_t>(nnz > 0 ? nnz : 1)));
-  }
+  a.row_at = row_at;
+  a.rows_max = lay.rows_max;
+  int32_t *old2new = symmetric ? reinterpret_cast<int32_t *>(ctx.ws + lay.old2new) : nullptr;
+  a.old2new = old2new;
+  a.tmp_key = symmetric ? reinterpret_cast<int32_t *>(ctx.ws + lay.tmp_key) : nullptr;
+  a.tmp_val = symmetric ? reinterpret_cast<float *>(ctx.ws + lay.tmp_val) : nullptr;
   CSG_CUDA(cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), ctx.stream));
   uint32_t *const outcome = reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
   ++ctx.outcome_ticket;
   len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, a.counters + CNT_MOVED,
                                                           symmetric ? outcome : nullptr, ctx.outcome_ticket);
   CSG_CUDA(cudaGetLastError());
-  CSG_CUDA(launch_behind(true, scan_block_sums_kernel, 1, 1024, 0, ctx.stream, nb, block_sums));
+  if (nb > SCAN_IN_PLACE) {
+    CSG_CUDA(launch_behind(true, scan_block_sums_kernel, 1, 1024, 0, ctx.stream, nb, block_sums));
+    count_launches(1);
+  }
   CSG_CUDA(launch_behind(true, ptr_new_kernel, nb, R_THREADS, 0, ctx.stream, n, nnz, d_ptr_old, d_new_order, block_sums,
-                         d_ptr_new, old2new, tile_row, row_delta));
-  count_launches(3);
+                         d_ptr_new, old2new, tile_row, row_at, lay.rows_max));
+  count_launches(2);
   if (nnz == 0) return true;
   bool local = false;
   if (symmetric) {
