@@ -51,18 +51,86 @@ bool ensure_workspace(Context &ctx, size_t bytes) {
   return true;
 }
 
-bool wait_outcome(Context &ctx, cudaStream_t st) {
-  volatile uint32_t *const h = reinterpret_cast<volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+bool wait_outcome(Context &ctx, cudaStream_t st, int word, uint32_t ticket) {
+  volatile uint32_t *const h = outcome_words(ctx, word);
   const auto start = std::chrono::steady_clock::now();
-  for (int spins = 0; h[0] != ctx.outcome_ticket; ++spins) {
+  for (int spins = 0; h[0] != ticket; ++spins) {
     // something went wrong on the device, or it is busy with other work: wait for the stream
     if ((spins & 1023) == 1023 && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(200)) {
       CSG_CUDA(cudaStreamSynchronize(st));
-      CSG_REQUIRE(h[0] == ctx.outcome_ticket, "internal: a kernel did not report its outcome");
+      CSG_REQUIRE(h[0] == ticket, "internal: a kernel did not report its outcome");
     }
   }
   std::atomic_thread_fence(std::memory_order_acquire);
   return true;
+}
+
+bool read_lists(Context &ctx, CsgScratch &s, int phase) {
+  const int word = phase == PHASE_PRIO ? OUTCOME_WORD_PRIO : OUTCOME_WORD;
+  if (!wait_outcome(ctx, phase == PHASE_PRIO ? ctx.side_stream : ctx.stream, word, s.ticket)) return false;
+  const volatile uint32_t *const h = outcome_words(ctx, word);
+  s.chain_rows = h[1];
+  s.chain_need = static_cast<uint64_t>(h[4]) << 32 | h[3];
+  s.no_heavy_rows = s.chain_rows == 0;
+  return true;
+}
+
+namespace {
+// ctx.chains[part] of `bytes` or more.  The one it replaces may be in use by the call's other stream, so it stays until the
+// call ends - unless its memory is needed.
+bool grow_chains(Context &ctx, int part, size_t bytes) {
+  if (bytes <= ctx.chains_bytes[part]) return true;
+  if (ctx.chains[part]) {
+    if (ctx.outgrown[part]) cudaFree(ctx.outgrown[part]);
+    ctx.outgrown[part] = ctx.chains[part];
+    ctx.chains[part] = nullptr;
+    ctx.chains_bytes[part] = 0;
+  }
+  for (const size_t want : {bytes + (bytes >> 3), bytes}) {  // (head room, so that similar calls reuse it)
+    if (cudaMalloc(&ctx.chains[part], want) == cudaSuccess) {
+      ctx.chains_bytes[part] = want;
+      return true;
+    }
+    cudaGetLastError();
+    ctx.chains[part] = nullptr;
+    for (char *&old : ctx.outgrown) {  // (cudaFree waits for the kernels that may use it)
+      if (old) cudaFree(old);
+      old = nullptr;
+    }
+  }
+  return false;
+}
+}  // namespace
+
+// Streams of all listed rows if s.stream_cap and the device's memory allow; else the heaviest rows that fit get a chain
+// and the kernel of the light rows computes the others, so results never depend on the size.
+bool plan_chains(Context &ctx, int32_t nnz, CsgScratch &s, int phase) {
+  const int part = phase == PHASE_PRIO ? 1 : 0;
+  uint64_t cap = s.chain_need < s.stream_cap ? s.chain_need : s.stream_cap;
+  if (cap < 1) cap = 1;
+  for (;; cap /= 2) {
+    size_t rows = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
+    if (rows > s.chain_rows) rows = s.chain_rows;
+    if (rows > s.heavy_max) rows = s.heavy_max;
+    const size_t parts = static_cast<size_t>(nnz) / SKETCH_PART_COLS + rows + 1;  // column slices of these rows
+    Arena ar;
+    const size_t o_stream = ar.take(8 * cap), o_off = ar.take(4 * (rows + 1)), o_state = ar.take(4 * rows * 2 * s.slots);
+    const size_t o_base = ar.take(4 * (rows + 2)), o_part = ar.take(4 * (parts + 1));
+    if (!grow_chains(ctx, part, ar.off)) {
+      if (cap > 1) continue;
+      set_error("device workspace of %zu bytes for the longest rows: %s", ar.off, cudaGetErrorString(cudaErrorMemoryAllocation));
+      return false;
+    }
+    char *const base = ctx.chains[part];
+    s.hstream = reinterpret_cast<int2 *>(base + o_stream);
+    s.heavy_off = reinterpret_cast<uint32_t *>(base + o_off);
+    s.heavy_state = reinterpret_cast<int32_t *>(base + o_state);
+    s.part_base = reinterpret_cast<uint32_t *>(base + o_base);
+    s.part_off = reinterpret_cast<uint32_t *>(base + o_part);
+    s.stream_cap = static_cast<uint32_t>(cap);
+    s.heavy_max = static_cast<uint32_t>(rows);
+    return true;
+  }
 }
 
 // sporder/src/sporder.cpp:147-161 and the checks of
@@ -113,26 +181,25 @@ size_t greedy_bitmap_words(int32_t n, int32_t chunk) {
 
 constexpr int32_t AHEAD_MIN_NNZ = 1 << 24;  // smaller calls do not pay for a second pipeline's launches
 
-// Stream elements the buffer of the heaviest rows gets for this call: never more than the
-// rows could stream at all (nnz * chunk span), than 2 GiB or than the caller's limit; at
-// least what the largest earlier call of the context asked for, and for a first call eight
-// elements per nonzero (at least 2^20: 8 MiB).
+// Stream elements the chains of a call may take: never more than the rows could stream at all
+// (nnz * chunk span), than 2 GiB or than the caller's limit.
 uint64_t stream_capacity(const Context &ctx, size_t nnz, size_t span) {
-  uint64_t cap = static_cast<uint64_t>(nnz) * 8;
-  if (cap < (uint64_t(1) << 20)) cap = uint64_t(1) << 20;
-  const uint64_t seen = ctx.stream_need_seen + (ctx.stream_need_seen >> 3);
-  if (cap < seen) cap = seen;
-  const uint64_t most = static_cast<uint64_t>(nnz) * span;
-  if (cap > most) cap = most;
+  uint64_t cap = static_cast<uint64_t>(nnz) * span;
   if (cap > STREAM_CAP_MAX) cap = STREAM_CAP_MAX;
   if (ctx.stream_limit && cap > ctx.stream_limit) cap = ctx.stream_limit;
   return cap < 1 ? 1 : cap;
 }
 
+// most rows with a chain on streams of `cap` elements
+uint32_t chain_rows_max(uint64_t cap, int32_t n) {
+  const uint64_t rows = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
+  return static_cast<uint32_t>(rows < static_cast<uint64_t>(n) ? rows : n);
+}
+
 // Lays out the scratch of one csg call in the context workspace.  `transpose_only` leaves
 // out everything behind the chunk-local transpose (the pillar count needs no more).
 // With `prio` the call runs one chunk ahead of the rest (run_csg): that part gets control
-// words, work lists and tile tables of its own and a share of the stream buffer.
+// words, work lists and tile tables of its own.
 bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint64_t *user_table,
                   CsgScratch *s, int32_t greedy_chunk = 0, bool transpose_only = false,
                   CsgScratch *prio = nullptr) {
@@ -157,39 +224,18 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   const size_t tiles_max = z / 4096 + heavy_max + 1;
   const size_t o_hc = ar.take(4 * heavy_max), o_htb = ar.take(4 * (heavy_max + 1));
   const size_t o_th = ar.take(4 * 256 * tiles_max), o_db = ar.take(4 * 256 * heavy_max);
-  // streams of the heaviest rows
   const size_t span = static_cast<size_t>(p.chunk < n ? p.chunk : n);
-  const size_t cap = transpose_only ? 1 : static_cast<size_t>(stream_capacity(ctx, z, span));
-  size_t hmax = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
-  if (hmax > static_cast<size_t>(n)) hmax = static_cast<size_t>(n);
-  const size_t o_hs = ar.take(8 * cap), o_ho = ar.take(4 * (hmax + 1));
-  const size_t o_hst = ar.take(4 * hmax * 2 * (p.M / 32) * 32);
-  const size_t pmax = transpose_only ? 1 : z / SKETCH_PART_COLS + hmax + 1;  // column slices of the heavy rows
-  const size_t o_pb = ar.take(4 * (hmax + 2)), o_po = ar.take(4 * (pmax + 1));
   const size_t o_table = (user_table || transpose_only) ? 0 : ar.take(8 * static_cast<size_t>(n) * p.k);
   // the part that runs ahead: one chunk's worth of lists, tile tables for up to all nonzeros
-  // (nothing bounds a chunk's share of them), and its share of the stream buffer - what it
-  // asked for in the context's last call plus an eighth, half the buffer on a first call
-  size_t cap_p = 0, hmax_p = 0, pmax_p = 0;
-  size_t o_p_list = 0, o_p_ctrl = 0, o_p_hc = 0, o_p_htb = 0, o_p_th = 0, o_p_db = 0, o_p_ho = 0, o_p_hst = 0,
-         o_p_pb = 0, o_p_po = 0;
+  // (nothing bounds a chunk's share of them)
+  size_t o_p_list = 0, o_p_ctrl = 0, o_p_hc = 0, o_p_htb = 0, o_p_th = 0, o_p_db = 0;
   if (prio) {
-    cap_p = ctx.stream_need_prio ? static_cast<size_t>(ctx.stream_need_prio + (ctx.stream_need_prio >> 3)) : cap / 2;
-    if (cap_p > cap - cap / 4) cap_p = cap - cap / 4;
-    if (cap_p < 1) cap_p = 1;
-    hmax_p = cap_p / HEAVY_WORK + 1;
-    if (hmax_p > span) hmax_p = span;
-    pmax_p = z / SKETCH_PART_COLS + hmax_p + 1;
     o_p_list = ar.take(4 * span);
     o_p_ctrl = ar.take(4 * CTRL_WORDS);
     o_p_hc = ar.take(4 * 2);
     o_p_htb = ar.take(4 * 4);
     o_p_th = ar.take(4 * 256 * (z / 4096 + 2));
     o_p_db = ar.take(4 * 256);
-    o_p_ho = ar.take(4 * (hmax_p + 1));
-    o_p_hst = ar.take(4 * hmax_p * 2 * (p.M / 32) * 32);
-    o_p_pb = ar.take(4 * (hmax_p + 2));
-    o_p_po = ar.take(4 * (pmax_p + 1));
   }
   if (!ensure_workspace(ctx, ar.off)) return false;
   s->keyA = reinterpret_cast<uint32_t *>(ctx.ws + o_keyA);
@@ -206,13 +252,9 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
   s->row_list = reinterpret_cast<int32_t *>(ctx.ws + o_list);
   s->ctrl = reinterpret_cast<uint32_t *>(ctx.ws + o_ctrl);
   s->table = user_table ? user_table : reinterpret_cast<uint64_t *>(ctx.ws + o_table);
-  s->hstream = reinterpret_cast<int2 *>(ctx.ws + o_hs);
-  s->heavy_off = reinterpret_cast<uint32_t *>(ctx.ws + o_ho);
-  s->heavy_state = reinterpret_cast<int32_t *>(ctx.ws + o_hst);
-  s->part_base = reinterpret_cast<uint32_t *>(ctx.ws + o_pb);
-  s->part_off = reinterpret_cast<uint32_t *>(ctx.ws + o_po);
+  const uint64_t cap = stream_capacity(ctx, z, span);
   s->stream_cap = static_cast<uint32_t>(cap);
-  s->heavy_max = static_cast<uint32_t>(hmax);
+  s->heavy_max = chain_rows_max(cap, n);
   s->slots = p.M;
   s->heavy_chunk = reinterpret_cast<int32_t *>(ctx.ws + o_hc);
   s->heavy_tile_base = reinterpret_cast<int32_t *>(ctx.ws + o_htb);
@@ -227,24 +269,16 @@ bool plan_scratch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, uint
     prio->heavy_tile_base = reinterpret_cast<int32_t *>(ctx.ws + o_p_htb);
     prio->tile_hist = reinterpret_cast<uint32_t *>(ctx.ws + o_p_th);
     prio->digit_base = reinterpret_cast<uint32_t *>(ctx.ws + o_p_db);
-    prio->heavy_off = reinterpret_cast<uint32_t *>(ctx.ws + o_p_ho);
-    prio->heavy_state = reinterpret_cast<int32_t *>(ctx.ws + o_p_hst);
-    prio->part_base = reinterpret_cast<uint32_t *>(ctx.ws + o_p_pb);
-    prio->part_off = reinterpret_cast<uint32_t *>(ctx.ws + o_p_po);
-    // the stream buffer is cut in two: the front for the part ahead
-    prio->stream_cap = static_cast<uint32_t>(cap_p);
-    prio->heavy_max = static_cast<uint32_t>(hmax_p);
-    s->hstream = s->hstream + cap_p;
-    s->stream_cap = static_cast<uint32_t>(cap - cap_p);
-    const size_t hmax_r = (cap - cap_p) / HEAVY_WORK + 1 + CHAIN_ROWS;
-    if (hmax_r < s->heavy_max) s->heavy_max = static_cast<uint32_t>(hmax_r);
+    // (the rest keeps a quarter of what the streams may take in any case)
+    prio->stream_cap = static_cast<uint32_t>(cap - cap / 4);
+    prio->heavy_max = static_cast<uint32_t>(span);
   }
   return true;
 }
 
 // End of a call that ran the transpose (and possibly the sketch): the control words come
 // back with the call's one synchronisation.  Malformed input and a refused stream slice are
-// errors; the stream need of the heavy rows is remembered for the context's next call.
+// errors.
 bool finish_call(Context &ctx, const CsgScratch &s, const CsgScratch *prio = nullptr) {
   uint32_t *h = reinterpret_cast<uint32_t *>(ctx.h_pinned);
   CSG_CUDA(cudaMemcpyAsync(h, s.ctrl, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
@@ -252,12 +286,12 @@ bool finish_call(Context &ctx, const CsgScratch &s, const CsgScratch *prio = nul
     CSG_CUDA(cudaMemcpyAsync(h + 16, prio->ctrl, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
   CSG_CUDA(cudaStreamSynchronize(ctx.stream));
   CSG_CUDA(cudaGetLastError());
-  uint64_t need_prio = 0;
-  if (prio) {  // the words of the part ahead: errors count like the others', its need is kept apart
+  for (char *&old : ctx.outgrown) {
+    if (old) CSG_CUDA(cudaFree(old));
+    old = nullptr;
+  }
+  if (prio) {  // the words of the part ahead: errors count like the others'
     const uint32_t *hp = h + 16;
-    need_prio = (static_cast<uint64_t>(hp[CTRL_HEAVY_NEED + 1]) << 32) | hp[CTRL_HEAVY_NEED];
-    if (need_prio > STREAM_CAP_MAX) need_prio = STREAM_CAP_MAX;
-    if (need_prio > ctx.stream_need_prio) ctx.stream_need_prio = need_prio;
     h[CTRL_BAD_INPUT] |= hp[CTRL_BAD_INPUT];
     h[CTRL_STREAM_OVERRUN] |= hp[CTRL_STREAM_OVERRUN];
     if (h[CTRL_CHECK] == 0 && hp[CTRL_CHECK] != 0)
@@ -278,9 +312,6 @@ bool finish_call(Context &ctx, const CsgScratch &s, const CsgScratch *prio = nul
   }
   CSG_REQUIRE(h[CTRL_STREAM_OVERRUN] == 0,
               "internal: a heavy row's stream slice did not fit its place in the stream buffer");
-  uint64_t need = ((static_cast<uint64_t>(h[CTRL_HEAVY_NEED + 1]) << 32) | h[CTRL_HEAVY_NEED]) + need_prio;
-  if (need > STREAM_CAP_MAX) need = STREAM_CAP_MAX;
-  if (need > ctx.stream_need_seen) ctx.stream_need_seen = need;
   return true;
 }
 
@@ -355,11 +386,20 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
       if (!launch_priority_pick(ctx, n, nnz, p.chunk, d_ptr, s, sp, ahead_chunk_nnz)) return false;
       CSG_CUDA(cudaEventRecord(ctx.ev[5], st));
       CSG_CUDA(cudaStreamWaitEvent(ctx.side_stream, ctx.ev[5], 0));
-      // the chunk ahead: queued first, so that the host's launches of the rest do not delay it
+      // the chunk ahead: queued first, so that the host's launches of the rest do not delay it; its chains as soon as
+      // its lists say how much room their streams take
       if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, sp, PHASE_PRIO, s.ctrl)) return false;
-      if (!launch_sketch(ctx, n, nnz, p, d_ptr, sp, row_base, false, PHASE_PRIO)) return false;
-      CSG_CUDA(cudaEventRecord(ctx.ev[7], ctx.side_stream));
       if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s, PHASE_REST, sp.ctrl)) return false;
+      if (!read_lists(ctx, sp, PHASE_PRIO)) return false;
+      if (!sp.no_heavy_rows) {
+        if (!launch_sketch(ctx, n, nnz, p, d_ptr, sp, row_base, false, PHASE_PRIO)) return false;
+        s.stream_cap -= sp.stream_cap < s.stream_cap ? sp.stream_cap : s.stream_cap - 1;
+        s.heavy_max = chain_rows_max(s.stream_cap, n);
+      } else {
+        CSG_CUDA(cudaEventRecord(ctx.ev[8], ctx.side_stream));
+      }
+      CSG_CUDA(cudaEventRecord(ctx.ev[7], ctx.side_stream));
+      if (!launch_lists(ctx, n, p.chunk, s, sp.ctrl) || !read_lists(ctx, s, PHASE_REST)) return false;
       if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
       CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[8], 0));
       if (!launch_sketch(ctx, n, nnz, p, d_ptr, s, row_base, false, PHASE_REST)) return false;
@@ -635,6 +675,10 @@ void sporder_context_destroy(sporder_context_t h) {
   cudaStreamSynchronize(c.stream);
   if (c.side_stream) cudaStreamSynchronize(c.side_stream);
   if (c.ws) cudaFree(c.ws);
+  for (int part = 0; part < 2; ++part) {
+    if (c.chains[part]) cudaFree(c.chains[part]);
+    if (c.outgrown[part]) cudaFree(c.outgrown[part]);
+  }
   if (c.stage) cudaFree(c.stage);
   for (auto &ev : c.ev)
     if (ev) cudaEventDestroy(ev);
@@ -661,7 +705,9 @@ void sporder_context_set_stream_limit(sporder_context_t h, uint64_t max_elements
   if (h) h->c.stream_limit = max_elements;
 }
 
-uint64_t sporder_context_workspace_bytes(sporder_context_t h) { return h ? h->c.ws_bytes : 0; }
+uint64_t sporder_context_workspace_bytes(sporder_context_t h) {
+  return h ? h->c.ws_bytes + h->c.chains_bytes[0] + h->c.chains_bytes[1] : 0;
+}
 
 const char *sporder_last_error(void) { return csg::g_has_err ? csg::g_err : nullptr; }
 

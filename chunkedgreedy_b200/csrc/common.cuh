@@ -53,13 +53,12 @@ struct Context {
   uint32_t outcome_ticket = 0;  // the newest one handed to a kernel (see OUTCOME_WORD)
   char *stage = nullptr;    // device copies of host inputs (host-buffer entry point), kept between calls
   size_t stage_bytes = 0;
-  // Buffer for the materialised candidate streams of the heaviest rows (sketch.cu), in stream
-  // elements of 8 bytes.  A call starts from a size in proportion to its input; every call
-  // reports what all its heavy rows together would have needed, and the next call of the
-  // context plans that much (rows that do not fit are still computed, by the slower kernel of
-  // the light rows, so results never depend on the size).
-  uint64_t stream_need_seen = 0;   // largest need any call of this context reported
-  uint64_t stream_need_prio = 0;   // ... and the share of it that the rows running ahead asked for
+  // Buffers for the chains of the heaviest rows (sketch.cu): their materialised candidate streams, sketches and lists
+  // of parts; [1] for the part of a call that runs ahead.  Grown to what the call's own rows need, which the host learns
+  // between the transposition and the sketch (plan_chains), so a call without such rows holds none.
+  char *chains[2] = {};
+  size_t chains_bytes[2] = {};
+  char *outgrown[2] = {};  // buffers a call replaced while kernels may run: freed when it ends
   // Second stream (higher priority) for the part of a large call that runs ahead of the rest:
   // the transposition and the chains of the chunk that holds the most nonzeros (see run_csg).
   cudaStream_t side_stream = nullptr;
@@ -70,9 +69,12 @@ struct Context {
 };
 
 // In h_pinned, written by the device: a ticket, then what a kernel found out that decides about the
-// launches behind it.  wait_outcome returns once the ticket is ctx.outcome_ticket.
-constexpr int OUTCOME_WORD = 48;
-bool wait_outcome(Context &ctx, cudaStream_t st);
+// launches behind it; the second place is that of the part that runs ahead.  wait_outcome returns once the ticket is there.
+constexpr int OUTCOME_WORD = 48, OUTCOME_WORD_PRIO = 56;
+inline volatile uint32_t *outcome_words(Context &ctx, int word) {
+  return reinterpret_cast<volatile uint32_t *>(ctx.h_pinned) + word;
+}
+bool wait_outcome(Context &ctx, cudaStream_t st, int word, uint32_t ticket);
 
 bool ensure_workspace(Context &ctx, size_t bytes);
 
@@ -110,13 +112,17 @@ struct CsgScratch {
   uint32_t *ctrl;  // [0]=chunk ticket [1]=row ticket [2]=rows listed [3..] see CTRL_* below
   uint64_t *table;  // n*k packed top-k entries
   uint32_t *gbitmaps;  // greedy bitmaps when they do not fit shared memory, else nullptr
-  // materialised candidate streams of the heaviest rows (see sketch.cu)
-  int2 *hstream;
-  uint32_t *heavy_off;
-  int32_t *heavy_state;
+  // materialised candidate streams of the heaviest rows (see sketch.cu): what they may take, what the lists asked for,
+  // and from plan_chains on the buffers and what they hold
   uint32_t stream_cap, heavy_max;
+  uint32_t chain_rows = 0;
+  uint64_t chain_need = 0;
+  int2 *hstream = nullptr;
+  uint32_t *heavy_off = nullptr;
+  int32_t *heavy_state = nullptr;
+  uint32_t *part_base = nullptr, *part_off = nullptr;
   int32_t slots;  // of a row's sketch
-  uint32_t *part_base, *part_off;
+  uint32_t ticket = 0;  // of the lists' outcome
   bool no_heavy_rows = false;  // known on the host already: nothing for the chain kernel
   bool one_stream = true;      // the call runs on one stream: its kernels may be programmatic dependent launches
   // compact_kernel's second list, tiled sort of heavy chunks (see transpose.cu)
@@ -133,7 +139,6 @@ enum {
   CTRL_HEAVY_ROWS = 6,     // rows at the head of row_list that the heavy sketch kernel takes
   CTRL_HEAVY_TICKET = 7,   // and the word after it: a second ticket
   CTRL_HEAVY_PARTS = 9,    // column slices of the heavy rows
-  CTRL_HEAVY_NEED = 10,    // and the word after it: stream elements of all rows of heavy weight (64-bit)
   CTRL_STREAM_OVERRUN = 12,  // set by heavy_expand_kernel when a slice would pass the stream buffer
   CTRL_CHECK = 13,         // checked build: site of the first index out of bounds, then the index (64-bit)
   CTRL_MID_END = 16,       // end of the rows in row_list that are not run by a lane (those past CTRL_HEAVY_ROWS: by a warp)
@@ -180,6 +185,12 @@ constexpr int32_t WARP_FEW_ROWS = 32768;
 bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
                       const int32_t *d_ind, CsgScratch &s, int phase = PHASE_ALL, uint32_t *ctrl_other = nullptr,
                       unsigned long long *d_count = nullptr);
+// work lists of the rows with candidates (part of launch_transpose but in a call that runs one chunk ahead)
+bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead);
+// waits for what the lists say about the call's longest rows: s.chain_rows, s.chain_need, s.no_heavy_rows
+bool read_lists(Context &ctx, CsgScratch &s, int phase);
+// buffers for the chains of the listed rows, no larger than they need; fewer chains where memory is short
+bool plan_chains(Context &ctx, int32_t nnz, CsgScratch &s, int phase);
 // start of a call that runs one chunk ahead: clears the counters of both parts and names the chunk
 bool launch_priority_pick(Context &ctx, int32_t n, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
                           CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz);

@@ -966,7 +966,7 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   a.tmp_key = symmetric ? reinterpret_cast<int32_t *>(ctx.ws + lay.tmp_key) : nullptr;
   a.tmp_val = symmetric ? reinterpret_cast<float *>(ctx.ws + lay.tmp_val) : nullptr;
   CSG_CUDA(cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), ctx.stream));
-  uint32_t *const outcome = reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
+  volatile uint32_t *const outcome = outcome_words(ctx, OUTCOME_WORD);
   ++ctx.outcome_ticket;
   len_block_sums_kernel<<<nb, R_THREADS, 0, ctx.stream>>>(n, d_ptr_old, d_new_order, block_sums, a.counters + CNT_MOVED,
                                                           symmetric ? outcome : nullptr, ctx.outcome_ticket);
@@ -981,8 +981,8 @@ bool launch_reorder(Context &ctx, int32_t n, int32_t nnz, const int32_t *d_ptr_o
   if (nnz == 0) return true;
   bool local = false;
   if (symmetric) {
-    if (!wait_outcome(ctx, ctx.stream)) return false;
-    local = reinterpret_cast<volatile uint32_t *>(outcome)[1] == 0u;
+    if (!wait_outcome(ctx, ctx.stream, OUTCOME_WORD, ctx.outcome_ticket)) return false;
+    local = outcome[1] == 0u;
   }
   if (!symmetric || local) {
     constexpr int64_t block = static_cast<int64_t>(FLAT_TILE) * FLAT_WARPS;

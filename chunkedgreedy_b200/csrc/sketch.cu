@@ -2068,6 +2068,7 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
 
 bool launch_sketch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, const int32_t *d_ptr,
                    CsgScratch &s, int32_t row_base, bool zero_table, int phase) {
+  if (!s.no_heavy_rows && !plan_chains(ctx, nnz, s, phase)) return false;
   SketchArgs a;
   a.n = n;
   a.nnz = nnz;

@@ -388,11 +388,23 @@ __global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, Tr
   }
 }
 
+// what the lists tell the host (read_lists)
+__device__ __forceinline__ void tell_lists(volatile uint32_t *outcome, uint32_t ticket, uint32_t chain_rows, uint32_t heavy_chunks,
+                                           unsigned long long need) {
+  outcome[1] = chain_rows;
+  outcome[2] = heavy_chunks;
+  outcome[3] = static_cast<uint32_t>(need);
+  outcome[4] = static_cast<uint32_t>(need >> 32);
+  __threadfence_system();
+  outcome[0] = ticket;
+}
+
 // Work list of the chunk ahead: its rows within a factor of four of its longest stream (and of
 // HEAVY_WORK candidates or more), longest first.  Those can decide when the call ends; the other
 // rows of the chunk go with everybody else's.  One block; a chunk has at most PRIO_MAX_CHUNK rows.
 constexpr int PRIO_MAX_CHUNK = 4096;
-__global__ void __launch_bounds__(1024) priority_rows_kernel(TransposeArgs ap, int32_t *row_list) {
+__global__ void __launch_bounds__(1024) priority_rows_kernel(TransposeArgs ap, int32_t *row_list, volatile uint32_t *outcome,
+                                                             uint32_t ticket) {
   __shared__ int32_t s_row[PRIO_MAX_CHUNK];
   __shared__ uint32_t s_work[PRIO_MAX_CHUNK];
   __shared__ uint32_t count, longest;
@@ -446,7 +458,7 @@ __global__ void __launch_bounds__(1024) priority_rows_kernel(TransposeArgs ap, i
     ap.ctrl[CTRL_ROW_TICKET] = count;
     ap.ctrl[CTRL_HEAVY_TICKET] = 0;
     ap.ctrl[CTRL_HEAVY_TICKET + 1] = 0;
-    *reinterpret_cast<unsigned long long *>(ap.ctrl + CTRL_HEAVY_NEED) = need;
+    tell_lists(outcome, ticket, count, 0, need);
   }
 }
 
@@ -870,35 +882,36 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     const float all = static_cast<float>(__shfl_sync(FULL, work_run, 31));
     work_run -= work_sum;
     run = incl - sum;
-    // time with the chains down to this bucket, and the least of them: of all choices (what the stream buffer should
-    // hold the next time), and of those that fit the buffer as it is
-    float best = 3.0e38f, best_fit = 3.0e38f;
-    uint32_t rows_fit = 0;
+    // time with the chains down to this bucket, and the least of them
+    float best = 3.0e38f;
+    uint32_t rows = 0;
+    uint32_t upto[4];
+    unsigned long long work_upto[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int b = WORK_BUCKETS - 1 - (4 * lane + j);
       run += c[j];
       work_run += work[j];
-      if (c[j] && run <= heavy) need = work_run;
-      if (!weigh || c[j] == 0 || b < work_bucket(CHAIN_WORK_MIN) || run > cost.rows_max) continue;
+      upto[j] = run;
+      work_upto[j] = work_run;
+      if (!weigh || c[j] == 0 || b < work_bucket(CHAIN_WORK_MIN) || run > cost.rows_max || work_run > cost.stream_cap) continue;
       const float s = static_cast<float>(work_run), r = static_cast<float>(run);
       const float chains = fmaxf(top * cost.alone, (s * cost.chain + r * cost.row) / cost.groups);
       const float lanes = run < listed ? fmaxf(bucket_floor(b) * cost.lane, (all - s) * cost.lanes) : 0.0f;
       const float time = fmaxf(chains, lanes) + 0.1f * fminf(chains, lanes) + r * cost.list + s * cost.expand;
-      if (work_run <= STREAM_CAP_MAX && time < best) {
+      if (time < best) {
         best = time;
-        need = max(need, work_run);
-      }
-      if (work_run <= cost.stream_cap && time < best_fit) {
-        best_fit = time;
-        rows_fit = run;
+        rows = run;
       }
     }
     if (weigh) {
-      const uint32_t time = __reduce_min_sync(FULL, __float_as_uint(best)), fit = __reduce_min_sync(FULL, __float_as_uint(best_fit));
-      if (__float_as_uint(best) != time && run > heavy) need = 0;
-      heavy = max(heavy, __reduce_max_sync(FULL, __float_as_uint(best_fit) == fit ? rows_fit : 0u));
+      const uint32_t time = __reduce_min_sync(FULL, __float_as_uint(best));
+      heavy = max(heavy, __reduce_max_sync(FULL, __float_as_uint(best) == time ? rows : 0u));
     }
+    // what their streams take, which the host makes room for (as far as it may: heavy_offsets_kernel)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c[j] && upto[j] <= heavy) need = work_upto[j];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) need = max(need, __shfl_xor_sync(FULL, need, off));
   }
@@ -911,12 +924,7 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     ctrl[CTRL_LANE_TICKET] = mid;
     ctrl[CTRL_HEAVY_TICKET] = 0;
     ctrl[CTRL_ROW_TICKET] = heavy;
-    *reinterpret_cast<unsigned long long *>(ctrl + CTRL_HEAVY_NEED) = need;
-    // for the host (wait_outcome)
-    outcome[1] = heavy;
-    outcome[2] = ctrl[CTRL_HEAVY_COUNT];
-    __threadfence_system();
-    outcome[0] = ticket;
+    tell_lists(outcome, ticket, heavy, ctrl[CTRL_HEAVY_COUNT], need);
   }
 }
 
@@ -1068,6 +1076,8 @@ bool launch_compact(Context &ctx, const TransposeArgs &a, cudaStream_t st) {
   return true;
 }
 
+}  // namespace
+
 // the rows with candidates, longest stream first
 bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead) {
   int grid = (n + 255) / 256;
@@ -1075,8 +1085,9 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
   CSG_CUDA(launch_behind(s.one_stream, bucket_count_kernel, grid, 256, 0, ctx.stream, n, s.row_work, s.ctrl, chunk, ctrl_ahead));
   const int32_t span = chunk < n ? chunk : n;
   const int octaves = span <= LANE_TABLE_ROWS ? 0 : span <= WARP_FEW_ROWS ? 4 : 3;
+  s.ticket = ++ctx.outcome_ticket;
   CSG_CUDA(launch_behind(s.one_stream, bucket_scan_kernel, 1, 32, 0, ctx.stream, s.ctrl,
-                         reinterpret_cast<uint32_t *>(ctx.h_pinned) + OUTCOME_WORD, ++ctx.outcome_ticket, octaves, ctrl_ahead,
+                         outcome_words(ctx, OUTCOME_WORD), s.ticket, octaves, ctrl_ahead,
                          chain_costs(ctx, s.slots, span <= LANE_TABLE_ROWS, s.heavy_max, s.stream_cap)));
   int steps = static_cast<int>((static_cast<int64_t>(n) + 256 * LIST_ROWS - 1) / (256 * LIST_ROWS));
   if (steps > ctx.num_sms * 32) steps = ctx.num_sms * 32;
@@ -1085,13 +1096,12 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
   count_launches(3);
   return true;
 }
-}  // namespace
 
 // phase PHASE_ALL: the whole transposition on the context's stream.  PHASE_PRIO (on the side
 // stream, `s` = the scratch of the part that runs ahead): the one chunk launch_priority_pick
 // named, then that chunk's list of heavy rows; ctx.ev[6] marks the end of its transposition.
-// PHASE_REST (context's stream): every other chunk, then - once ev[6] has passed, because the
-// lists read the work counters of all rows - the lists of everything the part ahead left.
+// PHASE_REST (context's stream): every other chunk; what follows in the stream is behind ev[6], because the lists
+// (launch_lists, once the chunk ahead has told what its streams take) read the work counters of all rows.
 // A PHASE_ALL call looks at the outcome of compact_kernel on the host: without chunks for the
 // tiled sort (none on meshes, roads and most small matrices) its dozen launches are left out.
 // d_count: only the number of (chunk, column) pairs is wanted, and added there.
@@ -1106,7 +1116,8 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   if (phase == PHASE_PRIO) {
     cudaStream_t st = ctx.side_stream;
     if (!launch_heavy(ctx, a, true, st)) return false;
-    priority_rows_kernel<<<1, 1024, 0, st>>>(a, s.row_list);
+    s.ticket = ++ctx.outcome_ticket;
+    priority_rows_kernel<<<1, 1024, 0, st>>>(a, s.row_list, outcome_words(ctx, OUTCOME_WORD_PRIO), s.ticket);
     CSG_CUDA(cudaGetLastError());
     count_launches(1);
     CSG_CUDA(cudaEventRecord(ctx.ev[6], st));  // the rest may read this chunk's work counters and its longest stream
@@ -1116,21 +1127,18 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
   if (phase == PHASE_REST) {
     if (!launch_compact(ctx, a, st) || !launch_heavy(ctx, a, false, st)) return false;
     CSG_CUDA(cudaStreamWaitEvent(st, ctx.ev[6], 0));
-    return launch_lists(ctx, n, chunk, s, ctrl_other);
+    return true;
   }
   CSG_CUDA(cudaMemsetAsync(s.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
   if (!launch_compact(ctx, a, st)) return false;
   if (d_count) return launch_heavy(ctx, a, false, st);
   if (!launch_lists(ctx, n, chunk, s, nullptr)) return false;
   // (the row list is still being written then, and the launches behind it are queued in time)
-  if (!wait_outcome(ctx, st)) return false;
-  const volatile uint32_t *const outcome = reinterpret_cast<const volatile uint32_t *>(ctx.h_pinned) + OUTCOME_WORD;
-  s.no_heavy_rows = outcome[1] == 0;
-  if (outcome[2] != 0) {
-    s.no_heavy_rows = false;
+  if (!read_lists(ctx, s, PHASE_ALL)) return false;
+  if (outcome_words(ctx, OUTCOME_WORD)[2] != 0) {
     if (!launch_heavy(ctx, a, false, st)) return false;
     CSG_CUDA(cudaMemsetAsync(s.ctrl + CTRL_BUCKET_COUNT, 0, 3 * sizeof(uint32_t) * WORK_BUCKETS, st));
-    return launch_lists(ctx, n, chunk, s, nullptr);
+    return launch_lists(ctx, n, chunk, s, nullptr) && read_lists(ctx, s, PHASE_ALL);
   }
   return true;
 }

@@ -174,9 +174,9 @@ SPORDER_API void sporder_context_set_stream(sporder_context_t ctx, void *stream)
 /* Upper bound, in stream elements of 8 bytes, on the buffer that holds the materialised
  * candidate streams of the heaviest rows (rows that stream tens of thousands of candidates are
  * computed fastest from such a copy).  0 = no bound beyond the built-in 2^28 elements (2 GiB).
- * Without a bound a call plans max(8 * nnz, 2^20) elements, or what the largest earlier
- * call of this context needed, never more than nnz * chunk_size.  Rows that do not fit are
- * computed by the kernel of the lighter rows; results are the same for every bound. */
+ * A call makes the buffer as large as its own rows need, once it knows them, and the context keeps
+ * it; a call without such rows holds none.  Rows that do not fit, because of a bound or for want
+ * of memory, are computed by the kernel of the lighter rows; results are the same for every bound. */
 SPORDER_API void sporder_context_set_stream_limit(sporder_context_t ctx, uint64_t max_elements);
 
 /* Calls of sporder_chunk_similarity_greedy (and its variants with a table, on host buffers or
