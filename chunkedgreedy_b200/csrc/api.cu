@@ -350,19 +350,19 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
   // there while the context's stream transposes everything else; the two meet before the
   // greedy stage.  Results do not depend on the split (the same kernels on the same rows).
   // By default for calls of 2^24 nonzeros in 64 chunks or more, whose chunk ahead must hold 2^17 nonzeros:
-  // smaller calls do not pay for the second pipeline's fifteen launches.  With 32 slots, where a chain is one warp,
-  // the chains of the two parts slow each other nearly everywhere, with 96 and 128 in tall chunks, and with 128
-  // where rows are long.  Time ahead over time not, R-MAT and its symmetrised form of 19 to 65 M nonzeros, chunks of
-  // 512 to 1024: 32 slots 1.57 (R-MAT scale 22 111 and 71 ms); 64 slots 0.90 to 0.95; 96 slots 0.81 to 0.95 at 10 to
-  // 31 nonzeros a row; 128 slots 0.84 to 0.96 up to 27, 1.02 to 1.07 from there on, 0.90 to 0.95 in chunks of 512;
-  // 160 and 256 slots (a warp per row) 0.97 to 0.99; in chunks of 4096, 96 slots 1.07, 128 slots 1.28, 64 slots 0.88 to
+  // smaller calls do not pay for the second pipeline's fifteen launches.  With 96 and 128 slots in tall chunks, and
+  // with 128 where rows are long, the chains of the two parts slow each other.  Time ahead over time not, R-MAT and
+  // its symmetrised form of 19 to 65 M nonzeros, chunks of 512 to 1024: 32 slots 0.89 to 0.96; 64 slots 0.87 to 0.96; 96
+  // slots 0.81 to 0.95 at 10 to 31 nonzeros a row; 128 slots 0.84 to 0.96 up to 27, 1.02 to 1.07 from there on, 0.90 to
+  // 0.95 in chunks of 512; 160 and 256 slots (a warp per row) 0.97 to 0.99; in chunks of 2048, 32 slots 0.82 to 0.88; in
+  // chunks of 4096, 32 slots 0.87 to 0.97, 96 slots 1.07, 128 slots 1.28, 64 slots 0.88 to
   // 1.15.  A caller's own threshold (sporder_context_set_ahead_threshold) applies to any call of two chunks.
   const int64_t chunks = (static_cast<int64_t>(n) + p.chunk - 1) / p.chunk;
   bool ahead = ctx.side_stream != nullptr && p.chunk <= 4096;
   int32_t ahead_chunk_nnz = 1 << 17;
   if (ctx.ahead_min_nnz == 0) {
-    const bool slowed = p.M == 32 || (p.chunk > 2048 && (p.M == 96 || p.M == 128)) ||
-                        (p.chunk > 512 && p.M == 128 && nnz >= 27ll * n);
+    const bool slowed =
+        (p.chunk > 2048 && (p.M == 96 || p.M == 128)) || (p.chunk > 512 && p.M == 128 && nnz >= 27ll * n);
     ahead = ahead && nnz >= AHEAD_MIN_NNZ && chunks >= 64 && !slowed;
   } else {
     ahead = ahead && ctx.ahead_min_nnz > 0 && nnz >= ctx.ahead_min_nnz && chunks >= 2;
@@ -370,11 +370,14 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
   }
   CsgScratch s, sp;
   if (!plan_scratch(ctx, n, nnz, p, d_table, &s, 0, false, ahead ? &sp : nullptr)) return false;
-  s.one_stream = sp.one_stream = !ahead;
   cudaStream_t st = ctx.stream;
   const bool zero_table = d_table != nullptr || stats != nullptr;
 
   if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[0], st));
+  // (a matrix without such a chunk goes on like any smaller call: mesh of 2 M rows, 64 slots 0.434 ms with both parts'
+  // launches, 0.277 so; asking costs it 0.014)
+  if (ahead && !launch_priority_pick(ctx, n, nnz, p.chunk, d_ptr, s, sp, ahead_chunk_nnz, &ahead)) return false;
+  s.one_stream = sp.one_stream = !ahead;
   if (!ahead) {
     if (!launch_transpose(ctx, n, ncols, nnz, p.chunk, d_ptr, d_ind, s)) return false;
     if (timing) CSG_CUDA(cudaEventRecord(ctx.ev[1], st));
@@ -383,7 +386,6 @@ bool run_csg(Context &ctx, int32_t n, int32_t ncols, int32_t row_base, int32_t n
     auto two_parts = [&]() -> bool {
       if (zero_table)
         CSG_CUDA(cudaMemsetAsync(s.table, 0, sizeof(uint64_t) * static_cast<size_t>(n) * p.k, st));
-      if (!launch_priority_pick(ctx, n, nnz, p.chunk, d_ptr, s, sp, ahead_chunk_nnz)) return false;
       CSG_CUDA(cudaEventRecord(ctx.ev[5], st));
       CSG_CUDA(cudaStreamWaitEvent(ctx.side_stream, ctx.ev[5], 0));
       // the chunk ahead: queued first, so that the host's launches of the rest do not delay it; its chains as soon as

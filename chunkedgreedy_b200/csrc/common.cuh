@@ -191,9 +191,9 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
 bool read_lists(Context &ctx, CsgScratch &s, int phase);
 // buffers for the chains of the listed rows, no larger than they need; fewer chains where memory is short
 bool plan_chains(Context &ctx, int32_t nnz, CsgScratch &s, int phase);
-// start of a call that runs one chunk ahead: clears the counters of both parts and names the chunk
+// start of a call that runs one chunk ahead: clears the counters of both parts and names the chunk, if there is one (on)
 bool launch_priority_pick(Context &ctx, int32_t n, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
-                          CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz);
+                          CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz, bool *on);
 bool launch_sketch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, const int32_t *d_ptr,
                    CsgScratch &s, int32_t row_base, bool zero_table, int phase = PHASE_ALL);
 bool launch_greedy(Context &ctx, int32_t n, const CsgParams &p, CsgScratch &s,

@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(S::THREADS) compact_kernel(TransposeArgs a) {
 // The chunk that runs ahead of the rest: the one with the most nonzeros, if it is a heavy
 // chunk of at least min_nnz nonzeros (a row that streams 65,536 candidates or more needs a
 // chunk about that big).  It becomes the only entry of `ap`'s list of heavy chunks.
-__global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, TransposeArgs ap, int32_t min_nnz) {
+__global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, TransposeArgs ap, int32_t min_nnz,
+                                                             volatile uint32_t *outcome, uint32_t ticket) {
   __shared__ unsigned long long best[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long mine = 0;  // (nonzeros << 32) | ~chunk: the first of equally heavy chunks wins
@@ -385,6 +386,9 @@ __global__ void __launch_bounds__(1024) pick_priority_kernel(TransposeArgs a, Tr
     ap.ctrl[CTRL_PRIO] = on ? q : PRIO_NONE;
     ap.ctrl[CTRL_HEAVY_COUNT] = on ? 1u : 0u;
     ap.heavy_chunk[0] = on ? static_cast<int32_t>(q) : 0;
+    outcome[1] = on ? 1u : 0u;
+    __threadfence_system();
+    outcome[0] = ticket;
   }
 }
 
@@ -1013,16 +1017,19 @@ TransposeArgs transpose_args(int32_t n, int32_t ncols, int32_t nnz, int32_t chun
 }  // namespace
 
 bool launch_priority_pick(Context &ctx, int32_t n, int32_t nnz, int32_t chunk, const int32_t *d_ptr,
-                          CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz) {
+                          CsgScratch &s, CsgScratch &prio, int32_t min_chunk_nnz, bool *on) {
   const TransposeArgs a = transpose_args(n, n, nnz, chunk, d_ptr, nullptr, s);
   const TransposeArgs ap = transpose_args(n, n, nnz, chunk, d_ptr, nullptr, prio);
   cudaStream_t st = ctx.stream;
   CSG_CUDA(cudaMemsetAsync(s.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
   CSG_CUDA(cudaMemsetAsync(prio.ctrl, 0, sizeof(uint32_t) * CTRL_WORDS, st));
-  CSG_CUDA(cudaMemsetAsync(s.row_work, 0, sizeof(uint32_t) * static_cast<size_t>(n), st));
-  pick_priority_kernel<<<1, 1024, 0, st>>>(a, ap, min_chunk_nnz);
+  prio.ticket = ++ctx.outcome_ticket;
+  pick_priority_kernel<<<1, 1024, 0, st>>>(a, ap, min_chunk_nnz, outcome_words(ctx, OUTCOME_WORD_PRIO), prio.ticket);
   CSG_CUDA(cudaGetLastError());
   count_launches(1);
+  if (!wait_outcome(ctx, st, OUTCOME_WORD_PRIO, prio.ticket)) return false;
+  *on = outcome_words(ctx, OUTCOME_WORD_PRIO)[1] != 0;
+  if (*on) CSG_CUDA(cudaMemsetAsync(s.row_work, 0, sizeof(uint32_t) * static_cast<size_t>(n), st));
   return true;
 }
 

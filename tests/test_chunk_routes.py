@@ -72,6 +72,31 @@ def test_rows_of_32_slots_against_oracle(n, hubs, members, k):
     _check(ptr, ind, limits=(0, 1), k=k, chunk_size=n)
 
 
+@pytest.mark.parametrize("k", [4, 8])
+@pytest.mark.parametrize("chunk", [512, 1024, 2048, 4096])
+def test_32_slots_one_chunk_ahead(chunk, k):
+    # the chunk with the most nonzeros transposed first, its rows of 65,536 candidates and more on the second stream
+    import chunkedgreedy_b200 as sp
+    rng = np.random.default_rng(chunk + k)
+    n = 4 * chunk + 100
+    rows = [list(rng.integers(0, n, 4)) for _ in range(n)]
+    for c in range(900):  # hubs of the second chunk
+        for r in rng.choice(chunk, 150, replace=False):
+            rows[chunk + r].append(c)
+    for r in range(chunk + 10, chunk + 40):
+        rows[r] += range(900)
+    ptr, ind = _csr(rows, n)
+    order, table = oracle.csg(ptr, ind, False, with_table=True, k=k, chunk_size=chunk)
+    ctx = sp.Context()
+    ctx.set_ahead_threshold(1)
+    for limit in (0, 0, 300_000):
+        ctx.set_stream_limit(limit)
+        got = sp.csg_table(torch.from_numpy(ptr).cuda(), torch.from_numpy(ind).cuda(), ctx=ctx, k=k, chunk_size=chunk)
+        assert np.array_equal(got[1].cpu().numpy().view(np.uint64), table)
+        assert np.array_equal(got[0].cpu().numpy(), order)
+    ctx.close()
+
+
 @pytest.mark.parametrize("k", [8, 16, 40])
 @pytest.mark.parametrize("chunk,skew", [(1024, 10), (1025, 10), (5000, 5), (40_000, 4)])
 def test_rows_by_warp_before_the_lanes(chunk, skew, k):
