@@ -189,6 +189,8 @@ bool launch_transpose(Context &ctx, int32_t n, int32_t ncols, int32_t nnz, int32
 bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const uint32_t *ctrl_ahead);
 // waits for what the lists say about the call's longest rows: s.chain_rows, s.chain_need, s.no_heavy_rows
 bool read_lists(Context &ctx, CsgScratch &s, int phase);
+// rows a block of the chain kernel (one to an SM) works on side by side; 0 beyond the slots that are resolved in rounds
+int chain_groups(const Context &ctx, int slots, int64_t span);
 // buffers for the chains of the listed rows, no larger than they need; fewer chains where memory is short
 bool plan_chains(Context &ctx, int32_t nnz, CsgScratch &s, int phase);
 // start of a call that runs one chunk ahead: clears the counters of both parts and names the chunk, if there is one (on)

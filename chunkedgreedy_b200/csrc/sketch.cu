@@ -1970,6 +1970,21 @@ __global__ void __launch_bounds__(S_THREADS) heavy_topk_kernel(SketchArgs a) {
   }
 }
 
+// shared memory of a block of heavy_rounds_kernel: as many groups as their key tables leave room for
+struct ChainBlock {
+  int groups, group_bytes, tab_bytes, room;
+};
+template <int CELLS>
+ChainBlock chain_block(const Context &ctx, int64_t span) {
+  ChainBlock b;
+  b.tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
+  b.group_bytes = GroupMemory<CELLS>::tab_offset(span > MATES) + b.tab_bytes;
+  b.room = ctx.smem_optin - 1024;
+  b.groups = Helpers<CELLS>::ROWS;
+  while (b.groups > 1 && b.groups * b.group_bytes > b.room) --b.groups;
+  return b;
+}
+
 template <int CELLS>
 bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_rows) {
   // A call that runs one chunk ahead has two of these sequences in flight: the chunk ahead on
@@ -1989,21 +2004,15 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
     if (phase == PHASE_PRIO) CSG_CUDA(cudaEventRecord(ctx.ev[8], st));
     // Sketches of up to ROUND_CELLS cells per lane are resolved in rounds, a group of warps per row.
     if constexpr (in_rounds) {
-      const int64_t span = a.chunk < a.n ? a.chunk : a.n;
-      const int tab_bytes = span <= ROUND_TAB_MAX ? static_cast<int>((span + 15) / 16 * 16) : 0;
-      // (groups per block: as many as their tables leave room for)
-      const int group_bytes = GroupMemory<CELLS>::tab_offset(span > MATES) + tab_bytes;
-      const int room = ctx.smem_optin - 1024;
-      int groups = Helpers<CELLS>::ROWS;
-      while (groups > 1 && groups * group_bytes > room) --groups;
-      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+      const ChainBlock block = chain_block<CELLS>(ctx, a.chunk < a.n ? a.chunk : a.n);
+      CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, block.room));
       // (all of an SM's memory as shared: a block of another split cannot move in beside this one)
       CSG_CUDA(cudaFuncSetAttribute(heavy_rounds_kernel<CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared));
       // (a plain launch: started beside the end of the expansion, blocks gather on the SMs that are through first, and
       // symmetrised R-MAT of scale 20 takes 29.4 ms instead of 27.7)
-      CSG_CUDA(launch_behind(false, heavy_rounds_kernel<CELLS>, ctx.num_sms, Helpers<CELLS>::THREADS * groups,
-                             groups * group_bytes, st, a, tab_bytes));
+      CSG_CUDA(launch_behind(false, heavy_rounds_kernel<CELLS>, ctx.num_sms, Helpers<CELLS>::THREADS * block.groups,
+                             block.groups * block.group_bytes, st, a, block.tab_bytes));
     }
     if constexpr (CELLS > ROUND_CELLS) {
       const int pad = ctx.smem_optin - 1024 - 2 * S_WARPS * S_RING * 4;
@@ -2065,6 +2074,17 @@ bool launch_cells(Context &ctx, const SketchArgs &a, int phase, bool no_heavy_ro
 }
 
 }  // namespace
+
+int chain_groups(const Context &ctx, int slots, int64_t span) {
+  static_assert(ROUND_CELLS == 4, "a case each");
+  switch (slots / 32) {
+    case 1: return chain_block<1>(ctx, span).groups;
+    case 2: return chain_block<2>(ctx, span).groups;
+    case 3: return chain_block<3>(ctx, span).groups;
+    case 4: return chain_block<4>(ctx, span).groups;
+    default: return 0;
+  }
+}
 
 bool launch_sketch(Context &ctx, int32_t n, int32_t nnz, const CsgParams &p, const int32_t *d_ptr,
                    CsgScratch &s, int32_t row_base, bool zero_table, int phase) {

@@ -798,14 +798,20 @@ struct ChainCosts {
 // and with chains for rows of 2^16 candidates or 296 rows, ms: R-MAT scale 22 21.4 and 23.5, top-k graph of scale 16
 // 22.8 and 27.3, scale 19 in chunks of 2,048 10.7 and 12.9; symmetrised R-MAT of scale 20 27.9 and 28.0, of 262,144
 // rows 12.2 and 16.2, of 65,536 rows 3.3 and 4.1.
-ChainCosts chain_costs(const Context &ctx, int slots, bool key_table, uint32_t rows_max, uint32_t stream_cap) {
+// Key tables of tall chunks leave room for three groups of 32 slots (from 44,600 rows on) or two (from 63,900): a chain is
+// the faster the fewer share its SM, but beside two the lanes get on, too.  Top-k graphs of 65,536 rows with k = 14, rule for four groups
+// and for those there are, ms: R-MAT 16 edges a row 26.8 and 20.0, 6 edges 8.5 and 5.8, symmetrised 23.6 and 14.6, power-law
+// band 1.27 both; of 50,000 rows the same.
+ChainCosts chain_costs(const Context &ctx, int slots, int32_t span, uint32_t rows_max, uint32_t stream_cap) {
+  const bool key_table = span <= LANE_TABLE_ROWS;
   ChainCosts c = {};
   c.rows_max = rows_max;
   c.stream_cap = stream_cap;
-  if (slots > 128) return c;
-  c.groups = (slots == 32 ? 4.0f : 2.0f) * static_cast<float>(ctx.num_sms);
-  c.chain = slots == 32 ? 0.050f : slots == 64 ? 0.030f : slots == 96 ? 0.035f : 0.052f;
+  const int groups = chain_groups(ctx, slots, span);
+  if (groups == 0) return c;
+  c.groups = static_cast<float>(groups * ctx.num_sms);
   c.alone = slots == 32 ? 0.028f : slots == 64 ? 0.018f : 0.021f;
+  c.chain = slots == 32 ? (groups > 2 ? 0.0125f * groups : 0.040f) : slots == 64 ? 0.030f : slots == 96 ? 0.035f : 0.052f;
   c.row = 3.0f;
   c.lane = key_table ? 0.24f : 0.40f;
   c.lanes = (key_table ? (slots <= 64 ? 5.5e-5f : 7.5e-5f) : 1.0e-4f) * 148.0f / static_cast<float>(ctx.num_sms);
@@ -1095,7 +1101,7 @@ bool launch_lists(Context &ctx, int32_t n, int32_t chunk, CsgScratch &s, const u
   s.ticket = ++ctx.outcome_ticket;
   CSG_CUDA(launch_behind(s.one_stream, bucket_scan_kernel, 1, 32, 0, ctx.stream, s.ctrl,
                          outcome_words(ctx, OUTCOME_WORD), s.ticket, octaves, ctrl_ahead,
-                         chain_costs(ctx, s.slots, span <= LANE_TABLE_ROWS, s.heavy_max, s.stream_cap)));
+                         chain_costs(ctx, s.slots, span, s.heavy_max, s.stream_cap)));
   int steps = static_cast<int>((static_cast<int64_t>(n) + 256 * LIST_ROWS - 1) / (256 * LIST_ROWS));
   if (steps > ctx.num_sms * 32) steps = ctx.num_sms * 32;
   CSG_CUDA(launch_behind(s.one_stream, row_list_kernel, steps, 256, 0, ctx.stream, n, s.row_work, s.ctrl, s.row_list, chunk,
