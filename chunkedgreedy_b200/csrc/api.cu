@@ -2,6 +2,7 @@
 // the csg pipeline driver and the thin wrappers around reorder and SpMM.
 #include "../../include/sporder_b200.h"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstring>
@@ -108,15 +109,14 @@ bool plan_chains(Context &ctx, int32_t nnz, CsgScratch &s, int phase) {
   const int part = phase == PHASE_PRIO ? 1 : 0;
   uint64_t cap = s.chain_need < s.stream_cap ? s.chain_need : s.stream_cap;
   if (cap < 1) cap = 1;
+  size_t rows = s.chain_rows < s.heavy_max ? s.chain_rows : s.heavy_max;
   for (;; cap /= 2) {
-    size_t rows = cap / HEAVY_WORK + 1 + CHAIN_ROWS;
-    if (rows > s.chain_rows) rows = s.chain_rows;
-    if (rows > s.heavy_max) rows = s.heavy_max;
     const size_t parts = static_cast<size_t>(nnz) / SKETCH_PART_COLS + rows + 1;  // column slices of these rows
     Arena ar;
     const size_t o_stream = ar.take(8 * cap), o_off = ar.take(4 * (rows + 1)), o_state = ar.take(4 * rows * 2 * s.slots);
     const size_t o_base = ar.take(4 * (rows + 2)), o_part = ar.take(4 * (parts + 1));
     if (!grow_chains(ctx, part, ar.off)) {
+      rows = std::min<size_t>(rows, cap / 2 / HEAVY_WORK + 1 + CHAIN_ROWS);
       if (cap > 1) continue;
       set_error("device workspace of %zu bytes for the longest rows: %s", ar.off, cudaGetErrorString(cudaErrorMemoryAllocation));
       return false;
@@ -310,6 +310,7 @@ bool finish_call(Context &ctx, const CsgScratch &s, const CsgScratch *prio = nul
     set_error("checked build: index out of bounds (%s: %lld); results unspecified", site[k], idx);
     return false;
   }
+  ctx.chain_rows = h[CTRL_HEAVY_ROWS] + (prio ? h[16 + CTRL_HEAVY_ROWS] : 0u);
   CSG_REQUIRE(h[CTRL_STREAM_OVERRUN] == 0,
               "internal: a heavy row's stream slice did not fit its place in the stream buffer");
   return true;
@@ -706,6 +707,12 @@ void sporder_context_set_ahead_threshold(sporder_context_t h, int64_t min_nnz) {
 void sporder_context_set_stream_limit(sporder_context_t h, uint64_t max_elements) {
   if (h) h->c.stream_limit = max_elements;
 }
+
+void sporder_context_set_chain_threshold(sporder_context_t h, uint32_t min_candidates) {
+  if (h) h->c.chain_min_work = min_candidates;
+}
+
+uint64_t sporder_context_chain_rows(sporder_context_t h) { return h ? h->c.chain_rows : 0; }
 
 uint64_t sporder_context_workspace_bytes(sporder_context_t h) {
   return h ? h->c.ws_bytes + h->c.chains_bytes[0] + h->c.chains_bytes[1] : 0;
