@@ -71,6 +71,15 @@ class Context:
         never.  Results never depend on it."""
         _lib.load().sporder_context_set_ahead_threshold(self._h, int(min_nnz))
 
+    def set_chain_threshold(self, min_candidates):
+        """Candidates from which a row goes to the kernel of the longest streams: 0 = the built-in
+        rule.  Results never depend on it."""
+        _lib.load().sporder_context_set_chain_threshold(self._h, int(min_candidates))
+
+    def chain_rows(self):
+        """Rows that kernel took in the last csg or similarity graph call."""
+        return int(_lib.load().sporder_context_chain_rows(self._h))
+
     def close(self):
         if getattr(self, "_h", None):
             _lib.load().sporder_context_destroy(self._h)

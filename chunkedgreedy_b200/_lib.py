@@ -58,6 +58,8 @@ SYMBOLS = {
     "sporder_context_workspace_bytes": (C.c_uint64, [_P]),
     "sporder_context_set_stream_limit": (None, [_P, C.c_uint64]),
     "sporder_context_set_ahead_threshold": (None, [_P, C.c_int64]),
+    "sporder_context_set_chain_threshold": (None, [_P, C.c_uint32]),
+    "sporder_context_chain_rows": (C.c_uint64, [_P]),
     "sporder_csg_with_table": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, C.c_bool, C.c_int32,
                                            C.c_float, C.c_int32, _P, _P, C.c_uint64,
                                            C.POINTER(CsgTiming), C.POINTER(CsgStats)]),

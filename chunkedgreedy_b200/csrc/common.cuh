@@ -66,6 +66,8 @@ struct Context {
   // never, positive = the caller's threshold (sporder_context_set_ahead_threshold)
   int64_t ahead_min_nnz = 0;
   uint64_t stream_limit = 0;       // caller's upper bound (sporder_context_set_stream_limit), 0 = none
+  uint32_t chain_min_work = 0;     // rows from so many candidates on get a chain, 0 = as their costs say
+  uint64_t chain_rows = 0;         // rows that got one in the last call
 };
 
 // In h_pinned, written by the device: a ticket, then what a kernel found out that decides about the

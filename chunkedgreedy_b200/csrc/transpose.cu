@@ -788,9 +788,10 @@ __global__ void __launch_bounds__(256) bucket_count_kernel(int32_t n, const uint
 // busy, `alone` for the longest, `row` for every row; a lane `lane` per candidate of its row, all of them together
 // `lanes`; `start` for the launches that a call without chains leaves out, `list` and `expand` for what they do per row and
 // candidate.  chain = 0: no such times, FEW_CHAIN_ROWS rows.
+// `forced` > 0: the caller's rule instead, every row in the buckets from that of so many candidates on.
 struct ChainCosts {
   float groups, chain, alone, row, lane, lanes, start, list, expand;
-  uint32_t rows_max, stream_cap;
+  uint32_t rows_max, stream_cap, forced;
 };
 
 // Measured: csg and top-k graphs of R-MAT matrices and their symmetrised forms, rows listed down to 2^12 .. 2^17
@@ -807,6 +808,7 @@ ChainCosts chain_costs(const Context &ctx, int slots, int32_t span, uint32_t row
   ChainCosts c = {};
   c.rows_max = rows_max;
   c.stream_cap = stream_cap;
+  if (ctx.chain_min_work) c.forced = ctx.chain_min_work > CHAIN_WORK_MIN ? ctx.chain_min_work : CHAIN_WORK_MIN;
   const int groups = chain_groups(ctx, slots, span);
   if (groups == 0) return c;
   c.groups = static_cast<float>(groups * ctx.num_sms);
@@ -867,13 +869,13 @@ __global__ void bucket_scan_kernel(uint32_t *ctrl, volatile uint32_t *outcome, u
     ctrl[CTRL_BUCKET_BASE + b] = run;
     run += c[j];
     ctrl[CTRL_BUCKET_FILL + b] = 0;
-    if (b >= work_bucket(HEAVY_WORK) || (cost.chain == 0.0f && b >= work_bucket(CHAIN_WORK_MIN) && run <= FEW_CHAIN_ROWS))
-      heavy = run;
+    const bool few = cost.chain == 0.0f && b >= work_bucket(CHAIN_WORK_MIN) && run <= FEW_CHAIN_ROWS;
+    if (cost.forced ? b >= work_bucket(cost.forced) : b >= work_bucket(HEAVY_WORK) || few) heavy = run;
     if (octaves > 0 && b >= least) mid = run;
   }
   heavy = __reduce_max_sync(FULL, heavy);
   // (where the lanes end their longest row before a chain kernel would have begun, there is nothing to weigh)
-  const bool weigh = cost.chain > 0.0f && top * cost.lane > cost.start;
+  const bool weigh = cost.forced == 0 && cost.chain > 0.0f && top * cost.lane > cost.start;
   unsigned long long need = 0;
   if (weigh || heavy > 0) {
     const unsigned long long *const bucket_work = reinterpret_cast<const unsigned long long *>(ctrl + CTRL_BUCKET_WORK);

@@ -189,6 +189,15 @@ SPORDER_API void sporder_context_set_stream_limit(sporder_context_t ctx, uint64_
  * reference counterpart. */
 SPORDER_API void sporder_context_set_ahead_threshold(sporder_context_t ctx, int64_t min_nnz);
 
+/* Which rows the kernel of the longest candidate streams takes, a group of warps each.  0: as
+ * many as its measured costs and those of the kernel beside it say; otherwise the rows with
+ * min_candidates candidates or more (no fewer than 64, rounded down to a quarter octave), as far
+ * as there is room for their streams.  Results are the same either way. */
+SPORDER_API void sporder_context_set_chain_threshold(sporder_context_t ctx, uint32_t min_candidates);
+
+/* Rows that kernel took in the context's last csg or similarity graph call. */
+SPORDER_API uint64_t sporder_context_chain_rows(sporder_context_t ctx);
+
 /* Bytes of device workspace the context currently holds (grow-only cache). */
 SPORDER_API uint64_t sporder_context_workspace_bytes(sporder_context_t ctx);
 
