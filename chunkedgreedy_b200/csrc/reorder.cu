@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(int32_t nb, RowCo
 // chain of launches (power-law band of 65,536 rows, rows only 58.2 and 53.4 us, mesh of 1,048,576 rows 88.7 and 83.1).
 constexpr int32_t SCAN_IN_PLACE = 2048;
 
+constexpr int TILES_BY_THREAD = 16;  // further tiles of a row that its thread names
+
 // Row pointers of the new matrix, and for the tiles of apply_flat_kernel the list of the rows that have entries (first
 // entry, where it was less where it is; one more entry behind the last) with the place in it that each tile begins at.
 __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
@@ -231,7 +233,17 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     if (tile[i] * FLAT_TILE < end[i]) tile_row[tile[i]] = static_cast<int32_t>(place[i]);
     several |= (++tile[i]) * FLAT_TILE < end[i];
   }
-  // the further tiles of a row, by its warp (a row of 98,000 entries in front of R-MAT scale 22 has 768)
+  // the further tiles of a row: the first of them by its own thread, since where one row has some its neighbours often
+  // have them too, those of the longest by its warp (a row of 98,000 entries in front of R-MAT scale 22 has 768)
+  for (int step = 0; step < TILES_BY_THREAD && several; ++step) {
+    several = false;
+#pragma unroll
+    for (int i = 0; i < R_SCAN_IPT; ++i) {
+      if (tile[i] * FLAT_TILE >= end[i]) continue;
+      tile_row[tile[i]] = static_cast<int32_t>(place[i]);
+      several |= (++tile[i]) * FLAT_TILE < end[i];
+    }
+  }
   if (!__any_sync(FULL, several)) return;
 #pragma unroll
   for (int i = 0; i < R_SCAN_IPT; ++i)

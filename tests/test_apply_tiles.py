@@ -104,3 +104,15 @@ def test_blocks_of_rows(n):
     # rows counted in blocks of 2,048, whose sums are added up by each block or by a kernel of its own
     lens = (torch.arange(n, device="cuda") % 3 == 0).long()
     _apply_both_ways(lens, torch.arange(0, n, 3, device="cuda"), _local_order(n, n))
+
+
+@pytest.mark.parametrize("tiles", [2, 16, 17, 18, 40])
+def test_neighbouring_rows_of_several_tiles(tiles):
+    # 70 rows of about so many tiles each: the first 16 further ones are named by the row's thread, the rest by its warp
+    n = 1 << 13
+    lens = torch.ones(n, dtype=torch.int64, device="cuda")
+    lens[3000:3070] = tiles * 128 + torch.arange(70, device="cuda") * 61 % 131 - 65
+    rows = torch.repeat_interleave(torch.arange(n, device="cuda"), lens)
+    nth = torch.arange(rows.numel(), device="cuda") - torch.repeat_interleave(torch.cumsum(lens, 0) - lens, lens)
+    cols = torch.sort(rows * n + (rows * 37 + nth) % n)[0] % n  # (ascending in every row)
+    _apply_both_ways(lens, cols, _local_order(n, tiles))
