@@ -99,3 +99,19 @@ def test_more_rows_than_a_limited_buffer_lists(k):
     most = room // 65536 + 1 + 4096
     assert (work >= LEAST).sum() > most
     assert _check(ptr, ind, (room,), k, 1000) == [most]
+
+
+@pytest.mark.parametrize("scale", [14, 15])
+@pytest.mark.parametrize("k", [8, 20])
+def test_no_more_rows_than_the_costs_hold_for(scale, k):
+    # the whole matrix as one chunk and long streams throughout: the rule by costs ends at 4,096 rows and one for every
+    # 65,536 candidates of those it takes
+    import chunkedgreedy_b200 as sp
+    from chunkedgreedy_b200 import synth
+    ptr, ind, _ = synth.rmat_gcn(scale, 8)
+    work = _candidates(ptr, ind, ptr.size)
+    ctx = sp.Context()
+    sp.similarity_graph(torch.from_numpy(ptr).cuda(), torch.from_numpy(ind).cuda(), k=k, ctx=ctx)
+    took = ctx.chain_rows()
+    ctx.close()
+    assert 0 < took <= 4096 + int(np.sort(work)[::-1][:took].sum()) // 65536
