@@ -742,8 +742,8 @@ struct LaneSketch {
 };
 
 // The rows between the chain kernel's and the lanes' own, before those: the long ones of chunks without a
-// byte table (bucket_scan_kernel says which), and rows that did not fit the stream buffer (rare: a first call
-// on much larger rows than the context has seen, or a caller's bound on the buffer).
+// byte table (bucket_scan_kernel says which), and rows that did not fit the stream buffer (rare: more than
+// 2^28 candidates, little memory left, or a caller's bound on the buffer).
 template <int CELLS>
 __device__ __noinline__ void rows_before_the_lanes(const SketchArgs &a, uint32_t end, uint32_t *mem) {
   mem += (threadIdx.x >> 5) * 2 * S_RING;
@@ -1372,7 +1372,7 @@ __device__ __forceinline__ int slot_of(const RoundRow &row, int32_t s) {
 }
 
 // One of the other warps: the place of its sixteen slots in the (weight, code) order, the
-// number of entries (x, i) below (mine, slot).  GROUP lanes to GROUP / 2 slots, as many parts of the entries.
+// number of entries (x, i) below (mine, slot).  Eight lanes to four slots, as many parts of the entries.
 // "x < mine" is counted as sat((mine - x) * 2^90), one fused multiply-add that is exactly 1 or 0:
 // weights lie in [2^-31, 2^32], so two different ones are at least 2^-54 apart.  An equal entry
 // is below for a smaller code: then the bar is the next float above.
@@ -1382,7 +1382,7 @@ __device__ __forceinline__ bool rank_slots(int base, int helper, int lane) {
   RoundState<CELLS> &st = GroupMemory<CELLS>::state(base);
   constexpr float BIG = 1.2379400392853803e27f;  // 2^90
   constexpr float ZERO = 8388608.0f;             // 2^23: counts are read off its last bits
-  constexpr int GROUP = 8, SLOTS = GROUP / 2, QUADS = 8 * CELLS / GROUP;
+  constexpr int GROUP = 8, SLOTS = 4, QUADS = CELLS;
   const int sub = lane % GROUP, first = helper * 16 + lane / GROUP * SLOTS, slot = first + sub % SLOTS, own = first / 4;
   const float4 *const v4 = reinterpret_cast<const float4 *>(st.w);
   float4 all[QUADS];  // (loaded in one go: left to itself the compiler waits for every load)
@@ -1404,18 +1404,16 @@ __device__ __forceinline__ bool rank_slots(int base, int helper, int lane) {
       // entries of the slots' own block of four in front of this slot, and others, have the bar of their block
       const bool before = b * GROUP + sub < own, upto = b * GROUP + sub <= own;
       const float bar = before ? le : lt, front = upto ? le : lt;
-      const int e = (first + i) & 3;
       const float x[4] = {all[b].x, all[b].y, all[b].z, all[b].w};
       float c[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) c[k] = __saturatef(fmaf(x[k], -BIG, k < (SLOTS == 4 ? i : e) ? front : bar));
+      for (int k = 0; k < 4; ++k) c[k] = __saturatef(fmaf(x[k], -BIG, k < i ? front : bar));
       acc[i] += (c[0] + c[1]) + (c[2] + c[3]);
     }
   }
   // counts of the slots in the bytes of one word
   uint32_t counts = __byte_perm(__float_as_uint(acc[0]), __float_as_uint(acc[1]), 0x0040) & 0xFFFFu;
-  if (SLOTS == 4)
-    counts = __byte_perm(counts, __byte_perm(__float_as_uint(acc[SLOTS - 2]), __float_as_uint(acc[SLOTS - 1]), 0x0040), 0x5410);
+  counts = __byte_perm(counts, __byte_perm(__float_as_uint(acc[2]), __float_as_uint(acc[3]), 0x0040), 0x5410);
 #pragma unroll
   for (int d = 1; d < GROUP; d <<= 1) counts += __shfl_xor_sync(FULL, counts, d);
   const int pos = static_cast<int>(counts >> (8 * (sub % SLOTS)) & 255u);
