@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(R_THREADS) ptr_new_kernel(
     several |= (++tile[i]) * FLAT_TILE < end[i];
   }
   // the further tiles of a row: the first of them by its own thread, since where one row has some its neighbours often
-  // have them too, those of the longest by its warp (a row of 98,000 entries in front of R-MAT scale 22 has 768)
+  // have them too (symmetrised R-MAT of 120,000 rows: 83 us the call, 89 with all of them by the warp), those of the longest
+  // by its warp (a row of 98,000 entries in front of R-MAT scale 22 has 768)
   for (int step = 0; step < TILES_BY_THREAD && several; ++step) {
     several = false;
 #pragma unroll
@@ -440,11 +441,11 @@ __device__ __forceinline__ void warp_row(const ApplyArgs &a, int32_t src, int32_
 // first entry; a tile reads on behind its end as far as its last run goes.
 // All rows cost the same per entry this way.  By blocks of 256 threads on tiles of 2048 entries, with ten barriers a
 // tile, the reordered R-MAT scale 22 took 955 us here, now 522; mesh of 1,048,576 rows 94 and 48.  Bound by the
-// latency of the gathers at 48 warps per SM (40 registers; 11 KB of shared memory a block leave the L1 its space: with
-// 27 KB 677 us).  Tiles of 64 / 96 / 256 entries: 10 / 4 / 30 % slower.
+// gathers and by the tiles' own instructions about equally at 45 warps per SM (scale 20: 7.2 warp instructions an entry, L1
+// 63 %, DRAM 18 %; 40 registers; 11 KB of shared memory a block leave the L1 its space: with 27 KB 677 us).  Tiles of 64 / 96 / 256 entries: 10 / 4 / 30 % slower.
 // A tile finds its rows in the list of those that have entries: at most 128, whatever lies between them.  Walked row by
-// row, 32 at a time, 4 M empty rows between two entries took one warp 88 ms (the whole call now 0.12), and half of the
-// rows of an R-MAT matrix are empty (scale 22 rows only 319 -> 276 us, scale 16 63 -> 55).
+// row, 32 at a time, 4 M empty rows between two entries took one warp 88 ms (the whole call now 0.07), and half of the
+// rows of an R-MAT matrix are empty (scale 22 rows only 319 -> 258 us).
 constexpr int FLAT_PER = FLAT_TILE / 32;    // windows of 32 entries
 // longest run ranked by comparing: 20 took 624 us for the whole call, 28 606, 48 581, 72 579, 128 585 (a bit map costs a
 // warp two trips over the run and a scan)
